@@ -191,3 +191,31 @@ def test_programmatic_dependent_launch_is_transparent(ctx, backend):
     assert np.array_equal(outs[0].view(np.uint16), outs[1].view(np.uint16))
     assert ctx.last_device_status() == 0
 
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("splitk", [1, 2, 4])
+@pytest.mark.parametrize("M,N", [(5, 8), (33, 136), (64, 1016), (77, 120), (300, 264)])
+def test_wa_outputs_that_fill_no_tile(ctx, backend, dtype, splitk, M, N):
+    """Outputs in multiples of 8 that leave the last tile of 128 (64 with SwiGLU) partly empty: every row
+    and column against the oracle, and nothing written behind the last output."""
+    K = 512
+    x = synth.activations(M, K, dtype, 48, f"war.{M}")
+    layer = synth.int4_layer(2 * N, K, 48, f"war.{N}")
+    half = synth.int4_layer(N, K, 48, f"war.{N}.p")
+    code = orc.dtype_code(x)
+    guard = np.full(M * N + 64, 0x5A5A, np.uint16)
+    for lay, flags in ((half, 0), (layer, B.FLAG_SWIGLU)):
+        xb, yb = ctx.upload(x), ctx.upload(guard)
+        with _Tuned(backend, gemm_tc_splitk=splitk):
+            ctx.qmatmul(xb, ctx.upload_layer(lay), yb, M, B.np_dtype_code(x), flags=flags)
+        assert backend.last_kernel_name().startswith("lux_qgemm_i4_tc_wa")
+        raw = yb.to_host(np.uint16, guard.shape)
+        assert (raw[M * N:] == 0x5A5A).all()
+        y = raw[:M * N].reshape(M, N).view(x.dtype)
+        if flags:
+            gu = orc.qmatmul(x, *lay.triple, bits=4, group=128, y_code=orc.F32, w_round=code)
+            assert orc.rel_l2(y, orc.swiglu(gu, h_code=code)) < TOL_16
+        else:
+            assert orc.rel_l2(y, _oracle(x, lay)) < TOL_16
+    assert ctx.last_device_status() == 0

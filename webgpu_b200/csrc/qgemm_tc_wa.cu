@@ -176,7 +176,9 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
     };
     if (warp >= 2) {
         const int r = quad * 32 + lane;                 // this thread's TMEM lane and its weight row
-        const int wrow = SW ? (r < OUT_W ? n0 + r : p.up_row_offset + n0 + r - OUT_W) : n0 + r;
+        // the lanes of a last tile that has fewer outputs read its last row again; they are not written
+        const int orow = min(n0 + (SW ? r & (OUT_W - 1) : r), p.Nout - 1);
+        const int wrow = SW && r >= OUT_W ? p.up_row_offset + orow : orow;
         wp = p.w + (size_t)wrow * (p.K / 2) + (k_base >> 1);
         sp = p.scales + (size_t)wrow * p.G + g_base;
         zrow = p.zeros ? p.zeros + (size_t)wrow * p.ZS : nullptr;
@@ -430,7 +432,7 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
 #pragma unroll 2
             for (int c = (warp - 2) * 4 + sub; c < KEEP; c += 32) {
                 const int m = m0 + keep0 + c;
-                if (m < p.M && keep0 + c < p.ncols) {
+                if (m < p.M && keep0 + c < p.ncols && n0 + l8 * 8 < p.Nout) {
                     const float4* gp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(stage) + c * BM + l8 * 8);
                     const float4 g0 = gp[0], g1 = gp[1], u0 = gp[OUT_W / 4], u1 = gp[OUT_W / 4 + 1];
                     uint4 v;
@@ -447,7 +449,7 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
 #pragma unroll 4
             for (int c = (warp - 2) * 2 + sub; c < KEEP; c += 16) {
                 const int m = m0 + keep0 + c;
-                if (m < p.M) {
+                if (m < p.M && n0 + l16 * 8 < p.Nout) {
                     const uint4 v = *reinterpret_cast<const uint4*>(stage + c * WA_STAGE_PITCH + l16 * 16);
                     *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(p.y) + ((size_t)m * p.Nout + n0 + l16 * 8) * 2) = v;
                 }
@@ -483,12 +485,12 @@ cudaError_t launch_wa(bool pdl, const CUtensorMap& mx, const WaParams& p, dim3 g
 
 }  // namespace
 
-// Takes int4 GEMMs without a push epilogue whose outputs come in whole tiles (128 weight rows;
-// with SwiGLU 64 outputs = 64 gate + 64 up rows); everything else stays with lux_qgemm_i4_tc.
+// Takes int4 GEMMs without a push epilogue whose outputs come in multiples of 8 (16-byte pieces of y); a last
+// tile (128 weight rows; with SwiGLU 64 outputs = 64 gate + 64 up rows) may be partly empty.
 LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     const int nout = a.swiglu ? a.N / 2 : a.N;
     const int out_w = a.swiglu ? BM / 2 : BM;                   // outputs per tile
-    if (a.push || nout % out_w || a.K % 128 || a.M < 1) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
+    if (a.push || nout % 8 || a.K % 128 || a.M < 1) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     if (a.scale_dtype != LUX_QDTYPE_F16 || a.x_dtype != a.y_dtype) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     if (a.x_dtype != LUX_QDTYPE_BF16 && a.x_dtype != LUX_QDTYPE_F16) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     if ((reinterpret_cast<uintptr_t>(a.w) & 15u) || (a.K / 2) % 16) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
@@ -500,7 +502,7 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     // Split K over a cluster of two or four CTAs when whole tiles alone would leave most slots idle
     // (`slots` = CTAs resident at once).
     auto plan = [&](int bn, int slots, int& ks_out) {
-        const int tiles = (nout / out_w) * ((a.M + bn - 1) / bn);
+        const int tiles = (nout + out_w - 1) / out_w * ((a.M + bn - 1) / bn);
         const bool can_split = a.K % 256 == 0 && (size_t)tiles * (2 * wa_slot_bytes(bn, 2)) <= ctx->d_splitk_bytes;
         const bool can_split4 = a.K % 512 == 0 && (size_t)tiles * (12 * wa_slot_bytes(bn, 4)) <= ctx->d_splitk_bytes;
         int ks = (tiles * 4 <= slots && can_split4) ? 4 : (tiles * 2 <= slots && can_split) ? 2 : 1;
@@ -548,7 +550,7 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     p.ncols = ncols;
     p.prefetch = g_tune.gemm_wa_prefetch < 0 ? 0 : (g_tune.gemm_wa_prefetch > 0 ? g_tune.gemm_wa_prefetch : 2);
 
-    dim3 grid(nout / out_w, (a.M + bn - 1) / bn, ks);
+    dim3 grid((nout + out_w - 1) / out_w, (a.M + bn - 1) / bn, ks);
     const int threads = (2 + 4 * groups) * 32;                  // groups >= 2: the epilogue needs warps 2..9
     const bool pdl = pdl_allowed(ctx, a.weights_volatile);
     auto go = [&](auto bf_tag, auto sw_tag, auto bn_tag) {
@@ -566,7 +568,8 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     cudaError_t e;
     if (a.swiglu) e = bf16 ? go_bn(std::true_type{}, std::true_type{}) : go_bn(std::false_type{}, std::true_type{});
     else          e = bf16 ? go_bn(std::true_type{}, std::false_type{}) : go_bn(std::false_type{}, std::false_type{});
-    count_launch(bf16 ? "lux_qgemm_i4_tc_wa_bf16" : "lux_qgemm_i4_tc_wa_f16");
+    if (nout % out_w) count_launch(bf16 ? "lux_qgemm_i4_tc_wa_edge_bf16" : "lux_qgemm_i4_tc_wa_edge_f16");     // partly empty last tile
+    else count_launch(bf16 ? "lux_qgemm_i4_tc_wa_bf16" : "lux_qgemm_i4_tc_wa_f16");
     return map_cuda(e, "lux_qgemm_i4_tc_wa");
 }
 
