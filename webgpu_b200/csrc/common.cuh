@@ -44,7 +44,7 @@ struct Context {
     void*          d_stage = nullptr;       // device staging for host-pointer ops
     size_t         d_stage_bytes = 0;
     uint32_t       last_status = 0;
-    uint32_t*      d_absmax = nullptr;      // device word for lux_cuda_dynamic_quantize's tensor-wide max (allocated with the context)
+    float*         d_absmax = nullptr;      // lux_cuda_dynamic_quantize: one maximum per block (ABSMAX_PARTS, allocated with the context)
     void*          d_splitk = nullptr;      // split-K exchange of the weights-in-TMEM GEMM: 128 KB per CTA pair,
     size_t         d_splitk_bytes = 0;      // allocated with the context (no entry point allocates for it)
     void*          d_int = nullptr;         // lux_cuda_matmul_int8 on the tcgen05 path: B transposed (and A unpacked), grown on demand
@@ -59,6 +59,8 @@ struct Context {
     // operands before griddepcontrol.wait (see launch_pdl below).
     bool           writer_pending = false;
 };
+
+constexpr int ABSMAX_PARTS = 1024;
 
 inline Context* as_ctx(LuxBackendContext* c) { return reinterpret_cast<Context*>(c); }
 inline Buffer*  as_buf(LuxBackendBuffer* b) { return reinterpret_cast<Buffer*>(b); }

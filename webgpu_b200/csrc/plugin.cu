@@ -104,7 +104,7 @@ static LuxBackendContext* cuda_create_context(int device_index) {
     // stream wait without another copy.
     ok = ok && cudaHostAlloc(&ctx->h_status, sizeof(uint32_t), cudaHostAllocMapped) == cudaSuccess;
     ok = ok && cudaHostGetDevicePointer((void**)&ctx->d_status, ctx->h_status, 0) == cudaSuccess;
-    ok = ok && cudaMalloc(&ctx->d_absmax, sizeof(uint32_t)) == cudaSuccess;
+    ok = ok && cudaMalloc(&ctx->d_absmax, ABSMAX_PARTS * sizeof(float)) == cudaSuccess;
     // Split-K partial sums of the tensor-core GEMM: one 128 KB slot per CTA pair, at most one pair
     // per two SMs.  Allocated here so that no matmul entry point ever allocates device memory.
     if (ok) {

@@ -27,32 +27,34 @@
 // wait is bounded (the abort flag, status 0x7C05000B).  No cluster, no multicast.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
 namespace luxcuda {
 
-bool encode_tensor_map_u8(void* map, int rank, const void* base, const uint64_t* dims, const uint64_t* strides_bytes,
-                          const uint32_t* box, bool swizzle128);
-
 namespace {
 
 using namespace tcptx;
 
-constexpr int I8_BM = 128, I8_BN = 256, I8_KB = 128;       // tile of C; k (= bytes) per stage
-constexpr int I8_A_BYTES = I8_BM * I8_KB, I8_B_BYTES = I8_BN * I8_KB;
+constexpr int I8_BM = 128, I8_KB = 128;                    // rows of a tile of C; k (= bytes) per stage
+constexpr int I8_A_BYTES = I8_BM * I8_KB;
+__host__ __device__ constexpr int i8_b_bytes(int bn) { return bn * I8_KB; }
 constexpr int I8_THREADS = 6 * 32;
 // MA = row tiles of 128 per CTA (1 or 2): two accumulators share every B tile, which cuts the bytes a CTA
 // pulls from L2 per multiply-add by a third (the one-tile form asks for 92 bytes per clock and SM at the
 // tensor pipe's rate and ran at half of it)
-__host__ __device__ constexpr int i8_stages(int ma) { return ma == 2 ? 3 : 4; }
-__host__ __device__ constexpr size_t i8_smem(int ma) { return 1024 + (size_t)i8_stages(ma) * (ma * I8_A_BYTES + I8_B_BYTES) + 256; }
+// BN = columns per CTA (256 or 128).
+__host__ __device__ constexpr int i8_stages(int ma, int bn) { return ma == 2 ? 3 : bn == 256 ? 4 : 6; }
+__host__ __device__ constexpr size_t i8_smem(int ma, int bn) {
+    return 1024 + (size_t)i8_stages(ma, bn) * (ma * I8_A_BYTES + i8_b_bytes(bn)) + 256;
+}
 
 // Instruction descriptor for kind::i8: D = s32 (bits 4-5 = 2), A and B signed 8-bit (bits 7-9 and
 // 10-12 = 1), both K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-__host__ __device__ constexpr uint32_t i8_idesc() {
-    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(I8_BN >> 3) << 17) | ((uint32_t)(I8_BM >> 4) << 24);
+__host__ __device__ constexpr uint32_t i8_idesc(int bn) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(I8_BM >> 4) << 24);
 }
 
 __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
@@ -81,10 +83,14 @@ __device__ __forceinline__ uint64_t make_mnmajor_sw128_desc(uint32_t smem_addr) 
     return ((uint64_t)hi << 32) | lo;
 }
 
-template <int MA>
+// Split K: the CTAs of a cluster (grid z) take slices of K for the same tile.  Slice 0 stores its sums, a cluster
+// barrier (release / acquire) publishes them, and the others add theirs with integer reductions in L2:
+// integer sums are the same in any order.
+template <int MA, int BN>
 __global__ void __launch_bounds__(I8_THREADS, 1)
 lux_matmul_int8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const I8Params p) {
-    constexpr int I8_STAGES = i8_stages(MA);
+    constexpr int I8_BN = BN, I8_B_BYTES = i8_b_bytes(BN);
+    constexpr int I8_STAGES = i8_stages(MA, BN);
     constexpr int A_STAGE = MA * I8_A_BYTES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -95,7 +101,9 @@ lux_matmul_int8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
     volatile uint32_t* abort_flag = tmem_slot + 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.x * I8_BN, m0 = blockIdx.y * (MA * I8_BM);
-    const int KB = (p.K + I8_KB - 1) / I8_KB;
+    const int stages_all = (p.K + I8_KB - 1) / I8_KB;
+    const int kb0 = (int)((long long)stages_all * blockIdx.z / gridDim.z);                 // first stage of this slice of K
+    const int KB = (int)((long long)stages_all * (blockIdx.z + 1) / gridDim.z) - kb0;
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
     auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(I8_STAGES + s); };
@@ -113,7 +121,7 @@ lux_matmul_int8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     }
     if (warp == 1) {
-        tmem_alloc(smem_u32(tmem_slot), MA * 256);
+        tmem_alloc(smem_u32(tmem_slot), MA * BN);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -127,19 +135,20 @@ lux_matmul_int8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
                 const int s = kb % I8_STAGES;
                 if (kb >= I8_STAGES && !mbar_wait_relaxed(empty(s), (uint32_t)((kb / I8_STAGES) - 1) & 1u, abort_flag)) break;
                 mbar_expect_tx(full(s), (uint32_t)(A_STAGE + I8_B_BYTES));        // boxes past an edge are zero-filled and still counted
-                tma_load_2d(smem_u32(a_ring + (size_t)s * A_STAGE), &map_a, kb * I8_KB, m0, full(s));
+                tma_load_2d(smem_u32(a_ring + (size_t)s * A_STAGE), &map_a, (kb0 + kb) * I8_KB, m0, full(s));
                 if (p.b_mn) {
-                    // two boxes of 128 columns of N x 128 rows of K, as they lie in B
-                    tma_load_2d(smem_u32(b_ring + (size_t)s * I8_B_BYTES), &map_b, n0, kb * I8_KB, full(s));
-                    tma_load_2d(smem_u32(b_ring + (size_t)s * I8_B_BYTES + I8_B_BYTES / 2), &map_b, n0 + 128, kb * I8_KB, full(s));
+                    // boxes of 128 columns of N x 128 rows of K, as they lie in B
+#pragma unroll
+                    for (int c = 0; c < BN; c += 128)
+                        tma_load_2d(smem_u32(b_ring + (size_t)s * I8_B_BYTES + c * I8_KB), &map_b, n0 + c, (kb0 + kb) * I8_KB, full(s));
                 } else {
-                    tma_load_2d(smem_u32(b_ring + (size_t)s * I8_B_BYTES), &map_b, kb * I8_KB, n0, full(s));
+                    tma_load_2d(smem_u32(b_ring + (size_t)s * I8_B_BYTES), &map_b, (kb0 + kb) * I8_KB, n0, full(s));
                 }
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = i8_idesc() | (p.b_mn ? (1u << 16) : 0u);       // bit 16: B is MN-major
+            const uint32_t idesc = i8_idesc(BN) | (p.b_mn ? (1u << 16) : 0u);       // bit 16: B is MN-major
             const uint64_t b_step = p.b_mn ? (uint64_t)((32 * 128) >> 4) : 2u;     // 32 k: 32 rows of the box, or 32 bytes of the swizzle row
             bool ok = true;
             for (int kb = 0; kb < KB; kb++) {
@@ -151,59 +160,74 @@ lux_matmul_int8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
                 const uint64_t b_desc = p.b_mn ? make_mnmajor_sw128_desc(b_addr) : make_kmajor_sw128_desc(b_addr);
 #pragma unroll
                 for (int a = 0; a < MA; a++) {
-                    // accumulator a: rows a * 128 .. of the A box, TMEM columns a * 256 ..
+                    // accumulator a: rows a * 128 .. of the A box, TMEM columns a * BN ..
                     const uint64_t a_desc = make_kmajor_sw128_desc(smem_u32(a_ring + (size_t)s * A_STAGE + (size_t)a * I8_A_BYTES));
 #pragma unroll
                     for (int k = 0; k < I8_KB / 32; k++)  // 32 k = 32 bytes inside the 128-byte swizzle row: +2 in the address field
-                        umma_i8(tmem_base + (uint32_t)(a * 256), a_desc + (uint64_t)(2 * k), b_desc + b_step * (uint64_t)k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        umma_i8(tmem_base + (uint32_t)(a * BN), a_desc + (uint64_t)(2 * k), b_desc + b_step * (uint64_t)k, idesc, (kb | k) != 0 ? 1u : 0u);
                 }
                 umma_commit(empty(s));
             }
             if (ok) umma_commit(acc_full);
         }
-    } else {
-        // epilogue warps: TMEM lane quarter = warp % 4 (a warp reaches only its own quarter)
+    }
+    __syncwarp();
+    // epilogue warps: TMEM lane quarter = warp % 4 (a warp reaches only its own quarter)
+    bool done = false;
+    auto epilogue = [&](auto add_tag) {
+        constexpr bool ADD = decltype(add_tag)::value;
         const int quad = warp & 3;
+        const bool vec = (p.N & 3) == 0;
+        uint32_t* patch = reinterpret_cast<uint32_t*>(a_ring) + (warp - 2) * (32 * 33);   // the loads are over: the ring is free
+#pragma unroll 1
+        for (int cc = 0; cc < MA * I8_BN; cc += 32) {
+            const int a = cc / I8_BN, c0 = cc - a * I8_BN;
+            const int row0 = m0 + a * I8_BM + quad * 32;
+            const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * I8_BN);
+            if (n0 + c0 >= p.N || m0 + a * I8_BM >= p.M) continue;   // warp-uniform
+            uint32_t v[32];
+            tmem_ld32(lane_addr + (uint32_t)c0, v);
+            tmem_ld_wait();
+            // through this warp's 32 x 33-word patch of the (idle) ring, so that a store instruction
+            // writes four whole 128-byte pieces of four rows instead of 16 bytes of 32 rows
+#pragma unroll
+            for (int j = 0; j < 32; j++) patch[lane * 33 + j] = v[j];
+            __syncwarp();
+            int* dst = p.c + (size_t)row0 * p.N + n0 + c0;
+            if (ADD) {
+                const int rows = min(32, p.M - row0);
+                if (n0 + c0 + lane < p.N)
+                    for (int r = 0; r < rows; r++)
+                        asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" ::"l"(dst + (size_t)r * p.N + lane), "r"(patch[r * 33 + lane]) : "memory");
+            } else if (vec && n0 + c0 + 32 <= p.N) {
+#pragma unroll
+                for (int it = 0; it < 8; it++) {
+                    const int r = it * 4 + (lane >> 3), q = lane & 7;
+                    const uint32_t* src = patch + r * 33 + q * 4;
+                    if (row0 + r < p.M)
+                        *reinterpret_cast<int4*>(dst + (size_t)r * p.N + q * 4) = make_int4((int)src[0], (int)src[1], (int)src[2], (int)src[3]);
+                }
+            } else {
+                const int rows = min(32, p.M - row0);
+                if (n0 + c0 + lane < p.N)
+                    for (int r = 0; r < rows; r++) dst[(size_t)r * p.N + lane] = (int)patch[r * 33 + lane];
+            }
+            __syncwarp();
+        }
+        tc_fence_before();
+    };
+    if (warp >= 2) {
         // (sleeping between polls: these four warps wait for the whole main loop, and tight polls next to
         // the MMA-issuing thread make its own satisfied waits several times dearer)
-        bool ok = warp_wait_relaxed(acc_full, 0u, abort_flag, lane);
-        if (ok) {
+        done = warp_wait_relaxed(acc_full, 0u, abort_flag, lane);
+        if (done) {
             tc_fence_after();
-            const bool vec = (p.N & 3) == 0;
-            uint32_t* patch = reinterpret_cast<uint32_t*>(a_ring) + (warp - 2) * (32 * 33);   // the loads are over: the ring is free
-#pragma unroll 1
-            for (int cc = 0; cc < MA * I8_BN; cc += 32) {
-                const int a = cc / I8_BN, c0 = cc - a * I8_BN;
-                const int row = m0 + a * I8_BM + quad * 32 + lane;
-                const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * 256);
-                if (n0 + c0 >= p.N || m0 + a * I8_BM >= p.M) continue;   // warp-uniform
-                uint32_t v[32];
-                tmem_ld32(lane_addr + (uint32_t)c0, v);
-                tmem_ld_wait();
-                if (vec && n0 + c0 + 32 <= p.N) {
-                    // through this warp's 32 x 33-word patch of the (idle) ring, so that a store instruction
-                    // writes four whole 128-byte pieces of four rows instead of 16 bytes of 32 rows
-#pragma unroll
-                    for (int j = 0; j < 32; j++) patch[lane * 33 + j] = v[j];
-                    __syncwarp();
-#pragma unroll
-                    for (int it = 0; it < 8; it++) {
-                        const int r = it * 4 + (lane >> 3), q = lane & 7;
-                        const int grow = m0 + a * I8_BM + quad * 32 + r;
-                        const uint32_t* src = patch + r * 33 + q * 4;
-                        if (grow < p.M)
-                            *reinterpret_cast<int4*>(p.c + (size_t)grow * p.N + n0 + c0 + q * 4) = make_int4((int)src[0], (int)src[1], (int)src[2], (int)src[3]);
-                    }
-                    __syncwarp();
-                } else if (row < p.M) {
-                    int* dst = p.c + (size_t)row * p.N + n0 + c0;
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (n0 + c0 + j < p.N) dst[j] = (int)v[j];
-                }
-            }
-            tc_fence_before();
+            if (blockIdx.z == 0) epilogue(std::false_type{});
         }
+    }
+    if (gridDim.z > 1) {
+        cluster_sync_all();              // slice 0's tile is published (every thread reaches this on every path)
+        if (done && blockIdx.z > 0) epilogue(std::true_type{});
     }
     __syncthreads();
     if (*abort_flag) {
@@ -213,7 +237,7 @@ lux_matmul_int8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
     }
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, MA * 256);
+        tmem_dealloc(tmem_base, MA * BN);
     }
 }
 
@@ -271,7 +295,7 @@ __global__ void __launch_bounds__(256) lux_unpack_s4_s8(const uint8_t* __restric
 // Returns NOT_SUPPORTED for shapes this kernel does not take (the caller falls back to the
 // mma.sync kernels): fewer than a tile's worth of work, K not a multiple of 16, unaligned views.
 LuxBackendError launch_matmul_int8_tcgen05(Context* ctx, const void* a, const void* b, int* c, int M, int N, int K, bool a_int4) {
-    if (K % 16 || (size_t)M * N < (size_t)I8_BM * I8_BN || K < 256) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
+    if (K % 16 || (size_t)M * N < (size_t)128 * 256 || K < 256) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     // B as it lies when its rows can be a tensor map's (N a multiple of 16 bytes); else through B^T
     const bool b_mn = N % 16 == 0 && g_tune.int_matmul_kernel != 2;
@@ -305,8 +329,26 @@ LuxBackendError launch_matmul_int8_tcgen05(Context* ctx, const void* a, const vo
     CUtensorMap ma_map, mb;
     const uint64_t adims[2] = {(uint64_t)K, (uint64_t)M}, bdims[2] = {(uint64_t)K, (uint64_t)N};
     const uint64_t strides[1] = {(uint64_t)K};
-    const int ma = M > I8_BM ? 2 : 1;
-    const uint32_t abox[2] = {(uint32_t)I8_KB, (uint32_t)(ma * I8_BM)}, bbox[2] = {(uint32_t)I8_KB, (uint32_t)I8_BN};
+    // Tile: the one whose waves of CTAs cost least.  A stage of 128 k takes the tensor pipe 1024 / 512 / 256 cycles in
+    // the three forms, but its operands (64 / 48 / 32 KB) arrive at about 50 bytes per clock and SM, which is
+    // what bounds all three: 1310 / 980 / 655.
+    // Against the first form alone (the second up to 128 rows): 512 x 4096 x 4096 29.4 -> 14.1 us, 128 x 4096 x 4096
+    // 19.2 -> 12.0, 256 x 1024 x 4096 (split four ways) 29.8 -> 10.3; 4096^3 keeps the first form.
+    const int stages = (K + I8_KB - 1) / I8_KB, sms = ctx->sm_count;
+    struct Form { int ma, bn, cost; };
+    const Form forms[3] = {{2, 256, 1310}, {1, 256, 980}, {1, 128, 655}};
+    auto ctas_of = [&](const Form& f) { return (long long)((N + f.bn - 1) / f.bn) * ((M + f.ma * I8_BM - 1) / (f.ma * I8_BM)); };
+    const Form* best = &forms[0];
+    long long best_cost = 0;
+    for (const Form& f : forms) {
+        const long long cost = (ctas_of(f) + sms - 1) / sms * f.cost;
+        if (best_cost == 0 || cost < best_cost) { best = &f; best_cost = cost; }
+    }
+    const int ma = best->ma, bn = best->bn;
+    // split K while that still finds idle SMs and leaves a slice at least four stages
+    unsigned ks = 1;
+    while (ks < 4 && ctas_of(*best) * (ks * 2) <= sms && stages >= (int)(ks * 2) * 4) ks *= 2;
+    const uint32_t abox[2] = {(uint32_t)I8_KB, (uint32_t)(ma * I8_BM)}, bbox[2] = {(uint32_t)I8_KB, (uint32_t)bn};
     if (!encode_tensor_map_u8(&ma_map, 2, a_int4 ? (const void*)a8 : a, adims, strides, abox, true)) return LUX_BACKEND_ERROR_INTERNAL;
     if (b_mn) {
         const uint64_t dims_mn[2] = {(uint64_t)N, (uint64_t)K}, strides_mn[1] = {(uint64_t)N};
@@ -318,19 +360,21 @@ LuxBackendError launch_matmul_int8_tcgen05(Context* ctx, const void* a, const vo
     static std::atomic<bool> configured[64];
     int dev = ctx->device & 63;
     if (!configured[dev].load(std::memory_order_relaxed)) {
-        if (cudaFuncSetAttribute(lux_matmul_int8_tcgen05<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8_smem(1)) != cudaSuccess ||
-            cudaFuncSetAttribute(lux_matmul_int8_tcgen05<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8_smem(2)) != cudaSuccess)
+        if (cudaFuncSetAttribute(lux_matmul_int8_tcgen05<2, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8_smem(2, 256)) != cudaSuccess ||
+            cudaFuncSetAttribute(lux_matmul_int8_tcgen05<1, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8_smem(1, 256)) != cudaSuccess ||
+            cudaFuncSetAttribute(lux_matmul_int8_tcgen05<1, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8_smem(1, 128)) != cudaSuccess)
             return map_cuda(cudaGetLastError(), "lux_matmul_int8_tcgen05");
         configured[dev].store(true, std::memory_order_relaxed);
     }
     I8Params p{c, ctx->d_status, M, N, K, b_mn ? 1 : 0};
-    const dim3 grid((N + I8_BN - 1) / I8_BN, (M + ma * I8_BM - 1) / (ma * I8_BM));
-    if (ma == 2) lux_matmul_int8_tcgen05<2><<<grid, I8_THREADS, i8_smem(2), ctx->stream>>>(ma_map, mb, p);
-    else lux_matmul_int8_tcgen05<1><<<grid, I8_THREADS, i8_smem(1), ctx->stream>>>(ma_map, mb, p);
+    const dim3 grid((N + bn - 1) / bn, (M + ma * I8_BM - 1) / (ma * I8_BM), ks);
+    auto kfn = ma == 2 ? lux_matmul_int8_tcgen05<2, 256> : bn == 256 ? lux_matmul_int8_tcgen05<1, 256> : lux_matmul_int8_tcgen05<1, 128>;
+    cudaError_t e = launch_pdl(false, kfn, grid, dim3(I8_THREADS), i8_smem(ma, bn), ctx->stream, ks, ma_map, mb, p);
+    if (e != cudaSuccess) return map_cuda(e, "lux_matmul_int8_tcgen05");
     count_launch(a_int4 ? "lux_matmul_int4_int8_tcgen05" : "lux_matmul_int8_tcgen05");
     return LUX_BACKEND_OK;
 }
 
-const void* kernel_addr_matmul_int8_tcgen05() { return (const void*)lux_matmul_int8_tcgen05<2>; }
+const void* kernel_addr_matmul_int8_tcgen05() { return (const void*)lux_matmul_int8_tcgen05<2, 256>; }
 
 }  // namespace luxcuda

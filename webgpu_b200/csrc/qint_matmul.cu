@@ -15,6 +15,7 @@
 // int4 weights are sign-extended to bytes while they are staged.  Shapes the tiled kernel does not
 // take (K % 16, N % 16, unaligned views) run in a plain one-thread-per-output kernel.
 #include "common.cuh"
+#include "round_div.cuh"
 
 #include <algorithm>
 
@@ -152,88 +153,105 @@ __global__ void __launch_bounds__(256) lux_matmul_int8_plain(const uint8_t* __re
     C[o] = sum;
 }
 
-__global__ void __launch_bounds__(256) lux_requantize_i32_i8(const int* __restrict__ in, int* __restrict__ out, size_t n,
-                                                            float in_scale, float out_scale, int zp) {
-    const size_t stride = (size_t)gridDim.x * 256;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += stride) {
-        const float v = __fmul_rn((float)in[i], in_scale);
+// VEC: both views 16-byte aligned, four values per access
+template <bool VEC>
+__global__ void __launch_bounds__(256) lux_requantize_i32_i8(const int* in, int* out, size_t n, float in_scale, float out_scale, int zp) {
+    auto one = [&](int x) {
+        const float v = __fmul_rn((float)x, in_scale);
         const float r = __fadd_rn(rintf(__fdiv_rn(v, out_scale)), (float)zp);
-        out[i] = min(max(__float2int_rz(r), -128), 127);
+        return min(max(__float2int_rz(r), -128), 127);
+    };
+    const size_t stride = (size_t)gridDim.x * 256;
+    size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (VEC) {
+        for (size_t j = i; j < n / 4; j += stride) {
+            const int4 x = reinterpret_cast<const int4*>(in)[j];
+            reinterpret_cast<int4*>(out)[j] = make_int4(one(x.x), one(x.y), one(x.z), one(x.w));
+        }
+        i += n / 4 * 4;
     }
+    for (; i < n; i += stride) out[i] = one(in[i]);
 }
 
-// phase 1 of dynamic_quantize: max |x| over the tensor, as the bit pattern of a non-negative float
-__global__ void __launch_bounds__(256) lux_absmax_f32(const float* __restrict__ x, size_t n, uint32_t* __restrict__ out_bits) {
+// max over the block's 256 threads of non-negative values, on every thread
+__device__ __forceinline__ float block_max(float m) {
+    __shared__ float part[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; w++) m = fmaxf(m, part[w]);
+    return m;
+}
+
+// phase 1 of dynamic_quantize: max |x| over the tensor.  One word per block, reduced by every block of phase 2:
+// nothing to clear first, and no thousands of atomics on one word.
+__global__ void __launch_bounds__(256) lux_absmax_f32(const float* __restrict__ x, size_t n, float* __restrict__ part) {
+    pdl_launch_dependents();                   // phase 2 may take its place; it waits for this grid
     float m = 0.0f;
     const size_t stride = (size_t)gridDim.x * 256, t0 = (size_t)blockIdx.x * 256 + threadIdx.x;
     if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
-        // 16-byte loads, two in flight per thread
+        // 16-byte loads, four in flight per thread
         const float4* x4 = reinterpret_cast<const float4*>(x);
+        auto amax = [](float4 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))); };
         const size_t n4 = n / 4;
         size_t i = t0;
-        for (; i + stride < n4; i += 2 * stride) {
-            const float4 a = __ldg(x4 + i), b = __ldg(x4 + i + stride);
-            m = fmaxf(m, fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
-                               fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w)))));
+        for (; i + 3 * stride < n4; i += 4 * stride) {
+            const float4 a = __ldg(x4 + i), b = __ldg(x4 + i + stride), c = __ldg(x4 + i + 2 * stride), d = __ldg(x4 + i + 3 * stride);
+            m = fmaxf(m, fmaxf(fmaxf(amax(a), amax(b)), fmaxf(amax(c), amax(d))));
         }
-        if (i < n4) {
-            const float4 a = __ldg(x4 + i);
-            m = fmaxf(m, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))));
-        }
+        for (; i < n4; i += stride) m = fmaxf(m, amax(__ldg(x4 + i)));
         for (size_t j = n4 * 4 + t0; j < n; j += stride) m = fmaxf(m, fabsf(x[j]));
     } else {
         for (size_t i = t0; i < n; i += stride) m = fmaxf(m, fabsf(x[i]));
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out_bits, __float_as_uint(m));
+    m = block_max(m);
+    if (threadIdx.x == 0) part[blockIdx.x] = m;
 }
 
 // phase 2: scale = max / 127 (or / 7), 1 if that is 0; q = clamp(i32(round(x / scale))); eight values per thread
 template <int BITS>
-__global__ void __launch_bounds__(256) lux_dynamic_quantize(const float* __restrict__ x, size_t n, const uint32_t* __restrict__ max_bits,
+__global__ void __launch_bounds__(256) lux_dynamic_quantize(const float* __restrict__ x, size_t n, const float* __restrict__ part, uint32_t parts,
                                                            uint8_t* __restrict__ out, float* __restrict__ scale_out) {
-    float scale = __fdiv_rn(__uint_as_float(*max_bits), BITS == 4 ? 7.0f : 127.0f);
+    pdl_wait();
+    float m = 0.0f;
+    for (uint32_t i = threadIdx.x; i < parts; i += 256) m = fmaxf(m, __ldcg(part + i));
+    float scale = __fdiv_rn(block_max(m), BITS == 4 ? 7.0f : 127.0f);
     if (scale == 0.0f) scale = 1.0f;
+    const float ri = __frcp_rn(scale);
+    const bool ok = round_div_ok(scale);
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
     const size_t octets = (n + 7) / 8;
     const size_t stride = (size_t)gridDim.x * 256;
     // 16-byte loads and (int8) 8-byte stores where the views allow them
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(out) & 7u) == 0;
     for (size_t o = (size_t)blockIdx.x * 256 + threadIdx.x; o < octets; o += stride) {
-        int q[8];
-        if (vec && o * 8 + 8 <= n) {
+        float v[8];
+        const bool whole = vec && o * 8 + 8 <= n;
+        if (whole) {
             const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * o), b = __ldg(reinterpret_cast<const float4*>(x) + 2 * o + 1);
-            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int j = 0; j < 8; j++) q[j] = __float2int_rz(rintf(__fdiv_rn(v[j], scale)));
-            if (BITS == 8) {
-                uint32_t lo = 0, hi = 0;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    lo |= (uint32_t)(min(max(q[j], -128), 127) & 0xFF) << (8 * j);
-                    hi |= (uint32_t)(min(max(q[4 + j], -128), 127) & 0xFF) << (8 * j);
-                }
-                *reinterpret_cast<uint2*>(out + o * 8) = make_uint2(lo, hi);
-                continue;
-            }
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const size_t i = o * 8 + j;
-                q[j] = i < n ? __float2int_rz(rintf(__fdiv_rn(x[i], scale))) : 0;
-            }
+            for (int j = 0; j < 8; j++) v[j] = o * 8 + j < n ? x[o * 8 + j] : 0.0f;
         }
+        uint32_t t[8];
         if (BITS == 4) {
-            uint32_t w = 0;
-#pragma unroll
-            for (int j = 0; j < 8; j++) w |= (uint32_t)((min(max(q[j], -8), 7) + 8) & 0xF) << (4 * j);   // pack_nax_int4_sym_x8
+            round_div<4>(v, scale, ri, ok, -8, 7, 8, t);
+            const uint32_t w = round_div_pack4(t);                                                       // pack_nax_int4_sym_x8
             if (o * 4 + 4 <= (n + 1) / 2) *reinterpret_cast<uint32_t*>(out + o * 4) = w;
             else for (size_t b = o * 4; b < (n + 1) / 2; b++) out[b] = (uint8_t)(w >> (8 * (b - o * 4)));
         } else {
+            round_div<8>(v, scale, ri, ok, -128, 127, 0, t);
+            if (whole) {
+                *reinterpret_cast<uint2*>(out + o * 8) =
+                    make_uint2(round_div_pack8(t[0], t[1], t[2], t[3]), round_div_pack8(t[4], t[5], t[6], t[7]));
+            } else {
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-                if (o * 8 + j < n) out[o * 8 + j] = (uint8_t)(min(max(q[j], -128), 127) & 0xFF);
+                for (int j = 0; j < 8; j++)
+                    if (o * 8 + j < n) out[o * 8 + j] = (uint8_t)(t[j] & 0xFFu);
+            }
         }
     }
 }
@@ -298,8 +316,10 @@ LuxBackendError lux_cuda_requantize_int32_to_int8(LuxBackendContext* context, Lu
     if (bi->size < n * 4 || bo->size < n * 4) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     if (n == 0) return LUX_BACKEND_OK;
     cudaSetDevice(ctx->device);
-    const size_t blocks = std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 16);
-    lux_requantize_i32_i8<<<(unsigned)blocks, 256, 0, ctx->stream>>>((const int*)bi->ptr, (int*)bo->ptr, n, input_scale, output_scale,
+    const bool vec = aligned16(bi->ptr) && aligned16(bo->ptr);
+    const size_t blocks = std::min<size_t>(((vec ? (n + 3) / 4 : n) + 255) / 256, (size_t)ctx->sm_count * 16);
+    auto kfn = vec ? lux_requantize_i32_i8<true> : lux_requantize_i32_i8<false>;
+    kfn<<<(unsigned)blocks, 256, 0, ctx->stream>>>((const int*)bi->ptr, (int*)bo->ptr, n, input_scale, output_scale,
                                                                       output_zero_point);
     count_launch();
     return finish_op(ctx, false, "lux_cuda_requantize_int32_to_int8");
@@ -315,14 +335,12 @@ LuxBackendError lux_cuda_dynamic_quantize(LuxBackendContext* context, LuxBackend
     if ((reinterpret_cast<uintptr_t>(bo->ptr) & 3u) != 0) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
     std::lock_guard<std::mutex> lock(ctx->mu);                 // the max word belongs to the context
-    LUX_CUDA_TRY(cudaMemsetAsync(ctx->d_absmax, 0, sizeof(uint32_t), ctx->stream));
-    const size_t blocks = std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 8);
-    lux_absmax_f32<<<(unsigned)blocks, 256, 0, ctx->stream>>>((const float*)bx->ptr, n, ctx->d_absmax);
+    const unsigned parts = (unsigned)std::min<size_t>((n + 2047) / 2048, std::min(ctx->sm_count * 4, ABSMAX_PARTS));
+    lux_absmax_f32<<<parts, 256, 0, ctx->stream>>>((const float*)bx->ptr, n, ctx->d_absmax);
     const size_t qblocks = std::min<size_t>(((n + 7) / 8 + 255) / 256, (size_t)ctx->sm_count * 8);
-    if (bits == 4)
-        lux_dynamic_quantize<4><<<(unsigned)qblocks, 256, 0, ctx->stream>>>((const float*)bx->ptr, n, ctx->d_absmax, (uint8_t*)bo->ptr, (float*)bs->ptr);
-    else
-        lux_dynamic_quantize<8><<<(unsigned)qblocks, 256, 0, ctx->stream>>>((const float*)bx->ptr, n, ctx->d_absmax, (uint8_t*)bo->ptr, (float*)bs->ptr);
+    auto kfn = bits == 4 ? lux_dynamic_quantize<4> : lux_dynamic_quantize<8>;
+    LUX_CUDA_TRY(launch_pdl(g_tune.pdl != 2, kfn, dim3((unsigned)qblocks), dim3(256), 0, ctx->stream, 1, (const float*)bx->ptr, n,
+                            (const float*)ctx->d_absmax, (uint32_t)parts, (uint8_t*)bo->ptr, (float*)bs->ptr));
     count_launch(2);
     ctx->writer_pending = true;
     return finish_op(ctx, false, "lux_cuda_dynamic_quantize");
