@@ -112,3 +112,40 @@ def test_quantize_argument_checks(ctx, backend):
     assert call(B.make_desc(0, 4, 200, 4, 128, B.F32, B.F32, B.F32)) == B.INVALID_ARGUMENT   # K % group
     assert call(B.make_desc(0, 4, 256, 4, 128, B.F32, B.F32, B.F32), ww=ctx.alloc(16)) == B.INVALID_ARGUMENT
     assert lib.lux_cuda_qquantize(ctx.handle, None, x.handle, w.handle, s.handle, None) == B.INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("bits,symmetric,shifted", [(4, False, False), (4, True, False), (4, False, True), (8, True, False)])
+@pytest.mark.parametrize("kind", ["half_integers", "far_from_zero", "denormal_scale", "non_finite"])
+def test_rounding_without_division_is_the_division_s(ctx, bits, symmetric, shifted, kind):
+    """The kernel divides only where the product with the reciprocal lies next to a half-integer: values on
+    and one ulp either side of every half-integer times the scale, quotients far beyond the clamp, scales
+    whose reciprocal overflows, and NaN / infinities, bit for bit against the oracle's divisions."""
+    group = 128 if bits == 4 else 32
+    rng = np.random.default_rng(21)
+    N, K = 16, 512
+    x = rng.standard_normal((N, K)).astype(np.float32)
+    if kind == "half_integers":
+        top = {(4, True): 7.0, (4, False): 15.0, (8, True): 127.0}[(bits, symmetric)]
+        for r in range(N):
+            s = np.float32(rng.uniform(0.01, 3.0))
+            s = np.float32(np.float16(s)) if bits == 4 else s
+            h = (rng.integers(0, int(top), K) + np.float32(0.5)).astype(np.float32) * s
+            x[r] = np.nextafter(h, np.float32(np.inf) if r % 3 == 1 else np.float32(-np.inf)) if r % 3 else h
+            if symmetric:
+                x[r] *= rng.choice([-1, 1], K).astype(np.float32)
+            x[r, ::group] = s * np.float32(top)              # fixes the group's scale
+            x[r, 1::group] = 0.0
+    elif kind == "far_from_zero":
+        x = x * np.float32(0.01) + np.float32(100.0) * rng.choice([-1, 1], (N, 1)).astype(np.float32)
+    elif kind == "denormal_scale":
+        x *= np.float32(1e-39)
+    else:
+        x[0, 3], x[1, 4], x[2, 5] = np.nan, np.inf, -np.inf
+    sd = B.F32
+    L = ctx.qquantize(x, bits, symmetric, sd, flags=B.FLAG_QUANT_SHIFTED if shifted else 0)
+    w, s, z = _to_host(L, N, K, bits, sd)
+    rw, rs, rz = orc.quantize(x, bits, group, symmetric, orc.F32, shifted=shifted)
+    finite = np.isfinite(rs)                                 # which NaN a scale holds is not specified
+    assert np.array_equal(s[finite].view(np.uint32), rs[finite].view(np.uint32))
+    assert rz is None or np.array_equal(z, rz)
+    assert np.array_equal(w.view(np.uint8), rw.view(np.uint8))

@@ -25,6 +25,7 @@
 // programmatic-launch trigger), and the entry point marks the context so that the next matmul is
 // launched fully ordered behind it.
 #include "common.cuh"
+#include "round_div.cuh"
 
 namespace luxcuda {
 
@@ -63,20 +64,24 @@ __device__ __forceinline__ void load8(const QuantParams& p, size_t idx, float (&
 }
 
 // BITS = 4: groups of 128 (16 lanes); BITS = 8: groups of 32 (4 lanes), symmetric only.
+// With a division per element, and the group's three per eight elements, the arithmetic took longer than the
+// memory: 14336 x 4096 f32 to int4 with zero-points 73 us (266 MB, 3.6 TB/s).  round_div.cuh divides only
+// next to half-integers and the group's divisions are spread over its lanes: 55 us (4.8 TB/s).
 // A warp takes QCH consecutive 256-element chunks of a row and requests all of them before it
 // reduces the first: 4 KB in flight per warp, so that a streaming kernel with this little
 // arithmetic keeps HBM busy.
 constexpr int QCH = 4;
 
 template <int BITS, bool SYM>
-__global__ void __launch_bounds__(256) lux_qquantize(const QuantParams p) {
+__global__ void __launch_bounds__(256, 4) lux_qquantize(const QuantParams p) {
     constexpr int GL = BITS == 4 ? 16 : 4;                  // lanes per group
     const int lane = threadIdx.x & 31;
-    const size_t wid = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int wpr = (p.chunks_per_row + QCH - 1) / QCH;     // warps per row
-    const size_t n = wid / (size_t)wpr;
-    if (n >= (size_t)p.N) return;
-    const int c0 = (int)(wid - n * (size_t)wpr) * QCH;
+    const uint32_t wid = blockIdx.x * 8u + (threadIdx.x >> 5);
+    const uint32_t wpr = (uint32_t)(p.chunks_per_row + QCH - 1) / QCH;     // warps per row
+    const uint32_t row = wid / wpr;
+    if (row >= (uint32_t)p.N) return;
+    const size_t n = row;
+    const int c0 = (int)(wid - row * wpr) * QCH;
     float v[QCH][8];
     bool live[QCH];
 #pragma unroll
@@ -85,71 +90,78 @@ __global__ void __launch_bounds__(256) lux_qquantize(const QuantParams p) {
         live[ch] = k0 < p.K;                                 // K is a multiple of the group size, so of 8
         if (live[ch]) load8(p, n * (size_t)p.K + k0, v[ch]);
     }
+    // group statistics of all chunks
+    float mx[QCH], mn[QCH];
+#pragma unroll
+    for (int ch = 0; ch < QCH; ch++) {
+        mx[ch] = -1e30f;                                     // the shader's seeds (:169-170)
+        mn[ch] = 1e30f;
+        if (live[ch]) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                mx[ch] = fmaxf(mx[ch], v[ch][i]);
+                mn[ch] = fminf(mn[ch], v[ch][i]);
+            }
+        }
+#pragma unroll
+        for (int o = GL / 2; o > 0; o >>= 1) {
+            mx[ch] = fmaxf(mx[ch], __shfl_xor_sync(0xffffffffu, mx[ch], o));
+            mn[ch] = fminf(mn[ch], __shfl_xor_sync(0xffffffffu, mn[ch], o));
+        }
+    }
+    // Scale, zero-point and reciprocal: each lane works them out for ONE of its group's positions in the QCH
+    // chunks (lane % QCH), so that a warp goes through those divisions once, not once per chunk.
+    static_assert(QCH == 4 && GL >= QCH, "one lane of a group per chunk");
+    const bool h1 = lane & 1, h2 = lane & 2;
+    const float amx = h2 ? (h1 ? mx[3] : mx[2]) : (h1 ? mx[1] : mx[0]), amn = h2 ? (h1 ? mn[3] : mn[2]) : (h1 ? mn[1] : mn[0]);
+    float scale;
+    int zp = 0;
+    if (SYM) {
+        scale = __fdiv_rn(fmaxf(fabsf(amx), fabsf(amn)), BITS == 4 ? 7.0f : 127.0f);
+    } else {
+        scale = __fdiv_rn(amx - amn, 15.0f);
+        zp = min(max(__float2int_rz(rintf(__fdiv_rn(-amn, scale))), 0), 15);   // before the guard, as in the shader
+    }
+    if (scale == 0.0f) scale = 1.0f;
+    // compact table: an f16 table stores the rounded scale, and the values are quantized with the
+    // number the table holds (what dequantize will multiply by)
+    const __half s16 = __float2half_rn(scale);
+    if (p.scale_dtype == LUX_QDTYPE_F16) scale = __half2float(s16);
+    const float ri = __frcp_rn(scale);
+    {
+        const int k0 = (c0 + (lane & 3)) * 256 + (lane & ~(GL - 1)) * 8;       // first element of this lane's group
+        if ((lane & (GL - 1)) < QCH && k0 < p.K) {
+            const size_t at = n * (size_t)p.G + k0 / (BITS == 4 ? 128 : 32);
+            if (p.scale_dtype == LUX_QDTYPE_F16) reinterpret_cast<__half*>(p.scales)[at] = s16;
+            else reinterpret_cast<float*>(p.scales)[at] = scale;
+        }
+        if (BITS == 4 && !SYM) {
+            // the two groups of a chunk share a byte (the second is absent in the last chunk of an odd row)
+            const int zp_hi = __shfl_down_sync(0xffffffffu, zp, 16);
+            if (lane < QCH && k0 < p.K) p.zeros[n * (size_t)p.ZS + c0 + lane] = (uint8_t)(zp | (k0 + 128 < p.K ? zp_hi << 4 : 0));
+        }
+    }
+    const bool ok = round_div_ok(scale);
 #pragma unroll
     for (int ch = 0; ch < QCH; ch++) {
         const int c = c0 + ch;
         const int k0 = c * 256 + lane * 8;
         if (c >= p.chunks_per_row) break;                    // warp-uniform
-        float mx = -1e30f, mn = 1e30f;                       // the shader's seeds (:169-170)
-        if (live[ch]) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                mx = fmaxf(mx, v[ch][i]);
-                mn = fminf(mn, v[ch][i]);
-            }
-        }
-#pragma unroll
-        for (int o = GL / 2; o > 0; o >>= 1) {
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        }
-        float scale;
-        int zp = 0;
-        if (SYM) {
-            const float amax = fmaxf(fabsf(mx), fabsf(mn));
-            scale = __fdiv_rn(amax, BITS == 4 ? 7.0f : 127.0f);
-        } else {
-            scale = __fdiv_rn(mx - mn, 15.0f);
-            zp = min(max(__float2int_rz(rintf(__fdiv_rn(-mn, scale))), 0), 15);   // before the guard, as in the shader
-        }
-        if (scale == 0.0f) scale = 1.0f;
-        // compact table: an f16 table stores the rounded scale, and the values are quantized with the
-        // number the table holds (what dequantize will multiply by)
-        const __half s16 = __float2half_rn(scale);
-        if (p.scale_dtype == LUX_QDTYPE_F16) scale = __half2float(s16);
-        const int g = k0 / (BITS == 4 ? 128 : 32);
-        if (live[ch] && (lane % GL) == 0) {
-            if (p.scale_dtype == LUX_QDTYPE_F16) reinterpret_cast<__half*>(p.scales)[n * (size_t)p.G + g] = s16;
-            else reinterpret_cast<float*>(p.scales)[n * (size_t)p.G + g] = scale;
-        }
-        if (BITS == 4 && !SYM) {
-            const int zp_hi = __shfl_sync(0xffffffffu, live[ch] ? zp : 0, 16);
-            if (lane == 0 && live[ch]) p.zeros[n * (size_t)p.ZS + c] = (uint8_t)(zp | (zp_hi << 4));
-        }
+        const int src = (lane & ~(GL - 1)) | ch;             // the lane that worked out this chunk's group
+        const float sc = __shfl_sync(0xffffffffu, scale, src), rc = __shfl_sync(0xffffffffu, ri, src);
+        const int zc = __shfl_sync(0xffffffffu, zp | (ok ? 256 : 0), src);
         if (!live[ch]) continue;
-        int q[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = __float2int_rz(rintf(__fdiv_rn(v[ch][i], scale)));   // saturating; NaN -> 0
-        if (BITS == 4) {
-            uint32_t word = 0;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                int nib;
-                if (SYM) nib = min(max(q[i], -8), 7) + 8;
-                else if (p.shifted) nib = min(max(min(max(q[i], -32), 32) + zp, 0), 15);   // pre-clamped: a saturated q must not wrap
-                else nib = min(max(q[i], 0), 15);                         // (clamp(q, 0, 15) - zp) + zp, clamped again
-                word |= (uint32_t)nib << (4 * i);
-            }
-            reinterpret_cast<uint32_t*>(p.w)[(n * (size_t)p.K + k0) >> 3] = word;
-        } else {
-            uint32_t lo = 0, hi = 0;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                lo |= ((uint32_t)min(max(q[i], -128), 127) & 0xFFu) << (8 * i);
-                hi |= ((uint32_t)min(max(q[4 + i], -128), 127) & 0xFFu) << (8 * i);
-            }
-            reinterpret_cast<uint2*>(p.w)[(n * (size_t)p.K + k0) >> 3] = make_uint2(lo, hi);
-        }
+        // stored value = clamp(rint(v / scale), lo, hi) + off:
+        //   int8 and symmetric int4: the signed range; asymmetric int4: clamp(.., 0, 15) (the shader takes
+        //   the zero-point out and back in around a second clamp); shifted: clamp(rint + zp, 0, 15)
+        const int off = BITS == 8 ? 0 : SYM ? 8 : p.shifted ? zc & 15 : 0;
+        uint32_t t[8];
+        round_div<BITS>(v[ch], sc, rc, zc >= 256, BITS == 8 ? -128 : -off, BITS == 8 ? 127 : 15 - off, off, t);
+        if (BITS == 4)
+            reinterpret_cast<uint32_t*>(p.w)[(n * (size_t)p.K + k0) >> 3] = round_div_pack4(t);
+        else
+            reinterpret_cast<uint2*>(p.w)[(n * (size_t)p.K + k0) >> 3] =
+                make_uint2(round_div_pack8(t[0], t[1], t[2], t[3]), round_div_pack8(t[4], t[5], t[6], t[7]));
     }
 }
 
