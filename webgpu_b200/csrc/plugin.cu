@@ -45,15 +45,21 @@ LuxBackendError finish_op(Context* ctx, bool no_sync, const char* what) {
 
 enum BinOp { OP_ADD = 0, OP_SUB = 1, OP_MUL = 2 };
 
-template <int OP>
-__global__ void lux_binary_f32(const float* __restrict__ a, const float* __restrict__ b,
-                               float* __restrict__ out, size_t n) {
+// 16-byte accesses where all three views allow them (VEC): one access per thread and operand covers four
+// elements, so that a prompt-sized call is one short wave of blocks (512 x 4096: 7.7 -> 6.3 us, 25 MB).
+template <int OP, bool VEC>
+__global__ void __launch_bounds__(256) lux_binary_f32(const float* a, const float* b, float* out, size_t n) {
+    auto op = [](float x, float y) { return OP == OP_ADD ? x + y : (OP == OP_SUB ? x - y : x * y); };
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (; i < n; i += stride) {
-        float x = a[i], y = b[i];
-        out[i] = OP == OP_ADD ? x + y : (OP == OP_SUB ? x - y : x * y);
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    if (VEC) {
+        for (size_t j = i; j < n / 4; j += stride) {
+            const float4 x = reinterpret_cast<const float4*>(a)[j], y = reinterpret_cast<const float4*>(b)[j];
+            reinterpret_cast<float4*>(out)[j] = make_float4(op(x.x, y.x), op(x.y, y.y), op(x.z, y.z), op(x.w, y.w));
+        }
+        i += n / 4 * 4;
     }
+    for (; i < n; i += stride) out[i] = op(a[i], b[i]);
 }
 
 // out[M,N] = a[M,K] . b[K,N], row-major, 32x32 tiles, f32 accumulate in ascending k.
@@ -282,9 +288,11 @@ static LuxBackendError binary_op(LuxBackendContext* context, LuxBackendBuffer* a
     if (ba->size < n * 4 || bb->size < n * 4 || bo->size < n * 4) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     if (n == 0) return LUX_BACKEND_OK;
     cudaSetDevice(ctx->device);
-    size_t blocks = std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 16);
-    lux_binary_f32<OP><<<(unsigned)blocks, 256, 0, ctx->stream>>>(
-        (const float*)ba->ptr, (const float*)bb->ptr, (float*)bo->ptr, n);
+    const bool vec = ((reinterpret_cast<uintptr_t>(ba->ptr) | reinterpret_cast<uintptr_t>(bb->ptr) | reinterpret_cast<uintptr_t>(bo->ptr)) & 15u) == 0;
+    const size_t items = vec ? (n + 3) / 4 : n;
+    const size_t blocks = std::min<size_t>((items + 255) / 256, (size_t)ctx->sm_count * 16);
+    auto kfn = vec ? lux_binary_f32<OP, true> : lux_binary_f32<OP, false>;
+    kfn<<<(unsigned)blocks, 256, 0, ctx->stream>>>((const float*)ba->ptr, (const float*)bb->ptr, (float*)bo->ptr, n);
     count_launch();
     return finish_op(ctx, false, "binary_f32");
 }
