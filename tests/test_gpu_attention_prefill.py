@@ -1,0 +1,129 @@
+"""lux_attn_prefill_mma_f32 and the f32 kernel behind it (many queries per head, head size 128) at the sizes where
+their tiling can go wrong: queries and keys one off a tile of 64 or a block of 128, one tile, several,
+masked and not, appended to a cache, heads that share a KV head, operands of very different magnitudes, NaN
+and infinities; against the oracle, and against the streaming kernel.  Tolerance as in test_gpu_attention.py:
+relative L2 <= 2e-6 (f32 sums in another order; the split into two f16 parts keeps 22 bits of each factor)."""
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from webgpu_b200 import backend as B
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-6
+KERNELS = {1: "lux_attn_prefill_mma_f32", 3: "lux_attn_prefill_f32"}      # by the tunable attn_prefill
+
+
+class _Tuned:
+    def __init__(self, backend, **kw):
+        self.backend, self.kw = backend, kw
+
+    def __enter__(self):
+        for k, v in self.kw.items():
+            self.backend.tune(k, v)
+
+    def __exit__(self, *exc):
+        for k in self.kw:
+            self.backend.tune(k, 0)
+
+
+def _qkv(seed, B_, H, Hkv, Sq, Skv, D=128):
+    rng = np.random.default_rng(seed)
+    return [rng.standard_normal(s, np.float32) for s in ((B_, H, Sq, D), (B_, Hkv, Skv, D), (B_, Hkv, Skv, D))]
+
+
+def _sdpa(ctx, q, k, v, causal, scale=None):
+    B_, H, Sq, D = q.shape
+    qb, kb, vb, ob, lb = ctx.upload(q), ctx.upload(k), ctx.upload(v), ctx.alloc(q.nbytes), ctx.alloc(B_ * H * Sq * 4)
+    ctx.sdpa(qb, kb, vb, ob, B_, H, k.shape[1], Sq, k.shape[2], D, 1 / np.sqrt(D) if scale is None else scale, lse=lb,
+             flags=B.FLAG_ATTN_CAUSAL if causal else 0)
+    return ob.to_host(np.float32, q.shape), lb.to_host(np.float32, (B_, H, Sq))
+
+
+@pytest.mark.parametrize("mode", [1, 3])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("B_,H,Hkv,Sq,Skv", [(1, 2, 2, 127, 128), (1, 1, 1, 129, 191), (1, 2, 1, 260, 300), (1, 2, 2, 1, 1), (1, 2, 1, 63, 63), (1, 2, 2, 64, 64), (2, 4, 2, 65, 65), (1, 4, 1, 17, 129),
+                                             (1, 3, 3, 130, 40), (2, 4, 4, 200, 257)])
+def test_tile_edges(ctx, backend, B_, H, Hkv, Sq, Skv, causal, mode):
+    q, k, v = _qkv(Sq * 1000 + Skv, B_, H, Hkv, Sq, Skv)
+    with _Tuned(backend, attn_prefill=mode):
+        got, lse = _sdpa(ctx, q, k, v, causal)
+        assert backend.last_kernel_name() == KERNELS[mode]
+    want, want_lse = orc.sdpa(q, k, v, 1 / np.sqrt(128), causal, want_lse=True)
+    assert orc.rel_l2(got, want) < TOL
+    np.testing.assert_allclose(got, want, rtol=1e-4, atol=1e-5)
+    np.testing.assert_allclose(lse, want_lse, rtol=1e-5, atol=1e-5)
+    assert ctx.last_device_status() == 0
+
+
+@pytest.mark.parametrize("Sq,cache_len,max_len", [(64, 0, 64), (65, 63, 200), (100, 301, 512)])
+def test_chunk_appended_to_a_cache(ctx, backend, Sq, cache_len, max_len):
+    """Causal rows start at cache_len, and two KV heads lie max_len rows apart: the streaming kernel's answer
+    to the same call is the reference (both sum in f32; 2e-6 as against the oracle)."""
+    q, k, v = _qkv(cache_len, 2, 8, 2, Sq, max_len)
+    qb, kb, vb, ob = ctx.upload(q), ctx.upload(k), ctx.upload(v), ctx.alloc(q.nbytes)
+    outs = []
+    for mode in (1, 3, 2):
+        with _Tuned(backend, attn_prefill=mode):
+            ctx.sdpa_kv_cache(qb, kb, vb, ob, 2, 8, 2, Sq, cache_len, max_len, 128, 1 / np.sqrt(128), flags=B.FLAG_ATTN_CAUSAL)
+            assert mode == 2 or backend.last_kernel_name() == KERNELS[mode]
+        outs.append(ob.to_host(np.float32, q.shape).copy())
+    assert orc.rel_l2(outs[0], outs[2]) < TOL and orc.rel_l2(outs[1], outs[2]) < TOL
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_values_a_row_must_not_see_do_not_reach_it(ctx, backend, bad):
+    """A causal row ignores later positions altogether: a NaN or infinity in V (or NaN in K) there leaves every
+    earlier row bit for bit as it was, and reaches every row that sees it."""
+    q, k, v = _qkv(5, 1, 2, 1, 150, 150)
+    v2, k2 = v.copy(), k.copy()
+    v2[0, 0, 70, 3] = bad
+    k2[0, 0, 100, 5] = np.nan
+    with _Tuned(backend, attn_prefill=3):
+        clean, _ = _sdpa(ctx, q, k, v, True)
+        got, lse = _sdpa(ctx, q, k2, v2, True)
+    assert np.array_equal(got[:, :, :70].view(np.uint32), clean[:, :, :70].view(np.uint32))
+    assert not np.isfinite(got[:, :, 70:100, 3]).any() and np.array_equal(got[:, :, 70:100, 4], clean[:, :, 70:100, 4])
+    # the tensor-core kernel leaves such a call to the f32 kernel: the same bits; the next call is its own again
+    with _Tuned(backend, attn_prefill=1):
+        got1, lse1 = _sdpa(ctx, q, k2, v2, True)
+        after, _ = _sdpa(ctx, q, k, v, True)
+    assert np.array_equal(got1.view(np.uint32), got.view(np.uint32)) and np.array_equal(lse1.view(np.uint32), lse.view(np.uint32))
+    assert orc.rel_l2(after, clean) < TOL
+
+
+@pytest.mark.parametrize("mode", [1, 3])
+def test_no_keys_and_large_scores(ctx, backend, mode):
+    q, k, v = _qkv(6, 1, 2, 2, 70, 70)
+    with _Tuned(backend, attn_prefill=mode):
+        got, lse = _sdpa(ctx, q * 100, k, v, False)
+        empty, _ = _sdpa(ctx, q, k[:, :, :0], v[:, :, :0], False)
+    want, want_lse = orc.sdpa(q * 100, k, v, 1 / np.sqrt(128), False, want_lse=True)
+    # scores reach 450, where a rounding of the score is worth 450 x 2^-24 = 3e-5 of a weight; a few such add up
+    assert orc.rel_l2(got, want) < 1e-4
+    np.testing.assert_allclose(lse, want_lse, rtol=1e-5, atol=1e-4)
+    assert not empty.any()
+
+
+def test_magnitudes_far_apart(ctx, backend):
+    """Rows of K, columns of V and the whole of Q at scales from 1e-12 to 1e12 of each other: every output column keeps
+    its own relative precision (a power of two per row and column is taken out before the f16 split)."""
+    q, k, v = _qkv(8, 1, 2, 1, 140, 200)
+    rng = np.random.default_rng(8)
+    ks = 10.0 ** rng.uniform(-12, 0, (1, 1, 200, 1))
+    vs = 10.0 ** rng.uniform(-12, 12, (1, 1, 1, 128))
+    k, v = (k * ks).astype(np.float32), (v * vs).astype(np.float32)
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, False)
+    want = orc.sdpa(q, k, v, 1 / np.sqrt(128), False)
+    err = np.sqrt((((got - want) / vs) ** 2).sum(axis=(0, 1, 2)) / ((want / vs) ** 2).sum(axis=(0, 1, 2)))
+    assert err.max() < 2 * TOL, err.max()                 # the worst of 128 columns, each with 280 values
+
+
+@pytest.mark.parametrize("H,S,kernel", [(32, 256, "lux_attn_prefill_mma_f32"), (8, 128, "lux_attn_stream_f32")])
+def test_default_choice(ctx, backend, H, S, kernel):
+    """Prompts with enough (head, 64 queries) blocks to fill the chip take it, small ones the key-splitting kernel."""
+    q, k, v = _qkv(7, 1, H, H, S, S)
+    got, _ = _sdpa(ctx, q, k, v, True)
+    assert backend.last_kernel_name() == kernel
+    assert orc.rel_l2(got[:, :2], orc.sdpa(q[:, :2], k[:, :2], v[:, :2], 1 / np.sqrt(128), True)) < TOL

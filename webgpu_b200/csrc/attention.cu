@@ -666,6 +666,24 @@ AttnKernel pick_stream(int vpl, int rt, bool full) {
     return nullptr;
 }
 
+// What lux_attn_prefill_f32 takes (q, k and v have been found aligned).
+bool prefill_fits(const AttnParams& p) {
+    return !p.block_size && p.head_dim == 128 && aligned16(p.out) && (uint64_t)p.batch * p.heads * ((p.seq_q + 63u) / 64u) <= 0x7fffffffu;
+}
+// Where it is the faster kernel: when its CTAs (one per 64 queries of a head, each walking its keys alone)
+// are enough to occupy the chip; the streaming kernel also splits the keys.
+bool prefill_pays(const AttnParams& p) {
+    if (p.seq_q < 64 || p.kv_len == 0) return false;
+    uint64_t total = 0, longest = 1;                               // 64-key tiles
+    for (uint32_t q0 = 0; q0 < p.seq_q; q0 += 64) {
+        const uint64_t last = std::min<uint64_t>(q0 + 63u, p.seq_q - 1u);
+        const uint64_t keys = p.causal ? std::min<uint64_t>(p.causal_base + last + 1u, p.kv_len) : p.kv_len;
+        total += (keys + 63) / 64;
+        longest = std::max(longest, (keys + 63) / 64);
+    }
+    return total * p.batch * p.heads >= 64 * longest;
+}
+
 // Fills the launch geometry of p and launches.  max_keys: the longest context any row can have.
 LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint32_t flags, const char* what) {
     cudaSetDevice(ctx->device);
@@ -683,6 +701,23 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
         lux_attn_plain_f32<<<(unsigned)out_rows, 256, smem, ctx->stream>>>(p);
         count_launch("lux_attn_plain_f32");
         return finish_op(ctx, (flags & LUX_QMATMUL_FLAG_NO_SYNC) != 0, what);
+    }
+    if (prefill_fits(p) && g_tune.attn_prefill != 2 && (g_tune.attn_prefill || prefill_pays(p))) {
+        PrefillArgs f{};
+        f.q = p.q; f.k = p.k; f.v = p.v; f.out = p.out; f.lse = p.lse;
+        f.status = p.status; f.status_wait = ATT_STATUS_WAIT;
+        f.batch = p.batch; f.heads = p.heads; f.kv_heads = p.kv_heads; f.group = p.group; f.seq_q = p.seq_q;
+        f.kv_len = p.kv_len; f.kv_stride = p.kv_stride; f.causal = p.causal; f.causal_base = p.causal_base;
+        f.qscale = p.qscale;
+        LuxBackendError e = LUX_BACKEND_OK;
+        if (g_tune.attn_prefill != 3) {
+            f.call = ctx->attn_calls.fetch_add(1u, std::memory_order_relaxed) + 1u;
+            if (f.call == 0) f.call = ATTN_REDO;                                   // 0 is what an unused word holds
+            f.redo = ctx->d_attn_redo + f.call % ATTN_REDO;
+            e = launch_attn_prefill_mma(ctx, f);
+        }
+        if (e == LUX_BACKEND_OK) e = launch_attn_prefill(ctx, f);
+        return e != LUX_BACKEND_OK ? e : finish_op(ctx, (flags & LUX_QMATMUL_FLAG_NO_SYNC) != 0, what);
     }
     int vpl = (int)((D + 31) / 32);
     if (vpl > 4) vpl = 8;

@@ -50,6 +50,9 @@ struct Context {
     void*          d_int = nullptr;         // lux_cuda_matmul_int8 on the tcgen05 path: B transposed (and A unpacked), grown on demand
     size_t         d_int_bytes = 0;
     void*          d_attn = nullptr;        // partial results of attention calls that split the keys over CTAs:
+    uint32_t*      d_attn_redo = nullptr;   // prompt attention: ATTN_REDO words, call n writes n into word n % ATTN_REDO when it meets
+                                            // non-finite inputs (a word per call, so that calls on different streams do not meet)
+    std::atomic<uint32_t> attn_calls{0};    // prompt-attention calls so far
     size_t         d_attn_bytes = 0;        // 16 MB, allocated with the context (a call takes fewer slices rather than allocate)
     std::mutex     mu;                      // guards the staging buffers
     int            sm_count = 148;
@@ -61,6 +64,7 @@ struct Context {
 };
 
 constexpr int ABSMAX_PARTS = 1024;
+constexpr uint32_t ATTN_REDO = 256;
 
 inline Context* as_ctx(LuxBackendContext* c) { return reinterpret_cast<Context*>(c); }
 inline Buffer*  as_buf(LuxBackendBuffer* b) { return reinterpret_cast<Buffer*>(b); }
@@ -124,6 +128,8 @@ struct Tunables {
     int gemm_min_m = 0;          // smallest batch the weights-in-TMEM GEMM takes from the streaming kernels (0 = built-in)
     int gemm_tc_kernel = 0;      // 0 auto, 1 lux_qgemm_i4_tc, 2 lux_qgemm_i4_tc_wa wherever it applies
     int int_matmul_kernel = 0;   // lux_cuda_matmul_int8 / _int4_int8: 0 tcgen05 for large shapes, 1 mma.sync kernels only, 2 tcgen05 always through B^T
+    int attn_prefill = 0;        // attention of many queries per head: 0 choose, 1 lux_attn_prefill_mma_f32 wherever it applies, 2 never,
+                                 // 3 lux_attn_prefill_f32 wherever it applies
     int attn_splits = 0;         // attention: slices of the keys per (sequence, KV head, row block); 0 = choose
     int gemm_wa_narrow = 0;      // weights-in-TMEM GEMM, batch <= 64: 0 narrow tile (two CTAs per SM) when the launch has more CTAs
                                  // than SMs, 1 always, 2 never
@@ -299,6 +305,24 @@ LuxBackendError launch_qgemv_i4_units(Context* ctx, const QArgs& a);    // NOT_S
 LuxBackendError launch_qgemm_i4_tc(Context* ctx, const QArgs& a);
 LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a);    // NOT_SUPPORTED if the shape does not fit
 LuxBackendError launch_qdequant(Context* ctx, const QArgs& a, int bits);
+
+// attention_prefill.cu: contiguous K and V, head size 128, all pointers 16-byte aligned
+struct PrefillArgs {
+    const float *q, *k, *v;
+    float* out;
+    float* lse;                  // may be null
+    uint32_t* status;
+    uint32_t status_wait;        // reported when a bounded wait gives up
+    uint32_t batch, heads, kv_heads, group, seq_q;
+    uint32_t kv_len, kv_stride;  // keys a row may see; rows between the bases of two KV heads
+    uint32_t causal, causal_base;// causal: query i sees min(causal_base + i + 1, kv_len) keys
+    uint32_t q_blocks;           // blocks of queries (set by the launchers)
+    float qscale;                // scale * log2(e)
+    uint32_t* redo;              // the tensor-core kernel writes `call` here where it met non-finite inputs, and the
+    uint32_t call;               // f32 kernel then does the call (null: unconditionally)
+};
+LuxBackendError launch_attn_prefill_mma(Context* ctx, PrefillArgs p);
+LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p);
 
 // tensor_ops.cu: the f32 slots the reference's shader library backs but its plugin leaves unwired
 LuxBackendError op_div_f32(LuxBackendContext*, LuxBackendBuffer* a, LuxBackendBuffer* b, LuxBackendBuffer* out, size_t n);
