@@ -227,7 +227,7 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
         // =============================== MMA issuer =====================================
         // One wait, eight MMAs and one commit per unit: a satisfied mbarrier wait and a commit
         // cost this thread ~200 and ~100 cycles, so they are paid once per 128 K, not per 64.
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(BF16, p.ncols);
             int s = 0;
             uint32_t ph = 0;

@@ -147,7 +147,7 @@ lux_matmul_int8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = i8_idesc(BN) | (p.b_mn ? (1u << 16) : 0u);       // bit 16: B is MN-major
             const uint64_t b_step = p.b_mn ? (uint64_t)((32 * 128) >> 4) : 2u;     // 32 k: 32 rows of the box, or 32 bytes of the swizzle row
             bool ok = true;
