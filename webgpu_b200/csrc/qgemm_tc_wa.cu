@@ -96,6 +96,17 @@ __device__ __forceinline__ void group_consts(__half sh, uint32_t zp, uint32_t& z
     }
 }
 
+// The 64 packed bytes of a weight row in a quantization group, by two 32-byte loads: with 16-byte ones each of a
+// warp's 32 rows hands over its 32-byte sectors in halves (config 4 `o` at 16 rows 8.3 -> 7.9 us, `down` at 128 rows
+// 21.4 -> 20.4; with L1 bypassed, where the halves become separate L2 reads, 26.4 against 18.8 us for `down` at 16).
+__device__ __forceinline__ void load_row64(const uint8_t* src, uint4 (&q)[4]) {
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(q[2 * i].x), "=r"(q[2 * i].y), "=r"(q[2 * i].z), "=r"(q[2 * i].w), "=r"(q[2 * i + 1].x), "=r"(q[2 * i + 1].y), "=r"(q[2 * i + 1].z), "=r"(q[2 * i + 1].w)
+            : "l"(src + 32 * i));
+}
+
 template <int CW> __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[CW]);
 template <> __device__ __forceinline__ void tmem_ld_cols<32>(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 template <> __device__ __forceinline__ void tmem_ld_cols<16>(uint32_t taddr, uint32_t (&r)[16]) {
@@ -161,28 +172,30 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
     uint4 nq[4];                                        // next unit's 64 packed bytes of this thread's row
     __half nsh = __float2half(0.f);
     uint32_t nzb = 0x88u;                               // byte holding the next unit's zero-point nibble (raw: no use of a loaded value inside fetch)
+    // Where the next unit of this thread lies: packed row, scale, zero-point byte; advanced by NG units per fetch.  The
+    // converters' instructions per unit are on the critical path (a build with some hundred more per unit lost
+    // 400 cycles of a unit's 940), so nothing is recomputed from the unit's number: config 4 at 16 rows, gate_up
+    // 26.3 -> 25.0 us, down 18.0 -> 17.4; at 128 rows 41.8 -> 40.3 and 20.4 -> 19.8.
     const uint8_t* wp = nullptr;
     const __half* sp = nullptr;
-    const uint8_t* zrow = nullptr;
-    auto fetch = [&](int u) {
-        const uint4* src = reinterpret_cast<const uint4*>(wp + (size_t)u * (WA_UNIT_K / 2));
-#pragma unroll
-        for (int i = 0; i < 4; i++) nq[i] = __ldg(src + i);
-        // the line two fetches ahead is asked for now, so that the register fetch finds it in L2
-        if (p.prefetch && u + p.prefetch < U)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(wp + (size_t)(u + p.prefetch) * (WA_UNIT_K / 2)));
-        nsh = __ldg(sp + u);
-        if (zrow) nzb = (uint32_t)__ldg(zrow + ((g_base + u) >> 1));
+    const uint8_t* zp = nullptr;                        // of unit pair g / 2; null without zero-points
+    int zodd = (g_base + grp) & 1;                      // whether the next unit is the second of its pair
+    auto fetch = [&](bool ahead) {
+        load_row64(wp, nq);
+        // the line some units ahead is asked for now, so that the register fetch finds it in L2
+        if (ahead) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp + (size_t)p.prefetch * (WA_UNIT_K / 2)));
+        nsh = __ldg(sp);
+        if (zp) nzb = (uint32_t)__ldg(zp);
     };
     if (warp >= 2) {
         const int r = quad * 32 + lane;                 // this thread's TMEM lane and its weight row
         // the lanes of a last tile that has fewer outputs read its last row again; they are not written
         const int orow = min(n0 + (SW ? r & (OUT_W - 1) : r), p.Nout - 1);
         const int wrow = SW && r >= OUT_W ? p.up_row_offset + orow : orow;
-        wp = p.w + (size_t)wrow * (p.K / 2) + (k_base >> 1);
-        sp = p.scales + (size_t)wrow * p.G + g_base;
-        zrow = p.zeros ? p.zeros + (size_t)wrow * p.ZS : nullptr;
-        if (grp < U) fetch(grp);
+        wp = p.w + (size_t)wrow * (p.K / 2) + (size_t)(g_base + grp) * (WA_UNIT_K / 2);
+        sp = p.scales + (size_t)wrow * p.G + g_base + grp;
+        zp = p.zeros ? p.zeros + (size_t)wrow * p.ZS + ((g_base + grp) >> 1) : nullptr;
+        if (grp < U) fetch(p.prefetch && grp + p.prefetch < U);
     } else if (tid == 1) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
     } else if (tid == 0) {
@@ -253,15 +266,22 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
         // =============================== converters =====================================
         // Group `grp` takes units grp, grp + NG, ...; NG <= P keeps a group at most one lap of the
         // ring ahead of the commit it waits for, which is what a one-bit phase can tell apart.
+        int s = grp;                                    // ring slot of unit u and the lap's parity
+        uint32_t ph = 0;
+        const int last_ahead = p.prefetch ? U - p.prefetch : 0;
         for (int u = grp; u < U && ok; u += NG) {
             uint4 cq[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) cq[i] = nq[i];
             uint32_t zc, sa, sb;
-            group_consts<BF16>(nsh, (nzb >> (((g_base + u) & 1) * 4)) & 0xFu, zc, sa, sb);
-            if (u + NG < U) fetch(u + NG);
-            const int s = u % P;
-            const uint32_t ph = (uint32_t)(u / P) & 1u;
+            group_consts<BF16>(nsh, (nzb >> (zodd * 4)) & 0xFu, zc, sa, sb);
+            if (u + NG < U) {
+                wp += NG * (WA_UNIT_K / 2);
+                sp += NG;
+                if (zp) zp += (NG + zodd) >> 1;
+                zodd = (zodd + NG) & 1;
+                fetch(u + NG < last_ahead);
+            }
             const uint32_t a_dst = tmem_a0 + ((uint32_t)(quad * 32) << 16) + (uint32_t)(s * WA_UNIT_A_COLS);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
@@ -285,6 +305,8 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(full(s));
+            s += NG;
+            if (s >= P) { s -= P; ph ^= 1u; }
         }
         if (ok && warp < 10) ok = warp_wait(acc_full, 0u, abort_flag, lane);
         if (ok) tc_fence_after();
@@ -493,7 +515,7 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     if (a.push || nout % 8 || a.K % 128 || a.M < 1) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     if (a.scale_dtype != LUX_QDTYPE_F16 || a.x_dtype != a.y_dtype) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     if (a.x_dtype != LUX_QDTYPE_BF16 && a.x_dtype != LUX_QDTYPE_F16) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(a.w) & 15u) || (a.K / 2) % 16) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(a.w) & 31u) || (a.K / 2) % 32) return LUX_BACKEND_ERROR_NOT_SUPPORTED;      // 32-byte loads of weight rows
     // x is fetched by TMA and y written in 16-byte pieces: a caller's oddly offset view stays with the
     // kernels that use plain loads and stores
     if ((reinterpret_cast<uintptr_t>(a.x) & 15u) || (reinterpret_cast<uintptr_t>(a.y) & 15u)) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
