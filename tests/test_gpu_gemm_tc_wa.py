@@ -219,3 +219,21 @@ def test_wa_outputs_that_fill_no_tile(ctx, backend, dtype, splitk, M, N):
         else:
             assert orc.rel_l2(y, _oracle(x, lay)) < TOL_16
     assert ctx.last_device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("M,N,K", [(5, 128, 1024), (16, 264, 2048), (33, 384, 1024), (64, 1024, 4096)])
+def test_wa_eight_k_splits(ctx, backend, dtype, M, N, K):
+    """Eight CTAs of a cluster take an eighth of K each and finish eight batch rows each (narrow tile only)."""
+    x = synth.activations(M, K, dtype, 50, f"wa8.{M}.{K}")
+    layer = synth.int4_layer(N, K, 50, f"wa8.{N}.{K}")
+    with _Tuned(backend, gemm_tc_kernel=2, gemm_tc_splitk=8, gemm_wa_narrow=1):
+        y = _run(ctx, x, layer)
+        assert backend.last_kernel_name().startswith("lux_qgemm_i4_tc_wa")
+        h = _run_swiglu(ctx, x, layer) if N % 16 == 0 else None
+    assert orc.rel_l2(y, _oracle(x, layer)) < TOL_16
+    if h is not None:
+        code = orc.dtype_code(x)
+        gu = orc.qmatmul(x, *layer.triple, bits=4, group=128, y_code=orc.F32, w_round=code)
+        assert orc.rel_l2(h, orc.swiglu(gu, h_code=code)) < TOL_16
+    assert ctx.last_device_status() == 0

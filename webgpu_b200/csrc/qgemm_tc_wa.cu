@@ -117,6 +117,9 @@ template <> __device__ __forceinline__ void tmem_ld_cols<16>(uint32_t taddr, uin
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr) : "memory");
 }
+template <> __device__ __forceinline__ void tmem_ld_cols<4>(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
 template <> __device__ __forceinline__ void tmem_ld_cols<8>(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -327,7 +330,7 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
     constexpr int KEEP = BN / KS;                               // columns this CTA writes
     const int keep0 = ksplit * KEEP;                            // the first of them
     constexpr int PER_WARP = KEEP / 2;                          // per epilogue warp
-    constexpr int CW = PER_WARP < 32 ? PER_WARP : 32;           // columns per TMEM read (32, 16 or 8)
+    constexpr int CW = PER_WARP < 32 ? PER_WARP : 32;           // columns per TMEM read (32, 16, 8 or 4)
     constexpr int NCH = PER_WARP / CW;                          // reads per warp
     constexpr int SLOT = wa_slot_bytes(BN, KS);                 // split-K: KEEP columns x 128 rows x f32
     // an exchange block: 16 bytes (4 columns) per weight row, rows consecutive, [column quads][128 rows]:
@@ -371,13 +374,13 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
         tmem_ld_cols<CW>(lane_addr + (uint32_t)(keep0 + c0), acc);
         tmem_ld_wait();
         if (KS >= 2) acc_add(acc, peer);
-        if (KS == 4) {
-            // sources 1 and 2 of this CTA's slot row (source 0 came in `peer`)
-            float4 r1[CW / 4], r2[CW / 4];
-            load_peer(r1, c0, more, q0);
-            load_peer(r2, c0, more + SLOT, q0);
-            acc_add(acc, r1);
-            acc_add(acc, r2);
+        if (KS >= 4) {
+            // the other sources of this CTA's slot row (source 0 came in `peer`)
+            float4 r[KS >= 4 ? KS - 2 : 1][CW / 4];
+#pragma unroll
+            for (int k = 0; k < KS - 2; k++) load_peer(r[k], c0, more + k * SLOT, q0);
+#pragma unroll
+            for (int k = 0; k < KS - 2; k++) acc_add(acc, r[k]);
         }
         if constexpr (SW) {
             // gate and up of one output sit on different lanes (r and r + 64): the sums go to
@@ -397,21 +400,21 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
         }
     };
 
-    if (KS == 4) {
-        // four CTAs, four quarters of K: CTA r finishes columns [KEEP r, KEEP r + KEEP); block (d, s) of
+    if (KS >= 4) {
+        // four (eight) CTAs, as many parts of K: CTA r finishes columns [KEEP r, KEEP r + KEEP); block (d, s) of
         // the tile's slot holds what the s-th CTA after d (cyclically) leaves for d.  One read per warp.
-        static_assert(KS != 4 || NCH == 1, "four K splits: one TMEM read per epilogue warp");
-        unsigned char* slot4 = p.splitk + (size_t)(blockIdx.x + gridDim.x * blockIdx.y) * (12 * SLOT);
+        static_assert(KS < 4 || NCH == 1, "four or eight K splits: one TMEM read per epilogue warp");
+        unsigned char* slots = p.splitk + (size_t)(blockIdx.x + gridDim.x * blockIdx.y) * (KS * (KS - 1) * SLOT);
         if (ep_warp && ok) {
 #pragma unroll 1
-            for (int dd = 1; dd < 4; dd++) {
-                const int d = (ksplit + dd) & 3;                    // destination; this CTA is its source 3 - dd
-                send_chunk(d * KEEP + eh * PER_WARP, slot4 + (size_t)(d * 3 + 3 - dd) * SLOT, eh * (PER_WARP / 4));
+            for (int dd = 1; dd < KS; dd++) {
+                const int d = (ksplit + dd) & (KS - 1);             // destination; this CTA is its source KS - 1 - dd
+                send_chunk(d * KEEP + eh * PER_WARP, slots + (size_t)(d * (KS - 1) + KS - 1 - dd) * SLOT, eh * (PER_WARP / 4));
             }
         }
         cluster_sync_all();          // release / acquire at cluster scope: every block is published
         if (ep_warp && ok) {
-            const unsigned char* row = slot4 + (size_t)(ksplit * 3) * SLOT;
+            const unsigned char* row = slots + (size_t)(ksplit * (KS - 1)) * SLOT;
             float4 r0[CW / 4];
             load_peer(r0, eh * PER_WARP, row, eh * (PER_WARP / 4));
             finalize_chunk(eh * PER_WARP, r0, row + SLOT, eh * (PER_WARP / 4));
@@ -525,11 +528,19 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     // (`slots` = CTAs resident at once).
     auto plan = [&](int bn, int slots, int& ks_out) {
         const int tiles = (nout + out_w - 1) / out_w * ((a.M + bn - 1) / bn);
-        const bool can_split = a.K % 256 == 0 && (size_t)tiles * (2 * wa_slot_bytes(bn, 2)) <= ctx->d_splitk_bytes;
-        const bool can_split4 = a.K % 512 == 0 && (size_t)tiles * (12 * wa_slot_bytes(bn, 4)) <= ctx->d_splitk_bytes;
-        int ks = (tiles * 4 <= slots && can_split4) ? 4 : (tiles * 2 <= slots && can_split) ? 2 : 1;
-        if (g_tune.gemm_tc_splitk == 1 || (g_tune.gemm_tc_splitk == 2 && can_split) || (g_tune.gemm_tc_splitk == 4 && can_split4))
-            ks = g_tune.gemm_tc_splitk;
+        auto can = [&](int ks) {
+            return a.K % (ks * WA_UNIT_K) == 0 && (size_t)tiles * ((ks == 2 ? 2 : ks * (ks - 1)) * (size_t)wa_slot_bytes(bn, ks)) <= ctx->d_splitk_bytes;
+        };
+        // Eight ways: narrow tile only, i.e. two CTAs per SM, whose units interleave (660 cycles a unit and SM instead
+        // of 940), where four ways would leave one per SM; each CTA keeps at least four units.  16 / 64 rows,
+        // four ways -> eight: 4096 x 14336 17.1 / 19.0 -> 14.8 / 16.4 us, 3072 x 8192 11.1 / 12.4 -> 10.1 / 10.9,
+        // 4096 x 4096 7.7 / 8.6 -> 7.2 / 8.2; 2048 x 7168 (128 CTAs either way) stays at 10.1.
+        int ks = 1;
+        if (bn == WA_BN_SMALL && tiles * 8 <= slots && can(8) && a.K >= 8 * 4 * WA_UNIT_K) ks = 8;
+        else if (tiles * 4 <= slots && can(4)) ks = 4;
+        else if (tiles * 2 <= slots && can(2)) ks = 2;
+        const int want = g_tune.gemm_tc_splitk;
+        if (want == 1 || ((want == 2 || want == 4 || (want == 8 && bn == WA_BN_SMALL)) && can(want))) ks = want;
         ks_out = ks;
         return tiles * ks;                                      // CTAs of the launch
     };
@@ -579,6 +590,8 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
         constexpr bool BF_ = decltype(bf_tag)::value;
         constexpr bool SW_ = decltype(sw_tag)::value;
         constexpr int BN_ = decltype(bn_tag)::value;
+        if constexpr (BN_ == WA_BN_SMALL)
+            if (ks == 8) return launch_wa<BF_, 8, SW_, BN_>(pdl, mx, p, grid, threads, smem, ctx->stream);
         return ks == 4 ? launch_wa<BF_, 4, SW_, BN_>(pdl, mx, p, grid, threads, smem, ctx->stream)
              : ks == 2 ? launch_wa<BF_, 2, SW_, BN_>(pdl, mx, p, grid, threads, smem, ctx->stream)
                        : launch_wa<BF_, 1, SW_, BN_>(pdl, mx, p, grid, threads, smem, ctx->stream);
