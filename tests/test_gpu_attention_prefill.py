@@ -120,10 +120,10 @@ def test_magnitudes_far_apart(ctx, backend):
     assert err.max() < 2 * TOL, err.max()                 # the worst of 128 columns, each with 280 values
 
 
-@pytest.mark.parametrize("H,S,kernel", [(32, 256, "lux_attn_prefill_mma_f32"), (8, 128, "lux_attn_stream_f32")])
-def test_default_choice(ctx, backend, H, S, kernel):
+@pytest.mark.parametrize("H,S,kernels", [(32, 256, ("lux_attn_prefill_mma_f32",)), (8, 128, ("lux_attn_stream_f32", "lux_attn_merge_f32"))])
+def test_default_choice(ctx, backend, H, S, kernels):
     """Prompts with enough (head, 64 queries) blocks to fill the chip take it, small ones the key-splitting kernel."""
     q, k, v = _qkv(7, 1, H, H, S, S)
     got, _ = _sdpa(ctx, q, k, v, True)
-    assert backend.last_kernel_name() == kernel
+    assert backend.last_kernel_name() in kernels
     assert orc.rel_l2(got[:, :2], orc.sdpa(q[:, :2], k[:, :2], v[:, :2], 1 / np.sqrt(128), True)) < TOL
