@@ -237,3 +237,19 @@ def test_wa_eight_k_splits(ctx, backend, dtype, M, N, K):
         gu = orc.qmatmul(x, *layer.triple, bits=4, group=128, y_code=orc.F32, w_round=code)
         assert orc.rel_l2(h, orc.swiglu(gu, h_code=code)) < TOL_16
     assert ctx.last_device_status() == 0
+
+
+@pytest.mark.parametrize("M", [16, 200])
+def test_wa_weights_at_a_16_byte_offset(ctx, backend, M):
+    """Weights that are 16- but not 32-byte aligned take 16-byte loads: the same bits as the aligned layer."""
+    x = synth.activations(M, 512, "f16", 51, f"wao.{M}")
+    layer = synth.int4_layer(256, 512, 51, "wao")
+    base = _run(ctx, x, layer)
+    L = ctx.upload_layer(layer)
+    w = np.ascontiguousarray(layer.triple[0]).view(np.uint8).ravel()
+    big = ctx.upload(np.concatenate([np.zeros(16, np.uint8), w]))
+    off = B.DeviceQLayer(4, 128, 256, 512, ctx.wrap(big.device_ptr + 16, w.size), L.scales, L.zeros, B.F16)
+    xb, yb = ctx.upload(x), ctx.alloc(M * 256 * 2)
+    ctx.qmatmul(xb, off, yb, M, B.F16)
+    assert backend.last_kernel_name() == "lux_qgemm_i4_tc_wa_f16"
+    assert np.array_equal(yb.to_host(np.uint16, (M, 256)), base.view(np.uint16))

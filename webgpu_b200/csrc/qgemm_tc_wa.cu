@@ -1,5 +1,5 @@
 // int4 g128 weight-only GEMM on tcgen05 with the converted WEIGHTS as the tensor-memory A
-// operand: the default for every batch the tensor-core route takes (M >= 33) without SwiGLU.
+// operand: the default from five batch rows up.
 //
 //   y[M, N] = x[M, K] . dequant(W[N, K])^T      x, y bf16 or f16; f32 accumulate in TMEM
 //
@@ -26,7 +26,7 @@
 //                 units g, g + NG, ... of the CTA's K range.
 //   warps 2..9    epilogue.
 //
-// Split-K: with KS = 2 (or 4) the CTAs of a cluster take the halves (quarters) of K for the same tile;
+// Split-K: with KS = 2 (4, 8) the CTAs of a cluster take the halves (quarters, eighths) of K for the same tile;
 // each then leaves the accumulator columns the other one finishes in the pair's slot of a
 // context-owned exchange buffer in global memory (L2-resident; no entry point allocates), one
 // cluster barrier publishes both halves, and each adds what it found to its own half and writes
@@ -76,6 +76,7 @@ struct WaParams {
     int groups;               // converter groups of four warps, <= stages
     int up_row_offset;        // SwiGLU: weight row of `up` = weight row of `gate` + this (= number of outputs)
     int ncols;                // batch rows per tile = UMMA N: 256, or the batch rounded up to 16 when it is smaller
+    int wide;                 // weight rows are 32-byte aligned
     int prefetch;             // units ahead of the register fetch at which a thread asks L2 for its row's line (0 = off)
 };
 
@@ -96,15 +97,21 @@ __device__ __forceinline__ void group_consts(__half sh, uint32_t zp, uint32_t& z
     }
 }
 
-// The 64 packed bytes of a weight row in a quantization group, by two 32-byte loads: with 16-byte ones each of a
-// warp's 32 rows hands over its 32-byte sectors in halves (config 4 `o` at 16 rows 8.3 -> 7.9 us, `down` at 128 rows
-// 21.4 -> 20.4; with L1 bypassed, where the halves become separate L2 reads, 26.4 against 18.8 us for `down` at 16).
-__device__ __forceinline__ void load_row64(const uint8_t* src, uint4 (&q)[4]) {
+// The 64 packed bytes of a weight row in a quantization group, by two 32-byte loads where the weights are 32-byte
+// aligned: with 16-byte ones each of a warp's 32 rows hands over its 32-byte sectors in halves (config 4 `o` at
+// 16 rows 8.3 -> 7.9 us, `down` at 128 rows 21.4 -> 20.4; with L1 bypassed, where the halves become separate L2
+// reads, 26.4 against 18.8 us for `down` at 16).
+__device__ __forceinline__ void load_row64(const uint8_t* src, uint4 (&q)[4], bool wide) {
+    if (wide) {
 #pragma unroll
-    for (int i = 0; i < 2; i++)
-        asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=r"(q[2 * i].x), "=r"(q[2 * i].y), "=r"(q[2 * i].z), "=r"(q[2 * i].w), "=r"(q[2 * i + 1].x), "=r"(q[2 * i + 1].y), "=r"(q[2 * i + 1].z), "=r"(q[2 * i + 1].w)
-            : "l"(src + 32 * i));
+        for (int i = 0; i < 2; i++)
+            asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                : "=r"(q[2 * i].x), "=r"(q[2 * i].y), "=r"(q[2 * i].z), "=r"(q[2 * i].w), "=r"(q[2 * i + 1].x), "=r"(q[2 * i + 1].y), "=r"(q[2 * i + 1].z), "=r"(q[2 * i + 1].w)
+                : "l"(src + 32 * i));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) q[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+    }
 }
 
 template <int CW> __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[CW]);
@@ -184,7 +191,7 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
     const uint8_t* zp = nullptr;                        // of unit pair g / 2; null without zero-points
     int zodd = (g_base + grp) & 1;                      // whether the next unit is the second of its pair
     auto fetch = [&](bool ahead) {
-        load_row64(wp, nq);
+        load_row64(wp, nq, p.wide);
         // the line some units ahead is asked for now, so that the register fetch finds it in L2
         if (ahead) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp + (size_t)p.prefetch * (WA_UNIT_K / 2)));
         nsh = __ldg(sp);
@@ -518,7 +525,7 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     if (a.push || nout % 8 || a.K % 128 || a.M < 1) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     if (a.scale_dtype != LUX_QDTYPE_F16 || a.x_dtype != a.y_dtype) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     if (a.x_dtype != LUX_QDTYPE_BF16 && a.x_dtype != LUX_QDTYPE_F16) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(a.w) & 31u) || (a.K / 2) % 32) return LUX_BACKEND_ERROR_NOT_SUPPORTED;      // 32-byte loads of weight rows
+    if ((reinterpret_cast<uintptr_t>(a.w) & 15u) || (a.K / 2) % 16) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     // x is fetched by TMA and y written in 16-byte pieces: a caller's oddly offset view stays with the
     // kernels that use plain loads and stores
     if ((reinterpret_cast<uintptr_t>(a.x) & 15u) || (reinterpret_cast<uintptr_t>(a.y) & 15u)) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
@@ -581,6 +588,7 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     p.stages = stages;
     p.groups = groups;
     p.ncols = ncols;
+    p.wide = (reinterpret_cast<uintptr_t>(a.w) & 31u) == 0;
     p.prefetch = g_tune.gemm_wa_prefetch < 0 ? 0 : (g_tune.gemm_wa_prefetch > 0 ? g_tune.gemm_wa_prefetch : 2);
 
     dim3 grid((nout + out_w - 1) / out_w, (a.M + bn - 1) / bn, ks);
