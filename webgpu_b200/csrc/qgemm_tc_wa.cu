@@ -76,7 +76,6 @@ struct WaParams {
     int groups;               // converter groups of four warps, <= stages
     int up_row_offset;        // SwiGLU: weight row of `up` = weight row of `gate` + this (= number of outputs)
     int ncols;                // batch rows per tile = UMMA N: 256, or the batch rounded up to 16 when it is smaller
-    int wide;                 // weight rows are 32-byte aligned
     int prefetch;             // units ahead of the register fetch at which a thread asks L2 for its row's line (0 = off)
 };
 
@@ -98,11 +97,12 @@ __device__ __forceinline__ void group_consts(__half sh, uint32_t zp, uint32_t& z
 }
 
 // The 64 packed bytes of a weight row in a quantization group, by two 32-byte loads where the weights are 32-byte
-// aligned: with 16-byte ones each of a warp's 32 rows hands over its 32-byte sectors in halves (config 4 `o` at
+// aligned (W32; a template parameter: deciding it per unit cost a decoder layer at 16 rows 4 us of 63): with 16-byte ones each of a warp's 32 rows hands over its 32-byte sectors in halves (config 4 `o` at
 // 16 rows 8.3 -> 7.9 us, `down` at 128 rows 21.4 -> 20.4; with L1 bypassed, where the halves become separate L2
 // reads, 26.4 against 18.8 us for `down` at 16).
-__device__ __forceinline__ void load_row64(const uint8_t* src, uint4 (&q)[4], bool wide) {
-    if (wide) {
+template <bool W32>
+__device__ __forceinline__ void load_row64(const uint8_t* src, uint4 (&q)[4]) {
+    if (W32) {
 #pragma unroll
         for (int i = 0; i < 2; i++)
             asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -134,7 +134,7 @@ template <> __device__ __forceinline__ void tmem_ld_cols<8>(uint32_t taddr, uint
         : "r"(taddr) : "memory");
 }
 
-template <bool BF16, int KS, bool SW, int BN>
+template <bool BF16, int KS, bool SW, int BN, bool W32>
 __global__ void __launch_bounds__(BN == WA_BN_SMALL ? WA_SMALL_THREADS : WA_MAX_THREADS, BN == WA_BN_SMALL ? 2 : 1)
 lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) {
     constexpr int X_BYTES = BN * 128;                 // x tile of a stage: BN rows x 64 K x 2 bytes
@@ -191,7 +191,7 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
     const uint8_t* zp = nullptr;                        // of unit pair g / 2; null without zero-points
     int zodd = (g_base + grp) & 1;                      // whether the next unit is the second of its pair
     auto fetch = [&](bool ahead) {
-        load_row64(wp, nq, p.wide);
+        load_row64<W32>(wp, nq);
         // the line some units ahead is asked for now, so that the register fetch finds it in L2
         if (ahead) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp + (size_t)p.prefetch * (WA_UNIT_K / 2)));
         nsh = __ldg(sp);
@@ -501,9 +501,9 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
     }
 }
 
-template <bool BF16, int KS, bool SW, int BN>
+template <bool BF16, int KS, bool SW, int BN, bool W32>
 cudaError_t launch_wa(bool pdl, const CUtensorMap& mx, const WaParams& p, dim3 grid, int threads, size_t smem, cudaStream_t st) {
-    auto kfn = lux_qgemm_i4_tc_wa<BF16, KS, SW, BN>;
+    auto kfn = lux_qgemm_i4_tc_wa<BF16, KS, SW, BN, W32>;
     static std::atomic<size_t> configured[64];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -565,14 +565,18 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     if (narrow) ks = ks_narrow;
     const int bn = narrow ? WA_BN_SMALL : WA_BN;
     const int stages = g_tune.gemm_tc_stages >= 2 && g_tune.gemm_tc_stages <= WA_MAX_UNITS ? g_tune.gemm_tc_stages : WA_MAX_UNITS;
-    int groups = g_tune.gemm_tc_groups >= 2 && g_tune.gemm_tc_groups <= WA_MAX_GROUPS ? g_tune.gemm_tc_groups : 2;
+    // Converter groups.  Up to 128 batch columns the MMAs of a unit take half the tensor time or less and the converters
+    // are what the unit waits for: three groups (2 -> 3, M = 72: 11008 x 4096 f16 18.6 -> 17.3 us, bf16 22.2 -> 19.5,
+    // 20480 x 4096 bf16 41.8 -> 36.5; M = 128 bf16 22.6 -> 21.2, f16 equal).  Wider batches lose 2 % with the third
+    // (M = 256: 26.6 -> 27.1), and two CTAs of the narrow tile have no registers for it.
+    const int ncols = a.M >= bn ? bn : (a.M + 15) / 16 * 16;
+    int groups = g_tune.gemm_tc_groups >= 2 && g_tune.gemm_tc_groups <= WA_MAX_GROUPS ? g_tune.gemm_tc_groups : ncols <= 128 ? 3 : 2;
     groups = narrow ? 2 : std::min(groups, stages);
     const size_t smem = 1024 + (size_t)stages * (2 * bn * 128) + 512;
 
     CUtensorMap mx;
     const uint64_t dims[2] = {(uint64_t)a.K * 2, (uint64_t)a.M};
     const uint64_t strides[1] = {(uint64_t)a.K * 2};
-    const int ncols = a.M >= bn ? bn : (a.M + 15) / 16 * 16;
     const uint32_t box[2] = {128, (uint32_t)ncols};
     if (!encode_tensor_map_u8(&mx, 2, a.x, dims, strides, box, true)) return LUX_BACKEND_ERROR_INTERNAL;
 
@@ -588,21 +592,25 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     p.stages = stages;
     p.groups = groups;
     p.ncols = ncols;
-    p.wide = (reinterpret_cast<uintptr_t>(a.w) & 31u) == 0;
     p.prefetch = g_tune.gemm_wa_prefetch < 0 ? 0 : (g_tune.gemm_wa_prefetch > 0 ? g_tune.gemm_wa_prefetch : 2);
 
     dim3 grid((nout + out_w - 1) / out_w, (a.M + bn - 1) / bn, ks);
     const int threads = (2 + 4 * groups) * 32;                  // groups >= 2: the epilogue needs warps 2..9
     const bool pdl = pdl_allowed(ctx, a.weights_volatile);
-    auto go = [&](auto bf_tag, auto sw_tag, auto bn_tag) {
+    auto go_w = [&](auto bf_tag, auto sw_tag, auto bn_tag, auto w32_tag) {
         constexpr bool BF_ = decltype(bf_tag)::value;
         constexpr bool SW_ = decltype(sw_tag)::value;
         constexpr int BN_ = decltype(bn_tag)::value;
+        constexpr bool W_ = decltype(w32_tag)::value;
         if constexpr (BN_ == WA_BN_SMALL)
-            if (ks == 8) return launch_wa<BF_, 8, SW_, BN_>(pdl, mx, p, grid, threads, smem, ctx->stream);
-        return ks == 4 ? launch_wa<BF_, 4, SW_, BN_>(pdl, mx, p, grid, threads, smem, ctx->stream)
-             : ks == 2 ? launch_wa<BF_, 2, SW_, BN_>(pdl, mx, p, grid, threads, smem, ctx->stream)
-                       : launch_wa<BF_, 1, SW_, BN_>(pdl, mx, p, grid, threads, smem, ctx->stream);
+            if (ks == 8) return launch_wa<BF_, 8, SW_, BN_, W_>(pdl, mx, p, grid, threads, smem, ctx->stream);
+        return ks == 4 ? launch_wa<BF_, 4, SW_, BN_, W_>(pdl, mx, p, grid, threads, smem, ctx->stream)
+             : ks == 2 ? launch_wa<BF_, 2, SW_, BN_, W_>(pdl, mx, p, grid, threads, smem, ctx->stream)
+                       : launch_wa<BF_, 1, SW_, BN_, W_>(pdl, mx, p, grid, threads, smem, ctx->stream);
+    };
+    const bool w32 = (reinterpret_cast<uintptr_t>(a.w) & 31u) == 0;
+    auto go = [&](auto bf_tag, auto sw_tag, auto bn_tag) {
+        return w32 ? go_w(bf_tag, sw_tag, bn_tag, std::true_type{}) : go_w(bf_tag, sw_tag, bn_tag, std::false_type{});
     };
     auto go_bn = [&](auto bf_tag, auto sw_tag) {
         return narrow ? go(bf_tag, sw_tag, std::integral_constant<int, WA_BN_SMALL>{})
@@ -617,9 +625,9 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
 }
 
 
-const void* kernel_addr_qgemm_i4_tc_wa_bf16() { return (const void*)lux_qgemm_i4_tc_wa<true, 2, false, WA_BN>; }
-const void* kernel_addr_qgemm_i4_tc_wa_f16() { return (const void*)lux_qgemm_i4_tc_wa<false, 2, false, WA_BN>; }
-const void* kernel_addr_qgemm_i4_tc_wa_bf16_swiglu() { return (const void*)lux_qgemm_i4_tc_wa<true, 1, true, WA_BN>; }
-const void* kernel_addr_qgemm_i4_tc_wa_f16_swiglu() { return (const void*)lux_qgemm_i4_tc_wa<false, 1, true, WA_BN>; }
+const void* kernel_addr_qgemm_i4_tc_wa_bf16() { return (const void*)lux_qgemm_i4_tc_wa<true, 2, false, WA_BN, true>; }
+const void* kernel_addr_qgemm_i4_tc_wa_f16() { return (const void*)lux_qgemm_i4_tc_wa<false, 2, false, WA_BN, true>; }
+const void* kernel_addr_qgemm_i4_tc_wa_bf16_swiglu() { return (const void*)lux_qgemm_i4_tc_wa<true, 1, true, WA_BN, true>; }
+const void* kernel_addr_qgemm_i4_tc_wa_f16_swiglu() { return (const void*)lux_qgemm_i4_tc_wa<false, 1, true, WA_BN, true>; }
 
 }  // namespace luxcuda
