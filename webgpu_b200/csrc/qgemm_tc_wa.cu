@@ -539,11 +539,12 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
             return a.K % (ks * WA_UNIT_K) == 0 && (size_t)tiles * ((ks == 2 ? 2 : ks * (ks - 1)) * (size_t)wa_slot_bytes(bn, ks)) <= ctx->d_splitk_bytes;
         };
         // Eight ways: narrow tile only, i.e. two CTAs per SM, whose units interleave (660 cycles a unit and SM instead
-        // of 940), where four ways would leave one per SM; each CTA keeps at least four units.  16 / 64 rows,
-        // four ways -> eight: 4096 x 14336 17.1 / 19.0 -> 14.8 / 16.4 us, 3072 x 8192 11.1 / 12.4 -> 10.1 / 10.9,
-        // 4096 x 4096 7.7 / 8.6 -> 7.2 / 8.2; 2048 x 7168 (128 CTAs either way) stays at 10.1.
+        // of 940), where four ways would leave one per SM; each CTA keeps at least eight units.  16 / 64 rows, four ways ->
+        // eight: 4096 x 14336 17.1 / 19.0 -> 14.8 / 16.4 us, 3072 x 8192 11.1 / 12.4 -> 10.1 / 10.9.  With four units
+        // each 4096 x 4096 alone gains too (7.7 -> 7.2), but in a decoder layer clusters of eight wait for the kernel
+        // before them to drain: the layer's four GEMMs at 16 rows 60.2 us with `o` split four ways, 63.0 with eight.
         int ks = 1;
-        if (bn == WA_BN_SMALL && tiles * 8 <= slots && can(8) && a.K >= 8 * 4 * WA_UNIT_K) ks = 8;
+        if (bn == WA_BN_SMALL && tiles * 8 <= slots && can(8) && a.K >= 8 * 8 * WA_UNIT_K) ks = 8;
         else if (tiles * 4 <= slots && can(4)) ks = 4;
         else if (tiles * 2 <= slots && can(2)) ks = 2;
         const int want = g_tune.gemm_tc_splitk;
