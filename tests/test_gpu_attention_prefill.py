@@ -92,6 +92,21 @@ def test_values_a_row_must_not_see_do_not_reach_it(ctx, backend, bad):
     assert orc.rel_l2(after, clean) < TOL
 
 
+@pytest.mark.parametrize("bad", [np.nan, -np.inf])
+@pytest.mark.parametrize("row", [0, 15, 16, 77, 127, 128, 149])
+def test_a_non_finite_query_is_noticed_by_every_warp(ctx, backend, row, bad):
+    """One value of Q, in the first or last row of a warp, a block and the call: the f32 kernel's bits, whichever
+    warp meets it and however early."""
+    q, k, v = _qkv(11, 1, 1, 1, 150, 150)
+    q[0, 0, row, row % 128] = bad
+    outs = []
+    for mode in (3, 1):
+        with _Tuned(backend, attn_prefill=mode):
+            outs.append(_sdpa(ctx, q, k, v, True))
+    for a, b in zip(*outs):
+        assert np.array_equal(a[:, :, row // 128 * 128:][:, :, :128].view(np.uint32), b[:, :, row // 128 * 128:][:, :, :128].view(np.uint32))
+
+
 @pytest.mark.parametrize("mode", [1, 3])
 def test_no_keys_and_large_scores(ctx, backend, mode):
     q, k, v = _qkv(6, 1, 2, 2, 70, 70)

@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
         *bad_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncthreads();                              // the flags are clear before a warp may raise one over its rows of Q
     pdl_wait();
     if (tid == 0 && tiles) load_tile(0);
 
