@@ -2,7 +2,7 @@
 their tiling can go wrong: queries and keys one off a tile of 64 or a block of 128, one tile, several,
 masked and not, appended to a cache, heads that share a KV head, operands of very different magnitudes, NaN
 and infinities; against the oracle, and against the streaming kernel.  Tolerance as in test_gpu_attention.py:
-relative L2 <= 2e-6 (f32 sums in another order; the split into two f16 parts keeps 22 bits of each factor)."""
+relative L2 <= 2e-6 (f32 sums in another order; the three bf16 parts of a factor keep all of its 24 bits)."""
 import numpy as np
 import pytest
 
@@ -122,7 +122,7 @@ def test_no_keys_and_large_scores(ctx, backend, mode):
 
 def test_magnitudes_far_apart(ctx, backend):
     """Rows of K, columns of V and the whole of Q at scales from 1e-12 to 1e12 of each other: every output column keeps
-    its own relative precision (a power of two per row and column is taken out before the f16 split)."""
+    its own relative precision (the parts have f32's exponents)."""
     q, k, v = _qkv(8, 1, 2, 1, 140, 200)
     rng = np.random.default_rng(8)
     ks = 10.0 ** rng.uniform(-12, 0, (1, 1, 200, 1))
@@ -133,6 +133,81 @@ def test_magnitudes_far_apart(ctx, backend):
     want = orc.sdpa(q, k, v, 1 / np.sqrt(128), False)
     err = np.sqrt((((got - want) / vs) ** 2).sum(axis=(0, 1, 2)) / ((want / vs) ** 2).sum(axis=(0, 1, 2)))
     assert err.max() < 2 * TOL, err.max()                 # the worst of 128 columns, each with 280 values
+
+
+def _sdpa64(q, k, v, causal, scale=None):
+    """Attention in 64 bits (weights exp(s - max), as they are)."""
+    q, k, v = (x.astype(np.float64) for x in (q, k, v))
+    g = q.shape[1] // k.shape[1]
+    k, v = np.repeat(k, g, axis=1), np.repeat(v, g, axis=1)
+    s = q @ k.transpose(0, 1, 3, 2) * (1 / np.sqrt(q.shape[-1]) if scale is None else scale)
+    if causal:
+        s = np.where(np.tril(np.ones(s.shape[-2:], bool)), s, -np.inf)
+    w = np.exp(s - s.max(axis=-1, keepdims=True))
+    return w @ v / w.sum(axis=-1, keepdims=True)
+
+
+@pytest.mark.parametrize("factor", [1e5, 1e8, 1e12, 1e30])
+@pytest.mark.parametrize("key", [63, 149])
+def test_large_finite_values_behind_the_mask_do_not_reach_earlier_rows(ctx, backend, key, factor):
+    """V of a later key, in the same tile, times up to 1e30: the rows that must not see it keep their precision."""
+    q, k, v = _qkv(12, 1, 2, 1, 150, 150)
+    want = _sdpa64(q, k, v, True)[:, :, :key]
+    v[0, 0, key] *= np.float32(factor)
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, True)
+    assert orc.rel_l2(got[:, :, :key], want) < TOL
+
+
+@pytest.mark.parametrize("lo,hi", [(-6, 6), (-6, 12), (-30, 0)])
+def test_keys_of_very_different_magnitude(ctx, backend, lo, hi):
+    """V growing from key to key: a causal row's result is as precise as the largest value that it SEES allows."""
+    q, k, v = _qkv(13, 1, 2, 1, 150, 150)
+    v = (v * 10.0 ** np.linspace(lo, hi, 150).reshape(1, 1, 150, 1)).astype(np.float32)
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, True)
+    want = _sdpa64(q, k, v, True)
+    err = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
+    # one row of 128 values at a time: the largest of 300 such errors, against TOL over a whole call
+    assert err.max() < 2 * TOL, err.max()
+
+
+@pytest.mark.parametrize("drop", [14, 18, 21, 30])
+def test_small_weights_under_a_dominant_key_without_a_value(ctx, backend, drop):
+    """One key takes the row's weight and its V is zero: the output is made of weights of e^-drop, down to 2^-43, alone."""
+    rng = np.random.default_rng(14)
+    q, k, v = _qkv(14, 1, 2, 1, 140, 140)
+    k *= np.float32(0.1)
+    k[0, 0, 0] = 0.0
+    q[..., 0], k[..., 0] = np.float32(np.sqrt(128)), np.float32(0)
+    k[0, 0, 0, 0] = drop                                   # its score is `drop`, the others' about 0
+    v[0, 0, 0] = 0.0
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, False)
+    # the exponent's argument, up to 30 log2(e) = 43, is rounded to 2^-19 of its weight at worst (an ulp of 43 is 2^-18)
+    assert orc.rel_l2(got, _sdpa64(q, k, v, False)) < 4e-6
+
+
+@pytest.mark.parametrize("qs,ks", [(1e15, 1e-15), (1e30, 1e-30), (1e37, 1e-37), (1e-30, 1e30), (1e-37, 1e37)])
+def test_scores_of_ordinary_size_from_extreme_operands(ctx, backend, qs, ks):
+    """Q and K far from 1 with ordinary products: no scale of the kernel's own overflows or takes bits away."""
+    q, k, v = _qkv(15, 1, 2, 1, 140, 140)
+    q, k = q * np.float32(qs), k * np.float32(ks)
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, True)
+    assert orc.rel_l2(got, _sdpa64(q, k, v, True)) < TOL
+
+
+@pytest.mark.parametrize("value", [np.float32(2) - np.float32(2) ** -23, np.float32(1), np.float32(3e-30)])
+def test_a_constant_v_comes_back(ctx, backend, value):
+    """Weights sum to one: with one value in all of V every output is that value to a few roundings, and not
+    all of them on one side of it."""
+    q, k, v = _qkv(16, 1, 4, 4, 300, 300)
+    v[:] = value
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, True)
+    r = got.astype(np.float64) / np.float64(value) - 1
+    assert np.abs(r).max() < 8 * 2.0 ** -24 and abs(r.mean()) < 2.0 ** -24
 
 
 @pytest.mark.parametrize("H,S,kernels", [(32, 256, ("lux_attn_prefill_mma_f32",)), (8, 128, ("lux_attn_stream_f32", "lux_attn_merge_f32"))])
