@@ -210,6 +210,74 @@ def test_a_constant_v_comes_back(ctx, backend, value):
     assert np.abs(r).max() < 8 * 2.0 ** -24 and abs(r.mean()) < 2.0 ** -24
 
 
+@pytest.mark.parametrize("where,bad", [("q", np.nan), ("k", np.inf), ("v", np.nan), ("v", 1e30)])
+def test_a_block_out_of_range_leaves_the_others_alone(ctx, backend, where, bad):
+    """What the tensor-core parts cannot carry is met in one sequence: its blocks that see it take the f32 kernel's bits, every
+    block that does not see it keeps its own."""
+    q, k, v = _qkv(17, 2, 2, 1, 300, 300)
+    dirty = {"q": q.copy(), "k": k.copy(), "v": v.copy()}
+    dirty[where][1, 0, 200, 5] = bad
+    with _Tuned(backend, attn_prefill=1):
+        clean, clean_lse = _sdpa(ctx, q, k, v, True)
+        got, lse = _sdpa(ctx, **dirty, causal=True)
+    with _Tuned(backend, attn_prefill=3):
+        want, want_lse = _sdpa(ctx, **dirty, causal=True)
+    seen = np.zeros((2, 2, 300), bool)                     # rows of blocks (128 queries) that meet it
+    seen[1, :1 if where == "q" else 2, 128:256 if where == "q" else 300] = True
+    for g, c, w in ((got, clean, want), (lse, clean_lse, want_lse)):
+        assert np.array_equal(g[seen].view(np.uint32), w[seen].view(np.uint32))
+        assert np.array_equal(g[~seen].view(np.uint32), c[~seen].view(np.uint32))
+
+
+def test_output_over_the_queries(ctx, backend):
+    """out == q, with and without a value out of range: a block reads its queries before it writes."""
+    q, k, v = _qkv(18, 1, 2, 1, 260, 260)
+    bad = v.copy()
+    bad[0, 0, 250, 7] = np.inf
+    for vv in (v, bad):
+        with _Tuned(backend, attn_prefill=1):
+            want, _ = _sdpa(ctx, q, k, vv, True)
+            qb = ctx.upload(q)
+            ctx.sdpa(qb, ctx.upload(k), ctx.upload(vv), qb, 1, 2, 1, 260, 260, 128, 1 / np.sqrt(128), flags=B.FLAG_ATTN_CAUSAL)
+        assert np.array_equal(qb.to_host(np.float32, q.shape).view(np.uint32), want.view(np.uint32))
+
+
+def test_replays_of_a_captured_call_do_not_remember(backend):
+    """Captured once, replayed with finite, non-finite and finite inputs: the last replay gives the first one's bits."""
+    import torch
+    c = backend.create_context(0)
+    try:
+        st = torch.cuda.Stream()
+        c.set_stream(st.cuda_stream)
+        q, k, v = (torch.from_numpy(x).cuda() for x in _qkv(19, 1, 2, 1, 150, 150))
+        o = torch.zeros_like(q)
+        bufs = [c.wrap(t.data_ptr(), t.numel() * 4) for t in (q, k, v, o)]
+        call = lambda: c.sdpa(*bufs, 1, 2, 1, 150, 150, 128, 1 / np.sqrt(128), flags=B.FLAG_NO_SYNC | B.FLAG_ATTN_CAUSAL)
+        with _Tuned(backend, attn_prefill=1):
+            torch.cuda.synchronize()
+            with torch.cuda.stream(st):
+                call()
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=st, capture_error_mode="relaxed"):
+                    call()
+            outs = []
+            for val in (None, float("nan"), None):
+                keep = v[0, 0, 100, 3].clone()
+                if val is not None:
+                    v[0, 0, 100, 3] = val
+                torch.cuda.synchronize()
+                g.replay()
+                torch.cuda.synchronize()
+                outs.append(o.cpu().numpy().copy())
+                v[0, 0, 100, 3] = keep
+        torch.cuda.synchronize()
+        del g
+        assert np.isnan(outs[1][0, :, 100:, 3]).all() and np.isfinite(outs[2]).all()
+        assert np.array_equal(outs[0].view(np.uint32), outs[2].view(np.uint32))
+    finally:
+        c.destroy()
+
+
 @pytest.mark.parametrize("H,S,kernels", [(32, 256, ("lux_attn_prefill_mma_f32",)), (8, 128, ("lux_attn_stream_f32", "lux_attn_merge_f32"))])
 def test_default_choice(ctx, backend, H, S, kernels):
     """Prompts with enough (head, 64 queries) blocks to fill the chip take it, small ones the key-splitting kernel."""

@@ -709,14 +709,7 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
         f.batch = p.batch; f.heads = p.heads; f.kv_heads = p.kv_heads; f.group = p.group; f.seq_q = p.seq_q;
         f.kv_len = p.kv_len; f.kv_stride = p.kv_stride; f.causal = p.causal; f.causal_base = p.causal_base;
         f.qscale = p.qscale;
-        LuxBackendError e = LUX_BACKEND_OK;
-        if (g_tune.attn_prefill != 3) {
-            f.call = ctx->attn_calls.fetch_add(1u, std::memory_order_relaxed) + 1u;
-            if (f.call == 0) f.call = ATTN_REDO;                                   // 0 is what an unused word holds
-            f.redo = ctx->d_attn_redo + f.call % ATTN_REDO;
-            e = launch_attn_prefill_mma(ctx, f);
-        }
-        if (e == LUX_BACKEND_OK) e = launch_attn_prefill(ctx, f);
+        const LuxBackendError e = launch_attn_prefill(ctx, f, g_tune.attn_prefill == 3);
         return e != LUX_BACKEND_OK ? e : finish_op(ctx, (flags & LUX_QMATMUL_FLAG_NO_SYNC) != 0, what);
     }
     int vpl = (int)((D + 31) / 32);

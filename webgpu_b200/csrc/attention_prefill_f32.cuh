@@ -1,17 +1,16 @@
-// attention_prefill.cu -- attention of many query rows per head (prompt processing) on the f32 FMA pipe, head size 128.
+// attention_prefill_f32.cuh -- attention of a block of 128 query rows on the f32 FMA pipe, head size 128.
 //
-// The kernel behind lux_attn_prefill_mma_f32: it does the calls in which that one met NaN or infinities, and
-// otherwise returns after reading one word (2 us behind a prompt of 450).  attn_prefill = 3 runs it alone.
+// What lux_attn_prefill_mma_f32 does with a block in which it met values that its bf16 parts cannot carry (2^60 and
+// more, infinities, NaN): the block starts over here, in the same CTA, before anything of it was written, and
+// no other block notices.  lux_attn_prefill_f32 runs it for every block (tunable attn_prefill = 3: the tests).
 //
 // What bounds it.  Both contractions are f32 products of f32 operands, so the FMA pipe is the floor: 128 lanes x 148
 // SMs (72 TFLOP/s at 1.9 GHz).  A 16-byte shared-memory read costs the SM four cycles however many lanes read
 // the same bytes, so the floor in practice is set by FMAs per read: 8 in lux_attn_stream_f32, 16 (scores) and
-// 26 (weighted sum) here.  2048 causal tokens, Llama-3-8B heads: 1684 -> 1090 us with blocks walked in a loop, 884 (39
-// TFLOP/s) with a CTA per block, which the empty launch behind every prompt would pay for.
+// 26 (weighted sum) here.  2048 causal tokens, Llama-3-8B heads, all blocks: 956 us (36 TFLOP/s; streaming kernel 1679).
 // The contractions are register-tiled like a matrix product:
-//   * a CTA of 128 threads owns 64 queries of one head and walks 64-key tiles; two CTAs share an SM, so
-//     that one's barriers, softmax and loads are hidden behind the other's FMAs;
-//   * a thread owns rows tr + 16 i (i < 4) with tr = tid / 8.  Scores: keys tc + 8 j (j < 8, tc = tid % 8),
+//   * a CTA of 256 threads owns 128 queries of one head and walks 64-key tiles;
+//   * a thread owns rows tr + 32 i (i < 4) with tr = tid / 8.  Scores: keys tc + 8 j (j < 8, tc = tid % 8),
 //     four keys at a time: 8 16-byte reads per 64 FMAs.  Weighted sum: columns 32 j + 4 tc .. + 3;
 //   * FMAs go through fma.rn.f32x2 (two IEEE f32 FMAs per instruction, the same rounding as fmaf).  The
 //     pairs are neighbouring head columns, as they lie in memory: a score is kept as its even- and its
@@ -19,7 +18,7 @@
 //   * rows of Q and K are 132 floats apart in shared memory: the four rows and eight keys that a warp
 //     reads in one instruction then lie in different banks.  K arrives by one bulk copy per row, V (read
 //     along its rows) by one per tile;
-//   * a warp owns its 16 rows through the softmax, so the weights pass from the score layout to the
+//   * a warp owns its 16 rows (four values of tr) through the softmax, so the weights pass from the score layout to the
 //     weighted-sum layout through a warp-private piece of shared memory, 32 keys at a time;
 //   * the next K tile is requested when the scores are done, the next V tile when the weighted sum is.
 // Long sums are cut so that no rounding chain is longer than in the streaming kernel's lanes: scores
@@ -27,10 +26,12 @@
 // every tile.
 // A masked (row, key) pair takes no part in the sums at all (a predicated FMA, not a zero weight): an
 // infinite or NaN value at a position that a row must not see does not reach it.
+#pragma once
+
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
-#include <algorithm>
+#include <type_traits>
 
 namespace luxcuda {
 namespace {
@@ -39,15 +40,15 @@ namespace prefill {
 using namespace tcptx;
 
 constexpr int PF_D = 128;                 // head size
-constexpr int PF_BM = 64;                 // queries per CTA
+constexpr int PF_BM = 128;                // queries per CTA
 constexpr int PF_BN = 64;                 // keys per tile
-constexpr int PF_THREADS = 128;
+constexpr int PF_THREADS = 256;
 constexpr int PF_PITCH = PF_D + 4;        // floats between rows of Q and K in shared memory
 constexpr int PF_PW = 32;                 // keys whose weights are passed on at a time
 constexpr int PF_PPITCH = PF_PW + 8;      // floats between rows of the weights
 constexpr int PF_Q_FLOATS = PF_BM * PF_PITCH, PF_K_FLOATS = PF_BN * PF_PITCH, PF_V_FLOATS = PF_BN * PF_D,
               PF_P_FLOATS = PF_BM * PF_PPITCH;
-// Q, K, V, weights, then two mbarriers and the abort flag: 110.6 KB, two CTAs per SM
+// Q, K, V, weights, then two mbarriers and the abort flag: 151 KB
 constexpr int PF_SMEM = (PF_Q_FLOATS + PF_K_FLOATS + PF_V_FLOATS + PF_P_FLOATS) * 4 + 32;
 
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
@@ -98,8 +99,9 @@ __device__ __forceinline__ float ex2(float x) {                // as in the stre
 constexpr float PF_NEG = -3.0e38f;        // "no key seen yet" in the base-2 score domain
 constexpr float PF_LN2 = 0.6931471805599453f;
 
-__global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const PrefillArgs p) {
-    extern __shared__ __align__(128) unsigned char smem[];
+// Block qb of head h of sequence b.  All threads of the CTA call it, with 128-byte aligned shared memory that no copy
+// in flight still writes.
+__device__ __forceinline__ void attend_f32(const PrefillArgs& p, unsigned char* smem, uint32_t qb, uint32_t h, uint32_t b) {
     float* qs = reinterpret_cast<float*>(smem);
     float* ks = qs + PF_Q_FLOATS;
     float* vs = ks + PF_K_FLOATS;
@@ -107,27 +109,19 @@ __global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const Pref
     uint64_t* bars = reinterpret_cast<uint64_t*>(ps + PF_P_FLOATS);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(bars + 2);
     const uint32_t bar_k = smem_u32(bars), bar_v = bar_k + 8u;
-    pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tr = tid >> 3, tc = tid & 7;
 
-    // The tensor-core kernel in front of this one leaves the call's number where it met something it cannot do.
-    pdl_wait();
-    if (p.redo && __ldcg(p.redo) != p.call) return;
+    fence_proxy_async_smem();             // copies are about to land where this thread may have written
+    __syncthreads();
     if (tid == 0) {
         mbar_init(bar_k, 1u);
         mbar_init(bar_v, 1u);
         *abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const uint32_t bh = p.batch * p.heads;
-    uint32_t done = 0;                    // tiles of earlier blocks: the barriers' phase
-    for (uint32_t block = blockIdx.x; block < p.q_blocks * bh; block += gridDim.x) {
     __syncthreads();
-    // blocks of late queries see the most keys under a causal mask: they come first.  Neighbouring blocks
-    // are heads of one KV head and share its tiles in L2.
-    const uint32_t qb = p.q_blocks - 1u - block / bh, rest = block % bh;
-    const uint32_t h = rest % p.heads, b = rest / p.heads, g = h / p.group;
+    const uint32_t g = h / p.group;
     const uint32_t q0 = qb * PF_BM;
     const uint32_t rows = min((uint32_t)PF_BM, p.seq_q - q0);
     auto row_len = [&](uint32_t qi) { return p.causal ? min(p.causal_base + qi + 1u, p.kv_len) : p.kv_len; };
@@ -166,13 +160,13 @@ __global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const Pref
     }
     __syncthreads();
 
-    uint64_t o[4][8];                     // row tr + 16 i, columns 32 (j / 2) + 4 tc + 2 (j % 2) and the next
+    uint64_t o[4][8];                     // row tr + 32 i, columns 32 (j / 2) + 4 tc + 2 (j % 2) and the next
     float m[4], l[4];
     uint32_t len[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint32_t qi = q0 + tr + 16 * i;
-        len[i] = tr + 16 * i < (int)rows ? row_len(qi) : 0u;        // a padding row sees nothing and is not written
+        const uint32_t qi = q0 + tr + 32 * i;
+        len[i] = tr + 32 * i < (int)rows ? row_len(qi) : 0u;        // a padding row sees nothing and is not written
         m[i] = PF_NEG;
         l[i] = 0.0f;
 #pragma unroll
@@ -195,7 +189,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const Pref
             float w[4][4];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const float4 t = lds4(paddr + (uint32_t)(16 * i * PF_PPITCH * 4) + kk * 4u);
+                const float4 t = lds4(paddr + (uint32_t)(32 * i * PF_PPITCH * 4) + kk * 4u);
                 w[i][0] = t.x; w[i][1] = t.y; w[i][2] = t.z; w[i][3] = t.w;
             }
 #pragma unroll
@@ -232,7 +226,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const Pref
         const uint32_t t0 = t * PF_BN;
         const bool edge = t0 + PF_BN > min_len;          // some row of the CTA does not see the whole tile
         float s[4][8];
-        ok = warp_wait(bar_k, (done + t) & 1u, abort_flag, lane);
+        ok = warp_wait(bar_k, t & 1u, abort_flag, lane);
         if (ok) {
 #pragma unroll
             for (int hf = 0; hf < 2; hf++) {
@@ -252,7 +246,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const Pref
                     for (int d = 0; d < 32; d += 4) {
                         Pair2 qv[4], kv[4];
 #pragma unroll
-                        for (int i = 0; i < 4; i++) qv[i] = lds_pairs(qaddr + (uint32_t)(16 * i * PF_PITCH * 4 + (d0 + d) * 4));
+                        for (int i = 0; i < 4; i++) qv[i] = lds_pairs(qaddr + (uint32_t)(32 * i * PF_PITCH * 4 + (d0 + d) * 4));
 #pragma unroll
                         for (int j = 0; j < 4; j++) kv[j] = lds_pairs(kaddr + (uint32_t)(8 * (4 * hf + j) * PF_PITCH * 4 + (d0 + d) * 4));
 #pragma unroll
@@ -317,14 +311,14 @@ __global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const Pref
             l[i] += ((s[i][0] + s[i][1]) + (s[i][2] + s[i][3])) + ((s[i][4] + s[i][5]) + (s[i][6] + s[i][7]));
         }
 
-        ok = warp_wait(bar_v, (done + t) & 1u, abort_flag, lane);
+        ok = warp_wait(bar_v, t & 1u, abort_flag, lane);
         if (ok) {
 #pragma unroll
             for (int hf = 0; hf < 2; hf++) {
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
-                    for (int j = 0; j < 4; j++) ps[(tr + 16 * i) * PF_PPITCH + tc + 8 * j] = s[i][4 * hf + j];
+                    for (int j = 0; j < 4; j++) ps[(tr + 32 * i) * PF_PPITCH + tc + 8 * j] = s[i][4 * hf + j];
                 __syncwarp();
                 if (edge) weighted(std::true_type{}, hf * PF_PW, t0);
                 else weighted(std::false_type{}, hf * PF_PW, t0);
@@ -346,7 +340,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const Pref
         l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
         l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
         l[i] += __shfl_xor_sync(0xffffffffu, l[i], 4);
-        const int r = tr + 16 * i;
+        const int r = tr + 32 * i;
         if (r >= (int)rows) continue;
         const size_t orow = ((size_t)b * p.heads + h) * p.seq_q + q0 + r;
         const bool any = l[i] > 0.0f;
@@ -360,31 +354,8 @@ __global__ void __launch_bounds__(PF_THREADS, 2) lux_attn_prefill_f32(const Pref
         }
         if (tc == 0 && p.lse) p.lse[orow] = l[i] > 0.0f ? fmaf(m[i], PF_LN2, logf(l[i])) : -3.402823e+38f;
     }
-    done += tiles;
-    }
 }
 
 }  // namespace prefill
 }  // namespace
-
-LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p) {
-    using namespace prefill;
-    static std::atomic<bool> configured[64];
-    const int dev = ctx->device & 63;
-    if (!configured[dev].load(std::memory_order_relaxed)) {
-        cudaError_t e = cudaFuncSetAttribute(lux_attn_prefill_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM);
-        if (e != cudaSuccess) return map_cuda(e, "lux_attn_prefill_f32");
-        configured[dev].store(true, std::memory_order_relaxed);
-    }
-    p.q_blocks = (p.seq_q + PF_BM - 1) / PF_BM;
-    const unsigned blocks = std::min<unsigned>(p.q_blocks * p.heads * p.batch, 2u * (unsigned)ctx->sm_count);
-    cudaError_t e = launch_pdl(g_tune.pdl != 2, lux_attn_prefill_f32, dim3(blocks), dim3(PF_THREADS), (size_t)PF_SMEM, ctx->stream, 1, p);
-    if (e != cudaSuccess) return map_cuda(e, "lux_attn_prefill_f32");
-    if (!p.redo) count_launch("lux_attn_prefill_f32");
-    else count_launch();
-    return LUX_BACKEND_OK;
-}
-
-const void* kernel_addr_attn_prefill_f32() { return (const void*)prefill::lux_attn_prefill_f32; }
-
 }  // namespace luxcuda

@@ -10,20 +10,19 @@
 // Range.  bf16 has f32's exponents, so a part depends on its own element alone: no scale is shared along a row, a
 // column or a tile, a masked key weighs exactly nothing however large its values, and a weight of 2^-100 keeps
 // its 24 bits.  A part below 2^-126 is lost, so an element's error is 2^-24 of it or 2^-126.  A block that
-// meets a magnitude of 2^60 or more (after Q's scale), an infinity or a NaN is left to the f32 kernel: with
+// meets a magnitude of 2^60 or more (after Q's scale), an infinity or a NaN is done on the f32 pipe: with
 // all below 2^60 no score and no sum overflows (2^120 x 128) and no bf16 rounding does, and 2^-126 x 2^60 x 128 is
 // nothing in a score.
 //
 // Accumulation.  The tensor core sums a step of 16 exactly and cuts the f32 result off (measured: mean loss 3.8e-8 of
-// it, otherwise no more than rounding's error).  Every step's h h products, of 16 bits each, therefore start from zero and are added to the running f32
-// sum by an ordinary rounded addition; the other products, 2^-8 of these and less, run in a chain of their own, where
-// the cut is 2^-8 as large, and are added once per tile.  Relative error against 64 bits (2-norm, N(0, 1) inputs,
-// Llama-3-8B heads; streaming kernel / this one): causal, 150 tokens 1.34e-7 / 1.04e-7, 512 1.65 / 1.22, 2048 2.25 /
-// 1.42; unmasked, 700 x 3 3.06 / 1.76, 1448 4.06 / 2.03.
+// it, otherwise no more than rounding's error).  Every step's h h products, of 16 bits each, therefore start from zero
+// and are added to the running f32 sum by an ordinary rounded addition; the other products, 2^-8 of these and less,
+// run in a chain of their own, where the cut is 2^-8 as large, and are added once per tile.  Relative error against
+// 64 bits (2-norm, N(0, 1) inputs, Llama-3-8B heads; streaming kernel / this one): causal, 150 tokens 1.34e-7 /
+// 1.04e-7, 512 1.65 / 1.22, 2048 2.25 / 1.42; unmasked, 700 x 3 3.06 / 1.76, 1448 4.06 / 2.03.
 //
-// Out-of-range inputs.  A CTA that meets one writes nothing and leaves this call's number in a word of the context;
-// lux_attn_prefill_f32, launched behind this kernel, returns at once unless it finds that number there, and
-// otherwise does the whole call.
+// Out-of-range inputs.  A CTA that meets one starts its block over on the f32 pipe (attention_prefill_f32.cuh); it has written
+// nothing by then, so this holds with out == q, and no other block, call or replay of a captured one takes part.
 //
 // Work.  A CTA of eight warps owns 128 queries of one head and walks 32-key tiles (three parts of 64 would not fit
 // shared memory twice): bulk copies bring a tile as f32, two tiles ahead; all warps split it into three bf16
@@ -31,13 +30,10 @@
 // before it works on the current one and the other after it, so that the splitting runs beside the tensor core.  A warp
 // owns 16 rows from the scores to the output; Q's fragments and the output stay in its registers, the weights go from
 // accumulator to operand layout without leaving them.  Causal, Llama-3-8B heads, against the streaming kernel:
-// 2048 tokens 1679 -> 683 us (50 TFLOP/s of f32 products, 302 of the tensor core's 568 at this instruction), 512
-// tokens 152 -> 95, 150 tokens 29.5 -> 29.7; unmasked 1448 tokens 1567 -> 785.  What is left is the tensor pipe (more
+// 2048 tokens 1679 -> 677 us (51 TFLOP/s of f32 products, 305 of the tensor core's 568 at this instruction), 512
+// tokens 152 -> 94, 150 tokens 29.5 -> 28.4; unmasked 1448 tokens 1567 -> 785.  What is left is the tensor pipe (more
 // than half the time) and the softmax, splitting and fragment loads beside it.
-#include "common.cuh"
-#include "tc_ptx.cuh"
-
-#include <algorithm>
+#include "attention_prefill_f32.cuh"
 
 namespace luxcuda {
 
@@ -346,16 +342,16 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
         ok = !__syncthreads_or(*bad_flag != 0u);
     }
     if (!ok) {
-        // inputs out of range: the kernel behind this one does the call; or a bounded wait gave up: report it.  Nothing is
-        // written, and the CTA stays until its copies have landed (or have had time to).
-        for (uint32_t t = asked > 2u ? asked - 2u : 0u; t < asked && !*abort_flag; t++) landed(t);
+        // values out of range: the block starts over on the f32 pipe; or a bounded wait gave up: report it, and give
+        // copies in flight time to land.  Nothing has been written.
+        for (uint32_t t = asked > 2u ? asked - 2u : 0u; t < asked; t++) landed(t);
         __syncthreads();
         if (*abort_flag) {
             if (tid == 0 && p.status) atomicOr(p.status, p.status_wait);
             for (int i = 0; i < 64; i++) __nanosleep(1000);
             __syncthreads();
-        } else if (tid == 0) {
-            atomicExch(p.redo, p.call);
+        } else {
+            prefill::attend_f32(p, smem, qb, h, b);
         }
         return;
     }
@@ -375,25 +371,40 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
     }
 }
 
+// Every block on the f32 pipe.
+__global__ void __launch_bounds__(prefill::PF_THREADS, 1) lux_attn_prefill_f32(const PrefillArgs p) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t bh = p.batch * p.heads, rest = blockIdx.x % bh;
+    prefill::attend_f32(p, smem, p.q_blocks - 1u - blockIdx.x / bh, rest % p.heads, rest / p.heads);
+}
+
+static_assert(THREADS == prefill::PF_THREADS && BM == prefill::PF_BM && SMEM >= prefill::PF_SMEM + 128, "a block can change over");
+
 }  // namespace pmma
 }  // namespace
 
-LuxBackendError launch_attn_prefill_mma(Context* ctx, PrefillArgs p) {
+LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) {
     using namespace pmma;
-    static std::atomic<bool> configured[64];
-    const int dev = ctx->device & 63;
-    if (!configured[dev].load(std::memory_order_relaxed)) {
-        cudaError_t e = cudaFuncSetAttribute(lux_attn_prefill_mma_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) return map_cuda(e, "lux_attn_prefill_mma_f32");
-        configured[dev].store(true, std::memory_order_relaxed);
+    auto kfn = f32_only ? lux_attn_prefill_f32 : lux_attn_prefill_mma_f32;
+    const char* name = f32_only ? "lux_attn_prefill_f32" : "lux_attn_prefill_mma_f32";
+    static std::atomic<bool> configured[2][64];
+    std::atomic<bool>& done = configured[f32_only][ctx->device & 63];
+    if (!done.load(std::memory_order_relaxed)) {
+        cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e != cudaSuccess) return map_cuda(e, name);
+        done.store(true, std::memory_order_relaxed);
     }
     p.q_blocks = (p.seq_q + pmma::BM - 1) / pmma::BM;
-    cudaError_t e = launch_pdl(g_tune.pdl != 2, lux_attn_prefill_mma_f32, dim3(p.q_blocks * p.heads * p.batch), dim3(THREADS), (size_t)SMEM, ctx->stream, 1, p);
-    if (e != cudaSuccess) return map_cuda(e, "lux_attn_prefill_mma_f32");
-    count_launch("lux_attn_prefill_mma_f32");
+    cudaError_t e = launch_pdl(g_tune.pdl != 2, kfn, dim3(p.q_blocks * p.heads * p.batch), dim3(THREADS), (size_t)SMEM, ctx->stream, 1, p);
+    if (e != cudaSuccess) return map_cuda(e, name);
+    count_launch(name);
     return LUX_BACKEND_OK;
 }
 
 const void* kernel_addr_attn_prefill_mma_f32() { return (const void*)pmma::lux_attn_prefill_mma_f32; }
+const void* kernel_addr_attn_prefill_f32() { return (const void*)pmma::lux_attn_prefill_f32; }
 
 }  // namespace luxcuda

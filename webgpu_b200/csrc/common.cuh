@@ -50,9 +50,6 @@ struct Context {
     void*          d_int = nullptr;         // lux_cuda_matmul_int8 on the tcgen05 path: B transposed (and A unpacked), grown on demand
     size_t         d_int_bytes = 0;
     void*          d_attn = nullptr;        // partial results of attention calls that split the keys over CTAs:
-    uint32_t*      d_attn_redo = nullptr;   // prompt attention: ATTN_REDO words, call n writes n into word n % ATTN_REDO when it meets
-                                            // non-finite inputs (a word per call, so that calls on different streams do not meet)
-    std::atomic<uint32_t> attn_calls{0};    // prompt-attention calls so far
     size_t         d_attn_bytes = 0;        // 16 MB, allocated with the context (a call takes fewer slices rather than allocate)
     std::mutex     mu;                      // guards the staging buffers
     int            sm_count = 148;
@@ -64,7 +61,6 @@ struct Context {
 };
 
 constexpr int ABSMAX_PARTS = 1024;
-constexpr uint32_t ATTN_REDO = 256;
 
 inline Context* as_ctx(LuxBackendContext* c) { return reinterpret_cast<Context*>(c); }
 inline Buffer*  as_buf(LuxBackendBuffer* b) { return reinterpret_cast<Buffer*>(b); }
@@ -306,7 +302,7 @@ LuxBackendError launch_qgemm_i4_tc(Context* ctx, const QArgs& a);
 LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a);    // NOT_SUPPORTED if the shape does not fit
 LuxBackendError launch_qdequant(Context* ctx, const QArgs& a, int bits);
 
-// attention_prefill.cu: contiguous K and V, head size 128, all pointers 16-byte aligned
+// attention_prefill_mma.cu: contiguous K and V, head size 128, all pointers 16-byte aligned
 struct PrefillArgs {
     const float *q, *k, *v;
     float* out;
@@ -316,13 +312,10 @@ struct PrefillArgs {
     uint32_t batch, heads, kv_heads, group, seq_q;
     uint32_t kv_len, kv_stride;  // keys a row may see; rows between the bases of two KV heads
     uint32_t causal, causal_base;// causal: query i sees min(causal_base + i + 1, kv_len) keys
-    uint32_t q_blocks;           // blocks of queries (set by the launchers)
+    uint32_t q_blocks;           // blocks of queries (set by the launcher)
     float qscale;                // scale * log2(e)
-    uint32_t* redo;              // the tensor-core kernel writes `call` here where it met non-finite inputs, and the
-    uint32_t call;               // f32 kernel then does the call (null: unconditionally)
 };
-LuxBackendError launch_attn_prefill_mma(Context* ctx, PrefillArgs p);
-LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p);
+LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only);
 
 // tensor_ops.cu: the f32 slots the reference's shader library backs but its plugin leaves unwired
 LuxBackendError op_div_f32(LuxBackendContext*, LuxBackendBuffer* a, LuxBackendBuffer* b, LuxBackendBuffer* out, size_t n);

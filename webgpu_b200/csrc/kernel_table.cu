@@ -78,7 +78,7 @@ const Entry kTable[] = {
     {"lux_qgemv_i4_g128_units_fx_batch4", luxcuda::kernel_addr_qgemv_i4_units_fx_batch4, 512, 1, 1},
     {"lux_matmul_int8_tcgen05",    luxcuda::kernel_addr_matmul_int8_tcgen05, 192, 1, 1},
     {"lux_attn_stream_f32",        luxcuda::kernel_addr_attn_stream_f32,    288, 1, 1},
-    {"lux_attn_prefill_f32",       luxcuda::kernel_addr_attn_prefill_f32,   128, 1, 1},
+    {"lux_attn_prefill_f32",       luxcuda::kernel_addr_attn_prefill_f32,   256, 1, 1},
     {"lux_attn_prefill_mma_f32",   luxcuda::kernel_addr_attn_prefill_mma_f32, 256, 1, 1},
     {"lux_attn_merge_f32",         luxcuda::kernel_addr_attn_merge_f32,     128, 1, 1},
     {"lux_attn_plain_f32",         luxcuda::kernel_addr_attn_plain_f32,     256, 1, 1},

@@ -121,14 +121,11 @@ static LuxBackendContext* cuda_create_context(int device_index) {
     }
     if (ok) {
         ctx->d_attn_bytes = 16u << 20;
-        ok = cudaMalloc(&ctx->d_attn, ctx->d_attn_bytes) == cudaSuccess && cudaMalloc(&ctx->d_attn_redo, ATTN_REDO * sizeof(uint32_t)) == cudaSuccess &&
-             cudaMemsetAsync(ctx->d_attn_redo, 0, ATTN_REDO * sizeof(uint32_t), ctx->own_stream) == cudaSuccess &&
-             cudaStreamSynchronize(ctx->own_stream) == cudaSuccess;
+        ok = cudaMalloc(&ctx->d_attn, ctx->d_attn_bytes) == cudaSuccess;
     }
     if (!ok) {
         cudaGetLastError();
         if (ctx->d_attn) cudaFree(ctx->d_attn);
-        if (ctx->d_attn_redo) cudaFree(ctx->d_attn_redo);
         if (ctx->d_splitk) cudaFree(ctx->d_splitk);
         if (ctx->d_absmax) cudaFree(ctx->d_absmax);
         if (ctx->h_status) cudaFreeHost(ctx->h_status);
@@ -152,7 +149,6 @@ static void cuda_destroy_context(LuxBackendContext* context) {
     if (ctx->d_stage) cudaFree(ctx->d_stage);
     if (ctx->d_int) cudaFree(ctx->d_int);
     if (ctx->d_attn) cudaFree(ctx->d_attn);
-    if (ctx->d_attn_redo) cudaFree(ctx->d_attn_redo);
     if (ctx->d_splitk) cudaFree(ctx->d_splitk);
     if (ctx->d_absmax) cudaFree(ctx->d_absmax);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
