@@ -285,3 +285,18 @@ def test_default_choice(ctx, backend, H, S, kernels):
     got, _ = _sdpa(ctx, q, k, v, True)
     assert backend.last_kernel_name() in kernels
     assert orc.rel_l2(got[:, :2], orc.sdpa(q[:, :2], k[:, :2], v[:, :2], 1 / np.sqrt(128), True)) < TOL
+
+
+@pytest.mark.parametrize("Sq,keys,takes", [(65, 4096, False), (128, 4096, False), (512, 4096, True), (65, 300, False), (256, 300, True)])
+def test_default_choice_over_a_cache(ctx, backend, Sq, keys, takes):
+    """A chunk of a prompt over a longer cache: its blocks of 128 queries walk all keys alone, so few of them go to the
+    kernel that also splits the keys; either way the answer is that kernel's to rounding."""
+    q, k, v = _qkv(20, 1, 32, 8, Sq, keys)
+    qb, kb, vb, ob = ctx.upload(q), ctx.upload(k), ctx.upload(v), ctx.alloc(q.nbytes)
+    outs = []
+    for mode in (0, 2):
+        with _Tuned(backend, attn_prefill=mode):
+            ctx.sdpa_kv_cache(qb, kb, vb, ob, 1, 32, 8, Sq, keys - Sq, keys, 128, 1 / np.sqrt(128), flags=B.FLAG_ATTN_CAUSAL)
+            assert mode or (backend.last_kernel_name() == "lux_attn_prefill_mma_f32") == takes
+        outs.append(ob.to_host(np.float32, q.shape).copy())
+    assert orc.rel_l2(outs[0], outs[1]) < TOL

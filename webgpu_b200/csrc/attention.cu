@@ -666,22 +666,40 @@ AttnKernel pick_stream(int vpl, int rt, bool full) {
     return nullptr;
 }
 
-// What lux_attn_prefill_f32 takes (q, k and v have been found aligned).
+// What lux_attn_prefill_mma_f32 takes (q, k and v have been found aligned).
 bool prefill_fits(const AttnParams& p) {
-    return !p.block_size && p.head_dim == 128 && aligned16(p.out) && (uint64_t)p.batch * p.heads * ((p.seq_q + 63u) / 64u) <= 0x7fffffffu;
+    return !p.block_size && p.head_dim == 128 && aligned16(p.out) && (uint64_t)p.batch * p.heads * ((p.seq_q + 127ull) / 128u) <= 0x7fffffffu;
 }
-// Where it is the faster kernel: when its CTAs (one per 64 queries of a head, each walking its keys alone)
-// are enough to occupy the chip; the streaming kernel also splits the keys.
-bool prefill_pays(const AttnParams& p) {
-    if (p.seq_q < 64 || p.kv_len == 0) return false;
-    uint64_t total = 0, longest = 1;                               // 64-key tiles
-    for (uint32_t q0 = 0; q0 < p.seq_q; q0 += 64) {
-        const uint64_t last = std::min<uint64_t>(q0 + 63u, p.seq_q - 1u);
-        const uint64_t keys = p.causal ? std::min<uint64_t>(p.causal_base + last + 1u, p.kv_len) : p.kv_len;
-        total += (keys + 63) / 64;
-        longest = std::max(longest, (keys + 63) / 64);
+// Which of the two kernels is the faster one, by what each takes in us on 148 SMs.  Over 178 shapes (64 .. 2049
+// queries, 64 .. 16384 keys, 4 .. 64 heads, batch 1 .. 8) the choice is nowhere slower than the streaming kernel by more
+// than 3 %, and at most 14 % slower than the faster of the two.
+// The prompt kernel: a CTA per SM owns 128 queries of a head and walks all their keys, 5.5 us a tile of 32, 4.6 where half
+// of its warps have no rows.  32 heads over 4096 keys, prompt / streaming: 65 rows 708 / 225 us, 128 712 /
+// 433, 200 709 / 647, 256 712 / 848, 512 713 / 1627.
+double prefill_us(const AttnParams& p, int sms) {
+    double total = 0.0, longest = 0.0;
+    uint64_t blocks = 0;
+    for (uint64_t q0 = 0; q0 < p.seq_q; q0 += 128, blocks++) {
+        const uint64_t rows = std::min<uint64_t>(128u, p.seq_q - q0);
+        const uint64_t keys = p.causal ? std::min<uint64_t>(p.causal_base + q0 + rows, p.kv_len) : p.kv_len;
+        const double us = (double)((keys + 31) / 32) * (rows > 64 ? 5.5 : 4.6);
+        total += us;
+        longest = std::max(longest, us);
     }
-    return total * p.batch * p.heads >= 64 * longest;
+    const double bh = (double)p.batch * p.heads;
+    return 6.0 + (blocks * bh <= sms ? longest : std::max(longest, total * bh / sms + longest / 4));
+}
+// The streaming kernel: two CTAs per SM, each 16 rows of a KV head against a slice of the keys, 0.115 us a key (0.6 of
+// it where a CTA has its SM to itself) and a start-up of 32.
+double stream_us(const AttnParams& p, uint32_t slices, uint32_t slice_keys, int sms) {
+    // causal rows see one key more each until they see all
+    const double climb = p.causal ? std::min<double>(p.seq_q, std::max(0.0, (double)p.kv_len - p.causal_base)) : 0.0;
+    const double keys = (climb * (p.causal_base + (climb + 1) / 2) + (p.seq_q - climb) * p.kv_len) / p.seq_q;
+    const double items = (double)p.batch * p.kv_heads * p.row_blocks, ctas = items * slices;
+    const double longest = std::min<double>(slice_keys, p.kv_len) + 32.0, slots = 2.0 * sms;
+    const double span = ctas <= slots ? longest * (0.6 + 0.4 * std::max(0.0, ctas - sms) / sms)
+                                      : std::max(longest, items * (keys + slices * 32.0) / slots + longest / 2);
+    return (slices > 1 ? 12.0 : 9.0) + 0.115 * span;      // launches (and the merge of slices)
 }
 
 // Fills the launch geometry of p and launches.  max_keys: the longest context any row can have.
@@ -701,16 +719,6 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
         lux_attn_plain_f32<<<(unsigned)out_rows, 256, smem, ctx->stream>>>(p);
         count_launch("lux_attn_plain_f32");
         return finish_op(ctx, (flags & LUX_QMATMUL_FLAG_NO_SYNC) != 0, what);
-    }
-    if (prefill_fits(p) && g_tune.attn_prefill != 2 && (g_tune.attn_prefill || prefill_pays(p))) {
-        PrefillArgs f{};
-        f.q = p.q; f.k = p.k; f.v = p.v; f.out = p.out; f.lse = p.lse;
-        f.status = p.status; f.status_wait = ATT_STATUS_WAIT;
-        f.batch = p.batch; f.heads = p.heads; f.kv_heads = p.kv_heads; f.group = p.group; f.seq_q = p.seq_q;
-        f.kv_len = p.kv_len; f.kv_stride = p.kv_stride; f.causal = p.causal; f.causal_base = p.causal_base;
-        f.qscale = p.qscale;
-        const LuxBackendError e = launch_attn_prefill(ctx, f, g_tune.attn_prefill == 3);
-        return e != LUX_BACKEND_OK ? e : finish_op(ctx, (flags & LUX_QMATMUL_FLAG_NO_SYNC) != 0, what);
     }
     int vpl = (int)((D + 31) / 32);
     if (vpl > 4) vpl = 8;
@@ -753,6 +761,18 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
             best = n;
         }
         if (ctas > 8.0 * sm) break;
+    }
+    geometry(best);
+    if (prefill_fits(p) && g_tune.attn_prefill != 2 && (g_tune.attn_prefill || (p.seq_q >= 64 && p.kv_len &&
+        prefill_us(p, ctx->sm_count) < 0.97 * stream_us(p, p.nsplit, p.split_keys, ctx->sm_count)))) {
+        PrefillArgs f{};
+        f.q = p.q; f.k = p.k; f.v = p.v; f.out = p.out; f.lse = p.lse;
+        f.status = p.status; f.status_wait = ATT_STATUS_WAIT;
+        f.batch = p.batch; f.heads = p.heads; f.kv_heads = p.kv_heads; f.group = p.group; f.seq_q = p.seq_q;
+        f.kv_len = p.kv_len; f.kv_stride = p.kv_stride; f.causal = p.causal; f.causal_base = p.causal_base;
+        f.qscale = p.qscale;
+        const LuxBackendError e = launch_attn_prefill(ctx, f, g_tune.attn_prefill == 3);
+        return e != LUX_BACKEND_OK ? e : finish_op(ctx, (flags & LUX_QMATMUL_FLAG_NO_SYNC) != 0, what);
     }
     geometry(g_tune.attn_splits > 0 ? std::max<uint32_t>((uint32_t)g_tune.attn_splits, min_split) : best);
     if (p.nsplit > 256) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;     // a context beyond 256 x 2046 pages
