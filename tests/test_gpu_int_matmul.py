@@ -105,6 +105,22 @@ def test_dynamic_quantize_bit_exact(ctx, n, bits):
     assert sb.to_host(np.float32, (1,))[0] == 1.0
 
 
+def test_matmul_int8_more_rows_than_a_grid_of_128_row_tiles(ctx, backend):
+    """65536 * 128 + 1 rows: tiles of 128 rows would be one more than a grid may have along y, tiles of 256 are not."""
+    import torch
+    M, N, K = 65536 * 128 + 1, 16, 256
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.randint(-128, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    b = RNG.integers(-128, 128, size=(K, N), dtype=np.int8)
+    c = torch.full((M, N), -1, device="cuda", dtype=torch.int32)
+    torch.cuda.synchronize()
+    ctx.matmul_int8(ctx.wrap(a.data_ptr(), M * K), ctx.upload(b), ctx.wrap(c.data_ptr(), M * N * 4), M, N, K)
+    assert backend.last_kernel_name() == "lux_matmul_int8_tcgen05"
+    bt = torch.from_numpy(b).cuda().double()
+    for r0 in range(0, M, 1 << 20):                          # exact in f64
+        assert torch.equal(c[r0:r0 + (1 << 20)], (a[r0:r0 + (1 << 20)].double() @ bt).to(torch.int32))
+
+
 def test_w8a8_linear_layer_end_to_end(ctx):
     """dynamic_quantize -> matmul_int8 -> scale back: the W8A8 linear layer the shaders compose,
     against the f32 product (quantization error only)."""

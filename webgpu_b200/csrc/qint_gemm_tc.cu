@@ -16,15 +16,16 @@
 //     through shared memory), which is then read K-major (measured, 4096^3: 83.5 us through B^T,
 //     73.0 us without; 256 x 28672 x 4096: 103.8 -> 48.5 us).  For int4 x int8 another kernel
 //     sign-extends A's two's complement nibbles (quantized.wgsl:150-158) to bytes;
-//   * a CTA owns a 256 x 256 tile of C (128 x 256 when M <= 128): two int32 accumulators of 256
-//     columns each in tensor memory, fed by the same B tile;
-//   * warp 0 (one thread): TMA producer, one 256 x 128-byte box of A and 32 KB of B per stage
-//     (128 k; 128-byte swizzle), three stages (four with one accumulator);
-//   * warp 1 (one thread): per stage one wait, four tcgen05.mma.kind::i8 (128 x 256 x 32) per
-//     accumulator and one tcgen05.commit that frees the stage;
+//   * a CTA owns a tile of C of 256 x 256 (two int32 accumulators of 256 columns each in tensor memory, fed
+//     by the same B tile), 128 x 256 or 128 x 128; where tiles leave SMs idle, two or four CTAs of a cluster take
+//     slices of K of the same tile;
+//   * warp 0 (one thread): TMA producer, one box of A and 16 or 32 KB of B per stage (128 k; 128-byte
+//     swizzle), three, four or six stages;
+//   * warp 1 (one thread): per stage one wait, four tcgen05.mma.kind::i8 (K = 32) per accumulator and
+//     one tcgen05.commit that frees the stage;
 //   * warps 2-5: epilogue, tcgen05.ld 32 columns at a time, 128-byte stores per thread.
 // K tails and ragged M / N are covered by the TMA's zero fill and by masked stores.  Every mbarrier
-// wait is bounded (the abort flag, status 0x7C05000B).  No cluster, no multicast.
+// wait is bounded (the abort flag, status 0x7C05000B).  No multicast.
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -341,6 +342,7 @@ LuxBackendError launch_matmul_int8_tcgen05(Context* ctx, const void* a, const vo
     const Form* best = &forms[0];
     long long best_cost = 0;
     for (const Form& f : forms) {
+        if ((M + (long long)f.ma * I8_BM - 1) / (f.ma * I8_BM) > 65535) continue;           // row tiles are the grid's y
         const long long cost = (ctas_of(f) + sms - 1) / sms * f.cost;
         if (best_cost == 0 || cost < best_cost) { best = &f; best_cost = cost; }
     }
