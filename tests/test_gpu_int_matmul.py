@@ -121,6 +121,21 @@ def test_matmul_int8_more_rows_than_a_grid_of_128_row_tiles(ctx, backend):
         assert torch.equal(c[r0:r0 + (1 << 20)], (a[r0:r0 + (1 << 20)].double() @ bt).to(torch.int32))
 
 
+def test_a_refused_launch_is_reported_once(ctx):
+    """More row tiles than any grid holds: that call fails, and the next one does not hear of it."""
+    import torch
+    M, N, K = 65535 * 256 + 1, 16, 256                       # the launch is refused: nothing reads the operands
+    a = torch.empty((M, K), device="cuda", dtype=torch.int8)
+    c = torch.empty((M, N), device="cuda", dtype=torch.int32)
+    b = ctx.upload(np.zeros((K, N), np.int8))
+    with pytest.raises(B.BackendError):
+        ctx.matmul_int8(ctx.wrap(a.data_ptr(), M * K), b, ctx.wrap(c.data_ptr(), M * N * 4), M, N, K)
+    x = RNG.standard_normal(64).astype(np.float32)
+    ob, sb = ctx.alloc(64), ctx.alloc(4)
+    ctx.dynamic_quantize(ctx.upload(x), ob, sb, 64, 8)
+    assert np.array_equal(ob.to_host(np.uint8, (64,)), orc.dynamic_quantize(x, 8)[0])
+
+
 def test_w8a8_linear_layer_end_to_end(ctx):
     """dynamic_quantize -> matmul_int8 -> scale back: the W8A8 linear layer the shaders compose,
     against the f32 product (quantization error only)."""

@@ -79,6 +79,7 @@ inline void count_launch(const char* kernel) {
 inline LuxBackendError map_cuda(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return LUX_BACKEND_OK;
     std::fprintf(stderr, "[lux-cuda] %s: %s\n", what, cudaGetErrorString(e));
+    (void)cudaGetLastError();                // a refused launch is remembered by the runtime: the next call must not report it again
     if (e == cudaErrorMemoryAllocation) return LUX_BACKEND_ERROR_OUT_OF_MEMORY;
     if (e == cudaErrorInvalidValue || e == cudaErrorInvalidDevice) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     return LUX_BACKEND_ERROR_INTERNAL;
