@@ -51,6 +51,35 @@ def test_matmul_int8_bit_exact(ctx, backend, M, N, K):
         assert np.array_equal(got, orc.matmul_int(a, b, M, N, K, 8))
 
 
+@pytest.mark.parametrize("form", [1, 2, 3])
+@pytest.mark.parametrize("splits", [1, 2, 4])
+@pytest.mark.parametrize("M,N,K", [(300, 272, 1008),       # B as it lies, a K tail, ragged tiles
+                                   (257, 513, 528),        # N odd: through B^T, stores of single words; slices of one and two stages
+                                   (600, 300, 2064),       # N a multiple of 4 only
+                                   (128, 256, 512)])       # whole tiles, slices of one stage
+def test_every_tile_and_split_bit_exact(ctx, backend, M, N, K, form, splits):
+    """The three tiles and the slices of K, whichever the sizes would choose; int4 x int8 through the same kernel."""
+    a = RNG.integers(-128, 128, size=(M, K), dtype=np.int8)
+    a4 = RNG.integers(-8, 8, size=(M, K), dtype=np.int8)
+    b = RNG.integers(-128, 128, size=(K, N), dtype=np.int8)
+    bb, bf = ctx.upload(b), b.astype(np.float64)
+    backend.tune("int_matmul_form", form)
+    backend.tune("int_matmul_splits", splits)
+    try:
+        for op, bits in ((a, 8), (a4, 4)):
+            ab = ctx.upload(op if bits == 8 else _pack_int4_twos(op))
+            cb = ctx.upload(np.full((M * N + 64,), 0x5A5A5A5A, np.int32))
+            ctx.matmul_int8(ab, bb, cb, M, N, K, a_bits=bits)
+            assert backend.last_kernel_name() == ("lux_matmul_int8_tcgen05" if bits == 8 else "lux_matmul_int4_int8_tcgen05")
+            got = cb.to_host(np.int32, (M * N + 64,))
+            assert np.array_equal(got[:M * N].reshape(M, N), (op.astype(np.float64) @ bf).astype(np.int32))
+            assert (got[M * N:] == 0x5A5A5A5A).all()
+    finally:
+        backend.tune("int_matmul_form", 0)
+        backend.tune("int_matmul_splits", 0)
+    assert ctx.last_device_status() == 0
+
+
 @pytest.mark.parametrize("M,N", [(32, 32), (128, 256)])
 def test_matmul_int8_extremes(ctx, M, N):
     K = 4096
@@ -119,6 +148,43 @@ def test_matmul_int8_more_rows_than_a_grid_of_128_row_tiles(ctx, backend):
     bt = torch.from_numpy(b).cuda().double()
     for r0 in range(0, M, 1 << 20):                          # exact in f64
         assert torch.equal(c[r0:r0 + (1 << 20)], (a[r0:r0 + (1 << 20)].double() @ bt).to(torch.int32))
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("n", [7, 4096, 100003])
+@pytest.mark.parametrize("kind", ["half_integers", "denormal", "inf", "nan", "unaligned"])
+def test_dynamic_quantize_rounds_as_a_division(ctx, bits, n, kind):
+    """Values on and one ulp either side of every half-integer times the scale, scales whose reciprocal overflows,
+    infinities and NaN (skipped by the maximum, quantized to 0), and a view that takes no 16-byte loads."""
+    rng = np.random.default_rng(n + bits)
+    x = rng.standard_normal(n).astype(np.float32)
+    top = np.float32(127 if bits == 8 else 7)
+    if kind == "half_integers":
+        s = np.float32(0.37)
+        h = (rng.integers(0, int(top), n) + np.float32(0.5)).astype(np.float32) * s
+        side = rng.integers(0, 3, n)
+        h = np.where(side == 0, h, np.nextafter(h, np.where(side == 1, np.float32(np.inf), np.float32(-np.inf))))
+        x = (h * rng.choice([-1, 1], n)).astype(np.float32)
+        x[n // 2] = s * top
+    elif kind == "denormal":
+        x *= np.float32(1e-40)
+    elif kind == "inf":
+        x[n // 3] = -np.inf
+    elif kind == "nan":
+        x[n // 3] = np.nan
+    nbytes = n if bits == 8 else (n + 1) // 2
+    if kind == "unaligned":
+        big = ctx.upload(np.concatenate([np.zeros(1, np.float32), x]))
+        xb = ctx.wrap(big.device_ptr + 4, x.nbytes)
+    else:
+        xb = ctx.upload(x)
+    ob, sb = ctx.alloc((nbytes + 3) // 4 * 4), ctx.alloc(4)
+    ctx.dynamic_quantize(xb, ob, sb, n, bits)
+    # which operand max() returns beside a NaN is the shader's choice and would depend on the order: the kernel's maximum
+    # never takes it, and its quotient counts as 0, which is what the oracle gives for 0 in its place
+    want, scale = orc.dynamic_quantize(np.where(np.isnan(x), np.float32(0), x), bits)
+    assert sb.to_host(np.float32, (1,)).view(np.uint32)[0] == np.float32(scale).view(np.uint32)
+    assert np.array_equal(ob.to_host(np.uint8, ((nbytes + 3) // 4 * 4,))[:nbytes], want)
 
 
 def test_a_refused_launch_is_reported_once(ctx):

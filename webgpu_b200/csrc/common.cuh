@@ -125,6 +125,8 @@ struct Tunables {
     int gemm_min_m = 0;          // smallest batch the weights-in-TMEM GEMM takes from the streaming kernels (0 = built-in)
     int gemm_tc_kernel = 0;      // 0 auto, 1 lux_qgemm_i4_tc, 2 lux_qgemm_i4_tc_wa wherever it applies
     int int_matmul_kernel = 0;   // lux_cuda_matmul_int8 / _int4_int8: 0 tcgen05 for large shapes, 1 mma.sync kernels only, 2 tcgen05 always through B^T
+    int int_matmul_form = 0;     // its tile on tcgen05: 0 choose, 1 256 x 256, 2 128 x 256, 3 128 x 128
+    int int_matmul_splits = 0;   // slices of K there: 0 choose, 1, 2 or 4 where K has as many stages of 128
     int attn_prefill = 0;        // attention of many queries per head: 0 choose, 1 lux_attn_prefill_mma_f32 wherever it applies, 2 never,
                                  // 3 lux_attn_prefill_f32 wherever it applies
     int attn_splits = 0;         // attention: slices of the keys per (sequence, KV head, row block); 0 = choose

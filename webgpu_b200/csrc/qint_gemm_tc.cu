@@ -346,10 +346,13 @@ LuxBackendError launch_matmul_int8_tcgen05(Context* ctx, const void* a, const vo
         const long long cost = (ctas_of(f) + sms - 1) / sms * f.cost;
         if (best_cost == 0 || cost < best_cost) { best = &f; best_cost = cost; }
     }
+    if (g_tune.int_matmul_form >= 1 && g_tune.int_matmul_form <= 3) best = &forms[g_tune.int_matmul_form - 1];
     const int ma = best->ma, bn = best->bn;
     // split K while that still finds idle SMs and leaves a slice at least four stages
     unsigned ks = 1;
     while (ks < 4 && ctas_of(*best) * (ks * 2) <= sms && stages >= (int)(ks * 2) * 4) ks *= 2;
+    const int want = g_tune.int_matmul_splits;
+    if ((want == 1 || want == 2 || want == 4) && stages >= want) ks = (unsigned)want;
     const uint32_t abox[2] = {(uint32_t)I8_KB, (uint32_t)(ma * I8_BM)}, bbox[2] = {(uint32_t)I8_KB, (uint32_t)bn};
     if (!encode_tensor_map_u8(&ma_map, 2, a_int4 ? (const void*)a8 : a, adims, strides, abox, true)) return LUX_BACKEND_ERROR_INTERNAL;
     if (b_mn) {
