@@ -244,6 +244,43 @@ def test_decode_steps_no_sync_chain(ctx):
         _close(ob.to_host(np.float32, want.shape), want)
 
 
+@pytest.mark.parametrize("B_,H,Hkv,cache_len,Sq,kernel", [(2, 8, 2, 600, 1, "lux_attn_merge_f32"),
+                                                          (1, 32, 8, 100, 256, "lux_attn_prefill_mma_f32")])
+def test_overlapped_launches_change_nothing(ctx, backend, B_, H, Hkv, cache_len, Sq, kernel):
+    """rope -> append -> attend, each step's queries the last step's output and every buffer used again by the next one, so
+    that a kernel which started on its operands too early would read or overwrite what another still needs: the
+    same bits enqueued at once, enqueued at once without programmatic launches, and with a wait after each call.
+    The decode step splits its keys over CTAs (shared partial results, merge); the other takes the prompt kernel."""
+    rng = np.random.default_rng(44)
+    D, steps = 128, 4
+    max_len = cache_len + steps * Sq
+    cos, sin = orc.rope_cache(max_len, D, 10000.0)
+    cb, sb = ctx.upload(cos), ctx.upload(sin)
+    kc, vc = (rng.standard_normal((B_, Hkv, max_len, D), np.float32) for _ in range(2))
+    q0 = rng.standard_normal((B_, H, Sq, D), np.float32)          # read as [batch, seq, heads, dim] by the rotation: any bytes do
+    k0, v0 = (rng.standard_normal((B_, Hkv, Sq, D), np.float32) for _ in range(2))
+    results = []
+    for flags, pdl in ((0, 0), (B.FLAG_NO_SYNC, 0), (B.FLAG_NO_SYNC, 2)):
+        kcb, vcb, qb, kb, vb, ob = (ctx.upload(x) for x in (kc, vc, q0, k0, v0, q0))
+        backend.tune("pdl", pdl)
+        try:
+            for step in range(steps):
+                pos = cache_len + step * Sq
+                ctx.rope(ob, qb, B_, Sq, H, D, cos=cb, sin=sb, position_offset=pos, flags=flags)
+                ctx.rope(kb, kb, B_, Sq, Hkv, D, cos=cb, sin=sb, position_offset=pos, flags=flags)
+                ctx.update_kv_cache(kb, vb, kcb, vcb, B_, Hkv, Sq, pos, max_len, D, flags=flags)
+                ctx.sdpa_kv_cache(qb, kcb, vcb, ob, B_, H, Hkv, Sq, pos, max_len, D, 1 / np.sqrt(D), flags=flags | B.FLAG_ATTN_CAUSAL)
+                assert backend.last_kernel_name() == kernel
+            ctx.sync()
+        finally:
+            backend.tune("pdl", 0)
+        results.append([b.to_host(np.float32, x.shape).copy() for b, x in ((ob, q0), (qb, q0), (kb, k0), (kcb, kc), (vcb, vc))])
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    assert np.isfinite(results[0][0]).all()
+
+
 # ---- paged KV cache -------------------------------------------------------------------------------
 
 
