@@ -1,4 +1,4 @@
-"""lux_attn_prefill_mma_f32 and the f32 kernel behind it (many queries per head, head size 128) at the sizes where
+"""lux_attn_prefill_mma_f32 and the f32 arithmetic it falls back to (many queries per head, head size 128) at the sizes where
 their tiling can go wrong: queries and keys one off a tile of 64 or a block of 128, one tile, several,
 masked and not, appended to a cache, heads that share a KV head, operands of very different magnitudes, NaN
 and infinities; against the oracle, and against the streaming kernel.  Tolerance as in test_gpu_attention.py:

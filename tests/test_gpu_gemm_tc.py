@@ -19,8 +19,8 @@ TOL_16 = 5e-3
 
 @pytest.fixture(autouse=True)
 def _b_operand_kernel(backend):
-    """This file covers lux_qgemm_i4_tc (converted weights as the shared-memory B operand), which
-    by default only takes the shapes lux_qgemm_i4_tc_wa does not: select it for every test here."""
+    """This file covers lux_qgemm_i4_tc (converted weights as the shared-memory B operand), all of whose
+    shapes lux_qgemm_i4_tc_wa takes by default: select it for every test here."""
     backend.tune("gemm_tc_kernel", 1)
     yield
     backend.tune("gemm_tc_kernel", 0)

@@ -751,8 +751,8 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
         geometry(n);
         if (p.nsplit != n) continue;                                   // rounding to chunks merged this count into a smaller one
         // (a decode step over up to 512 keys goes down to 64: a slice is then two chunks of the ring, and what counts
-        // is how soon it ends: one sequence, Llama-3-8B heads, 300 keys, 11.5 -> 9.5 us a call; at 2000 keys slices
-        // of 64 are 13.6 us against 12.7, and a prompt of 150 tokens, which fills the chip with its rows, 40 against 30)
+        // is how soon it ends: one sequence, Llama-3-8B heads, 300 keys, 10.4 -> 9.3 us a call; at 2000 keys slices
+        // of 64 are 12.6 us against 11.5, and a prompt of 150 tokens, which fills the chip with its rows, 43 against 29)
         if (n > min_split && p.split_keys < (max_keys <= 512 && p.row_blocks == 1 ? 64u : 128u)) break;
         const double ctas = (double)items * n, waves = std::ceil(ctas / sm);
         const double score = ctas / (waves * sm) * p.split_keys / (p.split_keys + 64.0);

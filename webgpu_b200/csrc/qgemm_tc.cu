@@ -1,5 +1,7 @@
 // int4 g128 weight-only GEMM on the 5th-generation tensor cores (tcgen05 + TMEM), for
-// batches too large for the streaming kernel (prefill, M >= 33).
+// batches too large for the streaming kernel (prefill, M >= 33).  Selected by the tunable gemm_tc_kernel = 1:
+// lux_qgemm_i4_tc_wa takes every shape that this kernel takes and is the faster one; the two are tested
+// against each other.
 //
 //   y[M, N] = x[M, K] . dequant(W[N, K])^T      x, y bf16 or f16; f32 accumulate in TMEM
 //

@@ -531,7 +531,7 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     if ((reinterpret_cast<uintptr_t>(a.x) & 15u) || (reinterpret_cast<uintptr_t>(a.y) & 15u)) return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     const bool bf16 = a.x_dtype == LUX_QDTYPE_BF16;
 
-    // Split K over a cluster of two or four CTAs when whole tiles alone would leave most slots idle
+    // Split K over a cluster of two, four or eight CTAs when whole tiles alone would leave most slots idle
     // (`slots` = CTAs resident at once).
     auto plan = [&](int bn, int slots, int& ks_out) {
         const int tiles = (nout + out_w - 1) / out_w * ((a.M + bn - 1) / bn);
@@ -620,7 +620,7 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
     cudaError_t e;
     if (a.swiglu) e = bf16 ? go_bn(std::true_type{}, std::true_type{}) : go_bn(std::false_type{}, std::true_type{});
     else          e = bf16 ? go_bn(std::true_type{}, std::false_type{}) : go_bn(std::false_type{}, std::false_type{});
-    if (nout % out_w) count_launch(bf16 ? "lux_qgemm_i4_tc_wa_edge_bf16" : "lux_qgemm_i4_tc_wa_edge_f16");     // partly empty last tile
+    if (nout % out_w) count_launch(bf16 ? "lux_qgemm_i4_tc_wa_edge_bf16" : "lux_qgemm_i4_tc_wa_edge_f16");     // partly empty last tile (the route sweep tells them apart)
     else count_launch(bf16 ? "lux_qgemm_i4_tc_wa_bf16" : "lux_qgemm_i4_tc_wa_f16");
     return map_cuda(e, "lux_qgemm_i4_tc_wa");
 }

@@ -127,7 +127,7 @@ LuxBackendError dispatch(Context* ctx, const Checked& c) {
             // The kernel that keeps the converted weights in tensor memory (one conversion per 256
             // batch rows, 128 x 256 MMAs; for smaller batches 128 x M) wherever the shape fits it:
             // measured faster than the B-operand kernel at every batch from 64 up (config 4 layers at
-            // M = 64: 12-38 us against 34-109 us; config 3: 18 us against 40 us).
+            // M = 64: 12-38 us against 34-109 us; config 3: 18 us against 40 us).  It takes every shape the other one takes.
             if (g_tune.gemm_tc_kernel == 2 || g_tune.gemm_tc_kernel == 0) {
                 LuxBackendError e = launch_qgemm_i4_tc_wa(ctx, c.a);
                 if (e != LUX_BACKEND_ERROR_NOT_SUPPORTED) return e;
