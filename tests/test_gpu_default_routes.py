@@ -159,3 +159,22 @@ def test_bf16_decode_takes_the_fixed_point_gemv(ctx, backend, name, M):
     yh = ctx.alloc(M * layer.N * 2)
     ctx.qmatmul(ctx.upload(synth.bf16_bits_to_f32(x).astype(np.float16)), L, yh, M, B.F16)
     assert orc.rel_l2(y, yh.to_host(np.float16, (M, layer.N)).astype(np.float32)) < 2.5e-3
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("M,N", [(5, 1016), (16, 136), (32, 72)])
+def test_small_f16_batches_with_ragged_outputs_keep_exact_weights(ctx, backend, M, N, swiglu):
+    """Outputs that fill no tile at 5..32 f16 rows run on the kernels that do not round the weights: the only error is the
+    rounding of the output, 2^-11 / sqrt(3) of a value's binade, 2.1e-4 of the norm; a rounding of the weights would add as
+    much again (2.9e-4 in all)."""
+    K = 1024
+    x = synth.activations(M, K, "f16", 61, f"rag.{M}.{N}")
+    layer = synth.int4_layer(2 * N if swiglu else N, K, 61, f"rag.{N}.{swiglu}")
+    xb, yb = ctx.upload(x), ctx.alloc(M * N * 2)
+    ctx.qmatmul(xb, ctx.upload_layer(layer), yb, M, B.F16, flags=B.FLAG_SWIGLU if swiglu else 0)
+    assert not backend.last_kernel_name().startswith("lux_qgemm")
+    y = yb.to_host(np.float16, (M, N)).astype(np.float64)
+    want = x.astype(np.float64) @ orc.qdequant(*layer.triple, 4, 128).astype(np.float64).T
+    if swiglu:
+        want = want[:, :N] / (1 + np.exp(-want[:, :N])) * want[:, N:]
+    assert np.linalg.norm(y - want) / np.linalg.norm(want) < 2.4e-4

@@ -207,7 +207,7 @@ def test_wa_outputs_that_fill_no_tile(ctx, backend, dtype, splitk, M, N):
     guard = np.full(M * N + 64, 0x5A5A, np.uint16)
     for lay, flags in ((half, 0), (layer, B.FLAG_SWIGLU)):
         xb, yb = ctx.upload(x), ctx.upload(guard)
-        with _Tuned(backend, gemm_tc_splitk=splitk):
+        with _Tuned(backend, gemm_tc_kernel=2, gemm_tc_splitk=splitk):
             ctx.qmatmul(xb, ctx.upload_layer(lay), yb, M, B.np_dtype_code(x), flags=flags)
         assert backend.last_kernel_name().startswith("lux_qgemm_i4_tc_wa")
         raw = yb.to_host(np.uint16, guard.shape)

@@ -1,5 +1,5 @@
 // int4 g128 weight-only GEMM on tcgen05 with the converted WEIGHTS as the tensor-memory A
-// operand: the default from five batch rows up.
+// operand: the default from five batch rows up (f16 up to 32 rows: for outputs in whole tiles).
 //
 //   y[M, N] = x[M, K] . dequant(W[N, K])^T      x, y bf16 or f16; f32 accumulate in TMEM
 //

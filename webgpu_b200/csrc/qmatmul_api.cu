@@ -103,8 +103,12 @@ LuxBackendError dispatch(Context* ctx, const Checked& c) {
             // (config 4 gate_up / down at batch 5: 27.4 / 19.8 us against 31.4 / 25.7 us, at batch 11:
             // 27.5 / 19.9 us against 46.3 / 69.6 us; its time does not depend on the batch up to 64).  Three
             // and four rows stay with the fixed-point kernel above (gate_up 19.1 us) or the ring kernel.
+            // Only outputs in whole tiles (128, with SwiGLU 64): it rounds the weights to f16, which the kernels below, where
+            // other outputs have always run, do not (error against 64 bits 2.9e-4, SwiGLU 3.6e-4, against 2.1e-4;
+            // it would be the faster one there too: 11016 x 4096 at 16 rows 15.6 us against 41).
             const int min_m = g_tune.gemm_min_m > 0 ? g_tune.gemm_min_m : 5;
-            if (a.M >= min_m && g_tune.gemv_i4_kernel == 0 && g_tune.gemm_tc_kernel != 1 && !a.push) {
+            const bool whole = (a.swiglu ? a.N / 2 % 64 : a.N % 128) == 0 || g_tune.gemm_tc_kernel == 2;
+            if (a.M >= min_m && whole && g_tune.gemv_i4_kernel == 0 && g_tune.gemm_tc_kernel != 1 && !a.push) {
                 LuxBackendError e = launch_qgemm_i4_tc_wa(ctx, a);
                 if (e != LUX_BACKEND_ERROR_NOT_SUPPORTED) return e;
             }
