@@ -172,9 +172,9 @@ def test_keys_of_very_different_magnitude(ctx, backend, lo, hi):
     assert err.max() < 2 * TOL, err.max()
 
 
-@pytest.mark.parametrize("drop", [14, 18, 21, 30])
+@pytest.mark.parametrize("drop", [14, 18, 21, 30, 60, 80])
 def test_small_weights_under_a_dominant_key_without_a_value(ctx, backend, drop):
-    """One key takes the row's weight and its V is zero: the output is made of weights of e^-drop, down to 2^-43, alone."""
+    """One key takes the row's weight and its V is zero: the output is made of weights of e^-drop, down to 2^-115, alone."""
     rng = np.random.default_rng(14)
     q, k, v = _qkv(14, 1, 2, 1, 140, 140)
     k *= np.float32(0.1)
@@ -184,8 +184,23 @@ def test_small_weights_under_a_dominant_key_without_a_value(ctx, backend, drop):
     v[0, 0, 0] = 0.0
     with _Tuned(backend, attn_prefill=1):
         got, _ = _sdpa(ctx, q, k, v, False)
-    # the exponent's argument, up to 30 log2(e) = 43, is rounded to 2^-19 of its weight at worst (an ulp of 43 is 2^-18)
-    assert orc.rel_l2(got, _sdpa64(q, k, v, False)) < 4e-6
+    # the maximum and the exponent's argument, drop log2(e) in size, are each rounded to half an ulp, and an absolute error
+    # there is a relative one of the weight: up to 2 ln(2) 2^-25 2^ceil(log2(drop log2(e))), 2.6e-6 at 30 and 5.3e-6 at 80
+    bound = 2 * np.log(2) * 2.0 ** -25 * 2 ** np.ceil(np.log2(drop / np.log(2)))
+    assert orc.rel_l2(got, _sdpa64(q, k, v, False)) < bound + 1e-6
+
+
+@pytest.mark.parametrize("columns", [slice(None), slice(5, 6)])
+@pytest.mark.parametrize("scale", [1e-28, 1e-31, 1e-34, 1e-37])
+def test_values_close_to_the_smallest_normal_number(ctx, backend, scale, columns):
+    """V (or one column of it) down to 1e-37: f32 keeps 24 bits there, and so does every column of the output."""
+    q, k, v = _qkv(21, 1, 2, 1, 140, 140)
+    v[..., columns] *= np.float32(scale)
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, True)
+    want = _sdpa64(q, k, v, True)
+    err = np.sqrt(((got - want) ** 2).sum(axis=(0, 1, 2)) / (want ** 2).sum(axis=(0, 1, 2)))
+    assert err.max() < 2 * TOL, err.max()                 # the worst of 128 columns, each with 280 values
 
 
 @pytest.mark.parametrize("qs,ks", [(1e15, 1e-15), (1e30, 1e-30), (1e37, 1e-37), (1e-30, 1e30), (1e-37, 1e37)])

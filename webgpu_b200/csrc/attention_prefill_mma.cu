@@ -8,11 +8,12 @@
 // each per sub-core) where the FMA pipe does 128.
 //
 // Range.  bf16 has f32's exponents, so a part depends on its own element alone: no scale is shared along a row, a
-// column or a tile, a masked key weighs exactly nothing however large its values, and a weight of 2^-100 keeps
-// its 24 bits.  A part below 2^-126 is lost, so an element's error is 2^-24 of it or 2^-126.  A block that
-// meets a magnitude of 2^60 or more (after Q's scale), an infinity or a NaN is done on the f32 pipe: with
-// all below 2^60 no score and no sum overflows (2^120 x 128) and no bf16 rounding does, and 2^-126 x 2^60 x 128 is
-// nothing in a score.
+// column or a tile, and a masked key weighs exactly nothing however large its values.  A part below 2^-126 may be
+// lost.  Weights are split times 2^30 (a weight is 2^-126 at least, or 0) and so keep their 24 bits; in a score
+// 2^-126 x 2^60 x 128 is nothing; and V can lose 2^-126 of an output, which matters to outputs below 2^-100 alone:
+// if V had non-zero values below 2^-100 and such an output comes out, the block is done on the f32 pipe.
+// So is one that meets a magnitude of 2^60 or more (after Q's scale), an infinity or a NaN: with all below 2^60
+// no score, no sum (2^120 x 128; 2^(8 + 30 + 60) a key) and no bf16 rounding overflows.
 //
 // Accumulation.  The tensor core sums a step of 16 exactly and cuts the f32 result off (measured: mean loss 3.8e-8 of
 // it, otherwise no more than rounding's error).  Every step's h h products, of 16 bits each, therefore start from zero
@@ -30,8 +31,8 @@
 // before it works on the current one and the other after it, so that the splitting runs beside the tensor core.  A warp
 // owns 16 rows from the scores to the output; Q's fragments and the output stay in its registers, the weights go from
 // accumulator to operand layout without leaving them.  Causal, Llama-3-8B heads, against the streaming kernel:
-// 2048 tokens 1679 -> 677 us (51 TFLOP/s of f32 products, 305 of the tensor core's 568 at this instruction), 512
-// tokens 152 -> 94, 150 tokens 29.5 -> 28.4; unmasked 1448 tokens 1567 -> 785.  What is left is the tensor pipe (more
+// 2048 tokens 1679 -> 673 us (51 TFLOP/s of f32 products, 307 of the tensor core's 568 at this instruction), 512
+// tokens 152 -> 93, 150 tokens 29.5 -> 28.3; unmasked 1448 tokens 1567 -> 774.  What is left is the tensor pipe (more
 // than half the time) and the softmax, splitting and fragment loads beside it.
 #include "attention_prefill_f32.cuh"
 
@@ -48,13 +49,15 @@ constexpr int BN = 32;                    // keys per tile
 constexpr int WARPS = 8, THREADS = WARPS * 32;
 constexpr int F32_TILE = BN * D * 4;      // K or V of a tile as it arrives
 constexpr int PART = BN * D * 2;          // one part of it: 32 rows of 256 bytes, 16-byte chunks ^ (row & 7)
-// two slots of {K, V} in f32, two buffers of {K h, m, l, V h, m, l}, two mbarriers, abort flag, bad flag
+// two slots of {K, V} in f32, two buffers of {K h, m, l, V h, m, l}, two mbarriers, abort flag, bad flag, tiny flag
 constexpr int OFF_F32 = 0, SLOT = 2 * F32_TILE, OFF_BUF = 2 * SLOT, BUF_BYTES = 6 * PART;
 constexpr int OFF_BAR = OFF_BUF + 2 * BUF_BYTES;
 constexpr int SMEM = OFF_BAR + 64 + 128;
 constexpr float NEG = -3.0e38f, LN2 = 0.6931471805599453f;
 constexpr float RAISE = 8.0f;             // the running maximum is raised when a score passes it by more: weights below 2^8
+constexpr float P_SCALE = 0x1p30f;        // of the weights before they are split
 constexpr uint32_t TOO_LARGE = (127u + 60u) << 23;           // |x| >= 2^60, infinity or NaN, as bits
+constexpr uint32_t TOO_SMALL = (127u - 100u) << 23;          // 0 < |v| < 2^-100
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -92,6 +95,7 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
     const uint32_t bars = sb + OFF_BAR;           // one per slot
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_BAR + 16);
     volatile uint32_t* bad_flag = abort_flag + 1;
+    volatile uint32_t* tiny_flag = abort_flag + 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
 
     pdl_launch_dependents();
@@ -119,6 +123,7 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
         mbar_init(bars + 8u, 1u);
         *abort_flag = 0u;
         *bad_flag = 0u;
+        *tiny_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();                              // the flags are clear before a warp may raise one over its rows of Q
@@ -164,13 +169,15 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
         const uint32_t nk = min((uint32_t)BN, lmax - t * BN);
         const unsigned char* src = smem + OFF_F32 + (t & 1u) * SLOT + warp * 8 * (D * 4) + lane * 16;
         unsigned char* buf = smem + OFF_BUF + (t & 1u) * BUF_BYTES + (warp >> 2) * (3 * PART);
-        uint32_t top = 0u;
+        uint32_t top = 0u, low = 0xffffffffu;         // largest magnitude; smallest non-zero one, less 1
 #pragma unroll 4
         for (int i = 0; i < 8; i++) {
             const int key = (warp & 3) * 8 + i;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if ((uint32_t)key < nk) v = *reinterpret_cast<const float4*>(src + i * (D * 4));
-            top = max(top, max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))));
+            const uint32_t b0 = abs_bits(v.x), b1 = abs_bits(v.y), b2 = abs_bits(v.z), b3 = abs_bits(v.w);
+            top = max(top, max(max(b0, b1), max(b2, b3)));
+            low = min(low, min(min(b0 - 1u, b1 - 1u), min(b2 - 1u, b3 - 1u)));
             uint2 w[3];
             split3(v.x, v.y, w[0].x, w[1].x, w[2].x);
             split3(v.z, v.w, w[0].y, w[1].y, w[2].y);
@@ -179,6 +186,7 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
             for (int c = 0; c < 3; c++) *reinterpret_cast<uint2*>(buf + c * PART + at) = w[c];
         }
         if (top >= TOO_LARGE) *bad_flag = 1u;
+        if (low < TOO_SMALL - 1u && warp >= WARPS / 2) *tiny_flag = 1u;
     };
     // c += a b without its h h part, for two independent pairs at once (their chains of five are interleaved)
     auto mma_rest = [&](float (&c0)[4], float (&c1)[4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4],
@@ -286,8 +294,8 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
             sum[0] += s[n][0] + s[n][1];
             sum[1] += s[n][2] + s[n][3];
             const int f = n >> 1, e = 2 * (n & 1);
-            split3(s[n][0], s[n][1], wp[0][f][e], wp[1][f][e], wp[2][f][e]);
-            split3(s[n][2], s[n][3], wp[0][f][e + 1], wp[1][f][e + 1], wp[2][f][e + 1]);
+            split3(s[n][0] * P_SCALE, s[n][1] * P_SCALE, wp[0][f][e], wp[1][f][e], wp[2][f][e]);
+            split3(s[n][2] * P_SCALE, s[n][3] * P_SCALE, wp[0][f][e + 1], wp[1][f][e + 1], wp[2][f][e + 1]);
         }
         l[0] += sum[0];
         l[1] += sum[1];
@@ -341,6 +349,22 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
     } else {
         ok = !__syncthreads_or(*bad_flag != 0u);
     }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+    }
+    if (ok && *tiny_flag) {                            // the same for all: last written before the last round's barrier
+        bool low = false;
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int n = 0; n < 16; n++) {
+                const float least = l[r] * (P_SCALE * 0x1p-100f);
+                low |= fabsf(o[n][2 * r]) < least || fabsf(o[n][2 * r + 1]) < least;
+            }
+        ok = !__syncthreads_or(low);
+    }
     if (!ok) {
         // values out of range: the block starts over on the f32 pipe; or a bounded wait gave up: report it, and give
         // copies in flight time to land.  Nothing has been written.
@@ -357,8 +381,6 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
     }
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
-        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
         const uint32_t row = (uint32_t)(warp * 16 + g + 8 * r);
         if (row >= rows) continue;
         const size_t orow = ((size_t)b * p.heads + h) * p.seq_q + q0 + row;
@@ -366,7 +388,7 @@ __global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const Pre
 #pragma unroll
         for (int n = 0; n < 16; n++)
             *reinterpret_cast<float2*>(p.out + orow * D + 8 * n + 2 * t4) =
-                any ? make_float2(o[n][2 * r] / l[r], o[n][2 * r + 1] / l[r]) : make_float2(0.f, 0.f);
+                any ? make_float2(o[n][2 * r] / l[r] * (1.0f / P_SCALE), o[n][2 * r + 1] / l[r] * (1.0f / P_SCALE)) : make_float2(0.f, 0.f);
         if (t4 == 0 && p.lse) p.lse[orow] = any ? fmaf(m[r], LN2, logf(l[r])) : -3.402823e+38f;
     }
 }
