@@ -18,10 +18,11 @@
  * lux_cuda_buffer_wrap), arguments validated before anything is launched, a LuxBackendError
  * comes back, nothing throws.  `flags` takes LUX_QMATMUL_FLAG_NO_SYNC (enqueue and return) and
  * the LUX_ATTN_* bits below.  All data is f32; head_dim is any positive value (multiples of 4 up
- * to 256 take the streaming kernel, the rest a plain one).
+ * to 256 take the streaming kernel, prompts of head_dim 128 a tensor-core one, the rest a plain one).
  *
  * Arithmetic: scores = (q . k) * scale; weights = softmax over the keys a row sees; out =
- * weights . v, all in f32.  Sums are taken in a different order than the one-workgroup-per-row
+ * weights . v, all in f32 (the tensor-core kernel forms an f32 product from six products of the
+ * factors' exact bf16 parts, to 2^-24 of it, and adds in f32).  Sums are taken in a different order than the one-workgroup-per-row
  * shaders take them (keys are split over warps and, for long contexts, over thread blocks, and
  * merged with the running-maximum rule of sdpa_flash, scaled_dot_product_attention.wgsl:217-362),
  * so results agree with the shaders to rounding, not bit for bit.  The shaders' safe_exp clamps

@@ -66,7 +66,7 @@ __device__ __forceinline__ void load8(const QuantParams& p, size_t idx, float (&
 // BITS = 4: groups of 128 (16 lanes); BITS = 8: groups of 32 (4 lanes), symmetric only.
 // With a division per element, and the group's three per eight elements, the arithmetic took longer than the
 // memory: 14336 x 4096 f32 to int4 with zero-points 72 us (266 MB, 3.7 TB/s).  round_div.cuh divides only
-// next to half-integers and the group's divisions are spread over its lanes: 59 us (4.5 TB/s).
+// next to half-integers and the group's divisions are spread over its lanes: 57 to 59 us (4.5 to 4.7 TB/s).
 // A warp takes QCH consecutive 256-element chunks of a row and requests all of them before it
 // reduces the first: 4 KB in flight per warp, so that a streaming kernel with this little
 // arithmetic keeps HBM busy.
