@@ -315,3 +315,56 @@ def test_default_choice_over_a_cache(ctx, backend, Sq, keys, takes):
             assert mode or (backend.last_kernel_name() == "lux_attn_prefill_mma_f32") == takes
         outs.append(ob.to_host(np.float32, q.shape).copy())
     assert orc.rel_l2(outs[0], outs[1]) < TOL
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("B_,H,Hkv,Sq,Skv", [(1, 1, 1, 65, 65), (1, 5, 1, 129, 640), (1, 3, 3, 257, 449), (1, 6, 2, 128, 512), (1, 4, 2, 385, 385), (2, 8, 2, 250, 1000)])
+def test_pairs_of_blocks(ctx, backend, B_, H, Hkv, Sq, Skv, causal):
+    """Two heads of a KV head, or two blocks of queries of one head (the last one alone, or seeing fewer tiles than its
+    partner), over as many tiles as the ring has slots and more; against 64 bits."""
+    q, k, v = _qkv(Sq + Skv, B_, H, Hkv, Sq, Skv)
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, causal)
+    assert orc.rel_l2(got, _sdpa64(q, k, v, causal)) < TOL and ctx.last_device_status() == 0
+
+
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+def test_an_odd_pair_with_one_block_out_of_range(ctx, backend, where):
+    """Two blocks of queries of one head make a pair: what only the later one meets leaves the earlier one its own bits."""
+    q, k, v = _qkv(22, 1, 1, 1, 250, 250)
+    dirty = {"q": q.copy(), "k": k.copy(), "v": v.copy()}
+    dirty[where][0, 0, 200, 5] = np.inf
+    with _Tuned(backend, attn_prefill=1):
+        clean, _ = _sdpa(ctx, q, k, v, True)
+        got, _ = _sdpa(ctx, **dirty, causal=True)
+    with _Tuned(backend, attn_prefill=3):
+        want, _ = _sdpa(ctx, **dirty, causal=True)
+    assert np.array_equal(got[:, :, :128].view(np.uint32), clean[:, :, :128].view(np.uint32))
+    assert np.array_equal(got[:, :, 128:].view(np.uint32), want[:, :, 128:].view(np.uint32))
+
+
+@pytest.mark.parametrize("B_,Hkv,Skv,kernel", [(3, 50, 1000, "lux_attn_prefill_mma_f32"), (1, 1, 131073, "lux_attn_prefill_f32")])
+def test_more_keys_than_the_scratch_holds(ctx, backend, B_, Hkv, Skv, kernel):
+    """128 k keys of all KV heads have their parts in the scratch at a time: more heads go in several passes, a longer
+    head goes to the f32 kernel; either way the streaming kernel's answer to rounding."""
+    q, k, v = _qkv(23, B_, Hkv, Hkv, 66, Skv)
+    outs = []
+    for mode in (1, 2):
+        with _Tuned(backend, attn_prefill=mode):
+            outs.append(_sdpa(ctx, q, k, v, False)[0])
+            assert mode == 2 or backend.last_kernel_name() == kernel
+    # an output is the mean of Skv values: its rounding errors grow with the square root of the chain of sums
+    assert orc.rel_l2(outs[0], outs[1]) < TOL * max(1.0, (Skv / 4096) ** 0.5)
+
+
+def test_no_less_precise_than_the_streaming_kernel(ctx, backend):
+    """Error against 64 bits over lengths of one tile to many, masked and not: the tensor core's chains are short, so it
+    stays below that of ordinary f32 sums."""
+    for Sq, causal in ((64, True), (150, True), (512, True), (700, False)):
+        q, k, v = _qkv(Sq, 1, 4, 1, Sq, Sq)
+        want = _sdpa64(q, k, v, causal)
+        errs = []
+        for mode in (1, 2):
+            with _Tuned(backend, attn_prefill=mode):
+                errs.append(orc.rel_l2(_sdpa(ctx, q, k, v, causal)[0], want))
+        assert errs[0] < errs[1], (Sq, causal, errs)

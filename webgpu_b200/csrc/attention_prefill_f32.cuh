@@ -99,7 +99,16 @@ __device__ __forceinline__ float ex2(float x) {                // as in the stre
 constexpr float PF_NEG = -3.0e38f;        // "no key seen yet" in the base-2 score domain
 constexpr float PF_LN2 = 0.6931471805599453f;
 
-// Block qb of head h of sequence b.  All threads of the CTA call it, with 128-byte aligned shared memory that no copy
+// The block's own barrier: its 256 threads may be part of a larger CTA.
+__device__ __forceinline__ void block_sync() { named_bar_sync_c<1>(PF_THREADS); }
+__device__ __forceinline__ bool block_or(bool v) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)v), "n"(PF_THREADS) : "memory");
+    return r != 0u;
+}
+
+// Block qb of head h of sequence b.  The first 256 threads of the CTA call it, with 128-byte aligned shared memory that no copy
 // in flight still writes.
 __device__ __forceinline__ void attend_f32(const PrefillArgs& p, unsigned char* smem, uint32_t qb, uint32_t h, uint32_t b) {
     float* qs = reinterpret_cast<float*>(smem);
@@ -113,14 +122,14 @@ __device__ __forceinline__ void attend_f32(const PrefillArgs& p, unsigned char* 
     const int tr = tid >> 3, tc = tid & 7;
 
     fence_proxy_async_smem();             // copies are about to land where this thread may have written
-    __syncthreads();
+    block_sync();
     if (tid == 0) {
         mbar_init(bar_k, 1u);
         mbar_init(bar_v, 1u);
         *abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();
+    block_sync();
     const uint32_t g = h / p.group;
     const uint32_t q0 = qb * PF_BM;
     const uint32_t rows = min((uint32_t)PF_BM, p.seq_q - q0);
@@ -158,7 +167,7 @@ __device__ __forceinline__ void attend_f32(const PrefillArgs& p, unsigned char* 
             *reinterpret_cast<float4*>(qs + r * PF_PITCH + c * 4) = make_float4(t.x * p.qscale, t.y * p.qscale, t.z * p.qscale, t.w * p.qscale);
         }
     }
-    __syncthreads();
+    block_sync();
 
     uint64_t o[4][8];                     // row tr + 32 i, columns 32 (j / 2) + 4 tc + 2 (j % 2) and the next
     float m[4], l[4];
@@ -273,7 +282,7 @@ __device__ __forceinline__ void attend_f32(const PrefillArgs& p, unsigned char* 
             }
         }
         // K has been read by every warp: the next tile may land
-        if (__syncthreads_or(!ok)) { ok = false; break; }
+        if (block_or(!ok)) { ok = false; break; }
         if (warp == 0 && t + 1 < tiles) load_k(t + 1);
 
         // running maximum per row (the 8 lanes of a row agree on it), raised only when a score passes it
@@ -325,14 +334,14 @@ __device__ __forceinline__ void attend_f32(const PrefillArgs& p, unsigned char* 
                 __syncwarp();
             }
         }
-        if (__syncthreads_or(!ok)) { ok = false; break; }
+        if (block_or(!ok)) { ok = false; break; }
         if (warp == 0 && t + 1 < tiles) load_v(t + 1);
     }
     if (!ok) {
         // a bounded wait gave up: report it, give copies in flight time to land, write nothing
         if (tid == 0 && p.status) atomicOr(p.status, p.status_wait);
         for (int i = 0; i < 64; i++) __nanosleep(1000);
-        __syncthreads();
+        block_sync();
         return;
     }
 #pragma unroll

@@ -3,9 +3,8 @@
 // The f32 FMA pipe (72 TFLOP/s) is not what a prompt has to be bound by.  An f32 number is the exact sum of three bf16
 // parts, h = bf16(x), m = bf16(x - h), l = x - h - m, and
 //     a b = ah bh + (ah bm + am bh) + (am bm + ah bl + al bh)
-// leaves out only am bl + al bm + al bl <= 2^-24 |a b|, what rounding the product to f32 would cost.  Six m16n8k16
-// products replace one f32 product, and mma.sync does 1011 of those multiply-adds per clock and SM (measured: 8.1 cycles
-// each per sub-core) where the FMA pipe does 128.
+// leaves out only am bl + al bm + al bl <= 2^-24 |a b|, what rounding the product to f32 would cost.  Six bf16 products
+// on tcgen05 (8192 flop per clock and SM) replace one f32 product.
 //
 // Range.  bf16 has f32's exponents, so a part depends on its own element alone: no scale is shared along a row, a
 // column or a tile, and a masked key weighs exactly nothing however large its values.  A part below 2^-126 may be
@@ -13,28 +12,35 @@
 // 2^-126 x 2^60 x 128 is nothing; and V can lose 2^-126 of an output, which matters to outputs below 2^-100 alone:
 // if V had non-zero values below 2^-100 and such an output comes out, the block is done on the f32 pipe.
 // So is one that meets a magnitude of 2^60 or more (after Q's scale), an infinity or a NaN: with all below 2^60
-// no score, no sum (2^120 x 128; 2^(8 + 30 + 60) a key) and no bf16 rounding overflows.
+// no score, no sum (2^120 x 128; 2^(8 + 30 + 60) a key) and no bf16 rounding overflows.  A block (a CTA: 128 queries of
+// one head) starts over by itself (attention_prefill_f32.cuh), before it has written anything: this holds with
+// out == q, and no other block, call or replay of a captured one takes part.
 //
-// Accumulation.  The tensor core sums a step of 16 exactly and cuts the f32 result off (measured: mean loss 3.8e-8 of
-// it, otherwise no more than rounding's error).  Every step's h h products, of 16 bits each, therefore start from zero
-// and are added to the running f32 sum by an ordinary rounded addition; the other products, 2^-8 of these and less,
-// run in a chain of their own, where the cut is 2^-8 as large, and are added once per tile.  Relative error against
-// 64 bits (2-norm, N(0, 1) inputs, Llama-3-8B heads; streaming kernel / this one): causal, 150 tokens 1.34e-7 /
-// 1.04e-7, 512 1.65 / 1.22, 2048 2.25 / 1.42; unmasked, 700 x 3 3.06 / 1.76, 1448 4.06 / 2.03.
+// Two kernels.  lux_attn_split_kv writes the parts of K and V once per call, tile by tile as the tensor core wants them in
+// shared memory, into the context's scratch (split in every CTA instead, an element would be converted 64 times in a
+// 2048-token prompt, and the parts' way through shared memory would take as long as the products).
+// lux_attn_prefill_mma_f32 is a pair of CTAs (two heads that share a KV head and their 128 queries, or two
+// blocks of queries of one head where heads do not pair up) that works on 64-key tiles with cta_group::2 products of
+// 256 rows: each CTA holds one half of every tile, so a tile crosses L2 -> SM once per pair (48 KB per CTA and 3.2 k cycles).
+//   warp 9      bulk copies of the pair's K and V halves, seven slots of 24 KB
+//   warp 8      issues: scores of tile t + 1, then the weighted sum of tile t (in the pair's second CTA it passes on
+//               "my half has landed" instead)
+//   warps 0..3  a thread per row: scores from tensor memory, softmax without any exchange, weights back as operand
+//   warps 4..7  a thread per row: the running output in registers; adds each tile's 128 columns
+// Tensor memory (512 columns): Q's h and m parts 128, scores 2 x 64, weights 96, weighted sum 128.  Q's l part, one
+// product in six, is read from shared memory.
 //
-// Out-of-range inputs.  A CTA that meets one starts its block over on the f32 pipe (attention_prefill_f32.cuh); it has written
-// nothing by then, so this holds with out == q, and no other block, call or replay of a captured one takes part.
+// Accumulation.  The tensor core cuts its f32 sums off at every step of 16 (measured on chains of 1 / 2 / 4 / 8 steps:
+// mean loss 1.1 / 2.4 / 4.9 / 9.4e-8 of the sum, in rms 2.5 / 3.9 / 6.5 / 11.6e-8), so chains are four steps of the large products, after
+// the small ones: a score is the f32 sum of two such chains, and the output is kept in f32 registers, to which each
+// tile of 64 keys is added by an ordinary rounded addition.
 //
-// Work.  A CTA of eight warps owns 128 queries of one head and walks 32-key tiles (three parts of 64 would not fit
-// shared memory twice): bulk copies bring a tile as f32, two tiles ahead; all warps split it into three bf16
-// tiles each of K and V that ldmatrix reads without conflicts, double-buffered; in each sub-core one warp splits the next tile
-// before it works on the current one and the other after it, so that the splitting runs beside the tensor core.  A warp
-// owns 16 rows from the scores to the output; Q's fragments and the output stay in its registers, the weights go from
-// accumulator to operand layout without leaving them.  Causal, Llama-3-8B heads, against the streaming kernel:
-// 2048 tokens 1679 -> 673 us (51 TFLOP/s of f32 products, 307 of the tensor core's 568 at this instruction), 512
-// tokens 152 -> 93, 150 tokens 29.5 -> 28.3; unmasked 1448 tokens 1567 -> 774.  What is left is the tensor pipe (more
-// than half the time) and the softmax, splitting and fragment loads beside it.
+// Measured, Llama-3-8B heads, against mma.sync products with the splitting in every CTA (bound by that instruction, 568
+// TFLOP/s, and by the splitting): causal, 2048 tokens 674 -> 184 us (187 TFLOP/s of f32 products, 1.1 PFLOP/s of
+// bf16 ones), 512 tokens 95 -> 38, 150 tokens 28.6 -> 18.7; unmasked 1448 tokens 774 -> 182.
 #include "attention_prefill_f32.cuh"
+
+#include <algorithm>
 
 namespace luxcuda {
 
@@ -44,42 +50,42 @@ namespace pmma {
 using namespace tcptx;
 
 constexpr int D = 128;                    // head size
-constexpr int BM = 128;                   // queries per CTA: 16 per warp
-constexpr int BN = 32;                    // keys per tile
-constexpr int WARPS = 8, THREADS = WARPS * 32;
-constexpr int F32_TILE = BN * D * 4;      // K or V of a tile as it arrives
-constexpr int PART = BN * D * 2;          // one part of it: 32 rows of 256 bytes, 16-byte chunks ^ (row & 7)
-// two slots of {K, V} in f32, two buffers of {K h, m, l, V h, m, l}, two mbarriers, abort flag, bad flag, tiny flag
-constexpr int OFF_F32 = 0, SLOT = 2 * F32_TILE, OFF_BUF = 2 * SLOT, BUF_BYTES = 6 * PART;
-constexpr int OFF_BAR = OFF_BUF + 2 * BUF_BYTES;
-constexpr int SMEM = OFF_BAR + 64 + 128;
+constexpr int BM = 128;                   // queries per CTA
+constexpr int BN = 64;                    // keys per tile
+constexpr int THREADS = 384;              // three warpgroups
+// registers per thread of the softmax, output and copy / issue warpgroups; their sum is three times the 168 of the launch
+constexpr int REGS_S = 208, REGS_O = 216, REGS_C = 80, REGS = 168;
+constexpr int PART = 64 * D;              // bytes of one part of a CTA's half tile: K 32 keys x 128, V 64 keys x 64 columns
+constexpr int SLOT = 3 * PART;            // K or V of a tile, one CTA's half
+constexpr int SLOTS = 7;
+constexpr size_t TILE_BYTES = 4 * SLOT;   // scratch per tile: K of rank 0, 1, V of rank 0, 1
+// Q's l part, ring, two rows of factors, denominators and maxima, barriers and flags
+constexpr int OFF_QL = 0, OFF_RING = BM * D * 2, OFF_ALPHA = OFF_RING + SLOTS * SLOT, OFF_STAT = OFF_ALPHA + 2 * BM * 4;
+constexpr int OFF_BAR = OFF_STAT + 2 * BM * 4, OFF_FLAG = OFF_BAR + 256;
+constexpr int SMEM = OFF_FLAG + 64 + 1024;
+constexpr int OUT_PITCH = D + 4;          // floats between the rows of the output in shared memory (over the ring)
+// tensor memory columns
+constexpr uint32_t T_QH = 0, T_QM = 64, T_S = 128, T_P = 256, T_O = 384;
 constexpr float NEG = -3.0e38f, LN2 = 0.6931471805599453f;
 constexpr float RAISE = 8.0f;             // the running maximum is raised when a score passes it by more: weights below 2^8
 constexpr float P_SCALE = 0x1p30f;        // of the weights before they are split
+constexpr float CHAIN_LOSS = 0x1p-24f;    // taken off half of the denominator: what the weighted sum's chains lose on average
 constexpr uint32_t TOO_LARGE = (127u + 60u) << 23;           // |x| >= 2^60, infinity or NaN, as bits
 constexpr uint32_t TOO_SMALL = (127u - 100u) << 23;          // 0 < |v| < 2^-100
+constexpr uint32_t FLAG_BAD = 1u, FLAG_TINY = 2u;            // of a tile of K or V
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void ldm4(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldm4t(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+using prefill::add2;
+using prefill::ex2;
+using prefill::mul2;
+using prefill::pair;
+using prefill::unpair;
+
+__device__ __forceinline__ uint32_t pack(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
 }
 // two values as pairs of their parts, the first in the low half; the two differences are exact
 __device__ __forceinline__ void split3(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-    auto pack = [](float x, float y) {
-        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
-        return *reinterpret_cast<const uint32_t*>(&v);
-    };
     h = pack(a, b);
     a -= __uint_as_float(h << 16);
     b -= __uint_as_float(h & 0xffff0000u);
@@ -88,309 +94,459 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& h, uint32_t& 
 }
 __device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 
-__global__ void __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const PrefillArgs p) {
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// ---- cta_group::2 wrappers: 256 rows, 128 of each CTA --------------------------------------------------
+__host__ __device__ constexpr uint32_t idesc2(int n, bool b_mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | (16u << 24);
+}
+__device__ __forceinline__ void mma2_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void mma2_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// arrives on the barrier of this offset in both CTAs when all products issued so far are complete
+__device__ __forceinline__ void commit2(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+// the same offset in the pair's first CTA
+__device__ __forceinline__ uint32_t in_leader(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+// Only tensor-memory reads and writes, already waited for, are ordered by it: a release at cluster scope would
+// first wait for every store of the thread (600 cycles and more, three times a tile: 235 -> 184 us at 2048 tokens without).
+__device__ __forceinline__ void arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// The parts of a tile of K (blockIdx.z 0) or V (1), rows past the end as zeros, in the layout of the ring's slots:
+//   K, rank r (keys 32 r ..): [part][64 columns][32 keys] rows of 128 bytes      (K-major operand, 128-byte swizzle)
+//   V, rank r (columns 64 r ..): [part][64 keys] rows of 128 bytes               (MN-major operand, 128-byte swizzle)
+// 4 bytes are read and 6 written per element: 2048 keys x 8 heads 42 MB.
+__global__ void __launch_bounds__(256) lux_attn_split_kv(const float* __restrict__ k, const float* __restrict__ v, unsigned char* __restrict__ parts,
+                                                         uint32_t* __restrict__ flags, uint32_t bk0, uint32_t kv_len, uint32_t kv_stride) {
+    __shared__ uint32_t seen;
+    const uint32_t t = blockIdx.x, bk = blockIdx.y, is_v = blockIdx.z, tid = threadIdx.x;
+    if (tid == 0) seen = 0u;
+    __syncthreads();
+    pdl_launch_dependents();
+    pdl_wait();
+    const float* src = (is_v ? v : k) + ((size_t)(bk0 + bk) * kv_stride + (size_t)t * BN) * D;
+    unsigned char* dst = parts + ((size_t)bk * gridDim.x + t) * TILE_BYTES + (is_v ? 2 * SLOT : 0);
+    const uint32_t nk = min((uint32_t)BN, kv_len - t * BN);
+    uint32_t top = 0u, low = 0xffffffffu;             // largest magnitude; smallest non-zero one, less 1
+    float4 x[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t e = tid + 256u * i, key = e >> 4, c = e & 15u;      // 16-byte chunk c of a row's parts: columns 8 c ..
+        x[i][0] = x[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (key < nk) {
+            x[i][0] = __ldg(reinterpret_cast<const float4*>(src + (size_t)key * D) + 2 * c);
+            x[i][1] = __ldg(reinterpret_cast<const float4*>(src + (size_t)key * D) + 2 * c + 1);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t e = tid + 256u * i, key = e >> 4, c = e & 15u;
+        uint32_t w[3][4];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float4 f = x[i][j];
+            const uint32_t b0 = abs_bits(f.x), b1 = abs_bits(f.y), b2 = abs_bits(f.z), b3 = abs_bits(f.w);
+            top = max(top, max(max(b0, b1), max(b2, b3)));
+            low = min(low, min(min(b0 - 1u, b1 - 1u), min(b2 - 1u, b3 - 1u)));
+            split3(f.x, f.y, w[0][2 * j], w[1][2 * j], w[2][2 * j]);
+            split3(f.z, f.w, w[0][2 * j + 1], w[1][2 * j + 1], w[2][2 * j + 1]);
+        }
+        const uint32_t at = is_v ? (c >> 3) * SLOT + key * 128u : (key >> 5) * SLOT + (c >> 3) * (PART / 2) + (key & 31u) * 128u;
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            *reinterpret_cast<uint4*>(dst + at + q * PART + (((c & 7u) ^ (key & 7u)) << 4)) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+    }
+    const uint32_t f = (top >= TOO_LARGE ? FLAG_BAD : 0u) | (is_v && low < TOO_SMALL - 1u ? FLAG_TINY : 0u);
+    if (f) atomicOr(&seen, f);
+    __syncthreads();
+    if (tid == 0) flags[((size_t)bk * gridDim.x + t) * 2 + is_v] = seen;
+}
+
+struct Geometry {
+    const unsigned char* parts;  // of the KV heads bk0 .. bk0 + nbk (batch x kv_heads), all_tiles tiles each
+    const uint32_t* flags;
+    uint32_t bk0, nbk, all_tiles;
+    uint32_t by_head;            // pairs are two heads (their number per KV head is even), else two blocks of queries
+    uint32_t units, levels;      // pairs per KV head and block of queries; blocks of queries (pairs of them)
+};
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const PrefillArgs p, const Geometry geo) {
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const uint32_t sb = smem_u32(smem);
-    const uint32_t bars = sb + OFF_BAR;           // one per slot
-    volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_BAR + 16);
-    volatile uint32_t* bad_flag = abort_flag + 1;
-    volatile uint32_t* tiny_flag = abort_flag + 2;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    float* alpha_s = reinterpret_cast<float*>(smem + OFF_ALPHA);
+    float* stat = reinterpret_cast<float*>(smem + OFF_STAT);
+    const uint32_t bars = sb + OFF_BAR;
+    auto kv_full = [&](uint32_t s) { return bars + 8u * s; };
+    auto kv_empty = [&](uint32_t s) { return bars + 8u * (SLOTS + s); };
+    const uint32_t s_full = bars + 8u * (2 * SLOTS), s_free = s_full + 8u, p_ready = s_full + 16u, o_full = s_full + 24u, o_free = s_full + 32u,
+                   alpha_ready = s_full + 40u;    // two of these
+    volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_FLAG);
+    volatile uint32_t* abort_flag = flag;
+    volatile uint32_t* seen = flag + 1;           // FLAG_BAD, FLAG_TINY of what this CTA reads
+    volatile uint32_t* peer_bad = flag + 2;
+    uint32_t* tmem_slot = const_cast<uint32_t*>(flag + 3);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cluster_ctarank();
 
     pdl_launch_dependents();
     // blocks of late queries see the most keys under a causal mask: they come first, so that the last
-    // wave is made of short ones.  Neighbouring CTAs are heads of one KV head and share its tiles in L2.
-    const uint32_t bh = p.batch * p.heads;
-    const uint32_t qb = p.q_blocks - 1u - blockIdx.x / bh, rest = blockIdx.x % bh;
-    const uint32_t h = rest % p.heads, b = rest / p.heads, kvh = h / p.group;
-    const uint32_t q0 = qb * BM, rows = min((uint32_t)BM, p.seq_q - q0);
+    // wave is made of short ones.  Neighbouring pairs are heads of one KV head and share its tiles in L2.
+    const uint32_t per_level = geo.nbk * geo.units;
+    const uint32_t level = geo.levels - 1u - (blockIdx.x >> 1) / per_level, rest = (blockIdx.x >> 1) % per_level;
+    const uint32_t unit = rest % geo.units, bkl = rest / geo.units, bk = geo.bk0 + bkl, b = bk / p.kv_heads;
+    const uint32_t h = bk % p.kv_heads * p.group + (geo.by_head ? 2u * unit + rank : unit);
+    const uint32_t qb = geo.by_head ? level : 2u * level + rank;
+    const uint32_t q0 = qb * BM, rows = q0 < p.seq_q ? min((uint32_t)BM, p.seq_q - q0) : 0u;
     auto row_len = [&](uint32_t qi) { return p.causal ? min(p.causal_base + qi + 1u, p.kv_len) : p.kv_len; };
-    const uint32_t lmax = row_len(q0 + rows - 1u);
-    const uint32_t tiles = (lmax + BN - 1u) / BN;
-    const float* kbase = p.k + ((size_t)b * p.kv_heads + kvh) * p.kv_stride * D;
-    const float* vbase = p.v + ((size_t)b * p.kv_heads + kvh) * p.kv_stride * D;
+    const uint32_t lmax = rows ? row_len(q0 + rows - 1u) : 0u, own_tiles = (lmax + BN - 1u) / BN;
+    const uint32_t pair_last = min(p.seq_q, (geo.by_head ? level + 1u : 2u * level + 2u) * BM) - 1u;
+    const uint32_t tiles = (row_len(pair_last) + BN - 1u) / BN;            // the pair walks them together
+    const unsigned char* tile0 = geo.parts + (size_t)bkl * geo.all_tiles * TILE_BYTES + rank * SLOT;
 
-    auto load_tile = [&](uint32_t t) {            // tile t goes to slot t & 1
-        const uint32_t t0 = t * BN, bytes = min((uint32_t)BN, lmax - t0) * D * 4u, bar = bars + 8u * (t & 1u);
-        const uint32_t dst = sb + OFF_F32 + (t & 1u) * SLOT;
-        mbar_expect_tx(bar, 2u * bytes);
-        bulk_g2s(dst, kbase + (size_t)t0 * D, bytes, bar);
-        bulk_g2s(dst + F32_TILE, vbase + (size_t)t0 * D, bytes, bar);
-    };
     if (tid == 0) {
-        mbar_init(bars, 1u);
-        mbar_init(bars + 8u, 1u);
+        for (uint32_t s = 0; s < SLOTS; s++) {
+            mbar_init(kv_full(s), rank == 0 ? 2u : 1u);         // the first CTA's: both halves
+            mbar_init(kv_empty(s), 1u);
+        }
+        mbar_init(s_full, 1u);
+        mbar_init(s_free, 8u);                    // four warps of each CTA
+        mbar_init(p_ready, 8u);
+        mbar_init(o_full, 1u);
+        mbar_init(o_free, 8u);
+        mbar_init(alpha_ready, 4u);
+        mbar_init(alpha_ready + 8u, 4u);
         *abort_flag = 0u;
-        *bad_flag = 0u;
-        *tiny_flag = 0u;
+        *seen = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();                              // the flags are clear before a warp may raise one over its rows of Q
+    if (warp == 8) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot, quad = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     pdl_wait();
-    if (tid == 0) {
-        if (tiles > 0) load_tile(0);
-        if (tiles > 1) load_tile(1);
-    }
-    auto landed = [&](uint32_t t) { return warp_wait(bars + 8u * (t & 1u), (t >> 1) & 1u, abort_flag, lane); };
 
-    // ---- Q: this lane's fragments of rows g and g + 8 of the warp's 16, scaled and split ------------------
-    uint32_t qp[3][8][4];
-    float m[2], l[2];
-    uint32_t len[2];
+    // the ring: K0, K1, V0, K2, V1, ... in both CTAs, in the order in which the products read them
+    auto slot_at = [&](uint32_t i) { return sb + OFF_RING + (i % SLOTS) * SLOT; };
+    const uint32_t entries = 2u * tiles;
+    auto request = [&](uint32_t i) {              // entry i: K (i + 1) / 2 for odd i (the last one V), else V i / 2 - 1; K 0 first
+        const bool is_k = i == 0 || ((i & 1u) && i + 1u < entries);
+        const uint32_t t = i == 0 ? 0u : is_k ? (i + 1u) / 2u : i + 1u < entries ? i / 2u - 1u : tiles - 1u;
+        const uint32_t bar = kv_full(i % SLOTS);
+        mbar_expect_tx(bar, SLOT);
+        bulk_g2s(slot_at(i), tile0 + (size_t)t * TILE_BYTES + (is_k ? 0 : 2 * SLOT), SLOT, bar);
+    };
+    if (warp == 9 && lane == 0)
+        for (uint32_t i = 0; i < min(entries, (uint32_t)SLOTS); i++) request(i);
+
+    // ---- Q: rows on lanes, scaled and split; warps 0..3 take columns 0..63, warps 4..7 the others ---------
+    const uint32_t row = (uint32_t)((warp & 3) * 32 + lane);
+    uint32_t found = 0u;
+    if (warp < 8) {
+        const int half = warp >> 2;
+        uint32_t qh[32], qm[32];
+        const float* src = p.q + (((size_t)b * p.heads + h) * p.seq_q + q0 + min(row, max(rows, 1u) - 1u)) * D + half * 64;
+        float4 x[16];
 #pragma unroll
-    for (int r = 0; r < 2; r++) {                     // row half r: columns 8 j + 2 t4 and the next
-        const uint32_t row = (uint32_t)(warp * 16 + g + 8 * r);
-        len[r] = row < rows ? row_len(q0 + row) : 0u;                // a padding row sees nothing and is not written
-        const float* src = p.q + (((size_t)b * p.heads + h) * p.seq_q + q0 + min(row, rows - 1u)) * D + 2 * t4;
-        float2 x[16];
+        for (int j = 0; j < 16; j++) x[j] = rows ? __ldg(reinterpret_cast<const float4*>(src) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
         uint32_t top = 0u;
+        unsigned char* ql = smem + OFF_QL + half * (BM * 128) + row * 128u;
 #pragma unroll
-        for (int j = 0; j < 16; j++) x[j] = __ldg(reinterpret_cast<const float2*>(src + 8 * j));
+        for (int c = 0; c < 8; c++) {
+            uint32_t l[4];
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            x[j] = make_float2(x[j].x * p.qscale, x[j].y * p.qscale);
-            top = max(top, max(abs_bits(x[j].x), abs_bits(x[j].y)));
-            const int f = j >> 1, e = 2 * (j & 1) + r;
-            split3(x[j].x, x[j].y, qp[0][f][e], qp[1][f][e], qp[2][f][e]);
+            for (int j = 0; j < 2; j++) {
+                const float4 v = x[2 * c + j];
+                const float4 y = make_float4(v.x * p.qscale, v.y * p.qscale, v.z * p.qscale, v.w * p.qscale);
+                top = max(top, max(max(abs_bits(y.x), abs_bits(y.y)), max(abs_bits(y.z), abs_bits(y.w))));
+                const int e = 4 * c + 2 * j;
+                split3(y.x, y.y, qh[e], qm[e], l[2 * j]);
+                split3(y.z, y.w, qh[e + 1], qm[e + 1], l[2 * j + 1]);
+            }
+            *reinterpret_cast<uint4*>(ql + (((uint32_t)c ^ (row & 7u)) << 4)) = make_uint4(l[0], l[1], l[2], l[3]);
         }
-        if (top >= TOO_LARGE) *bad_flag = 1u;
-        m[r] = NEG;
-        l[r] = 0.0f;
+        tmem_st32(quad + T_QH + half * 32, qh);
+        tmem_st32(quad + T_QM + half * 32, qm);
+        tmem_st_wait();
+        if (top >= TOO_LARGE) found = FLAG_BAD;
     }
-    float o[16][4];                                   // columns 8 n + 2 t4 (+ 1) of rows g (0, 1) and g + 8 (2, 3)
+    for (uint32_t i = tid; i < 2u * own_tiles; i += THREADS) found |= geo.flags[(size_t)bkl * geo.all_tiles * 2u + i];
+    if (found) atomicOr(const_cast<uint32_t*>(seen), found);
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {                               // a CTA without rows has nothing to lose
+        uint32_t there;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(const_cast<uint32_t*>(peer_bad))), "r"(rank ^ 1u));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(there), "r"((*seen & FLAG_BAD) || !rows ? 1u : 0u) : "memory");
+    }
+    cluster_sync_all();
+    tc_fence_after();
+    const bool bad = (*seen & FLAG_BAD) || !rows;
+    // both start over: no products.  One of them: the pair works on, for the other's sake.
+    const uint32_t walk = bad && *peer_bad ? 0u : tiles;
+    float* out_s = reinterpret_cast<float*>(smem + OFF_RING);
+    bool low = false;                             // an output that V's lost parts could matter to
+    static_assert(REGS_S + REGS_O + REGS_C <= 3 * REGS, "what the launch has");
+    if (warp >= 8) {
+        regs_dec<REGS_C>();
+        if (warp == 9) {
+            if (lane == 0) {
+                for (uint32_t i = SLOTS; walk && i < entries; i++) {
+                    if (!mbar_wait_relaxed(kv_empty(i % SLOTS), (i / SLOTS - 1u) & 1u, abort_flag)) break;
+                    request(i);
+                }
+                // nobody else waits for what was requested above
+                for (uint32_t i = 0; !walk && i < min(entries, (uint32_t)SLOTS); i++) mbar_wait(kv_full(i), 0u, abort_flag);
+            }
+        } else if (warp == 8 && rank == 0) {
+            if (elect_one()) {
+                constexpr uint32_t id_s = idesc2(BN, false), id_o = idesc2(D, true);
+                uint32_t i = 0;                   // ring entry
+                auto take = [&]() { return mbar_wait(kv_full(i % SLOTS), (i / SLOTS) & 1u, abort_flag); };
+                auto scores = [&]() {
+                    const uint64_t kd = make_kmajor_sw128_desc(slot_at(i)), ld = make_kmajor_sw128_desc(sb + OFF_QL);
+                    tc_fence_after();
 #pragma unroll
-    for (int n = 0; n < 16; n++)
+                    for (int c = 0; c < 2; c++) { // columns 64 c .. of the head
+                        const uint32_t d = tmem + T_S + c * BN;
+                        // l h, h l, m m, m h, h m, h h
 #pragma unroll
-        for (int e = 0; e < 4; e++) o[n][e] = 0.0f;
-
-    // ---- tile t, f32 -> parts in buffer t & 1: warps 0..3 take eight rows of K each, 4..7 of V -----------------
-    auto convert = [&](uint32_t t) {
-        const uint32_t nk = min((uint32_t)BN, lmax - t * BN);
-        const unsigned char* src = smem + OFF_F32 + (t & 1u) * SLOT + warp * 8 * (D * 4) + lane * 16;
-        unsigned char* buf = smem + OFF_BUF + (t & 1u) * BUF_BYTES + (warp >> 2) * (3 * PART);
-        uint32_t top = 0u, low = 0xffffffffu;         // largest magnitude; smallest non-zero one, less 1
-#pragma unroll 4
-        for (int i = 0; i < 8; i++) {
-            const int key = (warp & 3) * 8 + i;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if ((uint32_t)key < nk) v = *reinterpret_cast<const float4*>(src + i * (D * 4));
-            const uint32_t b0 = abs_bits(v.x), b1 = abs_bits(v.y), b2 = abs_bits(v.z), b3 = abs_bits(v.w);
-            top = max(top, max(max(b0, b1), max(b2, b3)));
-            low = min(low, min(min(b0 - 1u, b1 - 1u), min(b2 - 1u, b3 - 1u)));
-            uint2 w[3];
-            split3(v.x, v.y, w[0].x, w[1].x, w[2].x);
-            split3(v.z, v.w, w[0].y, w[1].y, w[2].y);
-            const int at = key * 256 + (((lane >> 1) ^ (key & 7)) << 4) + (lane & 1) * 8;
+                        for (int s = 0; s < 4; s++)
+                            mma2_ss(d, ld + (uint64_t)(c * (BM * 128 / 16) + 2 * s), kd + (uint64_t)(c * (PART / 32) + 2 * s), id_s, s != 0);
 #pragma unroll
-            for (int c = 0; c < 3; c++) *reinterpret_cast<uint2*>(buf + c * PART + at) = w[c];
-        }
-        if (top >= TOO_LARGE) *bad_flag = 1u;
-        if (low < TOO_SMALL - 1u && warp >= WARPS / 2) *tiny_flag = 1u;
-    };
-    // c += a b without its h h part, for two independent pairs at once (their chains of five are interleaved)
-    auto mma_rest = [&](float (&c0)[4], float (&c1)[4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4],
-                        const uint32_t (&b0)[3][2], const uint32_t (&b1)[3][2]) {
-        mma(c0, al, b0[0][0], b0[0][1]);
-        mma(c1, al, b1[0][0], b1[0][1]);
-        mma(c0, ah, b0[2][0], b0[2][1]);
-        mma(c1, ah, b1[2][0], b1[2][1]);
-        mma(c0, am, b0[1][0], b0[1][1]);
-        mma(c1, am, b1[1][0], b1[1][1]);
-        mma(c0, am, b0[0][0], b0[0][1]);
-        mma(c1, am, b1[0][0], b1[0][1]);
-        mma(c0, ah, b0[1][0], b0[1][1]);
-        mma(c1, ah, b1[1][0], b1[1][1]);
-    };
-
-    // ---- one tile's work of a warp ---------------------------------------------------------------
-    const uint32_t last_len = row_len(q0 + min((uint32_t)(warp * 16 + 15), rows - 1u));
-    const uint32_t first_len = row_len(q0 + min((uint32_t)(warp * 16), rows - 1u));
-    const bool live = (uint32_t)(warp * 16) < rows;
-    auto work = [&](uint32_t t) {
-        const uint32_t t0 = t * BN;
-        if (!live || t0 >= last_len) return;            // no row of the warp sees the tile
-        const uint32_t buf = sb + OFF_BUF + (t & 1u) * BUF_BYTES;
-        // scores: B fragments of 8 keys x 32 columns per ldmatrix (rows = keys, four 16-byte chunks), two groups of
-        // 8 keys at a time
-        float s[4][4];
-        const uint32_t krow = buf + (uint32_t)(lane & 7) * 256u, kchunk = (uint32_t)(lane >> 3), kx = (uint32_t)(lane & 7);
+                        for (int o = 1; o < 6; o++) {
+                            const int a = o == 2 || o == 3 ? 1 : 0, w = o == 1 ? 2 : o == 2 || o == 4 ? 1 : 0;
 #pragma unroll
-        for (int n = 0; n < 4; n += 2) {
-            float rest[2][4];
-#pragma unroll
-            for (int i = 0; i < 2; i++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) s[n + i][e] = rest[i][e] = 0.0f;
-#pragma unroll
-            for (int d = 0; d < 4; d++) {
-                uint32_t kf[2][3][4];
-#pragma unroll
-                for (int i = 0; i < 2; i++)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) ldm4(krow + (uint32_t)(c * PART + (n + i) * 8 * 256) + (((kchunk + 4u * d) ^ kx) << 4), kf[i][c]);
-#pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    const int f = 2 * d + k;
-                    float c[2][4] = {};
-                    uint32_t bf[2][3][2];
-#pragma unroll
-                    for (int i = 0; i < 2; i++) {
-#pragma unroll
-                        for (int part = 0; part < 3; part++) {
-                            bf[i][part][0] = kf[i][part][2 * k];
-                            bf[i][part][1] = kf[i][part][2 * k + 1];
+                            for (int s = 0; s < 4; s++)
+                                mma2_ts(d, tmem + (a ? T_QM : T_QH) + c * 32 + s * 8, kd + (uint64_t)(w * (PART / 16) + c * (PART / 32) + 2 * s), id_s, 1u);
                         }
-                        mma(c[i], qp[0][f], bf[i][0][0], bf[i][0][1]);
                     }
-                    mma_rest(rest[0], rest[1], qp[0][f], qp[1][f], qp[2][f], bf[0], bf[1]);
+                    commit2(s_full);
+                    commit2(kv_empty(i % SLOTS));
+                    i++;
+                };
+                auto weighted = [&]() {
+                    // MN-major: rows of 128 bytes are keys, eight of them a swizzle atom, one atom column wide
+                    const uint64_t vd = make_kmajor_sw128_desc(slot_at(i));
+                    tc_fence_after();
 #pragma unroll
-                    for (int i = 0; i < 2; i++)
+                    for (int o = 0; o < 6; o++) {
+                        const int a = o == 0 ? 2 : o == 2 || o == 3 ? 1 : 0, w = o == 1 ? 2 : o == 2 || o == 4 ? 1 : 0;
 #pragma unroll
-                        for (int e = 0; e < 4; e++) s[n + i][e] += c[i][e];
+                        for (int s = 0; s < 4; s++)
+                            mma2_ts(tmem + T_O, tmem + T_P + a * 32 + s * 8, vd + (uint64_t)(w * (PART / 16) + s * (16 * 128 / 16)), id_o, (o | s) != 0);
+                    }
+                    commit2(o_full);
+                    commit2(kv_empty(i % SLOTS));
+                    i++;
+                };
+                bool ok = walk > 0 && take();
+                if (ok) scores();
+                for (uint32_t t = 0; ok && t < walk; t++) {
+                    if (t + 1 < walk) {
+                        ok = take() && mbar_wait(s_free, t & 1u, abort_flag);
+                        if (!ok) break;
+                        scores();
+                    }
+                    ok = take() && mbar_wait(p_ready, t & 1u, abort_flag) && (t == 0 || mbar_wait(o_free, (t - 1u) & 1u, abort_flag));
+                    if (!ok) break;
+                    weighted();
                 }
             }
-#pragma unroll
-            for (int i = 0; i < 2; i++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) s[n + i][e] += rest[i][e];
-        }
-        const bool edge = t0 + BN > first_len;
-        float mt[2] = {NEG, NEG};
-#pragma unroll
-        for (int n = 0; n < 4; n++) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                if (edge && t0 + 8 * n + 2 * t4 + (e & 1) >= len[e >> 1]) s[n][e] = -__int_as_float(0x7f800000);
-                mt[e >> 1] = fmaxf(mt[e >> 1], s[n][e]);
-            }
-        }
-        bool up = false;
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            mt[r] = fmaxf(mt[r], __shfl_xor_sync(0xffffffffu, mt[r], 1));
-            mt[r] = fmaxf(mt[r], __shfl_xor_sync(0xffffffffu, mt[r], 2));
-            up |= mt[r] > m[r] + RAISE;
-        }
-        if (__any_sync(0xffffffffu, up)) {
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const float mn = fmaxf(m[r], mt[r]), alpha = ex2(m[r] - mn);
-                m[r] = mn;
-                l[r] *= alpha;
-#pragma unroll
-                for (int n = 0; n < 16; n++) {
-                    o[n][2 * r] *= alpha;
-                    o[n][2 * r + 1] *= alpha;
+        } else if (warp == 8) {
+            if (lane == 0)
+                for (uint32_t i = 0; i < (walk ? entries : min(entries, (uint32_t)SLOTS)); i++) {
+                    if (!mbar_wait(kv_full(i % SLOTS), (i / SLOTS) & 1u, abort_flag)) break;
+                    arrive_cluster(in_leader(kv_full(i % SLOTS)));
                 }
-            }
         }
-        uint32_t wp[3][2][4];                          // the weights' parts as A fragments of 16 keys
-        float sum[2] = {0.f, 0.f};
-#pragma unroll
-        for (int n = 0; n < 4; n++) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) s[n][e] = ex2(s[n][e] - m[e >> 1]);
-            sum[0] += s[n][0] + s[n][1];
-            sum[1] += s[n][2] + s[n][3];
-            const int f = n >> 1, e = 2 * (n & 1);
-            split3(s[n][0] * P_SCALE, s[n][1] * P_SCALE, wp[0][f][e], wp[1][f][e], wp[2][f][e]);
-            split3(s[n][2] * P_SCALE, s[n][3] * P_SCALE, wp[0][f][e + 1], wp[1][f][e + 1], wp[2][f][e + 1]);
-        }
-        l[0] += sum[0];
-        l[1] += sum[1];
-        // weighted sum: B fragments of 16 keys x 16 columns per transposing ldmatrix
-        const uint32_t vrow = buf + (uint32_t)(3 * PART) + (uint32_t)(lane & 15) * 256u, vchunk = (uint32_t)(lane >> 4), vx = (uint32_t)(lane & 7);
-#pragma unroll
-        for (int n2 = 0; n2 < 8; n2++) {               // 16 columns
-            float c[2][2][4] = {}, rest[2][4] = {};
-#pragma unroll
-            for (int k = 0; k < 2; k++) {              // 16 keys
-                uint32_t vf[3][4], bf[2][3][2];
-#pragma unroll
-                for (int part = 0; part < 3; part++) ldm4t(vrow + (uint32_t)(part * PART + 16 * k * 256) + (((vchunk + 2u * n2) ^ vx) << 4), vf[part]);
+        __syncwarp();
+        cluster_sync_all();
+        regs_inc<REGS>();
+    } else if (warp < 4) {
+        // ---- softmax: this thread's row of every tile ------------------------------------------------
+        regs_inc<REGS_S>();
+        const uint32_t len = row < rows ? row_len(q0 + row) : 0u;        // a padding row sees nothing and is not written
+        const uint32_t free_bar = in_leader(s_free), ready_bar = in_leader(p_ready);
+        float m = NEG, l = 0.0f;
+        for (uint32_t t = 0; t < walk; t++) {
+            if (!warp_wait(s_full, t & 1u, abort_flag, lane)) break;
+            const bool own = t < own_tiles;
+            uint64_t s2[BN / 2];
+            tc_fence_after();
+            if (own) {
+                uint32_t a[2][32], c[2][32];
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
-#pragma unroll
-                    for (int part = 0; part < 3; part++) {
-                        bf[i][part][0] = vf[part][2 * i];
-                        bf[i][part][1] = vf[part][2 * i + 1];
-                    }
-                    mma(c[i][k], wp[0][k], bf[i][0][0], bf[i][0][1]);
+                    tmem_ld32(quad + T_S + 32 * i, a[i]);
+                    tmem_ld32(quad + T_S + BN + 32 * i, c[i]);
                 }
-                mma_rest(rest[0], rest[1], wp[0][k], wp[1][k], wp[2][k], bf[0], bf[1]);
-            }
+                tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 2; i++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) o[2 * n2 + i][e] += c[i][0][e] + (c[i][1][e] + rest[i][e]);
-        }
-    };
-
-    // ---- rounds: in round t the warps split tile t + 1 and work on tile t, and tile t + 2 is on its way ---------
-    bool ok = true;
-    uint32_t asked = min(2u, tiles);                   // tiles requested so far
-    if (tiles) {
-        bool here = landed(0);
-        if (here) convert(0);
-        ok = !__syncthreads_or(!here || *bad_flag != 0u);
-        for (uint32_t t = 0; ok && t < tiles; t++) {
-            const bool more = t + 1 < tiles;
-            if (t + 2 < tiles) {                       // slot t & 1 was split in the last round
-                if (tid == 0) load_tile(t + 2);
-                asked = t + 3;
+                for (int j = 0; j < BN / 2; j++)
+                    s2[j] = add2(pair(__uint_as_float(a[j >> 4][2 * (j & 15)]), __uint_as_float(a[j >> 4][2 * (j & 15) + 1])),
+                                 pair(__uint_as_float(c[j >> 4][2 * (j & 15)]), __uint_as_float(c[j >> 4][2 * (j & 15) + 1])));
             }
-            here = true;
-            if (more && warp < WARPS / 2 && (here = landed(t + 1))) convert(t + 1);
-            work(t);
-            if (more && warp >= WARPS / 2 && (here = landed(t + 1))) convert(t + 1);
-            if (__syncthreads_or(!here || *bad_flag != 0u)) ok = false;
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_cluster(free_bar);
+            float alpha = 1.0f;
+            uint32_t wh[32], wm[32], wl[32];
+            if (own) {
+                const uint32_t t0 = t * BN;
+                float s[BN];
+#pragma unroll
+                for (int j = 0; j < BN / 2; j++) unpair(s2[j], s[2 * j], s[2 * j + 1]);
+                if (t0 + BN > len) {
+#pragma unroll
+                    for (int j = 0; j < BN; j++)
+                        if (t0 + j >= len) s[j] = -__int_as_float(0x7f800000);
+                }
+                float mt[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) mt[j] = fmaxf(s[j], s[j + 4]);
+#pragma unroll
+                for (int j = 8; j < BN; j++) mt[j & 3] = fmaxf(mt[j & 3], s[j]);
+                const float top = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3]));
+                if (top > m + RAISE) {
+                    alpha = ex2(m - top);
+                    m = top;
+                    l *= alpha;
+                }
+                const uint64_t m2 = pair(-m, -m), scale2 = pair(P_SCALE, P_SCALE);
+                uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+                for (int j = 0; j < BN / 2; j++) {
+                    float x, y;
+                    unpair(add2(pair(s[2 * j], s[2 * j + 1]), m2), x, y);
+                    const uint64_t e = pair(ex2(x), ex2(y));
+                    sum[j & 3] = add2(sum[j & 3], e);
+                    unpair(mul2(e, scale2), x, y);
+                    split3(x, y, wh[j], wm[j], wl[j]);
+                }
+                float x, y;
+                unpair(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), x, y);
+                l = fmaf(x, 1.0f - CHAIN_LOSS, l + y);
+            }
+            // the weighted sum before this one has read its weights
+            if (t && !warp_wait(o_full, (t - 1u) & 1u, abort_flag, lane)) break;
+            tc_fence_after();
+            alpha_s[(t & 1u) * BM + row] = alpha;
+            if (own) {
+                tmem_st32(quad + T_P, wh);
+                tmem_st32(quad + T_P + 32, wm);
+                tmem_st32(quad + T_P + 64, wl);
+                tmem_st_wait();
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(alpha_ready + 8u * (t & 1u));
+                arrive_cluster(ready_bar);
+            }
         }
+        stat[row] = l;
+        stat[BM + row] = m;
+        __syncwarp();
+        cluster_sync_all();
+        regs_dec<REGS>();
     } else {
-        ok = !__syncthreads_or(*bad_flag != 0u);
-    }
+        // ---- the output: this thread's row ------------------------------------------------------------
+        regs_inc<REGS_O>();
+        const uint32_t free_bar = in_leader(o_free);
+        uint64_t o[D / 2];
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
-        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
-    }
-    if (ok && *tiny_flag) {                            // the same for all: last written before the last round's barrier
-        bool low = false;
+        for (int j = 0; j < D / 2; j++) o[j] = 0ull;
+        for (uint32_t t = 0; t < walk; t++) {
+            if (!warp_wait(alpha_ready + 8u * (t & 1u), (t >> 1) & 1u, abort_flag, lane) || !warp_wait(o_full, t & 1u, abort_flag, lane)) break;
+            tc_fence_after();
+            if (t < own_tiles) {
+                const float alpha = alpha_s[(t & 1u) * BM + row];
+                if (__any_sync(0xffffffffu, alpha != 1.0f)) {
+                    const uint64_t a2 = pair(alpha, alpha);
 #pragma unroll
-        for (int r = 0; r < 2; r++)
+                    for (int j = 0; j < D / 2; j++) o[j] = mul2(o[j], a2);
+                }
 #pragma unroll
-            for (int n = 0; n < 16; n++) {
-                const float least = l[r] * (P_SCALE * 0x1p-100f);
-                low |= fabsf(o[n][2 * r]) < least || fabsf(o[n][2 * r + 1]) < least;
+                for (int i = 0; i < 4; i += 2) {
+                    uint32_t c[2][32];
+                    tmem_ld32(quad + T_O + 32 * i, c[0]);
+                    tmem_ld32(quad + T_O + 32 * i + 32, c[1]);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        o[16 * i + j] = add2(o[16 * i + j], pair(__uint_as_float(c[j >> 4][2 * (j & 15)]), __uint_as_float(c[j >> 4][2 * (j & 15) + 1])));
+                }
             }
-        ok = !__syncthreads_or(low);
-    }
-    if (!ok) {
-        // values out of range: the block starts over on the f32 pipe; or a bounded wait gave up: report it, and give
-        // copies in flight time to land.  Nothing has been written.
-        for (uint32_t t = asked > 2u ? asked - 2u : 0u; t < asked; t++) landed(t);
-        __syncthreads();
-        if (*abort_flag) {
-            if (tid == 0 && p.status) atomicOr(p.status, p.status_wait);
-            for (int i = 0; i < 64; i++) __nanosleep(1000);
-            __syncthreads();
-        } else {
-            prefill::attend_f32(p, smem, qb, h, b);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_cluster(free_bar);
         }
+        // every product has been waited for (the last tile's here): the ring and the tensor memory are free once both CTAs are here
+        __syncwarp();
+        cluster_sync_all();
+        if (!*abort_flag) {
+#pragma unroll
+            for (int j = 0; j < D / 4; j++) {
+                float4 v;
+                unpair(o[2 * j], v.x, v.y);
+                unpair(o[2 * j + 1], v.z, v.w);
+                *reinterpret_cast<float4*>(out_s + row * OUT_PITCH + 4 * j) = v;
+            }
+        }
+        if ((*seen & FLAG_TINY) && row < rows) {
+            const float least = stat[row] * (P_SCALE * 0x1p-100f);
+#pragma unroll
+            for (int j = 0; j < D / 2; j++) {
+                float x, y;
+                unpair(o[j], x, y);
+                low |= fabsf(x) < least || fabsf(y) < least;
+            }
+        }
+        __syncwarp();
+        regs_dec<REGS>();
+    }
+    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    const bool again = __syncthreads_or(low) || bad;
+    if (*abort_flag) {
+        // a bounded wait gave up: report it, and give copies in flight time to land.  Nothing has been written.
+        if (tid == 0 && p.status) atomicOr(p.status, p.status_wait);
+        for (int i = 0; i < 64; i++) __nanosleep(1000);
+        __syncthreads();
         return;
     }
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-        const uint32_t row = (uint32_t)(warp * 16 + g + 8 * r);
-        if (row >= rows) continue;
-        const size_t orow = ((size_t)b * p.heads + h) * p.seq_q + q0 + row;
-        const bool any = l[r] > 0.0f;                  // a row without keys is zero
-#pragma unroll
-        for (int n = 0; n < 16; n++)
-            *reinterpret_cast<float2*>(p.out + orow * D + 8 * n + 2 * t4) =
-                any ? make_float2(o[n][2 * r] / l[r] * (1.0f / P_SCALE), o[n][2 * r + 1] / l[r] * (1.0f / P_SCALE)) : make_float2(0.f, 0.f);
-        if (t4 == 0 && p.lse) p.lse[orow] = any ? fmaf(m[r], LN2, logf(l[r])) : -3.402823e+38f;
+    if (!rows) return;
+    if (again) {                                  // values out of range: the block starts over on the f32 pipe
+        if (tid < prefill::PF_THREADS) prefill::attend_f32(p, smem, qb, h, b);
+        return;
     }
+    const size_t orow = ((size_t)b * p.heads + h) * p.seq_q + q0;
+    for (uint32_t r = warp; r < rows; r += THREADS / 32) {
+        const float l = stat[r];
+        float4 v = *reinterpret_cast<const float4*>(out_s + r * OUT_PITCH + 4 * lane);
+        v = l > 0.0f ? make_float4(v.x / l * (1.0f / P_SCALE), v.y / l * (1.0f / P_SCALE), v.z / l * (1.0f / P_SCALE), v.w / l * (1.0f / P_SCALE))
+                     : make_float4(0.f, 0.f, 0.f, 0.f);                          // a row without keys is zero
+        *reinterpret_cast<float4*>(p.out + (orow + r) * D + 4 * lane) = v;
+    }
+    if (p.lse && tid < (int)rows) p.lse[orow + tid] = stat[tid] > 0.0f ? fmaf(stat[BM + tid], LN2, logf(stat[tid])) : -3.402823e+38f;
 }
 
 // Every block on the f32 pipe.
@@ -403,30 +559,65 @@ __global__ void __launch_bounds__(prefill::PF_THREADS, 1) lux_attn_prefill_f32(c
     prefill::attend_f32(p, smem, p.q_blocks - 1u - blockIdx.x / bh, rest % p.heads, rest / p.heads);
 }
 
-static_assert(THREADS == prefill::PF_THREADS && BM == prefill::PF_BM && SMEM >= prefill::PF_SMEM + 128, "a block can change over");
+static_assert(THREADS >= prefill::PF_THREADS && BM == prefill::PF_BM && SMEM >= prefill::PF_SMEM + 1024, "a block can start over");
+static_assert(BM * OUT_PITCH * 4 <= SLOTS * SLOT && (2 * SLOTS + 7) * 8 <= 256, "layout of the shared memory");
+
+cudaError_t allow_smem(const void* kfn, int which, int bytes, int device) {
+    static std::atomic<bool> configured[2][64];
+    std::atomic<bool>& done = configured[which][device & 63];
+    if (done.load(std::memory_order_relaxed)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.store(true, std::memory_order_relaxed);
+    return e;
+}
 
 }  // namespace pmma
 }  // namespace
 
 LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) {
     using namespace pmma;
-    auto kfn = f32_only ? lux_attn_prefill_f32 : lux_attn_prefill_mma_f32;
-    const char* name = f32_only ? "lux_attn_prefill_f32" : "lux_attn_prefill_mma_f32";
-    static std::atomic<bool> configured[2][64];
-    std::atomic<bool>& done = configured[f32_only][ctx->device & 63];
-    if (!done.load(std::memory_order_relaxed)) {
-        cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) return map_cuda(e, name);
-        done.store(true, std::memory_order_relaxed);
-    }
     p.q_blocks = (p.seq_q + pmma::BM - 1) / pmma::BM;
-    cudaError_t e = launch_pdl(g_tune.pdl != 2, kfn, dim3(p.q_blocks * p.heads * p.batch), dim3(THREADS), (size_t)SMEM, ctx->stream, 1, p);
-    if (e != cudaSuccess) return map_cuda(e, name);
-    count_launch(name);
-    return LUX_BACKEND_OK;
+    const uint32_t keys = p.causal ? (uint32_t)std::min<uint64_t>((uint64_t)p.causal_base + p.seq_q, p.kv_len) : p.kv_len;
+    Geometry geo{};
+    geo.all_tiles = (keys + BN - 1) / BN;
+    const size_t per_bk = geo.all_tiles * (TILE_BYTES + 8);
+    const uint32_t bks = p.batch * p.kv_heads, fit = per_bk ? (uint32_t)std::min<size_t>(ctx->d_parts_bytes / per_bk, 65535) : 65535u;
+    if (f32_only || fit == 0) {                        // (128 k keys per KV head fit the scratch)
+        const char* name = "lux_attn_prefill_f32";
+        cudaError_t e = allow_smem((const void*)lux_attn_prefill_f32, 0, prefill::PF_SMEM + 128, ctx->device);
+        if (e == cudaSuccess)
+            e = launch_pdl(g_tune.pdl != 2, lux_attn_prefill_f32, dim3(p.q_blocks * p.heads * p.batch), dim3(prefill::PF_THREADS),
+                           (size_t)prefill::PF_SMEM + 128, ctx->stream, 1, p);
+        if (e != cudaSuccess) return map_cuda(e, name);
+        count_launch(name);
+        return LUX_BACKEND_OK;
+    }
+    geo.by_head = p.group % 2 == 0;
+    geo.units = geo.by_head ? p.group / 2 : p.group;
+    geo.levels = geo.by_head ? p.q_blocks : (p.q_blocks + 1) / 2;
+    const char* name = "lux_attn_prefill_mma_f32";
+    cudaError_t e = allow_smem((const void*)lux_attn_prefill_mma_f32, 1, SMEM, ctx->device);
+    // as many (sequence, KV head) pairs at a time as have their parts in the scratch (in one call all, up to 128 k keys in total)
+    for (geo.bk0 = 0; e == cudaSuccess && geo.bk0 < bks; geo.bk0 += geo.nbk) {
+        geo.nbk = std::min(fit, bks - geo.bk0);
+        unsigned char* parts = (unsigned char*)ctx->d_parts;
+        uint32_t* flags = (uint32_t*)(parts + (size_t)geo.nbk * geo.all_tiles * TILE_BYTES);
+        geo.parts = parts;
+        geo.flags = flags;
+        if (geo.all_tiles) {
+            e = launch_pdl(g_tune.pdl != 2, lux_attn_split_kv, dim3(geo.all_tiles, geo.nbk, 2), dim3(256), (size_t)0, ctx->stream, 1, p.k, p.v, parts, flags,
+                           geo.bk0, keys, p.kv_stride);
+            if (e != cudaSuccess) break;
+            count_launch("lux_attn_split_kv");
+        }
+        e = launch_pdl(g_tune.pdl != 2, lux_attn_prefill_mma_f32, dim3(2u * geo.levels * geo.nbk * geo.units), dim3(THREADS), (size_t)SMEM, ctx->stream, 1, p, geo);
+        if (e == cudaSuccess) count_launch(name);
+    }
+    return e == cudaSuccess ? LUX_BACKEND_OK : map_cuda(e, name);
 }
 
 const void* kernel_addr_attn_prefill_mma_f32() { return (const void*)pmma::lux_attn_prefill_mma_f32; }
 const void* kernel_addr_attn_prefill_f32() { return (const void*)pmma::lux_attn_prefill_f32; }
+const void* kernel_addr_attn_split_kv() { return (const void*)pmma::lux_attn_split_kv; }
 
 }  // namespace luxcuda

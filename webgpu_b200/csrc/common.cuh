@@ -51,6 +51,8 @@ struct Context {
     size_t         d_int_bytes = 0;
     void*          d_attn = nullptr;        // partial results of attention calls that split the keys over CTAs:
     size_t         d_attn_bytes = 0;        // 16 MB, allocated with the context (a call takes fewer slices rather than allocate)
+    void*          d_parts = nullptr;       // bf16 parts of K and V of prompt attention: 1536 bytes a key and KV head,
+    size_t         d_parts_bytes = 0;       // 128 k of them, allocated with the context (a larger call goes in several passes)
     std::mutex     mu;                      // guards the staging buffers
     int            sm_count = 148;
     // A kernel of this library that WRITES a buffer a later matmul may bind as weights, scales or

@@ -38,6 +38,7 @@ const void* kernel_addr_matmul_int8_tcgen05();
 const void* kernel_addr_attn_stream_f32();
 const void* kernel_addr_attn_prefill_f32();
 const void* kernel_addr_attn_prefill_mma_f32();
+const void* kernel_addr_attn_split_kv();
 const void* kernel_addr_attn_merge_f32();
 const void* kernel_addr_attn_plain_f32();
 const void* kernel_addr_rope_f32();
@@ -79,7 +80,8 @@ const Entry kTable[] = {
     {"lux_matmul_int8_tcgen05",    luxcuda::kernel_addr_matmul_int8_tcgen05, 192, 1, 1},
     {"lux_attn_stream_f32",        luxcuda::kernel_addr_attn_stream_f32,    288, 1, 1},
     {"lux_attn_prefill_f32",       luxcuda::kernel_addr_attn_prefill_f32,   256, 1, 1},
-    {"lux_attn_prefill_mma_f32",   luxcuda::kernel_addr_attn_prefill_mma_f32, 256, 1, 1},
+    {"lux_attn_prefill_mma_f32",   luxcuda::kernel_addr_attn_prefill_mma_f32, 384, 1, 1},
+    {"lux_attn_split_kv",          luxcuda::kernel_addr_attn_split_kv,      256, 1, 1},
     {"lux_attn_merge_f32",         luxcuda::kernel_addr_attn_merge_f32,     128, 1, 1},
     {"lux_attn_plain_f32",         luxcuda::kernel_addr_attn_plain_f32,     256, 1, 1},
     {"lux_rope_f32",               luxcuda::kernel_addr_rope_f32,           256, 1, 1},

@@ -123,8 +123,13 @@ static LuxBackendContext* cuda_create_context(int device_index) {
         ctx->d_attn_bytes = 16u << 20;
         ok = cudaMalloc(&ctx->d_attn, ctx->d_attn_bytes) == cudaSuccess;
     }
+    if (ok) {
+        ctx->d_parts_bytes = (size_t)131072 / 64 * ((64u * 1536u) + 8u);
+        ok = cudaMalloc(&ctx->d_parts, ctx->d_parts_bytes) == cudaSuccess;
+    }
     if (!ok) {
         cudaGetLastError();
+        if (ctx->d_parts) cudaFree(ctx->d_parts);
         if (ctx->d_attn) cudaFree(ctx->d_attn);
         if (ctx->d_splitk) cudaFree(ctx->d_splitk);
         if (ctx->d_absmax) cudaFree(ctx->d_absmax);
@@ -148,6 +153,7 @@ static void cuda_destroy_context(LuxBackendContext* context) {
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->d_stage) cudaFree(ctx->d_stage);
     if (ctx->d_int) cudaFree(ctx->d_int);
+    if (ctx->d_parts) cudaFree(ctx->d_parts);
     if (ctx->d_attn) cudaFree(ctx->d_attn);
     if (ctx->d_splitk) cudaFree(ctx->d_splitk);
     if (ctx->d_absmax) cudaFree(ctx->d_absmax);
