@@ -368,3 +368,18 @@ def test_no_less_precise_than_the_streaming_kernel(ctx, backend):
             with _Tuned(backend, attn_prefill=mode):
                 errs.append(orc.rel_l2(_sdpa(ctx, q, k, v, causal)[0], want))
         assert errs[0] < errs[1], (Sq, causal, errs)
+
+
+def test_keys_and_values_at_a_16_byte_offset(ctx, backend):
+    """K and V that are 16- but not 32-byte aligned are read by 16-byte loads: the same bits."""
+    q, k, v = _qkv(24, 1, 4, 2, 130, 200)
+    with _Tuned(backend, attn_prefill=1):
+        want, _ = _sdpa(ctx, q, k, v, False)
+        bufs = []
+        for a in (k, v):
+            big = ctx.upload(np.concatenate([np.zeros(4, np.float32), a.ravel()]))
+            bufs += [big, ctx.wrap(big.device_ptr + 16, a.nbytes)]
+        ob = ctx.alloc(q.nbytes)
+        ctx.sdpa(ctx.upload(q), bufs[1], bufs[3], ob, 1, 4, 2, 130, 200, 128, 1 / np.sqrt(128))
+        assert backend.last_kernel_name() == "lux_attn_prefill_mma_f32"
+    assert np.array_equal(ob.to_host(np.uint32, q.shape), want.view(np.uint32))

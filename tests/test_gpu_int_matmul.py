@@ -226,3 +226,17 @@ def test_argument_checks(ctx, backend):
     assert lib.lux_cuda_matmul_int8(ctx.handle, a.handle, a.handle, c.handle, 0, 8, 8) == B.INVALID_ARGUMENT
     assert lib.lux_cuda_dynamic_quantize(ctx.handle, a.handle, a.handle, c.handle, 16, 5) == B.INVALID_ARGUMENT
     assert lib.lux_cuda_matmul_int8(None, a.handle, a.handle, c.handle, 1, 1, 1) == B.INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("n", [8, 4096, (1 << 16) + 5])
+def test_dynamic_quantize_from_a_16_byte_offset(ctx, bits, n):
+    """A tensor that is 16- but not 32-byte aligned is read by 16-byte loads: the oracle's bits as well."""
+    x = (RNG.standard_normal(n) * 2).astype(np.float32)
+    big = ctx.upload(np.concatenate([np.zeros(4, np.float32), x]))
+    nbytes = n if bits == 8 else (n + 1) // 2
+    ob, sb = ctx.alloc((nbytes + 3) // 4 * 4), ctx.alloc(4)
+    ctx.dynamic_quantize(ctx.wrap(big.device_ptr + 16, x.nbytes), ob, sb, n, bits)
+    want, scale = orc.dynamic_quantize(x, bits)
+    assert sb.to_host(np.float32, (1,)).view(np.uint32)[0] == np.float32(scale).view(np.uint32)
+    assert np.array_equal(ob.to_host(np.uint8, ((nbytes + 3) // 4 * 4,))[:nbytes], want)

@@ -149,3 +149,22 @@ def test_rounding_without_division_is_the_division_s(ctx, bits, symmetric, shift
     assert np.array_equal(s[finite].view(np.uint32), rs[finite].view(np.uint32))
     assert rz is None or np.array_equal(z, rz)
     assert np.array_equal(w.view(np.uint8), rw.view(np.uint8))
+
+
+@pytest.mark.parametrize("bits,zeros", [(4, True), (4, False), (8, False)])
+@pytest.mark.parametrize("N,K", [(5, 128), (33, 1280)])
+def test_quantize_from_a_16_byte_offset(ctx, backend, N, K, bits, zeros):
+    """A matrix that is 16- but not 32-byte aligned is read by 16-byte loads: the oracle's bits as well."""
+    import ctypes as C
+    x = _matrix(N, K, 9)
+    group = 128 if bits == 4 else 32
+    G = K // group
+    big = ctx.upload(np.concatenate([np.zeros(4, np.float32), x.ravel()]))
+    xb = ctx.wrap(big.device_ptr + 16, x.nbytes)
+    w, s, z = ctx.alloc(N * K * bits // 8), ctx.alloc(N * G * 4), ctx.alloc(N * ((G + 1) // 2)) if zeros else None
+    d = B.make_desc(0, N, K, bits, group, B.F32, B.F32, B.F32)
+    assert backend.lib.lux_cuda_qquantize(ctx.handle, C.byref(d), xb.handle, w.handle, s.handle, z.handle if z else None) == B.OK
+    rw, rs, rz = orc.quantize(x, bits, group, not zeros, orc.F32)
+    assert np.array_equal(w.to_host(np.uint8, (N, K * bits // 8)), rw.view(np.uint8))
+    assert np.array_equal(s.to_host(np.uint32, (N, G)), rs.view(np.uint32))
+    assert not zeros or np.array_equal(z.to_host(np.uint8, (N, (G + 1) // 2)), rz)

@@ -141,14 +141,20 @@ __global__ void __launch_bounds__(256) lux_attn_split_kv(const float* __restrict
     unsigned char* dst = parts + ((size_t)bk * gridDim.x + t) * TILE_BYTES + (is_v ? 2 * SLOT : 0);
     const uint32_t nk = min((uint32_t)BN, kv_len - t * BN);
     uint32_t top = 0u, low = 0xffffffffu;             // largest magnitude; smallest non-zero one, less 1
+    const bool wide = (reinterpret_cast<uintptr_t>(src) & 31u) == 0;
     float4 x[4][2];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const uint32_t e = tid + 256u * i, key = e >> 4, c = e & 15u;      // 16-byte chunk c of a row's parts: columns 8 c ..
         x[i][0] = x[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (key < nk) {
-            x[i][0] = __ldg(reinterpret_cast<const float4*>(src + (size_t)key * D) + 2 * c);
-            x[i][1] = __ldg(reinterpret_cast<const float4*>(src + (size_t)key * D) + 2 * c + 1);
+            const float* at = src + (size_t)key * D + 8 * c;
+            if (wide) {
+                load32(at, x[i][0], x[i][1]);
+            } else {
+                x[i][0] = __ldg(reinterpret_cast<const float4*>(at));
+                x[i][1] = __ldg(reinterpret_cast<const float4*>(at) + 1);
+            }
         }
     }
 #pragma unroll

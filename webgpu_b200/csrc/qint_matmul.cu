@@ -226,11 +226,18 @@ __global__ void __launch_bounds__(256) lux_dynamic_quantize(const float* __restr
     const size_t stride = (size_t)gridDim.x * 256;
     // 16-byte loads and (int8) 8-byte stores where the views allow them
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(out) & 7u) == 0;
+    const bool wide = (reinterpret_cast<uintptr_t>(x) & 31u) == 0;
     for (size_t o = (size_t)blockIdx.x * 256 + threadIdx.x; o < octets; o += stride) {
         float v[8];
         const bool whole = vec && o * 8 + 8 <= n;
         if (whole) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * o), b = __ldg(reinterpret_cast<const float4*>(x) + 2 * o + 1);
+            float4 a, b;
+            if (wide) {
+                load32(x + 8 * o, a, b);
+            } else {
+                a = __ldg(reinterpret_cast<const float4*>(x) + 2 * o);
+                b = __ldg(reinterpret_cast<const float4*>(x) + 2 * o + 1);
+            }
             v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         } else {
 #pragma unroll

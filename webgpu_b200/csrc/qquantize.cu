@@ -42,10 +42,19 @@ struct QuantParams {
     int chunks_per_row;     // ceil(K / 256)
 };
 
+// W32: f32 and 32-byte aligned, a lane's eight elements by one load (by two 16-byte ones each of a warp's requests takes
+// half of every sector it touches)
+template <bool W32>
 __device__ __forceinline__ void load8(const QuantParams& p, size_t idx, float (&v)[8]) {
-    if (p.x_dtype == LUX_QDTYPE_F32) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + idx));
-        const float4 b = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + idx) + 1);
+    if (W32 || p.x_dtype == LUX_QDTYPE_F32) {
+        const float* src = reinterpret_cast<const float*>(p.x) + idx;
+        float4 a, b;
+        if (W32) {
+            load32(src, a, b);
+        } else {
+            a = __ldg(reinterpret_cast<const float4*>(src));
+            b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        }
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     } else {
         const uint4 r = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.x) + idx));
@@ -72,7 +81,7 @@ __device__ __forceinline__ void load8(const QuantParams& p, size_t idx, float (&
 // arithmetic keeps HBM busy.
 constexpr int QCH = 4;
 
-template <int BITS, bool SYM>
+template <int BITS, bool SYM, bool W32>
 __global__ void __launch_bounds__(256, 4) lux_qquantize(const QuantParams p) {
     constexpr int GL = BITS == 4 ? 16 : 4;                  // lanes per group
     const int lane = threadIdx.x & 31;
@@ -88,7 +97,7 @@ __global__ void __launch_bounds__(256, 4) lux_qquantize(const QuantParams p) {
     for (int ch = 0; ch < QCH; ch++) {
         const int k0 = (c0 + ch) * 256 + lane * 8;
         live[ch] = k0 < p.K;                                 // K is a multiple of the group size, so of 8
-        if (live[ch]) load8(p, n * (size_t)p.K + k0, v[ch]);
+        if (live[ch]) load8<W32>(p, n * (size_t)p.K + k0, v[ch]);
     }
     // group statistics of all chunks
     float mx[QCH], mn[QCH];
@@ -167,8 +176,8 @@ __global__ void __launch_bounds__(256, 4) lux_qquantize(const QuantParams p) {
 
 }  // namespace
 
-const void* kernel_addr_qquantize_i4() { return (const void*)lux_qquantize<4, false>; }
-const void* kernel_addr_qquantize_i8() { return (const void*)lux_qquantize<8, true>; }
+const void* kernel_addr_qquantize_i4() { return (const void*)lux_qquantize<4, false, true>; }
+const void* kernel_addr_qquantize_i8() { return (const void*)lux_qquantize<8, true, true>; }
 
 }  // namespace luxcuda
 
@@ -205,12 +214,14 @@ extern "C" LuxBackendError lux_cuda_qquantize(LuxBackendContext* context, const 
     p.scale_dtype = (int)d->scale_dtype;
     p.shifted = (d->flags & LUX_QQUANT_FLAG_SHIFTED) ? 1 : 0;
     p.chunks_per_row = (int)((K + 255) / 256);
+    const bool w32 = d->x_dtype == LUX_QDTYPE_F32 && (reinterpret_cast<uintptr_t>(bx->ptr) & 31u) == 0;
     const size_t warps = N * (size_t)((p.chunks_per_row + QCH - 1) / QCH);
     const unsigned grid = (unsigned)((warps + 7) / 8);
     cudaSetDevice(ctx->device);
-    if (d->bits == 8) lux_qquantize<8, true><<<grid, 256, 0, ctx->stream>>>(p);
-    else if (bz) lux_qquantize<4, false><<<grid, 256, 0, ctx->stream>>>(p);
-    else lux_qquantize<4, true><<<grid, 256, 0, ctx->stream>>>(p);
+    auto kfn = d->bits == 8 ? (w32 ? lux_qquantize<8, true, true> : lux_qquantize<8, true, false>)
+               : bz         ? (w32 ? lux_qquantize<4, false, true> : lux_qquantize<4, false, false>)
+                            : (w32 ? lux_qquantize<4, true, true> : lux_qquantize<4, true, false>);
+    kfn<<<grid, 256, 0, ctx->stream>>>(p);
     count_launch("lux_qquantize");
     ctx->writer_pending = true;          // cleared by the wait in finish_op unless NO_SYNC
     return finish_op(ctx, (d->flags & LUX_QMATMUL_FLAG_NO_SYNC) != 0, "lux_cuda_qquantize");
