@@ -399,3 +399,49 @@ def test_decode_at_bench_size_properties(ctx):
     one = ctx.alloc(H * D * 4)
     ctx.sdpa_kv_cache(ctx.upload(q[3:4]), ctx.upload(kc[3:4]), ctx.upload(vc[3:4]), one, 1, H, Hkv, 1, L - 1, L, D, scale)
     _close(one.to_host(np.float32, (1, H, 1, D)), out[3:4])
+
+
+@pytest.mark.parametrize("lens,H,Hkv,D,block_size,max_blocks", [
+    ([1] * 70, 8, 8, 128, 16, None),                        # pieces of one chunk, more than 32 sequences, shares of many items
+    ([0] * 40 + [3000] + [0] * 33 + [33, 0, 64], 32, 8, 128, 16, None),      # a sequence far into the batch, empty ones around it
+    ([31, 32, 33, 127, 128, 129, 2000] * 5, 32, 8, 128, 32, 4096),           # items that end and begin inside shares, a wide table
+    ([700, 1, 5000], 4, 4, 64, 1, None),                    # one row per KV head, one key per page
+    ([900, 1200], 32, 2, 128, 24, None),                    # sixteen rows per KV head, a page size that does not divide the chunk
+    ([640, 10], 6, 2, 256, 16, None)])                      # one CTA per SM
+def test_paged_decode_dealt_out_evenly(ctx, lens, H, Hkv, D, block_size, max_blocks):
+    rng = np.random.default_rng(len(lens))
+    q, kc, vc, table, cl = _paged_case(rng, lens, H, Hkv, D, block_size, max_blocks)
+    init = np.full(q.shape, 7.0, np.float32)
+    scale = 1.0 / np.sqrt(D)
+    got = _paged(ctx, q, kc, vc, table, cl, scale, out_init=init)
+    assert ctx.backend.last_kernel_name() == "lux_attn_merge_f32" and ctx.last_device_status() == 0
+    assert (got[cl <= 0] == 7.0).all()
+    for i in np.flatnonzero(cl > 0):
+        # the context in 64 bits, page by page in the table's order
+        pages = table[i, :(cl[i] + block_size - 1) // block_size]
+        k, v = (x[pages].transpose(1, 0, 2, 3).reshape(Hkv, -1, D)[:, :cl[i]].astype(np.float64) for x in (kc, vc))
+        s = np.einsum("grd,gkd->grk", q[i].reshape(Hkv, H // Hkv, D).astype(np.float64), k) * scale
+        w = np.exp(s - s.max(axis=-1, keepdims=True))
+        want = np.einsum("grk,gkd->grd", w / w.sum(axis=-1, keepdims=True), v).reshape(H, D)
+        assert orc.rel_l2(got[i], want) < TOL
+
+
+@pytest.mark.parametrize("B_,H,Hkv,keys,Sq", [(1, 8, 8, 33, 1), (37, 8, 8, 32, 1), (37, 8, 8, 31, 1), (5, 32, 8, 1184, 1), (1, 32, 8, 148 * 64, 1),
+                                               (2, 8, 2, 700, 4), (3, 16, 2, 2049, 2)])
+def test_contiguous_decode_dealt_out_evenly(ctx, backend, B_, H, Hkv, keys, Sq):
+    """Shares that hold whole items, parts of one, and ends of two; rows of a step that appended several tokens see
+    different numbers of keys.  One slice per item (forced) is the reference (both sum in f32)."""
+    rng = np.random.default_rng(keys)
+    q = rng.standard_normal((B_, H, Sq, 128), np.float32)
+    kc, vc = (rng.standard_normal((B_, Hkv, keys, 128), np.float32) for _ in range(2))
+    outs = []
+    for splits in (0, 1):
+        backend.tune("attn_splits", splits)
+        try:
+            ob = ctx.alloc(q.nbytes)
+            ctx.sdpa_kv_cache(ctx.upload(q), ctx.upload(kc), ctx.upload(vc), ob, B_, H, Hkv, Sq, keys - Sq, keys, 128, 0.09, flags=B.FLAG_ATTN_CAUSAL)
+            outs.append(ob.to_host(np.float32, q.shape))
+        finally:
+            backend.tune("attn_splits", 0)
+    _close(outs[0], outs[1])
+    assert ctx.last_device_status() == 0

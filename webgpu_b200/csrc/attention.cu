@@ -11,8 +11,7 @@
 //     read from HBM once per KV head, not once per query head;
 //   * a producer warp streams 32-key chunks of K and V into a ring in shared memory with bulk
 //     copies (cp.async.bulk, one per contiguous run: a whole chunk for a contiguous cache, one per
-//     page for a paged one, the page numbers taken from a copy of the block table in shared
-//     memory), each chunk signalled through an mbarrier; two CTAs of nine warps share an SM, each
+//     page for a paged one, the page numbers read one chunk ahead), each chunk signalled through an mbarrier; two CTAs of nine warps share an SM, each
 //     with a ring of three chunks (D = 128);
 //   * eight consumer warps share a chunk: a key is handled by 8 lanes, each holding 16-byte columns
 //     of the row, so a warp takes 4 keys per step; every lane keeps two query rows in registers
@@ -25,9 +24,10 @@
 //     With every warp polling its mbarrier the kernel ran at 2.2-5.1 TB/s depending on how many
 //     warps happened to be waiting; parked, at 5.0-6.5 TB/s on the same shapes (polls travel the same
 //     queue as shared-memory loads and shuffles, and starved the warps that had work);
-//   * keys are split over CTAs when there are fewer (sequence, KV head) pairs than SM slots, and
-//     each CTA walks its chunks from a different starting point; a small second kernel, resident
-//     early through programmatic dependent launch, merges the slices.
+//   * a decode step is one wave of CTAs, each with the same number of chunks of the (sequence, KV head) items laid end to
+//     end, so that a CTA may finish one item and begin the next; for a paged cache each CTA works out its share from
+//     the lengths.  Blocks of more rows split their keys over CTAs where whole items would leave SM slots idle.
+//     A small second kernel, resident early through programmatic dependent launch, merges what several CTAs did of a row.
 // The one polling wait is bounded: if it gives up it sets the CTA's abort flag, every warp leaves
 // its loop (the consumers first release the stages the producer may be parked on), the device
 // status word reports 0x7C050008 and the output of that CTA is not written.
@@ -51,8 +51,10 @@ constexpr int ATT_THREADS = (ATT_CW + 1) * 32;  // + the producer warp
 constexpr int ATT_CK = 32;                      // keys per staged chunk
 constexpr int ATT_MAX_STAGES = 6;
 constexpr int ATT_CTAS_PER_SM = 2;
-constexpr int ATT_TABLE = 2048;                 // block-table entries a CTA keeps in shared memory
-constexpr int ATT_HEADER = 128;                 // barriers + abort flag
+constexpr uint64_t ATT_PAGES = 256ull * 2046;   // pages of the longest context taken
+constexpr int ATT_HEADER = 512;                 // barriers, abort flag, from byte 128 on each consumer warp's Piece
+// floats in which the warps of a row group leave their results: [warp][row][head_dim + 2], in whole 128-byte lines
+__host__ __device__ constexpr uint32_t att_merge_floats(uint32_t head_dim, uint32_t rt) { return (ATT_CW * rt * (head_dim + 2u) + 31u) / 32u * 32u; }
 constexpr size_t ATT_SMEM_BUDGET = 110u << 10;        // per CTA: two CTAs share an SM
 constexpr float ATT_NEG = -3.0e38f;             // "no key seen yet" in the base-2 score domain
 constexpr float ATT_LOG2E = 1.4426950408889634f;
@@ -69,7 +71,7 @@ struct AttnParams {
     float* lse;                  // may be null
     const int32_t* block_tables; // paged only
     const int32_t* context_lens; // paged only
-    float* part;                 // [out row][nsplit][head_dim + 2] when nsplit > 1
+    float* part;                 // partial results: [out row][nsplit][head_dim + 2], or [CTA][2][row][head_dim + 2]
     uint32_t* status;
     uint32_t batch, heads, kv_heads, group, seq_q, head_dim;
     uint32_t kv_len;             // keys a row may see (contiguous caches); paged: context_lens decides
@@ -77,7 +79,12 @@ struct AttnParams {
     uint32_t causal, causal_base;// causal: query i sees min(causal_base + i + 1, kv_len) keys
     uint32_t block_size, max_blocks_per_seq, num_blocks;   // paged (block_size 0: contiguous)
     uint32_t rgp;                // row groups per CTA (1, 2, 4 or 8): rows per CTA = RT * rgp
+    uint32_t rpb;                // rows per CTA
     uint32_t row_blocks, nsplit, split_keys, stages;
+    // One block of rows per KV head (a decode step): all 32-key chunks of all (sequence, KV head) items, one after the
+    // other, are dealt out evenly, each CTA taking the next `share` of them (0: the grid is one CTA per slice instead).
+    uint32_t share;              // contiguous: chunks per CTA; paged: the least, the lengths being known on the device only
+    int2* spans;                 // per item: its first CTA and how many CTAs work on it
     float qscale;                // scale * log2(e)
 };
 
@@ -92,51 +99,120 @@ __device__ __forceinline__ float ex2(float x) {
 // warp polling an mbarrier, whose polls share the queue that shared-memory loads and shuffles go
 // through.  With eight warps polling for every chunk the warps that had work ran 2-3 times slower.
 constexpr int ATT_BAR_READY = 1;           // consumer warps: the chunk has landed (warp 0 polled for it)
-constexpr int ATT_BAR_FREE0 = 2;           // + stage: every consumer warp is done with the stage (producer waits)
+constexpr int ATT_BAR_FREE0 = 2;           // + stage (6 at most): every consumer warp is done with the stage (producer waits)
+constexpr int ATT_BAR_MERGE = 8;           // consumer warps: the piece's results are in shared memory; have been read
 
 __device__ __forceinline__ uint32_t row_len(const AttnParams& p, uint32_t qi, uint32_t kv_len) {
     return p.causal ? min(p.causal_base + qi + 1u, kv_len) : kv_len;
 }
+
+// Keys that sequence b of a paged cache holds.
+__device__ __forceinline__ uint32_t paged_len(const AttnParams& p, uint32_t b) {
+    const int32_t cl = p.context_lens[b];
+    return cl <= 0 ? 0u : min((uint32_t)cl, p.max_blocks_per_seq * p.block_size);
+}
+__device__ __forceinline__ uint32_t chunks_of(uint32_t keys) { return (keys + ATT_CK - 1) / ATT_CK; }
+
+// What a CTA does next: chunks [lo, hi) of the n that the rows of (b, g, rb) see.
+struct Piece {
+    uint32_t b, g, rb, kv_len, lmax, lo, hi, n;
+    __device__ __forceinline__ void load(const volatile Piece* s) {
+        b = s->b; g = s->g; rb = s->rb; kv_len = s->kv_len; lmax = s->lmax; lo = s->lo; hi = s->hi; n = s->n;
+    }
+};
 
 template <int VPL, int RT, bool FULL>
 __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_f32(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t bar_full = smem_u32(smem);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + 16 * ATT_MAX_STAGES);
-    int32_t* table = reinterpret_cast<int32_t*>(smem + ATT_HEADER);
-    float* stages = reinterpret_cast<float*>(smem + ATT_HEADER + (p.block_size ? ATT_TABLE * 4 : 0));
+    float* mrg = reinterpret_cast<float*>(smem + ATT_HEADER);              // [warp][RT][D + 2]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t D = p.head_dim, NS = p.stages;
+    const uint32_t D = p.head_dim, NS = p.stages, MS = D + 2u;
+    float* stages = mrg + att_merge_floats(D, RT);
     const size_t stage_floats = (size_t)2 * ATT_CK * D;
 
     pdl_launch_dependents();                   // the merge kernel may take its place; it waits for this grid
     pdl_wait();                                // q, the cache and the tables may come from the kernels just before
 
-    uint32_t idx = blockIdx.x;
-    const uint32_t split = idx % p.nsplit; idx /= p.nsplit;
-    const uint32_t rb = idx % p.row_blocks; idx /= p.row_blocks;
-    const uint32_t g = idx % p.kv_heads, b = idx / p.kv_heads;
-
-    uint32_t kv_len = p.kv_len;
-    if (p.block_size) {
-        const int32_t cl = p.context_lens[b];
-        if (cl <= 0) return;                   // paged.wgsl:66-67: the rows stay as they are
-        kv_len = min((uint32_t)cl, p.max_blocks_per_seq * p.block_size);
-    }
     // rows of this CTA: row r of the KV head is (query qi = r / group, head g * group + r % group),
     // so a block of rows holds neighbouring queries and a causal block stops at its last row's keys
-    const uint32_t R = p.group * p.seq_q, rpb = RT * p.rgp, row0 = rb * rpb;
-    const uint32_t last_row = min(R, row0 + rpb) - 1u;
-    const uint32_t lmax = row_len(p, last_row / p.group, kv_len);
-    const uint32_t k_begin = split * p.split_keys;
-    const uint32_t k_end = min(lmax, k_begin + p.split_keys);
-    const uint32_t nchunks = k_end > k_begin ? (k_end - k_begin + ATT_CK - 1) / ATT_CK : 0u;
-    const uint32_t tbl0 = p.block_size ? k_begin / p.block_size : 0u;
-    // Every CTA walks its chunks from a different starting point (and wraps around), so that the CTAs
-    // of a wave, which start together and advance at the same pace, are not all at the same offset
-    // of equally spaced slices.
-    const uint32_t rot = nchunks ? (blockIdx.x * 2654435761u >> 8) % nchunks : 0u;
-    auto chunk_at = [&](uint32_t c) { const uint32_t cc = c + rot; return cc >= nchunks ? cc - nchunks : cc; };
+    const uint32_t R = p.group * p.seq_q, rpb = RT * p.rgp;
+    Piece first;
+    uint32_t total = 0u, share = p.share;      // chunks of this CTA; of every CTA
+    auto measure = [&](Piece& w) {             // what the rows of (b, g, rb) see
+        w.kv_len = p.block_size ? paged_len(p, w.b) : p.kv_len;
+        w.lmax = row_len(p, (min(R, (w.rb + 1u) * rpb) - 1u) / p.group, w.kv_len);
+        w.n = chunks_of(w.lmax);
+    };
+    if (!p.share) {
+        uint32_t idx = blockIdx.x;
+        const uint32_t split = idx % p.nsplit; idx /= p.nsplit;
+        first.rb = idx % p.row_blocks; idx /= p.row_blocks;
+        first.g = idx % p.kv_heads;
+        first.b = idx / p.kv_heads;
+        if (p.block_size && p.context_lens[first.b] <= 0) return;          // paged.wgsl:66-67: the rows stay as they are
+        measure(first);
+        first.lo = min(split * (p.split_keys / ATT_CK), first.n);
+        first.hi = min(first.lo + p.split_keys / ATT_CK, first.n);
+        total = first.hi - first.lo;
+    } else {
+        first.rb = 0u;
+        uint32_t all, at;                      // chunks of the call; the first one of this CTA
+        if (!p.block_size) {
+            first.b = 0u;
+            measure(first);
+            all = p.batch * p.kv_heads * first.n;
+            at = blockIdx.x * share;
+            const uint32_t item = at / first.n;
+            first.b = item / p.kv_heads;
+            first.g = item - first.b * p.kv_heads;
+            first.lo = at - item * first.n;
+        } else {
+            // every warp for itself, 32 sequences at a time: the sum, then the sequence in which this CTA starts
+            uint32_t sum = 0u;
+            for (uint32_t b0 = 0; b0 < p.batch; b0 += 32) sum += b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
+            for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+            all = sum * p.kv_heads;
+            share = max(share, (all + gridDim.x - 1u) / gridDim.x);
+            at = blockIdx.x * share;
+            if (at >= all) return;
+            uint32_t before = 0u;
+            for (uint32_t b0 = 0;; b0 += 32) {
+                const uint32_t n = b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
+                uint32_t upto = n;             // inclusive
+                for (int off = 1; off < 32; off <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, upto, off);
+                    if (lane >= off) upto += v;
+                }
+                const uint32_t hit = __ballot_sync(0xffffffffu, (before + upto) * p.kv_heads > at);
+                if (hit) {
+                    const int src = __ffs(hit) - 1;
+                    first.b = b0 + src;
+                    before += __shfl_sync(0xffffffffu, upto - n, src);
+                    break;
+                }
+                before += __shfl_sync(0xffffffffu, upto, 31);
+            }
+            measure(first);
+            const uint32_t in = at - before * p.kv_heads;
+            first.g = in / first.n;
+            first.lo = in - first.g * first.n;
+        }
+        total = min(share, all - at);
+        first.hi = min(first.lo + total, first.n);
+    }
+    auto next = [&](Piece& w, uint32_t left) { // the piece after w, `left` chunks still to do
+        if (++w.g == p.kv_heads) {
+            w.g = 0u;
+            do {
+                w.b++;
+                if (p.block_size) measure(w);
+            } while (w.n == 0u);               // (left > 0: there is one)
+        }
+        w.lo = 0u;
+        w.hi = min(left, w.n);
+    };
 
     if (tid == 0) {
         *abort_flag = 0u;
@@ -144,18 +220,6 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             mbar_init(bar_full + 8u * s, 1u);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (p.block_size && nchunks) {
-        const uint32_t nblk = (k_end - 1u) / p.block_size - tbl0 + 1u;      // <= ATT_TABLE by the launcher's split
-        const int32_t* src = p.block_tables + (size_t)b * p.max_blocks_per_seq + tbl0;
-        for (uint32_t i = tid; i < nblk; i += ATT_THREADS) {
-            int32_t e = src[i];
-            if ((uint32_t)e >= p.num_blocks) {
-                e = 0;
-                if (p.status) atomicOr(p.status, ATT_STATUS_BLOCK);
-            }
-            table[i] = e;
-        }
     }
     __syncthreads();
 
@@ -170,13 +234,27 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
 
     if (warp == ATT_CW) {
         // ---- producer: one chunk = keys [t0, t0 + nk) of K and of V ------------------------------
-        for (uint32_t c = 0; c < nchunks; c++) {
+        Piece w = first;
+        // paged: lane i holds the table's entry of the i-th page that the next chunk touches, read one chunk ahead
+        int32_t entry = 0;
+        auto lookup = [&](uint32_t t0) {
+            const uint32_t blk = t0 / p.block_size + (uint32_t)lane;
+            if (blk * p.block_size < min(w.lmax, t0 + ATT_CK)) {
+                entry = p.block_tables[(size_t)w.b * p.max_blocks_per_seq + blk];
+                if ((uint32_t)entry >= p.num_blocks) {
+                    entry = 0;
+                    if (p.status) atomicOr(p.status, ATT_STATUS_BLOCK);
+                }
+            }
+        };
+        if (p.block_size && total) lookup(w.lo * ATT_CK);
+        for (uint32_t c = 0, k = w.lo; c < total; c++) {
             const uint32_t s = c % NS;
             if (c >= NS) {
                 named_bar_sync<ATT_BAR_FREE0>(s, ATT_THREADS);          // all consumer warps have left the stage
                 if (*abort_flag) break;
             }
-            const uint32_t t0 = k_begin + chunk_at(c) * ATT_CK, nk = min((uint32_t)ATT_CK, k_end - t0);
+            const uint32_t t0 = k * ATT_CK, nk = min((uint32_t)ATT_CK, w.lmax - t0);
             const uint32_t bar = bar_full + 8u * s;
             float* ks = stages + s * stage_floats;
             float* vs = ks + (size_t)ATT_CK * D;
@@ -184,7 +262,7 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             __syncwarp();
             if (!p.block_size) {
                 if (lane == 0) {
-                    const size_t off = (((size_t)b * p.kv_heads + g) * p.kv_stride + t0) * D;
+                    const size_t off = (((size_t)w.b * p.kv_heads + w.g) * p.kv_stride + t0) * D;
                     bulk_g2s(smem_u32(ks), p.k + off, nk * D * 4u, bar);
                     bulk_g2s(smem_u32(vs), p.v + off, nk * D * 4u, bar);
                 }
@@ -193,32 +271,42 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                 const uint32_t blk = t0 / p.block_size + (uint32_t)lane;
                 const uint32_t ta = max(t0, blk * p.block_size), tb = min(t0 + nk, (blk + 1u) * p.block_size);
                 if (ta < tb) {
-                    const size_t off = (((size_t)table[blk - tbl0] * p.kv_heads + g) * p.block_size + (ta - blk * p.block_size)) * D;
+                    const size_t off = (((size_t)entry * p.kv_heads + w.g) * p.block_size + (ta - blk * p.block_size)) * D;
                     bulk_g2s(smem_u32(ks + (size_t)(ta - t0) * D), p.k + off, (tb - ta) * D * 4u, bar);
                     bulk_g2s(smem_u32(vs + (size_t)(ta - t0) * D), p.v + off, (tb - ta) * D * 4u, bar);
                 }
             }
+            if (++k == w.hi && c + 1 < total) {
+                next(w, total - c - 1u);
+                k = 0u;
+            }
+            if (p.block_size && c + 1 < total) lookup(k * ATT_CK);
         }
     } else {
         // ---- consumers -------------------------------------------------------------------------
         const uint32_t rg = (uint32_t)warp % p.rgp, kslot = (uint32_t)warp / p.rgp, wpg = ATT_CW / p.rgp;
+        uint32_t min_len;
+        auto begin = [&](const Piece& w) {                               // this lane's rows of the piece
+            min_len = 0xffffffffu;
 #pragma unroll
-        for (int i = 0; i < RT; i++) {
-            const uint32_t r = row0 + rg * RT + i;
-            const bool valid = r < R;
-            const uint32_t qi = valid ? r / p.group : 0u, head = g * p.group + (valid ? r % p.group : 0u);
-            len[i] = valid ? row_len(p, qi, kv_len) : 0xffffffffu;       // a padding row: q = 0, never written, never masks a chunk
-            const float* qr = p.q + (((size_t)b * p.heads + head) * p.seq_q + qi) * D;
-            m[i] = ATT_NEG;
-            l[i] = 0.0f;
+            for (int i = 0; i < RT; i++) {
+                const uint32_t r = w.rb * rpb + rg * RT + i;
+                const bool valid = r < R;
+                const uint32_t qi = valid ? r / p.group : 0u, head = w.g * p.group + (valid ? r % p.group : 0u);
+                len[i] = valid ? row_len(p, qi, w.kv_len) : 0xffffffffu; // a padding row: q = 0, never written, never masks a chunk
+                min_len = min(min_len, len[i]);
+                const float* qr = p.q + (((size_t)w.b * p.heads + head) * p.seq_q + qi) * D;
+                m[i] = ATT_NEG;
+                l[i] = 0.0f;
 #pragma unroll
-            for (int j = 0; j < VPL; j++) {
-                float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (valid && col_ok[j]) t = __ldg(reinterpret_cast<const float4*>(qr) + j * 8 + sub);
-                q[i][j] = make_float4(t.x * p.qscale, t.y * p.qscale, t.z * p.qscale, t.w * p.qscale);
-                o[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int j = 0; j < VPL; j++) {
+                    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (valid && col_ok[j]) t = __ldg(reinterpret_cast<const float4*>(qr) + j * 8 + sub);
+                    q[i][j] = make_float4(t.x * p.qscale, t.y * p.qscale, t.z * p.qscale, t.w * p.qscale);
+                    o[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
             }
-        }
+        };
         // One step: the warp's four keys (one per group of 8 lanes) against its RT rows.  The
         // running maximum of a lane is only raised when a score passes it by more than 8 (in the
         // base-2 domain), so weights stay below 2^8 and the common step has no rescaling in it:
@@ -291,141 +379,167 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                 }
             }
         };
-        uint32_t min_len = 0xffffffffu;
+        // the end of a piece: the four key slots of the warp, then the warps of each row group, are merged by the
+        // running-maximum rule, and the rows written: the outputs of a whole item, else partial results
+        auto finish = [&](const Piece& w) {
 #pragma unroll
-        for (int i = 0; i < RT; i++) min_len = min(min_len, len[i]);
+            for (int i = 0; i < RT; i++) {
+                float mm = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
+                mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, 16));
+                const float alpha = ex2(m[i] - mm);
+                m[i] = mm;
+                l[i] *= alpha;
+                l[i] += __shfl_xor_sync(0xffffffffu, l[i], 8);
+                l[i] += __shfl_xor_sync(0xffffffffu, l[i], 16);
+                float* dst = mrg + ((size_t)warp * RT + i) * MS;
+#pragma unroll
+                for (int j = 0; j < VPL; j++) {
+                    float* e = reinterpret_cast<float*>(&o[i][j]);
+#pragma unroll
+                    for (int x = 0; x < 4; x++) {
+                        float val = e[x] * alpha;
+                        val += __shfl_xor_sync(0xffffffffu, val, 8);
+                        val += __shfl_xor_sync(0xffffffffu, val, 16);
+                        if (kg == 0 && col_ok[j]) dst[(j * 8 + sub) * 4 + x] = val;
+                    }
+                }
+                if (lane == 0) {
+                    dst[D] = m[i];
+                    dst[D + 1] = l[i];
+                }
+            }
+            named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);
+            const uint32_t row0 = w.rb * rpb;
+            const bool whole = p.share ? w.lo == 0u && w.hi == w.n : p.nsplit == 1;
+            if (p.share && w.lo == 0u && tid == 0)                       // the item may go on in the CTAs after this one
+                p.spans[w.b * p.kv_heads + w.g] = make_int2((int)blockIdx.x, (int)(1u + (w.n - w.hi + share - 1u) / share));
+            for (uint32_t e = tid; e < rpb * D; e += ATT_CW * 32) {
+                const uint32_t ir = e / D, d = e - ir * D, r = row0 + ir;
+                if (r >= R) continue;
+                const uint32_t rgi = ir / RT, ii = ir % RT;
+                float M = ATT_NEG;
+                for (uint32_t v = 0; v < wpg; v++) M = fmaxf(M, mrg[((size_t)(v * p.rgp + rgi) * RT + ii) * MS + D]);
+                float L = 0.0f, acc = 0.0f;
+                for (uint32_t v = 0; v < wpg; v++) {
+                    const float* src = mrg + ((size_t)(v * p.rgp + rgi) * RT + ii) * MS;
+                    const float wgt = ex2(src[D] - M);
+                    L = fmaf(src[D + 1], wgt, L);
+                    acc = fmaf(src[d], wgt, acc);
+                }
+                const uint32_t qi = r / p.group, head = w.g * p.group + r % p.group;
+                const size_t orow = ((size_t)w.b * p.heads + head) * p.seq_q + qi;
+                if (whole) {
+                    p.out[orow * D + d] = L > 0.0f ? acc / L : 0.0f;
+                    if (d == 0 && p.lse) p.lse[orow] = L > 0.0f ? fmaf(M, ATT_LN2, logf(L)) : -3.402823e+38f;
+                } else {
+                    // two places per CTA: the item in which its share begins, and the one that begins in its share
+                    const size_t slot = p.share ? (size_t)(blockIdx.x * 2u + (w.lo == 0u ? 1u : 0u)) * rpb + ir
+                                                : orow * p.nsplit + blockIdx.x % p.nsplit;
+                    float* dst = p.part + slot * MS;
+                    dst[d] = acc;
+                    if (d == 0) {
+                        dst[D] = M;
+                        dst[D + 1] = L;
+                    }
+                }
+            }
+            named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);                // before the next piece is merged
+        };
         const uint32_t stage0 = smem_u32(stages), stage_bytes = 2u * ATT_CK * row_bytes, v_off = ATT_CK * row_bytes;
-        for (uint32_t c = 0; c < nchunks; c++) {
-            const uint32_t s = c % NS;
-            // one poller per CTA: warp 0 waits for the copies, the named barrier releases the other seven
-            if (warp == 0) warp_wait(bar_full + 8u * s, (c / NS) & 1u, abort_flag, lane);
-            named_bar_sync_c<ATT_BAR_READY>(ATT_CW * 32);
-            if (*abort_flag) {
-                // the producer may be parked on the stages this warp would still have released
-                for (uint32_t cc = c; cc < c + NS && cc + NS < nchunks; cc++) named_bar_arrive<ATT_BAR_FREE0>(cc % NS, ATT_THREADS);
-                break;
-            }
-            const uint32_t t0 = k_begin + chunk_at(c) * ATT_CK, nk = min((uint32_t)ATT_CK, k_end - t0);
-            const uint32_t kchunk = stage0 + s * stage_bytes + lane_off;
-            if (nk == ATT_CK && t0 + ATT_CK <= min_len) {
-                for (uint32_t kb = kslot * 4u; kb < ATT_CK; kb += wpg * 4u) {
-                    const uint32_t ka = kchunk + (kb + (uint32_t)kg) * row_bytes;
-                    step(std::false_type{}, ka, ka + v_off, true, 0u);
+        // The piece lies in shared memory while its chunks are worked on: the loop has no registers left for it.
+        Piece* const kept = reinterpret_cast<Piece*>(smem + 128) + warp;
+        Piece w = first;
+        uint32_t c = 0;
+        for (bool ok = true; ok;) {
+            begin(w);
+            if (lane == 0) *kept = w;
+            __syncwarp();
+            const uint32_t t_end = min(w.hi * ATT_CK, w.lmax);
+            for (uint32_t t0 = w.lo * ATT_CK; t0 < t_end; t0 += ATT_CK, c++) {
+                const uint32_t s = c % NS;
+                // one poller per CTA: warp 0 waits for the copies, the named barrier releases the other seven
+                if (warp == 0) warp_wait(bar_full + 8u * s, (c / NS) & 1u, abort_flag, lane);
+                named_bar_sync_c<ATT_BAR_READY>(ATT_CW * 32);
+                if (*abort_flag) {
+                    // the producer may be parked on the stages this warp would still have released
+                    for (uint32_t cc = c; cc < c + NS && cc + NS < total; cc++) named_bar_arrive<ATT_BAR_FREE0>(cc % NS, ATT_THREADS);
+                    ok = false;
+                    break;
                 }
-            } else {
-                for (uint32_t kb = kslot * 4u; kb < nk; kb += wpg * 4u) {
-                    const uint32_t key = kb + (uint32_t)kg, ka = kchunk + key * row_bytes;
-                    step(std::true_type{}, ka, ka + v_off, key < nk, t0 + key);
+                const uint32_t nk = min((uint32_t)ATT_CK, t_end - t0);
+                const uint32_t kchunk = stage0 + s * stage_bytes + lane_off;
+                if (nk == ATT_CK && t0 + ATT_CK <= min_len) {
+                    for (uint32_t kb = kslot * 4u; kb < ATT_CK; kb += wpg * 4u) {
+                        const uint32_t ka = kchunk + (kb + (uint32_t)kg) * row_bytes;
+                        step(std::false_type{}, ka, ka + v_off, true, 0u);
+                    }
+                } else {
+                    for (uint32_t kb = kslot * 4u; kb < nk; kb += wpg * 4u) {
+                        const uint32_t key = kb + (uint32_t)kg, ka = kchunk + key * row_bytes;
+                        step(std::true_type{}, ka, ka + v_off, key < nk, t0 + key);
+                    }
                 }
+                // done with the stage (not needed for the last NS chunks: nobody refills them)
+                if (c + NS < total) named_bar_arrive<ATT_BAR_FREE0>(s, ATT_THREADS);
             }
-            // done with the stage (not needed for the last NS chunks: nobody refills them)
-            if (c + NS < nchunks) named_bar_arrive<ATT_BAR_FREE0>(s, ATT_THREADS);
-        }
-        // the four key slots of the warp, merged by the running-maximum rule
-#pragma unroll
-        for (int i = 0; i < RT; i++) {
-            float mm = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
-            mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, 16));
-            const float alpha = ex2(m[i] - mm);
-            m[i] = mm;
-            l[i] *= alpha;
-            l[i] += __shfl_xor_sync(0xffffffffu, l[i], 8);
-            l[i] += __shfl_xor_sync(0xffffffffu, l[i], 16);
-#pragma unroll
-            for (int j = 0; j < VPL; j++) {
-                float* e = reinterpret_cast<float*>(&o[i][j]);
-#pragma unroll
-                for (int x = 0; x < 4; x++) {
-                    float val = e[x] * alpha;
-                    val += __shfl_xor_sync(0xffffffffu, val, 8);
-                    val += __shfl_xor_sync(0xffffffffu, val, 16);
-                    e[x] = val;
-                }
-            }
+            if (!ok) break;
+            w.load(kept);
+            finish(w);                                                   // (a slice past the rows' keys leaves an empty result)
+            if (c == total) break;
+            next(w, total - c);
+            __syncwarp();
         }
     }
 
-    __syncthreads();               // every chunk has landed and been read: the ring is free
+    __syncthreads();               // every chunk has landed and been read
     if (*abort_flag) {
         // A bounded wait gave up: report it and give copies still in flight time to land in this
-        // CTA's shared memory before it is released.  Nothing is written.
+        // CTA's shared memory before it is released.  The piece it was in is not written.
         if (tid == 0 && p.status) atomicOr(p.status, ATT_STATUS_WAIT);
         for (int i = 0; i < 64; i++) __nanosleep(1000);
         __syncthreads();
-        return;
-    }
-    // warps of one row group -> shared memory (over the ring), then one thread per output element
-    float* mrg = stages;                                   // [warp][RT][D + 2]
-    const uint32_t MS = D + 2u;
-    if (warp < ATT_CW && kg == 0) {
-#pragma unroll
-        for (int i = 0; i < RT; i++) {
-            float* dst = mrg + ((size_t)warp * RT + i) * MS;
-#pragma unroll
-            for (int j = 0; j < VPL; j++)
-                if (col_ok[j]) {
-                    // D + 2 floats per row: rows are 8-byte aligned, not 16
-                    float* d4 = dst + (j * 8 + sub) * 4;
-                    d4[0] = o[i][j].x; d4[1] = o[i][j].y; d4[2] = o[i][j].z; d4[3] = o[i][j].w;
-                }
-            if (sub == 0) {
-                dst[D] = m[i];
-                dst[D + 1] = l[i];
-            }
-        }
-    }
-    __syncthreads();
-    const uint32_t wpg = ATT_CW / p.rgp;
-    for (uint32_t e = tid; e < rpb * D; e += ATT_THREADS) {
-        const uint32_t ir = e / D, d = e - ir * D, r = row0 + ir;
-        if (r >= R) continue;
-        const uint32_t rgi = ir / RT, ii = ir % RT;
-        float M = ATT_NEG;
-        for (uint32_t w = 0; w < wpg; w++) M = fmaxf(M, mrg[((size_t)(w * p.rgp + rgi) * RT + ii) * MS + D]);
-        float L = 0.0f, acc = 0.0f;
-        for (uint32_t w = 0; w < wpg; w++) {
-            const float* src = mrg + ((size_t)(w * p.rgp + rgi) * RT + ii) * MS;
-            const float wgt = ex2(src[D] - M);
-            L = fmaf(src[D + 1], wgt, L);
-            acc = fmaf(src[d], wgt, acc);
-        }
-        const uint32_t qi = r / p.group, head = g * p.group + r % p.group;
-        const size_t orow = ((size_t)b * p.heads + head) * p.seq_q + qi;
-        if (p.nsplit == 1) {
-            p.out[orow * D + d] = L > 0.0f ? acc / L : 0.0f;
-            if (d == 0 && p.lse) p.lse[orow] = L > 0.0f ? fmaf(M, ATT_LN2, logf(L)) : -3.402823e+38f;
-        } else {
-            float* dst = p.part + (orow * p.nsplit + split) * MS;
-            dst[d] = acc;
-            if (d == 0) {
-                dst[D] = M;
-                dst[D + 1] = L;
-            }
-        }
     }
 }
 
-// Merge of the key slices of one output row (paged_attention_v2_reduce, paged.wgsl:351-405, with
+// Merge of the partial results of one output row (paged_attention_v2_reduce, paged.wgsl:351-405, with
 // the statistics in the base-2 domain).  One CTA per row; resident early, it waits for the slices.
-__global__ void __launch_bounds__(128) lux_attn_merge_f32(const float* __restrict__ part, float* __restrict__ out, float* __restrict__ lse,
-                                                          const int32_t* __restrict__ context_lens, uint32_t rows_per_seq,
-                                                          uint32_t nsplit, uint32_t D) {
-    __shared__ float wgt[256];
+constexpr int ATT_MAX_PARTS = 512;
+__global__ void __launch_bounds__(128) lux_attn_merge_f32(const AttnParams p) {
+    __shared__ float wgt[ATT_MAX_PARTS];
     __shared__ float stat[2];
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t row = blockIdx.x, MS = D + 2u;
-    if (context_lens && context_lens[row / rows_per_seq] <= 0) return;
-    const float* base = part + (size_t)row * nsplit * MS;
+    const uint32_t row = blockIdx.x, D = p.head_dim, MS = D + 2u, b = row / (p.heads * p.seq_q);
+    if (p.context_lens && p.context_lens[b] <= 0) return;
+    // partial result 0, partial result 1 and the step from it to each of the others
+    const float *base0, *base1;
+    size_t step;
+    uint32_t parts;
+    if (!p.share) {
+        base0 = p.part + (size_t)row * p.nsplit * MS;
+        base1 = base0 + MS;
+        step = MS;
+        parts = p.nsplit;
+    } else {
+        const uint32_t hq = row - b * (p.heads * p.seq_q), head = hq / p.seq_q, qi = hq - head * p.seq_q;
+        const uint32_t ir = qi * p.group + head % p.group;
+        const int2 span = p.spans[b * p.kv_heads + head / p.group];
+        if (span.y == 1) return;                       // one CTA saw all of it and wrote the row
+        base0 = p.part + ((size_t)(span.x * 2 + 1) * p.rpb + ir) * MS;
+        base1 = p.part + ((size_t)(span.x * 2 + 2) * p.rpb + ir) * MS;
+        step = (size_t)2 * p.rpb * MS;
+        parts = (uint32_t)span.y;
+    }
+    auto part = [&](uint32_t s) { return s == 0 ? base0 : base1 + (size_t)(s - 1u) * step; };
     if (threadIdx.x < 32) {
         float M = ATT_NEG;
-        for (uint32_t s = threadIdx.x; s < nsplit; s += 32) M = fmaxf(M, base[(size_t)s * MS + D]);
+        for (uint32_t s = threadIdx.x; s < parts; s += 32) M = fmaxf(M, part(s)[D]);
         for (int off = 16; off; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
         float L = 0.0f;
-        for (uint32_t s = threadIdx.x; s < nsplit; s += 32) {
-            const float w = exp2f(base[(size_t)s * MS + D] - M);
+        for (uint32_t s = threadIdx.x; s < parts; s += 32) {
+            const float w = exp2f(part(s)[D] - M);
             wgt[s] = w;
-            L = fmaf(base[(size_t)s * MS + D + 1], w, L);
+            L = fmaf(part(s)[D + 1], w, L);
         }
         for (int off = 16; off; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
         if (threadIdx.x == 0) {
@@ -437,10 +551,10 @@ __global__ void __launch_bounds__(128) lux_attn_merge_f32(const float* __restric
     const float L = stat[1], inv = L > 0.0f ? 1.0f / L : 0.0f;
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         float acc = 0.0f;
-        for (uint32_t s = 0; s < nsplit; s++) acc = fmaf(base[(size_t)s * MS + d], wgt[s], acc);
-        out[(size_t)row * D + d] = acc * inv;
+        for (uint32_t s = 0; s < parts; s++) acc = fmaf(part(s)[d], wgt[s], acc);
+        p.out[(size_t)row * D + d] = acc * inv;
     }
-    if (threadIdx.x == 0 && lse) lse[row] = L > 0.0f ? fmaf(stat[0], ATT_LN2, logf(L)) : -3.402823e+38f;
+    if (threadIdx.x == 0 && p.lse) p.lse[row] = L > 0.0f ? fmaf(stat[0], ATT_LN2, logf(L)) : -3.402823e+38f;
 }
 
 // Any head_dim, any alignment: one CTA per output row, 256 keys per step (a thread per key for the
@@ -670,12 +784,13 @@ AttnKernel pick_stream(int vpl, int rt, bool full) {
 bool prefill_fits(const AttnParams& p) {
     return !p.block_size && p.head_dim == 128 && aligned16(p.out) && (uint64_t)p.batch * p.heads * ((p.seq_q + 127ull) / 128u) <= 0x7fffffffu;
 }
-// Which of the two kernels is the faster one, by what each takes in us on 148 SMs.  Over 178 shapes (64 .. 2049
-// queries, 64 .. 16384 keys, 4 .. 64 heads, batch 1 .. 8) the choice is nowhere slower than the streaming kernel by more
-// than 3 %, and at most 14 % slower than the faster of the two.
-// The prompt kernel: a CTA per SM owns 128 queries of a head and walks all their keys, 5.5 us a tile of 32, 4.6 where half
-// of its warps have no rows.  32 heads over 4096 keys, prompt / streaming: 65 rows 708 / 225 us, 128 712 /
-// 433, 200 709 / 647, 256 712 / 848, 512 713 / 1627.
+// Which of the two kernels answers a call: by what the streaming kernel takes in us on 148 SMs and what the prompt kernel
+// took when its products were mma.sync ones.  Over 178 shapes (64 .. 2049 queries, 64 .. 16384 keys, 4 .. 64 heads,
+// batch 1 .. 8) that choice was nowhere slower than the streaming kernel by more than 3 %.  The prompt kernel has become two to
+// four times faster since (attention_prefill_mma.cu), so it is the faster one wherever it is chosen; the line has stayed, and with
+// it which kernel, and so which order of sums, a call gets.
+// The mma.sync form: a CTA per SM owned 128 queries of a head and walked all their keys, 5.5 us a tile of 32, 4.6 where half
+// of its warps had no rows.
 double prefill_us(const AttnParams& p, int sms) {
     double total = 0.0, longest = 0.0;
     uint64_t blocks = 0;
@@ -729,6 +844,7 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     const int rt = R >= 2 && vpl <= 4 ? 2 : 1;
     p.rgp = pow2ceil(std::min<uint32_t>((R + rt - 1) / rt, ATT_CW));
     const uint32_t rpb = rt * p.rgp;
+    p.rpb = rpb;
     p.row_blocks = (R + rpb - 1) / rpb;
     const size_t items = (size_t)p.batch * p.kv_heads * p.row_blocks;
     // Slices of the keys.  CTAs run two per SM, so the grid should fill whole waves of 2 x SMs; a slice
@@ -741,7 +857,7 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     uint32_t min_split = 1;
     if (p.block_size) {
         // a slice (a multiple of the chunk) spans at most split_keys / block_size + 2 pages
-        const uint64_t cap = (uint64_t)(ATT_TABLE - 2) * p.block_size / ATT_CK * ATT_CK;
+        const uint64_t cap = ATT_PAGES / 256 * p.block_size / ATT_CK * ATT_CK;
         min_split = (uint32_t)std::max<uint64_t>((max_keys + cap - 1) / cap, 1);
     }
     uint32_t best = min_split;
@@ -776,16 +892,35 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     }
     geometry(g_tune.attn_splits > 0 ? std::max<uint32_t>((uint32_t)g_tune.attn_splits, min_split) : best);
     if (p.nsplit > 256) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;     // a context beyond 256 x 2046 pages
-    const size_t part_bytes = p.nsplit > 1 ? out_rows * p.nsplit * (D + 2) * 4 : 0;
-    if (part_bytes > ctx->d_attn_bytes) {
-        // fewer slices than wanted rather than an allocation inside a call
-        const uint32_t fit = (uint32_t)(ctx->d_attn_bytes / (out_rows * (D + 2) * 4));
-        if (std::max(fit, 1u) < min_split) return LUX_BACKEND_ERROR_OUT_OF_MEMORY;
-        geometry(std::max(fit, 1u));
+    // A decode step deals its chunks out evenly over one wave of CTAs, wherever its items begin and end.  A share is no
+    // shorter than the shortest slice above.
+    const uint32_t slots = (uint32_t)ctx->sm_count * (D > 128 ? 1 : ATT_CTAS_PER_SM);
+    const uint32_t last_keys = p.causal ? (uint32_t)std::min<uint64_t>((uint64_t)p.causal_base + p.seq_q, p.kv_len) : p.kv_len;
+    const uint32_t n = (std::min(max_keys, last_keys) + ATT_CK - 1) / ATT_CK, least = max_keys <= 512 ? 2 : 4;
+    const uint64_t all = (uint64_t)items * n;
+    const size_t even_part = (size_t)slots * 2 * rpb * (D + 2) * 4;
+    size_t ctas = items * p.nsplit;
+    bool merge = p.nsplit > 1;
+    if (p.row_blocks == 1 && n && all < (1u << 31) && !g_tune.attn_splits && slots <= ATT_MAX_PARTS &&
+        even_part + items * sizeof(int2) <= ctx->d_attn_bytes) {
+        p.share = p.block_size ? least : std::max<uint32_t>(least, (uint32_t)((all + slots - 1) / slots));
+        ctas = std::min<uint64_t>((all + p.share - 1) / p.share, slots);
+        merge = p.block_size || p.share % n != 0;
+        p.part = (float*)ctx->d_attn;
+        p.spans = (int2*)((unsigned char*)ctx->d_attn + even_part);
+    } else if (merge) {
+        if (out_rows * p.nsplit * (D + 2) * 4 > ctx->d_attn_bytes) {
+            // fewer slices than wanted rather than an allocation inside a call
+            const uint32_t fit = (uint32_t)(ctx->d_attn_bytes / (out_rows * (D + 2) * 4));
+            if (std::max(fit, 1u) < min_split) return LUX_BACKEND_ERROR_OUT_OF_MEMORY;
+            geometry(std::max(fit, 1u));
+            ctas = items * p.nsplit;
+            merge = p.nsplit > 1;
+        }
+        p.part = (float*)ctx->d_attn;
     }
-    p.part = p.nsplit > 1 ? (float*)ctx->d_attn : nullptr;
     const size_t stage_bytes = (size_t)2 * ATT_CK * D * 4;
-    const size_t fixed = ATT_HEADER + (p.block_size ? ATT_TABLE * 4 : 0);
+    const size_t fixed = ATT_HEADER + att_merge_floats(D, rt) * 4;
     // heads wider than 128 take the whole SM's shared memory (one CTA per SM)
     const size_t budget = D > 128 ? 2 * ATT_SMEM_BUDGET : ATT_SMEM_BUDGET;
     p.stages = (uint32_t)std::min<size_t>(ATT_MAX_STAGES, (budget - fixed) / stage_bytes);
@@ -804,14 +939,12 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
             done = true;
         }
     }
-    const size_t ctas = items * p.nsplit;
     if (ctas > 0x7fffffffu) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     cudaError_t e = launch_pdl(g_tune.pdl != 2, kfn, dim3((unsigned)ctas), dim3(ATT_THREADS), smem, ctx->stream, 1, p);
     if (e != cudaSuccess) return map_cuda(e, what);
     count_launch("lux_attn_stream_f32");
-    if (p.nsplit > 1) {
-        e = launch_pdl(g_tune.pdl != 2, lux_attn_merge_f32, dim3((unsigned)out_rows), dim3(128), 0, ctx->stream, 1, (const float*)p.part,
-                                   p.out, p.lse, p.context_lens, p.heads * p.seq_q, p.nsplit, D);
+    if (merge) {
+        e = launch_pdl(g_tune.pdl != 2, lux_attn_merge_f32, dim3((unsigned)out_rows), dim3(128), 0, ctx->stream, 1, p);
         if (e != cudaSuccess) return map_cuda(e, what);
         count_launch("lux_attn_merge_f32");
     }
