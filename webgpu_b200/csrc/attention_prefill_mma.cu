@@ -69,7 +69,7 @@ constexpr uint32_t T_QH = 0, T_QM = 64, T_S = 128, T_P = 256, T_O = 384;
 constexpr float NEG = -3.0e38f, LN2 = 0.6931471805599453f;
 constexpr float RAISE = 8.0f;             // the running maximum is raised when a score passes it by more: weights below 2^8
 constexpr float P_SCALE = 0x1p30f;        // of the weights before they are split
-constexpr float CHAIN_LOSS = 0x1p-24f;    // taken off half of the denominator: what the weighted sum's chains lose on average
+constexpr float CHAIN_LOSS = 0x1p-24f;    // taken off the denominators: what the chains of the weighted sum lose on average (5 to 6e-8)
 constexpr uint32_t TOO_LARGE = (127u + 60u) << 23;           // |x| >= 2^60, infinity or NaN, as bits
 constexpr uint32_t TOO_SMALL = (127u - 100u) << 23;          // 0 < |v| < 2^-100
 constexpr uint32_t FLAG_BAD = 1u, FLAG_TINY = 2u;            // of a tile of K or V
@@ -450,7 +450,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
                 }
                 float x, y;
                 unpair(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), x, y);
-                l = fmaf(x, 1.0f - CHAIN_LOSS, l + y);
+                l = fmaf(x + y, 1.0f - CHAIN_LOSS, l);
             }
             // the weighted sum before this one has read its weights
             if (t && !warp_wait(o_full, (t - 1u) & 1u, abort_flag, lane)) break;
