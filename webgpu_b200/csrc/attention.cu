@@ -24,10 +24,11 @@
 //     With every warp polling its mbarrier the kernel ran at 2.2-5.1 TB/s depending on how many
 //     warps happened to be waiting; parked, at 5.0-6.5 TB/s on the same shapes (polls travel the same
 //     queue as shared-memory loads and shuffles, and starved the warps that had work);
-//   * a decode step is one wave of CTAs, each with the same number of chunks of the (sequence, KV head) items laid end to
-//     end, so that a CTA may finish one item and begin the next; for a paged cache each CTA works out its share from
-//     the lengths.  Blocks of more rows split their keys over CTAs where whole items would leave SM slots idle.
-//     A small second kernel, resident early through programmatic dependent launch, merges what several CTAs did of a row.
+//   * keys are split over CTAs when there are fewer (sequence, KV head) pairs than SM slots, and each CTA walks its chunks
+//     from a different starting point.  A decode step over a paged cache, whose sequences differ in length, is one wave of
+//     CTAs, each with the same number of chunks of the (sequence, KV head) items laid end to end, so that a CTA may finish
+//     one item and begin the next.  A small second kernel, resident early through programmatic dependent launch, merges
+//     what several CTAs did of a row.
 // The one polling wait is bounded: if it gives up it sets the CTA's abort flag, every warp leaves
 // its loop (the consumers first release the stages the producer may be parked on), the device
 // status word reports 0x7C050008 and the output of that CTA is not written.
@@ -52,6 +53,7 @@ constexpr int ATT_CK = 32;                      // keys per staged chunk
 constexpr int ATT_MAX_STAGES = 6;
 constexpr int ATT_CTAS_PER_SM = 2;
 constexpr uint64_t ATT_PAGES = 256ull * 2046;   // pages of the longest context taken
+constexpr uint32_t ATT_EVEN_KEYS = 992;         // EVEN: from so many keys per sequence on
 constexpr int ATT_HEADER = 512;                 // barriers, abort flag, from byte 128 on each consumer warp's Piece
 // floats in which the warps of a row group leave their results: [warp][row][head_dim + 2], in whole 128-byte lines
 __host__ __device__ constexpr uint32_t att_merge_floats(uint32_t head_dim, uint32_t rt) { return (ATT_CW * rt * (head_dim + 2u) + 31u) / 32u * 32u; }
@@ -81,9 +83,9 @@ struct AttnParams {
     uint32_t rgp;                // row groups per CTA (1, 2, 4 or 8): rows per CTA = RT * rgp
     uint32_t rpb;                // rows per CTA
     uint32_t row_blocks, nsplit, split_keys, stages;
-    // One block of rows per KV head (a decode step): all 32-key chunks of all (sequence, KV head) items, one after the
-    // other, are dealt out evenly, each CTA taking the next `share` of them (0: the grid is one CTA per slice instead).
-    uint32_t share;              // contiguous: chunks per CTA; paged: the least, the lengths being known on the device only
+    // EVEN kernels (a decode step over a paged cache): all 32-key chunks of all (sequence, KV head) items, one after the other, are
+    // dealt out evenly, each CTA taking the next so many of them, `share` at least (0: one CTA per slice of an item).
+    uint32_t share;
     int2* spans;                 // per item: its first CTA and how many CTAs work on it
     float qscale;                // scale * log2(e)
 };
@@ -116,12 +118,16 @@ __device__ __forceinline__ uint32_t chunks_of(uint32_t keys) { return (keys + AT
 // What a CTA does next: chunks [lo, hi) of the n that the rows of (b, g, rb) see.
 struct Piece {
     uint32_t b, g, rb, kv_len, lmax, lo, hi, n;
+    uint32_t ahead;              // EVEN: keys of the next sequence, asked for early
     __device__ __forceinline__ void load(const volatile Piece* s) {
-        b = s->b; g = s->g; rb = s->rb; kv_len = s->kv_len; lmax = s->lmax; lo = s->lo; hi = s->hi; n = s->n;
+        b = s->b; g = s->g; rb = s->rb; kv_len = s->kv_len; lmax = s->lmax; lo = s->lo; hi = s->hi; n = s->n; ahead = s->ahead;
     }
+    // Every CTA walks the chunks of a piece from a different starting point (and wraps around), so that the CTAs of a wave,
+    // which start together and advance at the same pace, are not all at the same offset of equally spaced slices.
+    __device__ __forceinline__ uint32_t start() const { return hi > lo ? lo + (blockIdx.x * 2654435761u >> 8) % (hi - lo) : lo; }
 };
 
-template <int VPL, int RT, bool FULL>
+template <int VPL, int RT, bool FULL, bool EVEN>
 __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_f32(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t bar_full = smem_u32(smem);
@@ -139,76 +145,64 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
     // so a block of rows holds neighbouring queries and a causal block stops at its last row's keys
     const uint32_t R = p.group * p.seq_q, rpb = RT * p.rgp;
     Piece first;
-    uint32_t total = 0u, share = p.share;      // chunks of this CTA; of every CTA
-    auto measure = [&](Piece& w) {             // what the rows of (b, g, rb) see
-        w.kv_len = p.block_size ? paged_len(p, w.b) : p.kv_len;
-        w.lmax = row_len(p, (min(R, (w.rb + 1u) * rpb) - 1u) / p.group, w.kv_len);
+    uint32_t total = 0u, share = 0u;           // chunks of this CTA; of every CTA
+    auto extent = [&](Piece& w, uint32_t kv_len) {   // what the rows of (b, g, rb) see
+        w.kv_len = kv_len;
+        w.lmax = row_len(p, (min(R, (w.rb + 1u) * rpb) - 1u) / p.group, kv_len);
         w.n = chunks_of(w.lmax);
     };
-    if (!p.share) {
+    if constexpr (!EVEN) {
         uint32_t idx = blockIdx.x;
         const uint32_t split = idx % p.nsplit; idx /= p.nsplit;
         first.rb = idx % p.row_blocks; idx /= p.row_blocks;
         first.g = idx % p.kv_heads;
         first.b = idx / p.kv_heads;
         if (p.block_size && p.context_lens[first.b] <= 0) return;          // paged.wgsl:66-67: the rows stay as they are
-        measure(first);
+        extent(first, p.block_size ? paged_len(p, first.b) : p.kv_len);
         first.lo = min(split * (p.split_keys / ATT_CK), first.n);
         first.hi = min(first.lo + p.split_keys / ATT_CK, first.n);
         total = first.hi - first.lo;
     } else {
-        first.rb = 0u;
-        uint32_t all, at;                      // chunks of the call; the first one of this CTA
-        if (!p.block_size) {
-            first.b = 0u;
-            measure(first);
-            all = p.batch * p.kv_heads * first.n;
-            at = blockIdx.x * share;
-            const uint32_t item = at / first.n;
-            first.b = item / p.kv_heads;
-            first.g = item - first.b * p.kv_heads;
-            first.lo = at - item * first.n;
-        } else {
-            // every warp for itself, 32 sequences at a time: the sum, then the sequence in which this CTA starts
-            uint32_t sum = 0u;
-            for (uint32_t b0 = 0; b0 < p.batch; b0 += 32) sum += b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
-            for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-            all = sum * p.kv_heads;
-            share = max(share, (all + gridDim.x - 1u) / gridDim.x);
-            at = blockIdx.x * share;
-            if (at >= all) return;
-            uint32_t before = 0u;
-            for (uint32_t b0 = 0;; b0 += 32) {
-                const uint32_t n = b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
-                uint32_t upto = n;             // inclusive
-                for (int off = 1; off < 32; off <<= 1) {
-                    const uint32_t v = __shfl_up_sync(0xffffffffu, upto, off);
-                    if (lane >= off) upto += v;
-                }
-                const uint32_t hit = __ballot_sync(0xffffffffu, (before + upto) * p.kv_heads > at);
-                if (hit) {
-                    const int src = __ffs(hit) - 1;
-                    first.b = b0 + src;
-                    before += __shfl_sync(0xffffffffu, upto - n, src);
-                    break;
-                }
-                before += __shfl_sync(0xffffffffu, upto, 31);
+        // every warp for itself, 32 sequences at a time: the sum, then the sequence in which this CTA starts
+        uint32_t sum = 0u;
+        for (uint32_t b0 = 0; b0 < p.batch; b0 += 32) sum += b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
+        for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        const uint32_t all = sum * p.kv_heads;
+        share = max(p.share, (all + gridDim.x - 1u) / gridDim.x);
+        const uint32_t at = blockIdx.x * share;
+        if (at >= all) return;
+        uint32_t before = 0u;
+        for (uint32_t b0 = 0;; b0 += 32) {
+            const uint32_t n = b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
+            uint32_t upto = n;                 // inclusive
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, upto, off);
+                if (lane >= off) upto += v;
             }
-            measure(first);
-            const uint32_t in = at - before * p.kv_heads;
-            first.g = in / first.n;
-            first.lo = in - first.g * first.n;
+            const uint32_t hit = __ballot_sync(0xffffffffu, (before + upto) * p.kv_heads > at);
+            if (hit) {
+                const int src = __ffs(hit) - 1;
+                first.b = b0 + src;
+                before += __shfl_sync(0xffffffffu, upto - n, src);
+                break;
+            }
+            before += __shfl_sync(0xffffffffu, upto, 31);
         }
+        first.rb = 0u;
+        extent(first, paged_len(p, first.b));
+        first.ahead = first.b + 1u < p.batch ? paged_len(p, first.b + 1u) : 0u;
+        const uint32_t in = at - before * p.kv_heads;
+        first.g = in / first.n;
+        first.lo = in - first.g * first.n;
         total = min(share, all - at);
         first.hi = min(first.lo + total, first.n);
     }
     auto next = [&](Piece& w, uint32_t left) { // the piece after w, `left` chunks still to do
         if (++w.g == p.kv_heads) {
             w.g = 0u;
-            do {
-                w.b++;
-                if (p.block_size) measure(w);
-            } while (w.n == 0u);               // (left > 0: there is one)
+            extent(w, w.ahead);
+            for (w.b++; w.n == 0u;) extent(w, paged_len(p, ++w.b));        // (left > 0: there is one)
+            w.ahead = w.b + 1u < p.batch ? paged_len(p, w.b + 1u) : 0u;
         }
         w.lo = 0u;
         w.hi = min(left, w.n);
@@ -247,8 +241,9 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                 }
             }
         };
-        if (p.block_size && total) lookup(w.lo * ATT_CK);
-        for (uint32_t c = 0, k = w.lo; c < total; c++) {
+        uint32_t k = w.start(), todo = w.hi - w.lo;
+        if (p.block_size && total) lookup(k * ATT_CK);
+        for (uint32_t c = 0; c < total; c++) {
             const uint32_t s = c % NS;
             if (c >= NS) {
                 named_bar_sync<ATT_BAR_FREE0>(s, ATT_THREADS);          // all consumer warps have left the stage
@@ -276,9 +271,11 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                     bulk_g2s(smem_u32(vs + (size_t)(ta - t0) * D), p.v + off, (tb - ta) * D * 4u, bar);
                 }
             }
-            if (++k == w.hi && c + 1 < total) {
+            if (++k == w.hi) k = w.lo;
+            if (EVEN && --todo == 0u && c + 1 < total) {
                 next(w, total - c - 1u);
-                k = 0u;
+                k = w.start();
+                todo = w.hi;
             }
             if (p.block_size && c + 1 < total) lookup(k * ATT_CK);
         }
@@ -410,8 +407,8 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             }
             named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);
             const uint32_t row0 = w.rb * rpb;
-            const bool whole = p.share ? w.lo == 0u && w.hi == w.n : p.nsplit == 1;
-            if (p.share && w.lo == 0u && tid == 0)                       // the item may go on in the CTAs after this one
+            const bool whole = EVEN ? w.lo == 0u && w.hi == w.n : p.nsplit == 1;
+            if (EVEN && w.lo == 0u && tid == 0)                       // the item may go on in the CTAs after this one
                 p.spans[w.b * p.kv_heads + w.g] = make_int2((int)blockIdx.x, (int)(1u + (w.n - w.hi + share - 1u) / share));
             for (uint32_t e = tid; e < rpb * D; e += ATT_CW * 32) {
                 const uint32_t ir = e / D, d = e - ir * D, r = row0 + ir;
@@ -433,8 +430,8 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                     if (d == 0 && p.lse) p.lse[orow] = L > 0.0f ? fmaf(M, ATT_LN2, logf(L)) : -3.402823e+38f;
                 } else {
                     // two places per CTA: the item in which its share begins, and the one that begins in its share
-                    const size_t slot = p.share ? (size_t)(blockIdx.x * 2u + (w.lo == 0u ? 1u : 0u)) * rpb + ir
-                                                : orow * p.nsplit + blockIdx.x % p.nsplit;
+                    const size_t slot = EVEN ? (size_t)(blockIdx.x * 2u + (w.lo == 0u ? 1u : 0u)) * rpb + ir
+                                             : orow * p.nsplit + blockIdx.x % p.nsplit;
                     float* dst = p.part + slot * MS;
                     dst[d] = acc;
                     if (d == 0) {
@@ -446,16 +443,11 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);                // before the next piece is merged
         };
         const uint32_t stage0 = smem_u32(stages), stage_bytes = 2u * ATT_CK * row_bytes, v_off = ATT_CK * row_bytes;
-        // The piece lies in shared memory while its chunks are worked on: the loop has no registers left for it.
-        Piece* const kept = reinterpret_cast<Piece*>(smem + 128) + warp;
-        Piece w = first;
         uint32_t c = 0;
-        for (bool ok = true; ok;) {
-            begin(w);
-            if (lane == 0) *kept = w;
-            __syncwarp();
-            const uint32_t t_end = min(w.hi * ATT_CK, w.lmax);
-            for (uint32_t t0 = w.lo * ATT_CK; t0 < t_end; t0 += ATT_CK, c++) {
+        auto walk = [&](const Piece& w) {                                // the chunks of a piece; false: a wait gave up
+            const uint32_t t_begin = w.lo * ATT_CK, t_end = min(w.hi * ATT_CK, w.lmax);
+            uint32_t t0 = w.start() * ATT_CK;
+            for (const uint32_t c_end = c + (w.hi - w.lo); c < c_end; c++) {
                 const uint32_t s = c % NS;
                 // one poller per CTA: warp 0 waits for the copies, the named barrier releases the other seven
                 if (warp == 0) warp_wait(bar_full + 8u * s, (c / NS) & 1u, abort_flag, lane);
@@ -463,8 +455,7 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                 if (*abort_flag) {
                     // the producer may be parked on the stages this warp would still have released
                     for (uint32_t cc = c; cc < c + NS && cc + NS < total; cc++) named_bar_arrive<ATT_BAR_FREE0>(cc % NS, ATT_THREADS);
-                    ok = false;
-                    break;
+                    return false;
                 }
                 const uint32_t nk = min((uint32_t)ATT_CK, t_end - t0);
                 const uint32_t kchunk = stage0 + s * stage_bytes + lane_off;
@@ -481,13 +472,29 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                 }
                 // done with the stage (not needed for the last NS chunks: nobody refills them)
                 if (c + NS < total) named_bar_arrive<ATT_BAR_FREE0>(s, ATT_THREADS);
+                t0 += ATT_CK;
+                if (t0 >= t_end) t0 = t_begin;
             }
-            if (!ok) break;
-            w.load(kept);
-            finish(w);                                                   // (a slice past the rows' keys leaves an empty result)
-            if (c == total) break;
-            next(w, total - c);
-            __syncwarp();
+            return true;
+        };
+        if constexpr (!EVEN) {
+            begin(first);
+            if (walk(first)) finish(first);                              // (a slice past the rows' keys leaves an empty result)
+        } else {
+            // the piece lies in shared memory while its chunks are worked on: the loop has no registers left for it
+            Piece* const kept = reinterpret_cast<Piece*>(smem + 128) + warp;
+            Piece w = first;
+            for (;;) {
+                begin(w);
+                if (lane == 0) *kept = w;
+                __syncwarp();
+                if (!walk(w)) break;
+                w.load(kept);
+                finish(w);
+                if (c == total) break;
+                next(w, total - c);
+                __syncwarp();
+            }
         }
     }
 
@@ -765,17 +772,18 @@ uint32_t pow2ceil(uint32_t v) {
 }
 
 using AttnKernel = void (*)(const AttnParams);
-template <int VPL, int RT> AttnKernel stream_kernel(bool full) {
-    return full ? lux_attn_stream_f32<VPL, RT, true> : lux_attn_stream_f32<VPL, RT, false>;
+template <int VPL, int RT> AttnKernel stream_kernel(bool full, bool even) {
+    if (even) return full ? lux_attn_stream_f32<VPL, RT, true, true> : lux_attn_stream_f32<VPL, RT, false, true>;
+    return full ? lux_attn_stream_f32<VPL, RT, true, false> : lux_attn_stream_f32<VPL, RT, false, false>;
 }
 // full: head_dim is exactly VPL * 32, so no lane has a column to skip
-AttnKernel pick_stream(int vpl, int rt, bool full) {
+AttnKernel pick_stream(int vpl, int rt, bool full, bool even) {
     switch (vpl * 10 + rt) {
-        case 11: return stream_kernel<1, 1>(full); case 12: return stream_kernel<1, 2>(full);
-        case 21: return stream_kernel<2, 1>(full); case 22: return stream_kernel<2, 2>(full);
-        case 31: return stream_kernel<3, 1>(full); case 32: return stream_kernel<3, 2>(full);
-        case 41: return stream_kernel<4, 1>(full); case 42: return stream_kernel<4, 2>(full);
-        case 81: return stream_kernel<8, 1>(full);
+        case 11: return stream_kernel<1, 1>(full, even); case 12: return stream_kernel<1, 2>(full, even);
+        case 21: return stream_kernel<2, 1>(full, even); case 22: return stream_kernel<2, 2>(full, even);
+        case 31: return stream_kernel<3, 1>(full, even); case 32: return stream_kernel<3, 2>(full, even);
+        case 41: return stream_kernel<4, 1>(full, even); case 42: return stream_kernel<4, 2>(full, even);
+        case 81: return stream_kernel<8, 1>(full, even);
     }
     return nullptr;
 }
@@ -892,20 +900,19 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     }
     geometry(g_tune.attn_splits > 0 ? std::max<uint32_t>((uint32_t)g_tune.attn_splits, min_split) : best);
     if (p.nsplit > 256) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;     // a context beyond 256 x 2046 pages
-    // A decode step deals its chunks out evenly over one wave of CTAs, wherever its items begin and end.  A share is no
-    // shorter than the shortest slice above.
-    const uint32_t slots = (uint32_t)ctx->sm_count * (D > 128 ? 1 : ATT_CTAS_PER_SM);
-    const uint32_t last_keys = p.causal ? (uint32_t)std::min<uint64_t>((uint64_t)p.causal_base + p.seq_q, p.kv_len) : p.kv_len;
-    const uint32_t n = (std::min(max_keys, last_keys) + ATT_CK - 1) / ATT_CK, least = max_keys <= 512 ? 2 : 4;
+    // A decode step over a paged cache deals its chunks out evenly over one wave of CTAs, wherever sequences begin and end
+    // (their lengths are known on the device only).  It costs a CTA some microseconds to end one item and begin another, so
+    // this is for caches that may hold 1000 keys of a sequence and more: equal items stay with the slices.
+    const uint32_t slots = (uint32_t)ctx->sm_count * (D > 128 ? 1 : ATT_CTAS_PER_SM), n = (max_keys + ATT_CK - 1) / ATT_CK;
     const uint64_t all = (uint64_t)items * n;
     const size_t even_part = (size_t)slots * 2 * rpb * (D + 2) * 4;
     size_t ctas = items * p.nsplit;
     bool merge = p.nsplit > 1;
-    if (p.row_blocks == 1 && n && all < (1u << 31) && !g_tune.attn_splits && slots <= ATT_MAX_PARTS &&
+    if (p.block_size && p.row_blocks == 1 && max_keys >= ATT_EVEN_KEYS && all < (1u << 31) && !g_tune.attn_splits && slots <= ATT_MAX_PARTS &&
         even_part + items * sizeof(int2) <= ctx->d_attn_bytes) {
-        p.share = p.block_size ? least : std::max<uint32_t>(least, (uint32_t)((all + slots - 1) / slots));
+        p.share = 4;                           // a share is no shorter than the shortest slice above
         ctas = std::min<uint64_t>((all + p.share - 1) / p.share, slots);
-        merge = p.block_size || p.share % n != 0;
+        merge = true;
         p.part = (float*)ctx->d_attn;
         p.spans = (int2*)((unsigned char*)ctx->d_attn + even_part);
     } else if (merge) {
@@ -926,13 +933,13 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     p.stages = (uint32_t)std::min<size_t>(ATT_MAX_STAGES, (budget - fixed) / stage_bytes);
     const size_t smem = fixed + p.stages * stage_bytes;
     const bool full = D == (uint32_t)vpl * 32u;
-    AttnKernel kfn = pick_stream(vpl, rt, full);
+    AttnKernel kfn = pick_stream(vpl, rt, full, p.share != 0);
     if (!kfn || p.stages < 2) return LUX_BACKEND_ERROR_INTERNAL;
     static std::mutex mu;
-    static bool attr_set[16][9][3][2];
+    static bool attr_set[16][9][3][2][2];
     {
         std::lock_guard<std::mutex> lk(mu);
-        bool& done = attr_set[ctx->device & 15][vpl][rt][full ? 1 : 0];
+        bool& done = attr_set[ctx->device & 15][vpl][rt][full ? 1 : 0][p.share ? 1 : 0];
         if (!done) {
             if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * ATT_SMEM_BUDGET)) != cudaSuccess)
                 return map_cuda(cudaGetLastError(), what);
@@ -965,7 +972,7 @@ size_t mul(std::initializer_list<uint64_t> v) {
 }  // namespace
 
 // entries of the kernel table (kernel_table.cu): the Llama-shaped instance of the streaming kernel
-const void* kernel_addr_attn_stream_f32() { return (const void*)lux_attn_stream_f32<4, 2, true>; }
+const void* kernel_addr_attn_stream_f32() { return (const void*)lux_attn_stream_f32<4, 2, true, false>; }
 const void* kernel_addr_attn_merge_f32() { return (const void*)lux_attn_merge_f32; }
 const void* kernel_addr_attn_plain_f32() { return (const void*)lux_attn_plain_f32; }
 const void* kernel_addr_rope_f32() { return (const void*)lux_rope_f32<uint32_t, 2>; }
