@@ -253,23 +253,3 @@ def test_wa_weights_at_a_16_byte_offset(ctx, backend, M):
     ctx.qmatmul(xb, off, yb, M, B.F16)
     assert backend.last_kernel_name() == "lux_qgemm_i4_tc_wa_f16"
     assert np.array_equal(yb.to_host(np.uint16, (M, 256)), base.view(np.uint16))
-
-
-@pytest.mark.parametrize("dtype", ["f16", "bf16"])
-@pytest.mark.parametrize("M", [17, 65, 128])
-@pytest.mark.parametrize("units", [1, 5, 6, 7, 13])
-def test_wa_tile_of_128_batch_rows(ctx, backend, dtype, M, units):
-    """One CTA per SM for up to 128 rows: a ring of six units, fewer and more units than slots; every ring depth and
-    number of converter groups gives the same bits."""
-    K = 128 * units
-    x = synth.activations(M, K, dtype, 52, f"wam.{M}.{K}")
-    layer = synth.int4_layer(256, K, 52, f"wam.{K}")
-    want = _oracle(x, layer)
-    base = None
-    for groups, stages in ((0, 0), (2, 6), (3, 4), (2, 3), (3, 2)):
-        with _Tuned(backend, gemm_tc_kernel=2, gemm_tc_splitk=1, gemm_wa_narrow=2, gemm_tc_groups=groups, gemm_tc_stages=stages):
-            y = _run(ctx, x, layer)
-        assert orc.rel_l2(y, want) < TOL_16
-        base = y if base is None else base
-        assert np.array_equal(y.view(np.uint16), base.view(np.uint16))
-    assert ctx.last_device_status() == 0

@@ -44,20 +44,17 @@ namespace {
 
 using namespace tcptx;
 
-// Three tile widths.  BN = 256 batch rows per CTA (= UMMA N = accumulator columns): one CTA per SM,
-// all 512 TMEM columns, 3 x 64 KB of x.  BN = 128 for batches of up to 128 rows: the columns and the shared memory that the
-// smaller accumulator and x tiles leave make the ring six units deep (6 x 64 columns, 6 x 32 KB).  BN = 64 for batches of up to 64 rows: 256 TMEM columns
+// Two tile widths.  BN = 256 batch rows per CTA (= UMMA N = accumulator columns): one CTA per SM,
+// all 512 TMEM columns, 3 x 64 KB of x.  BN = 64 for batches of up to 64 rows: 256 TMEM columns
 // (accumulator [0, 64) + A units [64, 256)) and 3 x 16 KB of x, so that TWO CTAs share an SM.  Below
 // ~128 batch rows the kernel is bound by its one MMA-issuing thread (wait + eight MMAs + commit per
 // 128 K whatever N is); a second CTA per SM is a second issuing thread per SM.
 constexpr int WA_BN = 256;                 // the wide tile (batch tiling of large batches uses it)
-constexpr int WA_BN_MID = 128;
 constexpr int WA_BN_SMALL = 64;
 constexpr int WA_A_COLS = BK / 2;          // TMEM columns of a converted 64-K block (2 K per column)
 constexpr int WA_UNIT_K = 128;             // K per ring slot: one quantization group = two 64-K blocks
 constexpr int WA_UNIT_A_COLS = 2 * WA_A_COLS;
-// ring depth: units of x in shared memory (192 KB per SM) and as many times 64 columns of A in TMEM
-__host__ __device__ constexpr int wa_units(int bn) { return bn == WA_BN_MID ? 6 : 3; }
+constexpr int WA_MAX_UNITS = 3;            // ring depth: 3 units of x in shared memory, 3 x 64 columns of A in TMEM
 constexpr int WA_MAX_GROUPS = 3;           // converter groups <= ring depth
 constexpr int WA_MAX_THREADS = (2 + 4 * WA_MAX_GROUPS) * 32;
 constexpr int WA_SMALL_THREADS = (2 + 4 * 2) * 32;   // the narrow tile always runs two converter groups
@@ -567,8 +564,8 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
         narrow = ctas > ctx->sm_count || g_tune.gemm_wa_narrow == 1;
     }
     if (narrow) ks = ks_narrow;
-    const int bn = narrow ? WA_BN_SMALL : a.M <= WA_BN_MID ? WA_BN_MID : WA_BN;
-    const int stages = g_tune.gemm_tc_stages >= 2 && g_tune.gemm_tc_stages <= wa_units(bn) ? g_tune.gemm_tc_stages : wa_units(bn);
+    const int bn = narrow ? WA_BN_SMALL : WA_BN;
+    const int stages = g_tune.gemm_tc_stages >= 2 && g_tune.gemm_tc_stages <= WA_MAX_UNITS ? g_tune.gemm_tc_stages : WA_MAX_UNITS;
     // Converter groups.  Up to 128 batch columns the MMAs of a unit take half the tensor time or less and the converters
     // are what the unit waits for: three groups (2 -> 3, M = 72: 11008 x 4096 f16 18.6 -> 17.3 us, bf16 22.2 -> 19.5,
     // 20480 x 4096 bf16 41.8 -> 36.5; M = 128 bf16 22.6 -> 21.2, f16 equal).  Wider batches lose 2 % with the third
@@ -617,9 +614,8 @@ LuxBackendError launch_qgemm_i4_tc_wa(Context* ctx, const QArgs& a) {
         return w32 ? go_w(bf_tag, sw_tag, bn_tag, std::true_type{}) : go_w(bf_tag, sw_tag, bn_tag, std::false_type{});
     };
     auto go_bn = [&](auto bf_tag, auto sw_tag) {
-        return bn == WA_BN_SMALL ? go(bf_tag, sw_tag, std::integral_constant<int, WA_BN_SMALL>{})
-             : bn == WA_BN_MID   ? go(bf_tag, sw_tag, std::integral_constant<int, WA_BN_MID>{})
-                                 : go(bf_tag, sw_tag, std::integral_constant<int, WA_BN>{});
+        return narrow ? go(bf_tag, sw_tag, std::integral_constant<int, WA_BN_SMALL>{})
+                      : go(bf_tag, sw_tag, std::integral_constant<int, WA_BN>{});
     };
     cudaError_t e;
     if (a.swiglu) e = bf16 ? go_bn(std::true_type{}, std::true_type{}) : go_bn(std::false_type{}, std::true_type{});
