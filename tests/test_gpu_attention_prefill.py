@@ -383,3 +383,35 @@ def test_keys_and_values_at_a_16_byte_offset(ctx, backend):
         ctx.sdpa(ctx.upload(q), bufs[1], bufs[3], ob, 1, 4, 2, 130, 200, 128, 1 / np.sqrt(128))
         assert backend.last_kernel_name() == "lux_attn_prefill_mma_f32"
     assert np.array_equal(ob.to_host(np.uint32, q.shape), want.view(np.uint32))
+
+
+def test_calls_on_two_streams_share_the_scratch_in_order(backend):
+    """Calls enqueued on one stream, then on another, without a wait: each keeps the bits that it has alone, though both
+    split their K and V into the same scratch."""
+    import torch
+    c = backend.create_context(0)
+    try:
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        data, want = [], []
+        for i, S in enumerate((1500, 700)):
+            t = [torch.from_numpy(x).cuda() for x in _qkv(60 + i, 1, 8, 2, S, S)]
+            t.append(torch.zeros_like(t[0]))
+            data.append((S, t, [c.wrap(x.data_ptr(), x.numel() * 4) for x in t]))
+        call = lambda S, b, fl: c.sdpa(*b, 1, 8, 2, S, S, 128, 1 / np.sqrt(128), flags=fl | B.FLAG_ATTN_CAUSAL)
+        with _Tuned(backend, attn_prefill=1):
+            torch.cuda.synchronize()
+            for S, t, b in data:
+                call(S, b, 0)
+                want.append(t[3].cpu().numpy().copy())
+                t[3].zero_()
+            torch.cuda.synchronize()
+            for _ in range(3):
+                for st, (S, t, b) in zip(streams, data):
+                    c.set_stream(st.cuda_stream)
+                    call(S, b, B.FLAG_NO_SYNC)
+        torch.cuda.synchronize()
+        for w, (S, t, b) in zip(want, data):
+            assert np.array_equal(t[3].cpu().numpy().view(np.uint32), w.view(np.uint32))
+    finally:
+        c.set_stream(0)
+        c.destroy()

@@ -29,6 +29,7 @@ LuxBackendError finish_op(Context* ctx, bool no_sync, const char* what) {
         return LUX_BACKEND_ERROR_DEVICE_LOST;
     }
     ctx->writer_pending = false;             // everything enqueued so far has completed
+    ctx->parts_pending = false;
     if (ctx->h_status && *(volatile uint32_t*)ctx->h_status != 0) {
         ctx->last_status = *(volatile uint32_t*)ctx->h_status;
         *(volatile uint32_t*)ctx->h_status = 0;
@@ -154,6 +155,7 @@ static void cuda_destroy_context(LuxBackendContext* context) {
     if (ctx->d_stage) cudaFree(ctx->d_stage);
     if (ctx->d_int) cudaFree(ctx->d_int);
     if (ctx->d_parts) cudaFree(ctx->d_parts);
+    if (ctx->parts_event) cudaEventDestroy(ctx->parts_event);
     if (ctx->d_attn) cudaFree(ctx->d_attn);
     if (ctx->d_splitk) cudaFree(ctx->d_splitk);
     if (ctx->d_absmax) cudaFree(ctx->d_absmax);
@@ -475,7 +477,21 @@ extern "C" {
 LuxBackendError lux_cuda_context_set_stream(LuxBackendContext* context, void* stream) {
     auto* ctx = as_ctx(context);
     if (!ctx) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
-    ctx->stream = stream ? reinterpret_cast<cudaStream_t>(stream) : ctx->own_stream;
+    const cudaStream_t next = stream ? reinterpret_cast<cudaStream_t>(stream) : ctx->own_stream;
+    if (next != ctx->stream && ctx->parts_pending) {
+        // A prompt's attention may still be reading its scratch on the old stream: what follows on the new one waits for
+        // it.  (Not across a capture, whose events belong to its graph.)
+        cudaStreamCaptureStatus a = cudaStreamCaptureStatusNone, b = cudaStreamCaptureStatusNone;
+        cudaSetDevice(ctx->device);
+        bool ok = cudaStreamIsCapturing(ctx->stream, &a) == cudaSuccess && cudaStreamIsCapturing(next, &b) == cudaSuccess;
+        if (ok && a == cudaStreamCaptureStatusNone && b == cudaStreamCaptureStatusNone) {
+            ok = (ctx->parts_event || cudaEventCreateWithFlags(&ctx->parts_event, cudaEventDisableTiming) == cudaSuccess) &&
+                 cudaEventRecord(ctx->parts_event, ctx->stream) == cudaSuccess && cudaStreamWaitEvent(next, ctx->parts_event, 0) == cudaSuccess;
+        }
+        if (!ok) cudaGetLastError();
+        ctx->parts_pending = false;
+    }
+    ctx->stream = next;
     return LUX_BACKEND_OK;
 }
 

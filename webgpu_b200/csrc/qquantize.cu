@@ -27,6 +27,8 @@
 #include "common.cuh"
 #include "round_div.cuh"
 
+#include <type_traits>
+
 namespace luxcuda {
 
 namespace {
@@ -37,31 +39,34 @@ struct QuantParams {
     void* scales;           // [N, G] f32 or f16
     uint8_t* zeros;         // int4 asymmetric: [N, ZS]; else null
     int N, K, G, ZS;
-    int x_dtype, scale_dtype;
+    int scale_dtype;
     int shifted;            // LUX_QQUANT_FLAG_SHIFTED
     int chunks_per_row;     // ceil(K / 256)
 };
 
-// W32: f32 and 32-byte aligned, a lane's eight elements by one load (by two 16-byte ones each of a warp's requests takes
-// half of every sector it touches)
-template <bool W32>
-__device__ __forceinline__ void load8(const QuantParams& p, size_t idx, float (&v)[8]) {
-    if (W32 || p.x_dtype == LUX_QDTYPE_F32) {
-        const float* src = reinterpret_cast<const float*>(p.x) + idx;
-        float4 a, b;
-        if (W32) {
-            load32(src, a, b);
-        } else {
-            a = __ldg(reinterpret_cast<const float4*>(src));
-            b = __ldg(reinterpret_cast<const float4*>(src) + 1);
-        }
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+// Where a lane's eight elements come from: f32 by one 32-byte load where the matrix is 32-byte aligned (by two 16-byte ones each of a
+// warp's requests takes half of every sector it touches), f16, bf16.
+enum Source { SRC_F32, SRC_F32_WIDE, SRC_F16, SRC_BF16 };
+template <int SRC>
+__device__ __forceinline__ void request8(const QuantParams& p, size_t idx, float4 (&r)[SRC <= SRC_F32_WIDE ? 2 : 1]) {
+    if constexpr (SRC == SRC_F32_WIDE) {
+        load32(reinterpret_cast<const float*>(p.x) + idx, r[0], r[1]);
+    } else if constexpr (SRC == SRC_F32) {
+        r[0] = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + idx));
+        r[1] = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + idx) + 1);
     } else {
-        const uint4 r = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.x) + idx));
-        const uint32_t u[4] = {r.x, r.y, r.z, r.w};
+        r[0] = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const uint16_t*>(p.x) + idx));
+    }
+}
+template <int SRC>
+__device__ __forceinline__ void widen8(const float4 (&r)[SRC <= SRC_F32_WIDE ? 2 : 1], float (&v)[8]) {
+    if constexpr (SRC <= SRC_F32_WIDE) {
+        v[0] = r[0].x; v[1] = r[0].y; v[2] = r[0].z; v[3] = r[0].w; v[4] = r[1].x; v[5] = r[1].y; v[6] = r[1].z; v[7] = r[1].w;
+    } else {
+        const uint32_t u[4] = {__float_as_uint(r[0].x), __float_as_uint(r[0].y), __float_as_uint(r[0].z), __float_as_uint(r[0].w)};
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            if (p.x_dtype == LUX_QDTYPE_F16) {
+            if (SRC == SRC_F16) {
                 const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&u[i]));
                 v[2 * i] = f.x; v[2 * i + 1] = f.y;
             } else {
@@ -75,13 +80,14 @@ __device__ __forceinline__ void load8(const QuantParams& p, size_t idx, float (&
 // BITS = 4: groups of 128 (16 lanes); BITS = 8: groups of 32 (4 lanes), symmetric only.
 // With a division per element, and the group's three per eight elements, the arithmetic took longer than the
 // memory: 14336 x 4096 f32 to int4 with zero-points 72 us (266 MB, 3.7 TB/s).  round_div.cuh divides only
-// next to half-integers and the group's divisions are spread over its lanes: 57 to 59 us (4.5 to 4.7 TB/s).
+// next to half-integers and the group's divisions are spread over its lanes: 57 to 59 us (4.5 to 4.7 TB/s); with 32-byte loads
+// 49.6 (5.4; timed alone, where 16-byte ones took 54.9).
 // A warp takes QCH consecutive 256-element chunks of a row and requests all of them before it
 // reduces the first: 4 KB in flight per warp, so that a streaming kernel with this little
 // arithmetic keeps HBM busy.
 constexpr int QCH = 4;
 
-template <int BITS, bool SYM, bool W32>
+template <int BITS, bool SYM, int SRC>
 __global__ void __launch_bounds__(256, 4) lux_qquantize(const QuantParams p) {
     constexpr int GL = BITS == 4 ? 16 : 4;                  // lanes per group
     const int lane = threadIdx.x & 31;
@@ -91,14 +97,20 @@ __global__ void __launch_bounds__(256, 4) lux_qquantize(const QuantParams p) {
     if (row >= (uint32_t)p.N) return;
     const size_t n = row;
     const int c0 = (int)(wid - row * wpr) * QCH;
-    float v[QCH][8];
+    // all requests before the first value is used (16-bit values widened one chunk at a time, each as it arrived, had one
+    // chunk of a warp in flight: 14336 x 4096 bf16 to int4 70 us, more than f32)
+    float4 raw[QCH][SRC <= SRC_F32_WIDE ? 2 : 1];
     bool live[QCH];
 #pragma unroll
     for (int ch = 0; ch < QCH; ch++) {
         const int k0 = (c0 + ch) * 256 + lane * 8;
         live[ch] = k0 < p.K;                                 // K is a multiple of the group size, so of 8
-        if (live[ch]) load8<W32>(p, n * (size_t)p.K + k0, v[ch]);
+        if (live[ch]) request8<SRC>(p, n * (size_t)p.K + k0, raw[ch]);
     }
+    float v[QCH][8];
+#pragma unroll
+    for (int ch = 0; ch < QCH; ch++)
+        if (live[ch]) widen8<SRC>(raw[ch], v[ch]);
     // group statistics of all chunks
     float mx[QCH], mn[QCH];
 #pragma unroll
@@ -176,8 +188,8 @@ __global__ void __launch_bounds__(256, 4) lux_qquantize(const QuantParams p) {
 
 }  // namespace
 
-const void* kernel_addr_qquantize_i4() { return (const void*)lux_qquantize<4, false, true>; }
-const void* kernel_addr_qquantize_i8() { return (const void*)lux_qquantize<8, true, true>; }
+const void* kernel_addr_qquantize_i4() { return (const void*)lux_qquantize<4, false, SRC_F32_WIDE>; }
+const void* kernel_addr_qquantize_i8() { return (const void*)lux_qquantize<8, true, SRC_F32_WIDE>; }
 
 }  // namespace luxcuda
 
@@ -210,17 +222,20 @@ extern "C" LuxBackendError lux_cuda_qquantize(LuxBackendContext* context, const 
     p.scales = bs->ptr;
     p.zeros = bz ? (uint8_t*)bz->ptr : nullptr;
     p.N = (int)N; p.K = (int)K; p.G = (int)G; p.ZS = (int)ZS;
-    p.x_dtype = (int)d->x_dtype;
     p.scale_dtype = (int)d->scale_dtype;
     p.shifted = (d->flags & LUX_QQUANT_FLAG_SHIFTED) ? 1 : 0;
     p.chunks_per_row = (int)((K + 255) / 256);
-    const bool w32 = d->x_dtype == LUX_QDTYPE_F32 && (reinterpret_cast<uintptr_t>(bx->ptr) & 31u) == 0;
+    const int src = d->x_dtype == LUX_QDTYPE_F16 ? SRC_F16 : d->x_dtype == LUX_QDTYPE_BF16 ? SRC_BF16
+                    : (reinterpret_cast<uintptr_t>(bx->ptr) & 31u) ? SRC_F32 : SRC_F32_WIDE;
     const size_t warps = N * (size_t)((p.chunks_per_row + QCH - 1) / QCH);
     const unsigned grid = (unsigned)((warps + 7) / 8);
     cudaSetDevice(ctx->device);
-    auto kfn = d->bits == 8 ? (w32 ? lux_qquantize<8, true, true> : lux_qquantize<8, true, false>)
-               : bz         ? (w32 ? lux_qquantize<4, false, true> : lux_qquantize<4, false, false>)
-                            : (w32 ? lux_qquantize<4, true, true> : lux_qquantize<4, true, false>);
+    auto pick = [&](auto of) {
+        constexpr int SRC = decltype(of)::value;
+        return d->bits == 8 ? lux_qquantize<8, true, SRC> : bz ? lux_qquantize<4, false, SRC> : lux_qquantize<4, true, SRC>;
+    };
+    auto kfn = src == SRC_F16 ? pick(std::integral_constant<int, SRC_F16>{}) : src == SRC_BF16 ? pick(std::integral_constant<int, SRC_BF16>{})
+               : src == SRC_F32 ? pick(std::integral_constant<int, SRC_F32>{}) : pick(std::integral_constant<int, SRC_F32_WIDE>{});
     kfn<<<grid, 256, 0, ctx->stream>>>(p);
     count_launch("lux_qquantize");
     ctx->writer_pending = true;          // cleared by the wait in finish_op unless NO_SYNC
