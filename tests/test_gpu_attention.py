@@ -402,12 +402,13 @@ def test_decode_at_bench_size_properties(ctx):
 
 
 @pytest.mark.parametrize("lens,H,Hkv,D,block_size,max_blocks", [
-    ([1] * 70, 8, 8, 128, 16, None),                        # pieces of one chunk, more than 32 sequences, shares of many items
+    ([1] * 70, 8, 8, 128, 16, 100),                         # pieces of one chunk, more than 32 sequences, shares of many items
     ([0] * 40 + [3000] + [0] * 33 + [33, 0, 64], 32, 8, 128, 16, None),      # a sequence far into the batch, empty ones around it
     ([31, 32, 33, 127, 128, 129, 2000] * 5, 32, 8, 128, 32, 4096),           # items that end and begin inside shares, a wide table
     ([700, 1, 5000], 4, 4, 64, 1, None),                    # one row per KV head, one key per page
     ([900, 1200], 32, 2, 128, 24, None),                    # sixteen rows per KV head, a page size that does not divide the chunk
-    ([640, 10], 6, 2, 256, 16, None)])                      # one CTA per SM
+    ([2000] * 3, 32, 8, 128, 20, None),                     # all as long as the table allows: slices
+    ([640, 10], 6, 2, 256, 16, 70)])                        # one CTA per SM
 def test_paged_decode_dealt_out_evenly(ctx, lens, H, Hkv, D, block_size, max_blocks):
     rng = np.random.default_rng(len(lens))
     q, kc, vc, table, cl = _paged_case(rng, lens, H, Hkv, D, block_size, max_blocks)

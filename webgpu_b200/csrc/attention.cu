@@ -84,9 +84,10 @@ struct AttnParams {
     uint32_t rpb;                // rows per CTA
     uint32_t row_blocks, nsplit, split_keys, stages;
     // EVEN kernels (a decode step over a paged cache): all 32-key chunks of all (sequence, KV head) items, one after the other, are
-    // dealt out evenly, each CTA taking the next so many of them, `share` at least (0: one CTA per slice of an item).
+    // dealt out evenly, each CTA taking the next so many of them, `share` at least (0: one CTA per slice of an item).  If
+    // all sequences are as long as the cache allows, the slices are dealt out instead: the same sums as over a contiguous cache.
     uint32_t share;
-    int2* spans;                 // per item: its first CTA and how many CTAs work on it
+    int2* spans;                 // per item: its first CTA and how many CTAs work on it; 0: slices
     float qscale;                // scale * log2(e)
 };
 
@@ -122,9 +123,9 @@ struct Piece {
     __device__ __forceinline__ void load(const volatile Piece* s) {
         b = s->b; g = s->g; rb = s->rb; kv_len = s->kv_len; lmax = s->lmax; lo = s->lo; hi = s->hi; n = s->n; ahead = s->ahead;
     }
-    // Every CTA walks the chunks of a piece from a different starting point (and wraps around), so that the CTAs of a wave,
+    // Every CTA (or slice: `key`) walks the chunks of a piece from a different starting point (and wraps around), so that the CTAs of a wave,
     // which start together and advance at the same pace, are not all at the same offset of equally spaced slices.
-    __device__ __forceinline__ uint32_t start() const { return hi > lo ? lo + (blockIdx.x * 2654435761u >> 8) % (hi - lo) : lo; }
+    __device__ __forceinline__ uint32_t start(uint32_t key) const { return hi > lo ? lo + (key * 2654435761u >> 8) % (hi - lo) : lo; }
 };
 
 template <int VPL, int RT, bool FULL, bool EVEN>
@@ -151,6 +152,16 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
         w.lmax = row_len(p, (min(R, (w.rb + 1u) * rpb) - 1u) / p.group, kv_len);
         w.n = chunks_of(w.lmax);
     };
+    bool slices = false;                       // EVEN: the slices of equal items, dealt out in turn
+    const uint32_t slice_count = p.batch * p.kv_heads * p.nsplit;
+    auto slice = [&](Piece& w, uint32_t i) {   // slice i, w's extent being set; kept in `ahead`
+        const uint32_t item = i / p.nsplit, chunks = p.split_keys / ATT_CK;
+        w.ahead = i;
+        w.b = item / p.kv_heads;
+        w.g = item - w.b * p.kv_heads;
+        w.lo = (i - item * p.nsplit) * chunks;
+        w.hi = min(w.lo + chunks, w.n);
+    };
     if constexpr (!EVEN) {
         uint32_t idx = blockIdx.x;
         const uint32_t split = idx % p.nsplit; idx /= p.nsplit;
@@ -165,14 +176,28 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
     } else {
         // every warp for itself, 32 sequences at a time: the sum, then the sequence in which this CTA starts
         uint32_t sum = 0u;
-        for (uint32_t b0 = 0; b0 < p.batch; b0 += 32) sum += b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
+        bool full = true;
+        for (uint32_t b0 = 0; b0 < p.batch; b0 += 32) {
+            const uint32_t n = b0 + lane < p.batch ? paged_len(p, b0 + lane) : 0u;
+            sum += chunks_of(n);
+            full = full && (b0 + lane >= p.batch || n == p.kv_len);
+        }
         for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        slices = __all_sync(0xffffffffu, full);
         const uint32_t all = sum * p.kv_heads;
         share = max(p.share, (all + gridDim.x - 1u) / gridDim.x);
         const uint32_t at = blockIdx.x * share;
-        if (at >= all) return;
         uint32_t before = 0u;
-        for (uint32_t b0 = 0;; b0 += 32) {
+        if (slices) {
+            if (blockIdx.x >= slice_count) return;
+            first.rb = 0u;
+            extent(first, p.kv_len);
+            slice(first, blockIdx.x);
+            for (uint32_t i = blockIdx.x; i < slice_count; i += gridDim.x) total += min(p.split_keys / ATT_CK, first.n - i % p.nsplit * (p.split_keys / ATT_CK));
+        } else if (at >= all) {
+            return;
+        }
+        for (uint32_t b0 = 0; !slices; b0 += 32) {
             const uint32_t n = b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
             uint32_t upto = n;                 // inclusive
             for (int off = 1; off < 32; off <<= 1) {
@@ -188,16 +213,22 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             }
             before += __shfl_sync(0xffffffffu, upto, 31);
         }
-        first.rb = 0u;
-        extent(first, paged_len(p, first.b));
-        first.ahead = first.b + 1u < p.batch ? paged_len(p, first.b + 1u) : 0u;
-        const uint32_t in = at - before * p.kv_heads;
-        first.g = in / first.n;
-        first.lo = in - first.g * first.n;
-        total = min(share, all - at);
-        first.hi = min(first.lo + total, first.n);
+        if (!slices) {
+            first.rb = 0u;
+            extent(first, paged_len(p, first.b));
+            first.ahead = first.b + 1u < p.batch ? paged_len(p, first.b + 1u) : 0u;
+            const uint32_t in = at - before * p.kv_heads;
+            first.g = in / first.n;
+            first.lo = in - first.g * first.n;
+            total = min(share, all - at);
+            first.hi = min(first.lo + total, first.n);
+        }
     }
     auto next = [&](Piece& w, uint32_t left) { // the piece after w, `left` chunks still to do
+        if (slices) {
+            slice(w, w.ahead + gridDim.x);
+            return;
+        }
         if (++w.g == p.kv_heads) {
             w.g = 0u;
             extent(w, w.ahead);
@@ -241,7 +272,7 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                 }
             }
         };
-        uint32_t k = w.start(), todo = w.hi - w.lo;
+        uint32_t k = w.start(slices ? w.ahead : blockIdx.x), todo = w.hi - w.lo;
         if (p.block_size && total) lookup(k * ATT_CK);
         for (uint32_t c = 0; c < total; c++) {
             const uint32_t s = c % NS;
@@ -274,8 +305,8 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             if (++k == w.hi) k = w.lo;
             if (EVEN && --todo == 0u && c + 1 < total) {
                 next(w, total - c - 1u);
-                k = w.start();
-                todo = w.hi;
+                k = w.start(slices ? w.ahead : blockIdx.x);
+                todo = w.hi - w.lo;
             }
             if (p.block_size && c + 1 < total) lookup(k * ATT_CK);
         }
@@ -408,8 +439,8 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);
             const uint32_t row0 = w.rb * rpb;
             const bool whole = EVEN ? w.lo == 0u && w.hi == w.n : p.nsplit == 1;
-            if (EVEN && w.lo == 0u && tid == 0)                       // the item may go on in the CTAs after this one
-                p.spans[w.b * p.kv_heads + w.g] = make_int2((int)blockIdx.x, (int)(1u + (w.n - w.hi + share - 1u) / share));
+            if (EVEN && w.lo == 0u && tid == 0)                          // the item may go on in the CTAs after this one
+                p.spans[w.b * p.kv_heads + w.g] = make_int2((int)blockIdx.x, slices && !whole ? 0 : (int)(1u + (w.n - w.hi + share - 1u) / share));
             for (uint32_t e = tid; e < rpb * D; e += ATT_CW * 32) {
                 const uint32_t ir = e / D, d = e - ir * D, r = row0 + ir;
                 if (r >= R) continue;
@@ -430,8 +461,9 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                     if (d == 0 && p.lse) p.lse[orow] = L > 0.0f ? fmaf(M, ATT_LN2, logf(L)) : -3.402823e+38f;
                 } else {
                     // two places per CTA: the item in which its share begins, and the one that begins in its share
-                    const size_t slot = EVEN ? (size_t)(blockIdx.x * 2u + (w.lo == 0u ? 1u : 0u)) * rpb + ir
-                                             : orow * p.nsplit + blockIdx.x % p.nsplit;
+                    const size_t slot = EVEN && !slices ? (size_t)(blockIdx.x * 2u + (w.lo == 0u ? 1u : 0u)) * rpb + ir
+                                        : EVEN          ? orow * p.nsplit + w.ahead % p.nsplit
+                                                        : orow * p.nsplit + blockIdx.x % p.nsplit;
                     float* dst = p.part + slot * MS;
                     dst[d] = acc;
                     if (d == 0) {
@@ -446,7 +478,7 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
         uint32_t c = 0;
         auto walk = [&](const Piece& w) {                                // the chunks of a piece; false: a wait gave up
             const uint32_t t_begin = w.lo * ATT_CK, t_end = min(w.hi * ATT_CK, w.lmax);
-            uint32_t t0 = w.start() * ATT_CK;
+            uint32_t t0 = w.start(slices ? w.ahead : blockIdx.x) * ATT_CK;
             for (const uint32_t c_end = c + (w.hi - w.lo); c < c_end; c++) {
                 const uint32_t s = c % NS;
                 // one poller per CTA: warp 0 waits for the copies, the named barrier releases the other seven
@@ -522,16 +554,16 @@ __global__ void __launch_bounds__(128) lux_attn_merge_f32(const AttnParams p) {
     const float *base0, *base1;
     size_t step;
     uint32_t parts;
-    if (!p.share) {
+    const uint32_t hq = row - b * (p.heads * p.seq_q), head = hq / p.seq_q, qi = hq - head * p.seq_q;
+    const int2 span = p.share ? p.spans[b * p.kv_heads + head / p.group] : make_int2(0, 0);
+    if (span.y == 1) return;                           // one CTA saw all of it and wrote the row
+    if (span.y == 0) {
         base0 = p.part + (size_t)row * p.nsplit * MS;
         base1 = base0 + MS;
         step = MS;
         parts = p.nsplit;
     } else {
-        const uint32_t hq = row - b * (p.heads * p.seq_q), head = hq / p.seq_q, qi = hq - head * p.seq_q;
         const uint32_t ir = qi * p.group + head % p.group;
-        const int2 span = p.spans[b * p.kv_heads + head / p.group];
-        if (span.y == 1) return;                       // one CTA saw all of it and wrote the row
         base0 = p.part + ((size_t)(span.x * 2 + 1) * p.rpb + ir) * MS;
         base1 = p.part + ((size_t)(span.x * 2 + 2) * p.rpb + ir) * MS;
         step = (size_t)2 * p.rpb * MS;
@@ -905,7 +937,7 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     // this is for caches that may hold 1000 keys of a sequence and more: equal items stay with the slices.
     const uint32_t slots = (uint32_t)ctx->sm_count * (D > 128 ? 1 : ATT_CTAS_PER_SM), n = (max_keys + ATT_CK - 1) / ATT_CK;
     const uint64_t all = (uint64_t)items * n;
-    const size_t even_part = (size_t)slots * 2 * rpb * (D + 2) * 4;
+    const size_t even_part = std::max((size_t)slots * 2 * rpb, out_rows * p.nsplit) * (D + 2) * 4 / 16 * 16 + 16;
     size_t ctas = items * p.nsplit;
     bool merge = p.nsplit > 1;
     if (p.block_size && p.row_blocks == 1 && max_keys >= ATT_EVEN_KEYS && all < (1u << 31) && !g_tune.attn_splits && slots <= ATT_MAX_PARTS &&
