@@ -135,8 +135,8 @@ __global__ void __launch_bounds__(256) lux_attn_split_kv(const float* __restrict
     const uint32_t t = blockIdx.x, bk = blockIdx.y, is_v = blockIdx.z, tid = threadIdx.x;
     if (tid == 0) seen = 0u;
     __syncthreads();
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();                          // after the wait: what comes next starts behind everything before this kernel
     const float* src = (is_v ? v : k) + ((size_t)(bk0 + bk) * kv_stride + (size_t)t * BN) * D;
     unsigned char* dst = parts + ((size_t)bk * gridDim.x + t) * TILE_BYTES + (is_v ? 2 * SLOT : 0);
     const uint32_t nk = min((uint32_t)BN, kv_len - t * BN);
@@ -247,7 +247,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot, quad = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    pdl_wait();
+    // Q comes from kernels before lux_attn_split_kv, which has waited for them before it let this one start: it may be read
+    // while K and V are still being split (from L2: this SM may have read an earlier call's).  Without keys nothing is split, and the wait comes first.
+    if (!geo.all_tiles) pdl_wait();
 
     // the ring: K0, K1, V0, K2, V1, ... in both CTAs, in the order in which the products read them
     auto slot_at = [&](uint32_t i) { return sb + OFF_RING + (i % SLOTS) * SLOT; };
@@ -259,8 +261,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         mbar_expect_tx(bar, SLOT);
         bulk_g2s(slot_at(i), tile0 + (size_t)t * TILE_BYTES + (is_k ? 0 : 2 * SLOT), SLOT, bar);
     };
-    if (warp == 9 && lane == 0)
-        for (uint32_t i = 0; i < min(entries, (uint32_t)SLOTS); i++) request(i);
+    if (warp == 9) {
+        pdl_wait();
+        if (lane == 0)
+            for (uint32_t i = 0; i < min(entries, (uint32_t)SLOTS); i++) request(i);
+    }
 
     // ---- Q: rows on lanes, scaled and split; warps 0..3 take columns 0..63, warps 4..7 the others ---------
     const uint32_t row = (uint32_t)((warp & 3) * 32 + lane);
@@ -271,7 +276,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         const float* src = p.q + (((size_t)b * p.heads + h) * p.seq_q + q0 + min(row, max(rows, 1u) - 1u)) * D + half * 64;
         float4 x[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) x[j] = rows ? __ldg(reinterpret_cast<const float4*>(src) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < 16; j++) x[j] = rows ? __ldcg(reinterpret_cast<const float4*>(src) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
         uint32_t top = 0u;
         unsigned char* ql = smem + OFF_QL + half * (BM * 128) + row * 128u;
 #pragma unroll
@@ -293,6 +298,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         tmem_st_wait();
         if (top >= TOO_LARGE) found = FLAG_BAD;
     }
+    pdl_wait();
     for (uint32_t i = tid; i < 2u * own_tiles; i += THREADS) found |= geo.flags[(size_t)bkl * geo.all_tiles * 2u + i];
     if (found) atomicOr(const_cast<uint32_t*>(seen), found);
     fence_proxy_async_smem();
