@@ -1,11 +1,13 @@
 // round_div.cuh -- clamp(rint(v / scale)) without a division per element, bit for bit the division's result.
 //
-// With ri = RN(1 / scale) and r = RN(v ri), r and RN(v / scale) are both within 1.5 * 2^-23 |v / scale| of each
-// other, so they round to the same integer unless r lies that close to a half-integer; only then (and
-// for NaN) is the division carried out.  Quotients that matter are at most 64 (4 bits) or 256 (8 bits) in
-// magnitude, which makes the distance 2^-16 or 2^-14; anything larger is clamped alike on both ways.
-// The rounding itself is the addition of 1.5 * 2^23, whose low mantissa bits then are the integer (FRND
-// and F2I run at a quarter of the rate of an add).
+// With ri = RN(1 / scale), v ri and RN(v / scale) are both within 1.5 * 2^-23 |v / scale| of each other, so they round to the
+// same integer unless v ri lies that close to a half-integer; only then (and for NaN) is the division carried
+// out.  Quotients that matter are at most 64 (4 bits) or 256 (8 bits) in magnitude, which makes the distance 2^-16 or
+// 2^-14; anything larger is clamped alike on both ways.
+// The rounding itself is the addition of 1.5 * 2^23 (FRND and F2I run at a quarter of the rate of an add), in one FMA with the
+// product; its low mantissa bits then are the integer.  How far v ri is from it, another FMA, is 1/2 at most, and only the
+// largest of a thread's distances is compared: six instructions an element, where a rounded product, clamped, rounded and
+// compared on its own took ten.
 #pragma once
 
 #include "common.cuh"
@@ -23,16 +25,16 @@ __device__ __forceinline__ bool round_div_ok(float scale) { return scale >= 0x1p
 template <int BITS, int N>
 __device__ __forceinline__ void round_div(const float (&v)[N], float scale, float ri, bool ok, int lo, int hi, int off, uint32_t (&t)[N]) {
     constexpr float NEAR = BITS == 4 ? 0x1p-16f : 0x1p-14f;
-    const float flo = (float)lo, fhi = (float)hi, add = ROUND_MAGIC + (float)off;
-    bool clear = ok;
+    const float add = ROUND_MAGIC + (float)off, flo = add + (float)lo, fhi = add + (float)hi;
+    float worst = 0.0f;
 #pragma unroll
     for (int i = 0; i < N; i++) {
-        const float r = __fmul_rn(v[i], ri);
-        const float y = __fadd_rn(fminf(fmaxf(r, flo), fhi), add);
-        const float d = __fsub_rn(r, __fsub_rn(y, add));
-        clear &= fabsf(__fsub_rn(fabsf(d), 0.5f)) > NEAR;      // false for NaN
-        t[i] = __float_as_uint(y);
+        const float y = __fmaf_rn(v[i], ri, add);
+        const float d = __fmaf_rn(v[i], ri, -__fsub_rn(y, add));
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(worst) : "f"(fabsf(d)));
+        t[i] = __float_as_uint(fminf(fmaxf(y, flo), fhi));
     }
+    const bool clear = ok && worst <= 0.5f - NEAR;            // false for NaN
     if (!clear) {
 #pragma unroll
         for (int i = 0; i < N; i++)
