@@ -33,11 +33,15 @@
 // Accumulation.  The tensor core cuts its f32 sums off at every step of 16 (measured on chains of 1 / 2 / 4 / 8 steps:
 // mean loss 1.1 / 2.4 / 4.9 / 9.4e-8 of the sum, in rms 2.5 / 3.9 / 6.5 / 11.6e-8), so chains are four steps of the large products, after
 // the small ones: a score is the f32 sum of two such chains, and the output is kept in f32 registers, to which each
-// tile of 64 keys is added by an ordinary rounded addition.
+// tile of 64 keys is added by an ordinary rounded addition.  What a chain loses on average is taken off the denominator too.
+// Relative error against 64 bits, in 1e-7 (2-norm, N(0, 1) inputs, Llama-3-8B heads; streaming kernel / mma.sync form of this
+// one / this one): causal, 150 tokens 1.37 / 1.06 / 1.05, 512 1.65 / 1.20 / 1.15, 2048 2.24 / 1.39 / 1.28; unmasked,
+// 700 x 3 3.07 / 1.76 / 1.56, 1448 4.03 / 2.02 / 1.76.
 //
-// Measured, Llama-3-8B heads, against mma.sync products with the splitting in every CTA (bound by that instruction, 568
-// TFLOP/s, and by the splitting): causal, 2048 tokens 674 -> 184 us (187 TFLOP/s of f32 products, 1.1 PFLOP/s of
-// bf16 ones), 512 tokens 95 -> 38, 150 tokens 28.6 -> 18.7; unmasked 1448 tokens 774 -> 182.
+// Measured, Llama-3-8B heads, against the form with mma.sync products and the splitting in every CTA (bound by that instruction,
+// 568 TFLOP/s, and by the splitting): causal, 2048 tokens 674 -> 177 us (194 TFLOP/s of f32 products, 1.17 PFLOP/s of
+// bf16 ones: 0.84 of what cuBLAS sustains under the power cap), 512 tokens 95 -> 34, 150 tokens 28.7 -> 18.3; unmasked
+// 1448 tokens 775 -> 176.  Two softmax warps per row instead of one: 175.5, so the tensor pipe is what is left.
 #include "attention_prefill_f32.cuh"
 
 #include <algorithm>
