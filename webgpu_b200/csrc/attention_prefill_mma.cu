@@ -280,7 +280,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         const float* src = p.q + (((size_t)b * p.heads + h) * p.seq_q + q0 + min(row, max(rows, 1u) - 1u)) * D + half * 64;
         float4 x[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) x[j] = rows ? __ldcg(reinterpret_cast<const float4*>(src) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < 16; j++) x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (rows && (reinterpret_cast<uintptr_t>(p.q) & 31u) == 0) {         // whole sectors at a time, as L1 does not keep them
+#pragma unroll
+            for (int j = 0; j < 16; j += 2)
+                asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                             : "=f"(x[j].x), "=f"(x[j].y), "=f"(x[j].z), "=f"(x[j].w), "=f"(x[j + 1].x), "=f"(x[j + 1].y), "=f"(x[j + 1].z), "=f"(x[j + 1].w)
+                             : "l"(src + 4 * j) : "memory");
+        } else if (rows) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) x[j] = __ldcg(reinterpret_cast<const float4*>(src) + j);
+        }
         uint32_t top = 0u;
         unsigned char* ql = smem + OFF_QL + half * (BM * 128) + row * 128u;
 #pragma unroll
