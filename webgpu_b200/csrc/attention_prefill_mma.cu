@@ -39,9 +39,10 @@
 // 700 x 3 3.07 / 1.76 / 1.56, 1448 4.03 / 2.02 / 1.76.
 //
 // Measured, Llama-3-8B heads, against the form with mma.sync products and the splitting in every CTA (bound by that instruction,
-// 568 TFLOP/s, and by the splitting): causal, 2048 tokens 674 -> 177 us (194 TFLOP/s of f32 products, 1.17 PFLOP/s of
-// bf16 ones: 0.84 of what cuBLAS sustains under the power cap), 512 tokens 95 -> 34, 150 tokens 28.7 -> 18.3; unmasked
-// 1448 tokens 775 -> 176.  Two softmax warps per row instead of one: 175.5, so the tensor pipe is what is left.
+// 568 TFLOP/s, and by the splitting): causal, 2048 tokens 674 -> 168 us (205 TFLOP/s of f32 products, 1.23 PFLOP/s of
+// bf16 ones: 0.89 of what cuBLAS sustains under the power cap), 512 tokens 95 -> 30.5, 150 tokens 28.7 -> 16.9; unmasked
+// 700 tokens x 3 511 -> 139.  The tensor pipe is busy for 62 % of the time, at 1.63 GHz; two softmax warps per row instead of one
+// gave 1 %.
 #include "attention_prefill_f32.cuh"
 
 #include <algorithm>
@@ -252,7 +253,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
     tc_fence_after();
     const uint32_t tmem = *tmem_slot, quad = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     // Q comes from kernels before lux_attn_split_kv, which has waited for them before it let this one start: it may be read
-    // while K and V are still being split (from L2: this SM may have read an earlier call's).  Without keys nothing is split, and the wait comes first.
+    // while K and V are still being split (from L2: this SM may have read an earlier call's; 512 tokens 33.4 -> 30.3 us).  Without keys nothing is split, and the wait comes first.
     if (!geo.all_tiles) pdl_wait();
 
     // the ring: K0, K1, V0, K2, V1, ... in both CTAs, in the order in which the products read them
@@ -281,7 +282,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         float4 x[16];
 #pragma unroll
         for (int j = 0; j < 16; j++) x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (rows && (reinterpret_cast<uintptr_t>(p.q) & 31u) == 0) {         // whole sectors at a time, as L1 does not keep them
+        if (rows && (reinterpret_cast<uintptr_t>(p.q) & 31u) == 0) {         // whole sectors at a time, as L1 does not keep them (2048 tokens 178 -> 168 us)
 #pragma unroll
             for (int j = 0; j < 16; j += 2)
                 asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
