@@ -624,7 +624,6 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
     geo.levels = geo.by_head ? p.q_blocks : (p.q_blocks + 1) / 2;
     const char* name = "lux_attn_prefill_mma_f32";
     cudaError_t e = allow_smem((const void*)lux_attn_prefill_mma_f32, 1, SMEM, ctx->device);
-    ctx->parts_pending = true;
     // as many (sequence, KV head) pairs at a time as have their parts in the scratch (in one call all, up to 128 k keys in total)
     for (geo.bk0 = 0; e == cudaSuccess && geo.bk0 < bks; geo.bk0 += geo.nbk) {
         geo.nbk = std::min(fit, bks - geo.bk0);

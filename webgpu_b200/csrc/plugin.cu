@@ -126,10 +126,12 @@ static LuxBackendContext* cuda_create_context(int device_index) {
     }
     if (ok) {
         ctx->d_parts_bytes = (size_t)131072 / 64 * ((64u * 1536u) + 8u);
-        ok = cudaMalloc(&ctx->d_parts, ctx->d_parts_bytes) == cudaSuccess;
+        ok = cudaMalloc(&ctx->d_parts, ctx->d_parts_bytes) == cudaSuccess &&
+             cudaEventCreateWithFlags(&ctx->parts_event, cudaEventDisableTiming) == cudaSuccess;
     }
     if (!ok) {
         cudaGetLastError();
+        if (ctx->parts_event) cudaEventDestroy(ctx->parts_event);
         if (ctx->d_parts) cudaFree(ctx->d_parts);
         if (ctx->d_attn) cudaFree(ctx->d_attn);
         if (ctx->d_splitk) cudaFree(ctx->d_splitk);
@@ -479,17 +481,13 @@ LuxBackendError lux_cuda_context_set_stream(LuxBackendContext* context, void* st
     if (!ctx) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     const cudaStream_t next = stream ? reinterpret_cast<cudaStream_t>(stream) : ctx->own_stream;
     if (next != ctx->stream && ctx->parts_pending) {
-        // A prompt's attention may still be reading its scratch on the old stream: what follows on the new one waits for
-        // it.  (Not across a capture, whose events belong to its graph.)
-        cudaStreamCaptureStatus a = cudaStreamCaptureStatusNone, b = cudaStreamCaptureStatusNone;
+        // A prompt's attention may still be reading its scratch: what follows on the new stream waits for it.  (Not into a
+        // capture, whose events belong to its graph; the old stream may be gone by now and is not touched.)
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
         cudaSetDevice(ctx->device);
-        bool ok = cudaStreamIsCapturing(ctx->stream, &a) == cudaSuccess && cudaStreamIsCapturing(next, &b) == cudaSuccess;
-        if (ok && a == cudaStreamCaptureStatusNone && b == cudaStreamCaptureStatusNone) {
-            ok = (ctx->parts_event || cudaEventCreateWithFlags(&ctx->parts_event, cudaEventDisableTiming) == cudaSuccess) &&
-                 cudaEventRecord(ctx->parts_event, ctx->stream) == cudaSuccess && cudaStreamWaitEvent(next, ctx->parts_event, 0) == cudaSuccess;
-        }
-        if (!ok) cudaGetLastError();
-        ctx->parts_pending = false;
+        if (cudaStreamIsCapturing(next, &st) != cudaSuccess ||
+            (st == cudaStreamCaptureStatusNone && cudaStreamWaitEvent(next, ctx->parts_event, 0) != cudaSuccess))
+            cudaGetLastError();
     }
     ctx->stream = next;
     return LUX_BACKEND_OK;
