@@ -184,10 +184,11 @@ template <int BASE> __device__ __forceinline__ void named_bar_arrive(uint32_t i,
 }
 #endif
 
-// 32 consecutive bytes of data that no kernel writes while this one runs, in one access (32-byte aligned)
+// 32 consecutive bytes in one access (32-byte aligned).  Volatile, with a clobber, and not a read of constant data (.nc): the
+// kernel before may still be writing them until pdl_wait() has returned, and a plain asm may move above that.
 __device__ __forceinline__ void load32(const void* src, float4& a, float4& b) {
-    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(src));
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(src) : "memory");
 }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
