@@ -37,6 +37,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "attention_span.h"
 #include "common.cuh"
 #include "tc_ptx.cuh"
 #include "lux/gpu/attention_ext.h"
@@ -87,7 +88,8 @@ struct AttnParams {
     // dealt out evenly, each CTA taking the next so many of them, `share` at least (0: one CTA per slice of an item).  If
     // all sequences are as long as the cache allows, the slices are dealt out instead: the same sums as over a contiguous cache.
     uint32_t share;
-    int2* spans;                 // per item: its first CTA and how many CTAs work on it; 0: slices
+    AttnSpan* spans;             // per item; ctas 0: slices
+    uint32_t ctas;               // of the grid
     float qscale;                // scale * log2(e)
 };
 
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             const uint32_t row0 = w.rb * rpb;
             const bool whole = EVEN ? w.lo == 0u && w.hi == w.n : p.nsplit == 1;
             if (EVEN && w.lo == 0u && tid == 0)                          // the item may go on in the CTAs after this one
-                p.spans[w.b * p.kv_heads + w.g] = make_int2((int)blockIdx.x, slices && !whole ? 0 : (int)(1u + (w.n - w.hi + share - 1u) / share));
+                p.spans[w.b * p.kv_heads + w.g] = AttnSpan{(int32_t)blockIdx.x, slices && !whole ? 0 : (int32_t)(1u + (w.n - w.hi + share - 1u) / share)};
             for (uint32_t e = tid; e < rpb * D; e += ATT_CW * 32) {
                 const uint32_t ir = e / D, d = e - ir * D, r = row0 + ir;
                 if (r >= R) continue;
@@ -555,19 +557,23 @@ __global__ void __launch_bounds__(128) lux_attn_merge_f32(const AttnParams p) {
     size_t step;
     uint32_t parts;
     const uint32_t hq = row - b * (p.heads * p.seq_q), head = hq / p.seq_q, qi = hq - head * p.seq_q;
-    const int2 span = p.share ? p.spans[b * p.kv_heads + head / p.group] : make_int2(0, 0);
-    if (span.y == 1) return;                           // one CTA saw all of it and wrote the row
-    if (span.y == 0) {
+    const AttnSpan span = p.share ? p.spans[b * p.kv_heads + head / p.group] : AttnSpan{0, 0};
+    if (span.ctas == 1) return;                        // one CTA saw all of it and wrote the row
+    if (span.ctas == 0) {
         base0 = p.part + (size_t)row * p.nsplit * MS;
         base1 = base0 + MS;
         step = MS;
         parts = p.nsplit;
     } else {
+        if (!span_fits(span, p.ctas)) {                // never written: a wait gave up in the CTA in which the item begins
+            if (threadIdx.x == 0 && p.status) atomicOr(p.status, ATT_STATUS_WAIT);
+            return;
+        }
         const uint32_t ir = qi * p.group + head % p.group;
-        base0 = p.part + ((size_t)(span.x * 2 + 1) * p.rpb + ir) * MS;
-        base1 = p.part + ((size_t)(span.x * 2 + 2) * p.rpb + ir) * MS;
+        base0 = p.part + ((size_t)span_place(span, 0) * p.rpb + ir) * MS;
+        base1 = p.part + ((size_t)span_place(span, 1) * p.rpb + ir) * MS;
         step = (size_t)2 * p.rpb * MS;
-        parts = (uint32_t)span.y;
+        parts = (uint32_t)span.ctas;
     }
     auto part = [&](uint32_t s) { return s == 0 ? base0 : base1 + (size_t)(s - 1u) * step; };
     if (threadIdx.x < 32) {
@@ -946,12 +952,12 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     size_t ctas = items * p.nsplit;
     bool merge = p.nsplit > 1;
     if (p.block_size && p.row_blocks == 1 && max_keys >= ATT_EVEN_KEYS && all < (1u << 31) && !g_tune.attn_splits && slots <= ATT_MAX_PARTS &&
-        even_part + items * sizeof(int2) <= ctx->d_attn_bytes) {
+        even_part + items * sizeof(AttnSpan) <= ctx->d_attn_bytes) {
         p.share = 4;                           // a share is no shorter than the shortest slice above
         ctas = std::min<uint64_t>((all + p.share - 1) / p.share, slots);
         merge = true;
         p.part = (float*)ctx->d_attn;
-        p.spans = (int2*)((unsigned char*)ctx->d_attn + even_part);
+        p.spans = (AttnSpan*)((unsigned char*)ctx->d_attn + even_part);
     } else if (merge) {
         if (out_rows * p.nsplit * (D + 2) * 4 > ctx->d_attn_bytes) {
             // fewer slices than wanted rather than an allocation inside a call
@@ -984,6 +990,7 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
         }
     }
     if (ctas > 0x7fffffffu) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
+    p.ctas = (uint32_t)ctas;
     cudaError_t e = launch_pdl(g_tune.pdl != 2, kfn, dim3((unsigned)ctas), dim3(ATT_THREADS), smem, ctx->stream, 1, p);
     if (e != cudaSuccess) return map_cuda(e, what);
     count_launch("lux_attn_stream_f32");
