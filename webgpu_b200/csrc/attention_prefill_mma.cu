@@ -44,6 +44,7 @@
 // 700 tokens x 3 511 -> 139.  The tensor pipe is busy for 62 % of the time, at 1.63 GHz; two softmax warps per row instead of one
 // gave 1 %.
 #include "attention_prefill_f32.cuh"
+#include "attention_ring.h"
 
 #include <algorithm>
 
@@ -128,6 +129,25 @@ __device__ __forceinline__ uint32_t in_leader(uint32_t addr) {
 // first wait for every store of the thread (600 cycles and more, three times a tile: 235 -> 184 us at 2048 tokens without).
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Passes on to the leader what this thread has waited for: copies that have landed in this CTA's shared memory.
+__device__ __forceinline__ void arrive_release_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// mbar_wait that takes over what such an arrival passes on
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
+    for (uint32_t it = 0; it < WAIT_LIMIT; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((it & 31u) == 31u && *abort_flag) return false;
+    }
+    *abort_flag = 1u;
+    return false;
 }
 
 // The parts of a tile of K (blockIdx.z 0) or V (1), rows past the end as zeros, in the layout of the ring's slots:
@@ -259,12 +279,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
     // the ring: K0, K1, V0, K2, V1, ... in both CTAs, in the order in which the products read them
     auto slot_at = [&](uint32_t i) { return sb + OFF_RING + (i % SLOTS) * SLOT; };
     const uint32_t entries = 2u * tiles;
-    auto request = [&](uint32_t i) {              // entry i: K (i + 1) / 2 for odd i (the last one V), else V i / 2 - 1; K 0 first
-        const bool is_k = i == 0 || ((i & 1u) && i + 1u < entries);
-        const uint32_t t = i == 0 ? 0u : is_k ? (i + 1u) / 2u : i + 1u < entries ? i / 2u - 1u : tiles - 1u;
+    auto request = [&](uint32_t i) {
+        const RingEntry e = ring_entry(i, tiles);
         const uint32_t bar = kv_full(i % SLOTS);
         mbar_expect_tx(bar, SLOT);
-        bulk_g2s(slot_at(i), tile0 + (size_t)t * TILE_BYTES + (is_k ? 0 : 2 * SLOT), SLOT, bar);
+        bulk_g2s(slot_at(i), tile0 + (size_t)e.tile * TILE_BYTES + (e.is_v ? 2 * SLOT : 0), SLOT, bar);
     };
     if (warp == 9) {
         pdl_wait();
@@ -347,7 +366,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
             if (elect_one()) {
                 constexpr uint32_t id_s = idesc2(BN, false), id_o = idesc2(D, true);
                 uint32_t i = 0;                   // ring entry
-                auto take = [&]() { return mbar_wait(kv_full(i % SLOTS), (i / SLOTS) & 1u, abort_flag); };
+                auto take = [&]() { return mbar_wait_cluster(kv_full(i % SLOTS), (i / SLOTS) & 1u, abort_flag); };
+                // Only slots that are filled again are given back: an arrival in the second CTA that nobody there waits for
+                // could come after that CTA has ended.
+                auto give_back = [&]() {
+                    if (ring_refilled(i, entries, SLOTS)) commit2(kv_empty(i % SLOTS));
+                    i++;
+                };
                 auto scores = [&]() {
                     const uint64_t kd = make_kmajor_sw128_desc(slot_at(i)), ld = make_kmajor_sw128_desc(sb + OFF_QL);
                     tc_fence_after();
@@ -367,8 +392,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
                         }
                     }
                     commit2(s_full);
-                    commit2(kv_empty(i % SLOTS));
-                    i++;
+                    give_back();
                 };
                 auto weighted = [&]() {
                     // MN-major: rows of 128 bytes are keys, eight of them a swizzle atom, one atom column wide
@@ -382,8 +406,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
                             mma2_ts(tmem + T_O, tmem + T_P + a * 32 + s * 8, vd + (uint64_t)(w * (PART / 16) + s * (16 * 128 / 16)), id_o, (o | s) != 0);
                     }
                     commit2(o_full);
-                    commit2(kv_empty(i % SLOTS));
-                    i++;
+                    give_back();
                 };
                 bool ok = walk > 0 && take();
                 if (ok) scores();
@@ -402,7 +425,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
             if (lane == 0)
                 for (uint32_t i = 0; i < (walk ? entries : min(entries, (uint32_t)SLOTS)); i++) {
                     if (!mbar_wait(kv_full(i % SLOTS), (i / SLOTS) & 1u, abort_flag)) break;
-                    arrive_cluster(in_leader(kv_full(i % SLOTS)));
+                    arrive_release_cluster(in_leader(kv_full(i % SLOTS)));
                 }
         }
         __syncwarp();
