@@ -427,6 +427,50 @@ def test_paged_decode_dealt_out_evenly(ctx, lens, H, Hkv, D, block_size, max_blo
         assert orc.rel_l2(got[i], want) < TOL
 
 
+def _even(backend, mode, call):
+    backend.tune("attn_even", mode)
+    try:
+        return call()
+    finally:
+        backend.tune("attn_even", 0)
+
+
+@pytest.mark.parametrize("lens,H,Hkv,D,block_size,max_blocks", [
+    ([5], 4, 4, 128, 16, 8),                                # one chunk
+    ([33, 0, 65], 8, 2, 64, 1, 100),                        # one key per page: a chunk takes every lane's page
+    ([700, 1, 5000], 4, 4, 64, 1, None),
+    ([900, 1200], 32, 2, 128, 24, None),                    # a page size that does not divide the chunk
+    ([1100, 900, 31], 6, 2, 256, 16, 80),                   # one CTA per SM
+    ([3000, 2999, 1], 8, 8, 128, 2, None),                  # many windows of 32 page numbers per piece
+    ([4000, 100], 16, 4, 96, 4096, 1),                      # one page, larger than the context
+    ([129] * 40, 8, 8, 32, 8, 20)])                         # more than 32 sequences, all equal, none full
+def test_even_shares_of_small_paged_caches(ctx, backend, lens, H, Hkv, D, block_size, max_blocks):
+    """Shares forced where the cache is too small for them by choice, against slices (both sum in f32)."""
+    rng = np.random.default_rng(len(lens) + D)
+    q, kc, vc, table, cl = _paged_case(rng, lens, H, Hkv, D, block_size, max_blocks)
+    init = np.full(q.shape, 7.0, np.float32)
+    got, want = (_even(backend, mode, lambda: _paged(ctx, q, kc, vc, table, cl, 1 / np.sqrt(D), out_init=init)) for mode in (1, 2))
+    assert (got[cl <= 0] == 7.0).all() and ctx.last_device_status() == 0
+    _close(got, want)
+
+
+def test_how_a_paged_cache_is_dealt_out_follows_what_is_missing(ctx, backend):
+    """8 sequences of up to 2560 keys, 5120 chunks over 8 KV heads: with up to 7 x 296 of them missing they get the slices' bits
+    (a full cache: those of a contiguous one), with more the even shares'."""
+    rng = np.random.default_rng(5)
+    full = [2560] * 8
+    q, kc, vc, table, _ = _paged_case(rng, full, 32, 8, 128, 16)
+    for lens, form in ((full, 2), (full[:-1] + [2559], 2), ([2560, 2200] * 4, 2), ([2560, 512] * 4, 2), ([2560, 480] * 4, 1),
+                       ([2560, 0, 3, 40] * 2, 1)):
+        cl = np.asarray(lens, np.int32)
+        got, shares, slices = (_even(backend, mode, lambda: _paged(ctx, q, kc, vc, table, cl, 0.09).copy()) for mode in (0, 1, 2))
+        rows = cl > 0
+        assert np.array_equal(got[rows].view(np.uint32), (shares if form == 1 else slices)[rows].view(np.uint32))
+        _close(shares[rows], slices[rows])
+        if sum((2560 - n) // 32 for n in lens):              # (mode 1 deals a full cache out by slices)
+            assert not np.array_equal(shares[rows].view(np.uint32), slices[rows].view(np.uint32))
+
+
 @pytest.mark.parametrize("B_,H,Hkv,keys,Sq", [(1, 8, 8, 33, 1), (37, 8, 8, 32, 1), (37, 8, 8, 31, 1), (5, 32, 8, 1184, 1), (1, 32, 8, 148 * 64, 1),
                                                (2, 8, 2, 700, 4), (3, 16, 2, 2049, 2)])
 def test_contiguous_decode_dealt_out_evenly(ctx, backend, B_, H, Hkv, keys, Sq):

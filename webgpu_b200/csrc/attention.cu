@@ -11,7 +11,8 @@
 //     read from HBM once per KV head, not once per query head;
 //   * a producer warp streams 32-key chunks of K and V into a ring in shared memory with bulk
 //     copies (cp.async.bulk, one per contiguous run: a whole chunk for a contiguous cache, one per
-//     page for a paged one, the page numbers read one chunk ahead), each chunk signalled through an mbarrier; two CTAs of nine warps share an SM, each
+//     page for a paged one, the page numbers taken from a copy of the block table in shared
+//     memory), each chunk signalled through an mbarrier; two CTAs of nine warps share an SM, each
 //     with a ring of three chunks (D = 128);
 //   * eight consumer warps share a chunk: a key is handled by 8 lanes, each holding 16-byte columns
 //     of the row, so a warp takes 4 keys per step; every lane keeps two query rows in registers
@@ -24,11 +25,13 @@
 //     With every warp polling its mbarrier the kernel ran at 2.2-5.1 TB/s depending on how many
 //     warps happened to be waiting; parked, at 5.0-6.5 TB/s on the same shapes (polls travel the same
 //     queue as shared-memory loads and shuffles, and starved the warps that had work);
-//   * keys are split over CTAs when there are fewer (sequence, KV head) pairs than SM slots, and each CTA walks its chunks
-//     from a different starting point.  A decode step over a paged cache, whose sequences differ in length, is one wave of
-//     CTAs, each with the same number of chunks of the (sequence, KV head) items laid end to end, so that a CTA may finish
-//     one item and begin the next.  A small second kernel, resident early through programmatic dependent launch, merges
-//     what several CTAs did of a row.
+//   * keys are split over CTAs when there are fewer (sequence, KV head) pairs than SM slots, and
+//     each CTA walks its chunks from a different starting point; a small second kernel, resident
+//     early through programmatic dependent launch, merges the slices;
+//   * a large paged cache whose sequences differ much in length is dealt out in even shares instead
+//     (lux_attn_even_f32): one wave of CTAs, each with the same number of chunks of the (sequence,
+//     KV head) items laid end to end, so that a CTA may finish one item and begin the next.  The
+//     lengths are known on the device only: both kernels are launched and one of them leaves at once.
 // The one polling wait is bounded: if it gives up it sets the CTA's abort flag, every warp leaves
 // its loop (the consumers first release the stages the producer may be parked on), the device
 // status word reports 0x7C050008 and the output of that CTA is not written.
@@ -53,10 +56,11 @@ constexpr int ATT_THREADS = (ATT_CW + 1) * 32;  // + the producer warp
 constexpr int ATT_CK = 32;                      // keys per staged chunk
 constexpr int ATT_MAX_STAGES = 6;
 constexpr int ATT_CTAS_PER_SM = 2;
-constexpr uint64_t ATT_PAGES = 256ull * 2046;   // pages of the longest context taken
-constexpr uint32_t ATT_EVEN_KEYS = 992;         // EVEN: from so many keys per sequence on
-constexpr int ATT_HEADER = 512;                 // barriers, abort flag, from byte 128 on each consumer warp's Piece
-// floats in which the warps of a row group leave their results: [warp][row][head_dim + 2], in whole 128-byte lines
+constexpr int ATT_TABLE = 2048;                 // block-table entries a CTA keeps in shared memory
+constexpr int ATT_HEADER = 128;                 // barriers, abort flag
+constexpr int ATT_EVEN_HEADER = 512;            // lux_attn_even_f32: and, from byte 128 on, each consumer warp's Piece
+constexpr int ATT_MAX_PARTS = 512;              // CTAs of lux_attn_even_f32
+// floats in which the warps of a CTA of the even form leave their results: [warp][row][head_dim + 2], in whole 128-byte lines
 __host__ __device__ constexpr uint32_t att_merge_floats(uint32_t head_dim, uint32_t rt) { return (ATT_CW * rt * (head_dim + 2u) + 31u) / 32u * 32u; }
 constexpr size_t ATT_SMEM_BUDGET = 110u << 10;        // per CTA: two CTAs share an SM
 constexpr float ATT_NEG = -3.0e38f;             // "no key seen yet" in the base-2 score domain
@@ -84,12 +88,11 @@ struct AttnParams {
     uint32_t rgp;                // row groups per CTA (1, 2, 4 or 8): rows per CTA = RT * rgp
     uint32_t rpb;                // rows per CTA
     uint32_t row_blocks, nsplit, split_keys, stages;
-    // EVEN kernels (a decode step over a paged cache): all 32-key chunks of all (sequence, KV head) items, one after the other, are
-    // dealt out evenly, each CTA taking the next so many of them, `share` at least (0: one CTA per slice of an item).  If
-    // all sequences are as long as the cache allows, the slices are dealt out instead: the same sums as over a contiguous cache.
-    uint32_t share;
-    AttnSpan* spans;             // per item; ctas 0: slices
-    uint32_t ctas;               // of the grid
+    // a paged cache that may be dealt out in even shares
+    uint32_t full_chunks;        // 32-key chunks of a full cache, over all KV heads
+    uint32_t slack;              // even shares if more of them than this are missing
+    uint32_t share, ctas;        // chunks per CTA, at least; CTAs of lux_attn_even_f32
+    AttnSpan* spans;             // per (sequence, KV head); ctas 0: slices
     float qscale;                // scale * log2(e)
 };
 
@@ -116,130 +119,284 @@ __device__ __forceinline__ uint32_t paged_len(const AttnParams& p, uint32_t b) {
     const int32_t cl = p.context_lens[b];
     return cl <= 0 ? 0u : min((uint32_t)cl, p.max_blocks_per_seq * p.block_size);
 }
-__device__ __forceinline__ uint32_t chunks_of(uint32_t keys) { return (keys + ATT_CK - 1) / ATT_CK; }
+__host__ __device__ __forceinline__ uint32_t chunks_of(uint32_t keys) { return (keys + ATT_CK - 1) / ATT_CK; }
 
-// What a CTA does next: chunks [lo, hi) of the n that the rows of (b, g, rb) see.
-struct Piece {
-    uint32_t b, g, rb, kv_len, lmax, lo, hi, n;
-    uint32_t ahead;              // EVEN: keys of the next sequence, asked for early
-    __device__ __forceinline__ void load(const volatile Piece* s) {
-        b = s->b; g = s->g; rb = s->rb; kv_len = s->kv_len; lmax = s->lmax; lo = s->lo; hi = s->hi; n = s->n; ahead = s->ahead;
+// 32-key chunks of all sequences and KV heads of a paged cache; every warp for itself.
+__device__ __forceinline__ uint32_t all_chunks(const AttnParams& p) {
+    uint32_t sum = 0u;
+    for (uint32_t b = threadIdx.x & 31u; b < p.batch; b += 32) sum += chunks_of(paged_len(p, b));
+    for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    return sum * p.kv_heads;
+}
+// Whether so many chunks are dealt out in even shares, not in slices.
+__device__ __forceinline__ bool ragged(const AttnParams& p, uint32_t all) { return p.full_chunks - all > p.slack; }
+
+// The rows of a consumer warp of lux_attn_even_f32: a lane's columns of RT query rows, their running maxima, denominators and
+// outputs.  (lux_attn_stream_f32 has the same arithmetic written out in its loop: through this struct its registers were
+// allotted otherwise and contiguous caches took 1 to 2 % longer, 32 x 2048 keys 93.5 -> 95.5 us a step.)
+template <int VPL, int RT, bool FULL>
+struct Rows {
+    float4 q[RT][VPL], o[RT][VPL];
+    float m[RT], l[RT];
+    uint32_t len[RT], min_len;
+    bool col_ok[VPL];
+
+    __device__ __forceinline__ void columns(uint32_t D, int sub) {
+#pragma unroll
+        for (int j = 0; j < VPL; j++) col_ok[j] = (uint32_t)(j * 8 + sub) * 4u < D;
     }
-    // Every CTA (or slice: `key`) walks the chunks of a piece from a different starting point (and wraps around), so that the CTAs of a wave,
-    // which start together and advance at the same pace, are not all at the same offset of equally spaced slices.
-    __device__ __forceinline__ uint32_t start(uint32_t key) const { return hi > lo ? lo + (key * 2654435761u >> 8) % (hi - lo) : lo; }
+    // rows row0 .. row0 + RT of KV head g of sequence b, which see kv_len keys
+    __device__ __forceinline__ void begin(const AttnParams& p, uint32_t b, uint32_t g, uint32_t row0, uint32_t kv_len, int sub) {
+        min_len = 0xffffffffu;
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            const uint32_t r = row0 + i;
+            const bool valid = r < p.group * p.seq_q;
+            const uint32_t qi = valid ? r / p.group : 0u, head = g * p.group + (valid ? r % p.group : 0u);
+            len[i] = valid ? row_len(p, qi, kv_len) : 0xffffffffu;       // a padding row: q = 0, never written, never masks a chunk
+            min_len = min(min_len, len[i]);
+            const float* qr = p.q + (((size_t)b * p.heads + head) * p.seq_q + qi) * p.head_dim;
+            m[i] = ATT_NEG;
+            l[i] = 0.0f;
+#pragma unroll
+            for (int j = 0; j < VPL; j++) {
+                float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (valid && col_ok[j]) t = __ldg(reinterpret_cast<const float4*>(qr) + j * 8 + sub);
+                q[i][j] = make_float4(t.x * p.qscale, t.y * p.qscale, t.z * p.qscale, t.w * p.qscale);
+                o[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    }
+    static __device__ __forceinline__ float4 lds4(uint32_t addr) {
+        float4 r;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(addr));
+        return r;
+    }
+    // One step: the warp's four keys (one per group of 8 lanes) against its RT rows.  The
+    // running maximum of a lane is only raised when a score passes it by more than 8 (in the
+    // base-2 domain), so weights stay below 2^8 and the common step has no rescaling in it:
+    // scores, one exp2 per row, the weighted sum.  MASKED steps (the last chunk of a slice, a
+    // causal edge) check each key against the chunk and each row's length.
+    template <bool MASKED>
+    __device__ __forceinline__ void step(uint32_t kaddr, uint32_t vaddr, bool inb, uint32_t t) {
+        float sc[RT];
+#pragma unroll
+        for (int i = 0; i < RT; i++) sc[i] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < VPL; j++) {
+            float4 kk = make_float4(0.f, 0.f, 0.f, 0.f);
+            if ((FULL || col_ok[j]) && (!MASKED || inb)) kk = lds4(kaddr + (uint32_t)j * 128u);
+#pragma unroll
+            for (int i = 0; i < RT; i++)
+                sc[i] = fmaf(q[i][j].x, kk.x, fmaf(q[i][j].y, kk.y, fmaf(q[i][j].z, kk.z, fmaf(q[i][j].w, kk.w, sc[i]))));
+        }
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            sc[i] += __shfl_xor_sync(0xffffffffu, sc[i], 1);
+            sc[i] += __shfl_xor_sync(0xffffffffu, sc[i], 2);
+            sc[i] += __shfl_xor_sync(0xffffffffu, sc[i], 4);
+        }
+        bool vis[RT], up = false, any = false;
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            vis[i] = !MASKED || (inb && t < len[i]);
+            up |= vis[i] && sc[i] > m[i] + 8.0f;
+            any |= vis[i];
+        }
+        if (__any_sync(0xffffffffu, up)) {
+#pragma unroll
+            for (int i = 0; i < RT; i++) {
+                const float mn = vis[i] ? fmaxf(m[i], sc[i]) : m[i];
+                const float alpha = ex2(m[i] - mn);
+                l[i] *= alpha;
+#pragma unroll
+                for (int j = 0; j < VPL; j++) {
+                    o[i][j].x *= alpha; o[i][j].y *= alpha; o[i][j].z *= alpha; o[i][j].w *= alpha;
+                }
+                m[i] = mn;
+            }
+        }
+        float pw[RT];
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            pw[i] = ex2(sc[i] - m[i]);
+            if (MASKED && !vis[i]) pw[i] = 0.0f;
+            l[i] += pw[i];
+        }
+        if (!MASKED || any) {
+#pragma unroll
+            for (int j = 0; j < VPL; j++) {
+                float4 vv = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (FULL || col_ok[j]) vv = lds4(vaddr + (uint32_t)j * 128u);
+#pragma unroll
+                for (int i = 0; i < RT; i++) {
+                    o[i][j].x = fmaf(pw[i], vv.x, o[i][j].x);
+                    o[i][j].y = fmaf(pw[i], vv.y, o[i][j].y);
+                    o[i][j].z = fmaf(pw[i], vv.z, o[i][j].z);
+                    o[i][j].w = fmaf(pw[i], vv.w, o[i][j].w);
+                }
+            }
+        }
+    }
+    // a warp's part of a chunk of nk keys from key t0 on, at kchunk in shared memory (V: v_off further)
+    __device__ __forceinline__ void chunk(uint32_t kchunk, uint32_t v_off, uint32_t row_bytes, uint32_t t0, uint32_t nk, uint32_t kslot, uint32_t wpg, int kg) {
+        if (nk == ATT_CK && t0 + ATT_CK <= min_len) {
+            for (uint32_t kb = kslot * 4u; kb < ATT_CK; kb += wpg * 4u) {
+                const uint32_t ka = kchunk + (kb + (uint32_t)kg) * row_bytes;
+                step<false>(ka, ka + v_off, true, 0u);
+            }
+        } else {
+            for (uint32_t kb = kslot * 4u; kb < nk; kb += wpg * 4u) {
+                const uint32_t key = kb + (uint32_t)kg, ka = kchunk + key * row_bytes;
+                step<true>(ka, ka + v_off, key < nk, t0 + key);
+            }
+        }
+    }
+    // the four key slots of the warp, merged by the running-maximum rule
+    __device__ __forceinline__ void fold(int i) {
+        float mm = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
+        mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, 16));
+        const float alpha = ex2(m[i] - mm);
+        m[i] = mm;
+        l[i] *= alpha;
+        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 8);
+        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 16);
+#pragma unroll
+        for (int j = 0; j < VPL; j++) {
+            float* e = reinterpret_cast<float*>(&o[i][j]);
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                float val = e[x] * alpha;
+                val += __shfl_xor_sync(0xffffffffu, val, 8);
+                val += __shfl_xor_sync(0xffffffffu, val, 16);
+                e[x] = val;
+            }
+        }
+    }
+    // row i to shared memory: outputs by column, its maximum and denominator at [D] and [D + 1] (rows are 8-byte aligned, not 16)
+    __device__ __forceinline__ void store(int i, float* dst, uint32_t D, int lane) const {
+        if (lane >= 8) return;
+#pragma unroll
+        for (int j = 0; j < VPL; j++)
+            if (col_ok[j]) {
+                float* d4 = dst + (j * 8 + lane) * 4;
+                d4[0] = o[i][j].x; d4[1] = o[i][j].y; d4[2] = o[i][j].z; d4[3] = o[i][j].w;
+            }
+        if (lane == 0) {
+            dst[D] = m[i];
+            dst[D + 1] = l[i];
+        }
+    }
 };
 
-template <int VPL, int RT, bool FULL, bool EVEN>
+// One output element of row ir of the CTA's block: column d of what the wpg warps of its row group left in mrg.
+template <int RT>
+__device__ __forceinline__ void merge_warps(const float* mrg, uint32_t ir, uint32_t d, uint32_t D, uint32_t rgp, uint32_t wpg, float& M, float& L, float& acc) {
+    const uint32_t rgi = ir / RT, ii = ir % RT, MS = D + 2u;
+    M = ATT_NEG;
+    for (uint32_t w = 0; w < wpg; w++) M = fmaxf(M, mrg[((size_t)(w * rgp + rgi) * RT + ii) * MS + D]);
+    L = 0.0f;
+    acc = 0.0f;
+    for (uint32_t w = 0; w < wpg; w++) {
+        const float* src = mrg + ((size_t)(w * rgp + rgi) * RT + ii) * MS;
+        const float wgt = ex2(src[D] - M);
+        L = fmaf(src[D + 1], wgt, L);
+        acc = fmaf(src[d], wgt, acc);
+    }
+}
+
+// The producer's page numbers: lane i holds the table's entries of pages base + i and base + 32 + i of a sequence, and of page i of
+// the piece that comes next, so that no entry is waited for (read one chunk ahead, with the memory busy, they came later than the
+// ring had room: 16 sequences of 4096 keys, 16-token pages, 113 us a step against 101).
+struct Pages {
+    uint32_t b, base;
+    int32_t cur, ahead, next;
+    __device__ __forceinline__ int32_t ask(const AttnParams& p, uint32_t seq, uint32_t page, uint32_t keys) const {
+        if (page >= p.max_blocks_per_seq || page * p.block_size >= keys) return 0;
+        return p.block_tables[(size_t)seq * p.max_blocks_per_seq + page];
+    }
+    // pages from `page` on of a sequence of so many keys, asked for earlier
+    __device__ __forceinline__ void begin(const AttnParams& p, uint32_t seq, uint32_t page, uint32_t keys, int lane) {
+        b = seq;
+        base = page;
+        cur = next;
+        ahead = ask(p, b, base + 32u + lane, keys);
+    }
+    // keys [t0, t0 + nk): one copy per page the chunk touches; lane i takes the i-th page
+    __device__ __forceinline__ void copy(const AttnParams& p, uint32_t g, uint32_t t0, uint32_t nk, uint32_t keys, float* ks, float* vs, uint32_t bar, int lane) {
+        const uint32_t first = t0 / p.block_size;
+        if (first >= base + 32u) {
+            base += 32u;
+            cur = ahead;
+            ahead = ask(p, b, base + 32u + lane, keys);
+        }
+        const uint32_t blk = first + (uint32_t)lane, i = blk - base;
+        const int32_t lo = __shfl_sync(0xffffffffu, cur, i & 31u), hi = __shfl_sync(0xffffffffu, ahead, i & 31u);
+        int32_t entry = i < 32u ? lo : hi;
+        if (blk <= (t0 + nk - 1u) / p.block_size) {
+            const uint32_t ta = max(t0, blk * p.block_size), tb = min(t0 + nk, (blk + 1u) * p.block_size);
+            if ((uint32_t)entry >= p.num_blocks) {
+                entry = 0;
+                if (p.status) atomicOr(p.status, ATT_STATUS_BLOCK);
+            }
+            const size_t off = (((size_t)entry * p.kv_heads + g) * p.block_size + (ta - blk * p.block_size)) * p.head_dim;
+            bulk_g2s(smem_u32(ks + (size_t)(ta - t0) * p.head_dim), p.k + off, (tb - ta) * p.head_dim * 4u, bar);
+            bulk_g2s(smem_u32(vs + (size_t)(ta - t0) * p.head_dim), p.v + off, (tb - ta) * p.head_dim * 4u, bar);
+        }
+    }
+};
+
+// A bounded wait gave up: report it and give copies still in flight time to land in this CTA's shared memory before it
+// is released.
+__device__ __forceinline__ void report_abort(const AttnParams& p) {
+    if (threadIdx.x == 0 && p.status) atomicOr(p.status, ATT_STATUS_WAIT);
+    for (int i = 0; i < 64; i++) __nanosleep(1000);
+    __syncthreads();
+}
+
+// One CTA per slice of the keys of (sequence, KV head, block of rows).
+// GATED: unless the cache is ragged; then lux_attn_even_f32, launched beside it, does all.
+template <int VPL, int RT, bool FULL, bool GATED>
 __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_f32(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t bar_full = smem_u32(smem);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + 16 * ATT_MAX_STAGES);
-    float* mrg = reinterpret_cast<float*>(smem + ATT_HEADER);              // [warp][RT][D + 2]
+    int32_t* table = reinterpret_cast<int32_t*>(smem + ATT_HEADER);
+    float* stages = reinterpret_cast<float*>(smem + ATT_HEADER + (p.block_size ? ATT_TABLE * 4 : 0));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t D = p.head_dim, NS = p.stages, MS = D + 2u;
-    float* stages = mrg + att_merge_floats(D, RT);
+    const uint32_t D = p.head_dim, NS = p.stages;
     const size_t stage_floats = (size_t)2 * ATT_CK * D;
 
     pdl_launch_dependents();                   // the merge kernel may take its place; it waits for this grid
     pdl_wait();                                // q, the cache and the tables may come from the kernels just before
 
+    if (GATED && ragged(p, all_chunks(p))) return;
+    uint32_t idx = blockIdx.x;
+    const uint32_t split = idx % p.nsplit; idx /= p.nsplit;
+    if (GATED && split == 0u && tid == 0) p.spans[idx] = AttnSpan{0, p.nsplit == 1 ? 1 : 0};
+    const uint32_t rb = idx % p.row_blocks; idx /= p.row_blocks;
+    const uint32_t g = idx % p.kv_heads, b = idx / p.kv_heads;
+
+    uint32_t kv_len = p.kv_len;
+    if (p.block_size) {
+        const int32_t cl = p.context_lens[b];
+        if (cl <= 0) return;                   // paged.wgsl:66-67: the rows stay as they are
+        kv_len = min((uint32_t)cl, p.max_blocks_per_seq * p.block_size);
+    }
     // rows of this CTA: row r of the KV head is (query qi = r / group, head g * group + r % group),
     // so a block of rows holds neighbouring queries and a causal block stops at its last row's keys
-    const uint32_t R = p.group * p.seq_q, rpb = RT * p.rgp;
-    Piece first;
-    uint32_t total = 0u, share = 0u;           // chunks of this CTA; of every CTA
-    auto extent = [&](Piece& w, uint32_t kv_len) {   // what the rows of (b, g, rb) see
-        w.kv_len = kv_len;
-        w.lmax = row_len(p, (min(R, (w.rb + 1u) * rpb) - 1u) / p.group, kv_len);
-        w.n = chunks_of(w.lmax);
-    };
-    bool slices = false;                       // EVEN: the slices of equal items, dealt out in turn
-    const uint32_t slice_count = p.batch * p.kv_heads * p.nsplit;
-    auto slice = [&](Piece& w, uint32_t i) {   // slice i, w's extent being set; kept in `ahead`
-        const uint32_t item = i / p.nsplit, chunks = p.split_keys / ATT_CK;
-        w.ahead = i;
-        w.b = item / p.kv_heads;
-        w.g = item - w.b * p.kv_heads;
-        w.lo = (i - item * p.nsplit) * chunks;
-        w.hi = min(w.lo + chunks, w.n);
-    };
-    if constexpr (!EVEN) {
-        uint32_t idx = blockIdx.x;
-        const uint32_t split = idx % p.nsplit; idx /= p.nsplit;
-        first.rb = idx % p.row_blocks; idx /= p.row_blocks;
-        first.g = idx % p.kv_heads;
-        first.b = idx / p.kv_heads;
-        if (p.block_size && p.context_lens[first.b] <= 0) return;          // paged.wgsl:66-67: the rows stay as they are
-        extent(first, p.block_size ? paged_len(p, first.b) : p.kv_len);
-        first.lo = min(split * (p.split_keys / ATT_CK), first.n);
-        first.hi = min(first.lo + p.split_keys / ATT_CK, first.n);
-        total = first.hi - first.lo;
-    } else {
-        // every warp for itself, 32 sequences at a time: the sum, then the sequence in which this CTA starts
-        uint32_t sum = 0u;
-        bool full = true;
-        for (uint32_t b0 = 0; b0 < p.batch; b0 += 32) {
-            const uint32_t n = b0 + lane < p.batch ? paged_len(p, b0 + lane) : 0u;
-            sum += chunks_of(n);
-            full = full && (b0 + lane >= p.batch || n == p.kv_len);
-        }
-        for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        slices = __all_sync(0xffffffffu, full);
-        const uint32_t all = sum * p.kv_heads;
-        share = max(p.share, (all + gridDim.x - 1u) / gridDim.x);
-        const uint32_t at = blockIdx.x * share;
-        uint32_t before = 0u;
-        if (slices) {
-            if (blockIdx.x >= slice_count) return;
-            first.rb = 0u;
-            extent(first, p.kv_len);
-            slice(first, blockIdx.x);
-            for (uint32_t i = blockIdx.x; i < slice_count; i += gridDim.x) total += min(p.split_keys / ATT_CK, first.n - i % p.nsplit * (p.split_keys / ATT_CK));
-        } else if (at >= all) {
-            return;
-        }
-        for (uint32_t b0 = 0; !slices; b0 += 32) {
-            const uint32_t n = b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
-            uint32_t upto = n;                 // inclusive
-            for (int off = 1; off < 32; off <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, upto, off);
-                if (lane >= off) upto += v;
-            }
-            const uint32_t hit = __ballot_sync(0xffffffffu, (before + upto) * p.kv_heads > at);
-            if (hit) {
-                const int src = __ffs(hit) - 1;
-                first.b = b0 + src;
-                before += __shfl_sync(0xffffffffu, upto - n, src);
-                break;
-            }
-            before += __shfl_sync(0xffffffffu, upto, 31);
-        }
-        if (!slices) {
-            first.rb = 0u;
-            extent(first, paged_len(p, first.b));
-            first.ahead = first.b + 1u < p.batch ? paged_len(p, first.b + 1u) : 0u;
-            const uint32_t in = at - before * p.kv_heads;
-            first.g = in / first.n;
-            first.lo = in - first.g * first.n;
-            total = min(share, all - at);
-            first.hi = min(first.lo + total, first.n);
-        }
-    }
-    auto next = [&](Piece& w, uint32_t left) { // the piece after w, `left` chunks still to do
-        if (slices) {
-            slice(w, w.ahead + gridDim.x);
-            return;
-        }
-        if (++w.g == p.kv_heads) {
-            w.g = 0u;
-            extent(w, w.ahead);
-            for (w.b++; w.n == 0u;) extent(w, paged_len(p, ++w.b));        // (left > 0: there is one)
-            w.ahead = w.b + 1u < p.batch ? paged_len(p, w.b + 1u) : 0u;
-        }
-        w.lo = 0u;
-        w.hi = min(left, w.n);
-    };
+    const uint32_t R = p.group * p.seq_q, rpb = RT * p.rgp, row0 = rb * rpb;
+    const uint32_t last_row = min(R, row0 + rpb) - 1u;
+    const uint32_t lmax = row_len(p, last_row / p.group, kv_len);
+    const uint32_t k_begin = split * p.split_keys;
+    const uint32_t k_end = min(lmax, k_begin + p.split_keys);
+    const uint32_t nchunks = k_end > k_begin ? (k_end - k_begin + ATT_CK - 1) / ATT_CK : 0u;
+    const uint32_t tbl0 = p.block_size ? k_begin / p.block_size : 0u;
+    // Every CTA walks its chunks from a different starting point (and wraps around), so that the CTAs
+    // of a wave, which start together and advance at the same pace, are not all at the same offset
+    // of equally spaced slices.
+    const uint32_t rot = nchunks ? (blockIdx.x * 2654435761u >> 8) % nchunks : 0u;
+    auto chunk_at = [&](uint32_t c) { const uint32_t cc = c + rot; return cc >= nchunks ? cc - nchunks : cc; };
 
     if (tid == 0) {
         *abort_flag = 0u;
@@ -247,6 +404,18 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             mbar_init(bar_full + 8u * s, 1u);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (p.block_size && nchunks) {
+        const uint32_t nblk = (k_end - 1u) / p.block_size - tbl0 + 1u;      // <= ATT_TABLE by the launcher's split
+        const int32_t* src = p.block_tables + (size_t)b * p.max_blocks_per_seq + tbl0;
+        for (uint32_t i = tid; i < nblk; i += ATT_THREADS) {
+            int32_t e = src[i];
+            if ((uint32_t)e >= p.num_blocks) {
+                e = 0;
+                if (p.status) atomicOr(p.status, ATT_STATUS_BLOCK);
+            }
+            table[i] = e;
+        }
     }
     __syncthreads();
 
@@ -261,28 +430,13 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
 
     if (warp == ATT_CW) {
         // ---- producer: one chunk = keys [t0, t0 + nk) of K and of V ------------------------------
-        Piece w = first;
-        // paged: lane i holds the table's entry of the i-th page that the next chunk touches, read one chunk ahead
-        int32_t entry = 0;
-        auto lookup = [&](uint32_t t0) {
-            const uint32_t blk = t0 / p.block_size + (uint32_t)lane;
-            if (blk * p.block_size < min(w.lmax, t0 + ATT_CK)) {
-                entry = p.block_tables[(size_t)w.b * p.max_blocks_per_seq + blk];
-                if ((uint32_t)entry >= p.num_blocks) {
-                    entry = 0;
-                    if (p.status) atomicOr(p.status, ATT_STATUS_BLOCK);
-                }
-            }
-        };
-        uint32_t k = w.start(slices ? w.ahead : blockIdx.x), todo = w.hi - w.lo;
-        if (p.block_size && total) lookup(k * ATT_CK);
-        for (uint32_t c = 0; c < total; c++) {
+        for (uint32_t c = 0; c < nchunks; c++) {
             const uint32_t s = c % NS;
             if (c >= NS) {
                 named_bar_sync<ATT_BAR_FREE0>(s, ATT_THREADS);          // all consumer warps have left the stage
                 if (*abort_flag) break;
             }
-            const uint32_t t0 = k * ATT_CK, nk = min((uint32_t)ATT_CK, w.lmax - t0);
+            const uint32_t t0 = k_begin + chunk_at(c) * ATT_CK, nk = min((uint32_t)ATT_CK, k_end - t0);
             const uint32_t bar = bar_full + 8u * s;
             float* ks = stages + s * stage_floats;
             float* vs = ks + (size_t)ATT_CK * D;
@@ -290,7 +444,7 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
             __syncwarp();
             if (!p.block_size) {
                 if (lane == 0) {
-                    const size_t off = (((size_t)w.b * p.kv_heads + w.g) * p.kv_stride + t0) * D;
+                    const size_t off = (((size_t)b * p.kv_heads + g) * p.kv_stride + t0) * D;
                     bulk_g2s(smem_u32(ks), p.k + off, nk * D * 4u, bar);
                     bulk_g2s(smem_u32(vs), p.v + off, nk * D * 4u, bar);
                 }
@@ -299,44 +453,32 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                 const uint32_t blk = t0 / p.block_size + (uint32_t)lane;
                 const uint32_t ta = max(t0, blk * p.block_size), tb = min(t0 + nk, (blk + 1u) * p.block_size);
                 if (ta < tb) {
-                    const size_t off = (((size_t)entry * p.kv_heads + w.g) * p.block_size + (ta - blk * p.block_size)) * D;
+                    const size_t off = (((size_t)table[blk - tbl0] * p.kv_heads + g) * p.block_size + (ta - blk * p.block_size)) * D;
                     bulk_g2s(smem_u32(ks + (size_t)(ta - t0) * D), p.k + off, (tb - ta) * D * 4u, bar);
                     bulk_g2s(smem_u32(vs + (size_t)(ta - t0) * D), p.v + off, (tb - ta) * D * 4u, bar);
                 }
             }
-            if (++k == w.hi) k = w.lo;
-            if (EVEN && --todo == 0u && c + 1 < total) {
-                next(w, total - c - 1u);
-                k = w.start(slices ? w.ahead : blockIdx.x);
-                todo = w.hi - w.lo;
-            }
-            if (p.block_size && c + 1 < total) lookup(k * ATT_CK);
         }
     } else {
         // ---- consumers -------------------------------------------------------------------------
         const uint32_t rg = (uint32_t)warp % p.rgp, kslot = (uint32_t)warp / p.rgp, wpg = ATT_CW / p.rgp;
-        uint32_t min_len;
-        auto begin = [&](const Piece& w) {                               // this lane's rows of the piece
-            min_len = 0xffffffffu;
 #pragma unroll
-            for (int i = 0; i < RT; i++) {
-                const uint32_t r = w.rb * rpb + rg * RT + i;
-                const bool valid = r < R;
-                const uint32_t qi = valid ? r / p.group : 0u, head = w.g * p.group + (valid ? r % p.group : 0u);
-                len[i] = valid ? row_len(p, qi, w.kv_len) : 0xffffffffu; // a padding row: q = 0, never written, never masks a chunk
-                min_len = min(min_len, len[i]);
-                const float* qr = p.q + (((size_t)w.b * p.heads + head) * p.seq_q + qi) * D;
-                m[i] = ATT_NEG;
-                l[i] = 0.0f;
+        for (int i = 0; i < RT; i++) {
+            const uint32_t r = row0 + rg * RT + i;
+            const bool valid = r < R;
+            const uint32_t qi = valid ? r / p.group : 0u, head = g * p.group + (valid ? r % p.group : 0u);
+            len[i] = valid ? row_len(p, qi, kv_len) : 0xffffffffu;       // a padding row: q = 0, never written, never masks a chunk
+            const float* qr = p.q + (((size_t)b * p.heads + head) * p.seq_q + qi) * D;
+            m[i] = ATT_NEG;
+            l[i] = 0.0f;
 #pragma unroll
-                for (int j = 0; j < VPL; j++) {
-                    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (valid && col_ok[j]) t = __ldg(reinterpret_cast<const float4*>(qr) + j * 8 + sub);
-                    q[i][j] = make_float4(t.x * p.qscale, t.y * p.qscale, t.z * p.qscale, t.w * p.qscale);
-                    o[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
+            for (int j = 0; j < VPL; j++) {
+                float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (valid && col_ok[j]) t = __ldg(reinterpret_cast<const float4*>(qr) + j * 8 + sub);
+                q[i][j] = make_float4(t.x * p.qscale, t.y * p.qscale, t.z * p.qscale, t.w * p.qscale);
+                o[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
-        };
+        }
         // One step: the warp's four keys (one per group of 8 lanes) against its RT rows.  The
         // running maximum of a lane is only raised when a score passes it by more than 8 (in the
         // base-2 domain), so weights stay below 2^8 and the common step has no rescaling in it:
@@ -409,78 +551,236 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                 }
             }
         };
-        // the end of a piece: the four key slots of the warp, then the warps of each row group, are merged by the
-        // running-maximum rule, and the rows written: the outputs of a whole item, else partial results
-        auto finish = [&](const Piece& w) {
+        uint32_t min_len = 0xffffffffu;
 #pragma unroll
-            for (int i = 0; i < RT; i++) {
-                float mm = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
-                mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, 16));
-                const float alpha = ex2(m[i] - mm);
-                m[i] = mm;
-                l[i] *= alpha;
-                l[i] += __shfl_xor_sync(0xffffffffu, l[i], 8);
-                l[i] += __shfl_xor_sync(0xffffffffu, l[i], 16);
-                float* dst = mrg + ((size_t)warp * RT + i) * MS;
-#pragma unroll
-                for (int j = 0; j < VPL; j++) {
-                    float* e = reinterpret_cast<float*>(&o[i][j]);
-#pragma unroll
-                    for (int x = 0; x < 4; x++) {
-                        float val = e[x] * alpha;
-                        val += __shfl_xor_sync(0xffffffffu, val, 8);
-                        val += __shfl_xor_sync(0xffffffffu, val, 16);
-                        if (kg == 0 && col_ok[j]) dst[(j * 8 + sub) * 4 + x] = val;
-                    }
+        for (int i = 0; i < RT; i++) min_len = min(min_len, len[i]);
+        const uint32_t stage0 = smem_u32(stages), stage_bytes = 2u * ATT_CK * row_bytes, v_off = ATT_CK * row_bytes;
+        for (uint32_t c = 0; c < nchunks; c++) {
+            const uint32_t s = c % NS;
+            // one poller per CTA: warp 0 waits for the copies, the named barrier releases the other seven
+            if (warp == 0) warp_wait(bar_full + 8u * s, (c / NS) & 1u, abort_flag, lane);
+            named_bar_sync_c<ATT_BAR_READY>(ATT_CW * 32);
+            if (*abort_flag) {
+                // the producer may be parked on the stages this warp would still have released
+                for (uint32_t cc = c; cc < c + NS && cc + NS < nchunks; cc++) named_bar_arrive<ATT_BAR_FREE0>(cc % NS, ATT_THREADS);
+                break;
+            }
+            const uint32_t t0 = k_begin + chunk_at(c) * ATT_CK, nk = min((uint32_t)ATT_CK, k_end - t0);
+            const uint32_t kchunk = stage0 + s * stage_bytes + lane_off;
+            if (nk == ATT_CK && t0 + ATT_CK <= min_len) {
+                for (uint32_t kb = kslot * 4u; kb < ATT_CK; kb += wpg * 4u) {
+                    const uint32_t ka = kchunk + (kb + (uint32_t)kg) * row_bytes;
+                    step(std::false_type{}, ka, ka + v_off, true, 0u);
                 }
-                if (lane == 0) {
-                    dst[D] = m[i];
-                    dst[D + 1] = l[i];
+            } else {
+                for (uint32_t kb = kslot * 4u; kb < nk; kb += wpg * 4u) {
+                    const uint32_t key = kb + (uint32_t)kg, ka = kchunk + key * row_bytes;
+                    step(std::true_type{}, ka, ka + v_off, key < nk, t0 + key);
                 }
             }
-            named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);
-            const uint32_t row0 = w.rb * rpb;
-            const bool whole = EVEN ? w.lo == 0u && w.hi == w.n : p.nsplit == 1;
-            if (EVEN && w.lo == 0u && tid == 0)                          // the item may go on in the CTAs after this one
-                p.spans[w.b * p.kv_heads + w.g] = AttnSpan{(int32_t)blockIdx.x, slices && !whole ? 0 : (int32_t)(1u + (w.n - w.hi + share - 1u) / share)};
-            for (uint32_t e = tid; e < rpb * D; e += ATT_CW * 32) {
-                const uint32_t ir = e / D, d = e - ir * D, r = row0 + ir;
-                if (r >= R) continue;
-                const uint32_t rgi = ir / RT, ii = ir % RT;
-                float M = ATT_NEG;
-                for (uint32_t v = 0; v < wpg; v++) M = fmaxf(M, mrg[((size_t)(v * p.rgp + rgi) * RT + ii) * MS + D]);
-                float L = 0.0f, acc = 0.0f;
-                for (uint32_t v = 0; v < wpg; v++) {
-                    const float* src = mrg + ((size_t)(v * p.rgp + rgi) * RT + ii) * MS;
-                    const float wgt = ex2(src[D] - M);
-                    L = fmaf(src[D + 1], wgt, L);
-                    acc = fmaf(src[d], wgt, acc);
-                }
-                const uint32_t qi = r / p.group, head = w.g * p.group + r % p.group;
-                const size_t orow = ((size_t)w.b * p.heads + head) * p.seq_q + qi;
-                if (whole) {
-                    p.out[orow * D + d] = L > 0.0f ? acc / L : 0.0f;
-                    if (d == 0 && p.lse) p.lse[orow] = L > 0.0f ? fmaf(M, ATT_LN2, logf(L)) : -3.402823e+38f;
-                } else {
-                    // two places per CTA: the item in which its share begins, and the one that begins in its share
-                    const size_t slot = EVEN && !slices ? (size_t)(blockIdx.x * 2u + (w.lo == 0u ? 1u : 0u)) * rpb + ir
-                                        : EVEN          ? orow * p.nsplit + w.ahead % p.nsplit
-                                                        : orow * p.nsplit + blockIdx.x % p.nsplit;
-                    float* dst = p.part + slot * MS;
-                    dst[d] = acc;
-                    if (d == 0) {
-                        dst[D] = M;
-                        dst[D + 1] = L;
-                    }
+            // done with the stage (not needed for the last NS chunks: nobody refills them)
+            if (c + NS < nchunks) named_bar_arrive<ATT_BAR_FREE0>(s, ATT_THREADS);
+        }
+        // the four key slots of the warp, merged by the running-maximum rule
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            float mm = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
+            mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, 16));
+            const float alpha = ex2(m[i] - mm);
+            m[i] = mm;
+            l[i] *= alpha;
+            l[i] += __shfl_xor_sync(0xffffffffu, l[i], 8);
+            l[i] += __shfl_xor_sync(0xffffffffu, l[i], 16);
+#pragma unroll
+            for (int j = 0; j < VPL; j++) {
+                float* e = reinterpret_cast<float*>(&o[i][j]);
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                    float val = e[x] * alpha;
+                    val += __shfl_xor_sync(0xffffffffu, val, 8);
+                    val += __shfl_xor_sync(0xffffffffu, val, 16);
+                    e[x] = val;
                 }
             }
-            named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);                // before the next piece is merged
-        };
+        }
+    }
+
+    __syncthreads();               // every chunk has landed and been read: the ring is free
+    if (*abort_flag) {
+        // A bounded wait gave up: report it and give copies still in flight time to land in this
+        // CTA's shared memory before it is released.  Nothing is written.
+        if (tid == 0 && p.status) atomicOr(p.status, ATT_STATUS_WAIT);
+        for (int i = 0; i < 64; i++) __nanosleep(1000);
+        __syncthreads();
+        return;
+    }
+    // warps of one row group -> shared memory (over the ring), then one thread per output element
+    float* mrg = stages;                                   // [warp][RT][D + 2]
+    const uint32_t MS = D + 2u;
+    if (warp < ATT_CW && kg == 0) {
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            float* dst = mrg + ((size_t)warp * RT + i) * MS;
+#pragma unroll
+            for (int j = 0; j < VPL; j++)
+                if (col_ok[j]) {
+                    // D + 2 floats per row: rows are 8-byte aligned, not 16
+                    float* d4 = dst + (j * 8 + sub) * 4;
+                    d4[0] = o[i][j].x; d4[1] = o[i][j].y; d4[2] = o[i][j].z; d4[3] = o[i][j].w;
+                }
+            if (sub == 0) {
+                dst[D] = m[i];
+                dst[D + 1] = l[i];
+            }
+        }
+    }
+    __syncthreads();
+    const uint32_t wpg = ATT_CW / p.rgp;
+    for (uint32_t e = tid; e < rpb * D; e += ATT_THREADS) {
+        const uint32_t ir = e / D, d = e - ir * D, r = row0 + ir;
+        if (r >= R) continue;
+        const uint32_t rgi = ir / RT, ii = ir % RT;
+        float M = ATT_NEG;
+        for (uint32_t w = 0; w < wpg; w++) M = fmaxf(M, mrg[((size_t)(w * p.rgp + rgi) * RT + ii) * MS + D]);
+        float L = 0.0f, acc = 0.0f;
+        for (uint32_t w = 0; w < wpg; w++) {
+            const float* src = mrg + ((size_t)(w * p.rgp + rgi) * RT + ii) * MS;
+            const float wgt = ex2(src[D] - M);
+            L = fmaf(src[D + 1], wgt, L);
+            acc = fmaf(src[d], wgt, acc);
+        }
+        const uint32_t qi = r / p.group, head = g * p.group + r % p.group;
+        const size_t orow = ((size_t)b * p.heads + head) * p.seq_q + qi;
+        if (p.nsplit == 1) {
+            p.out[orow * D + d] = L > 0.0f ? acc / L : 0.0f;
+            if (d == 0 && p.lse) p.lse[orow] = L > 0.0f ? fmaf(M, ATT_LN2, logf(L)) : -3.402823e+38f;
+        } else {
+            float* dst = p.part + (orow * p.nsplit + split) * MS;
+            dst[d] = acc;
+            if (d == 0) {
+                dst[D] = M;
+                dst[D + 1] = L;
+            }
+        }
+    }
+}
+
+// What a CTA of the even form does next: chunks [lo, hi) of the n of (sequence b, KV head g).
+struct Piece {
+    uint32_t b, g, keys, lo, hi, n;
+    uint32_t ahead;              // keys of the next sequence, asked for early
+    __device__ __forceinline__ void load(const volatile Piece* s) {
+        b = s->b; g = s->g; keys = s->keys; lo = s->lo; hi = s->hi; n = s->n; ahead = s->ahead;
+    }
+};
+
+// A decode step over a paged cache, dealt out evenly: all 32-key chunks of all (sequence, KV head) items, one after the other,
+// each CTA taking the next so many of them.
+template <int VPL, int RT, bool FULL>
+__global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_even_f32(const AttnParams p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const uint32_t bar_full = smem_u32(smem);
+    volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + 16 * ATT_MAX_STAGES);
+    float* mrg = reinterpret_cast<float*>(smem + ATT_EVEN_HEADER);         // [warp][RT][D + 2]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t D = p.head_dim, NS = p.stages, MS = D + 2u;
+    float* stages = mrg + att_merge_floats(D, RT);
+    const size_t stage_floats = (size_t)2 * ATT_CK * D;
+
+    pdl_launch_dependents();                   // the merge kernel may take its place; it waits for this grid
+    pdl_wait();                                // q, the cache and the tables may come from the kernels just before
+
+    const uint32_t R = p.group, rpb = RT * p.rgp;        // rows: the heads of a KV head
+    const uint32_t all = all_chunks(p);
+    if (!ragged(p, all)) return;
+    // every warp for itself, 32 sequences at a time: the sequence in which this CTA starts
+    const uint32_t share = max(p.share, (all + gridDim.x - 1u) / gridDim.x), at = blockIdx.x * share;
+    if (at >= all) return;
+    Piece first;
+    uint32_t before = 0u;
+    for (uint32_t b0 = 0;; b0 += 32) {
+        const uint32_t n = b0 + lane < p.batch ? chunks_of(paged_len(p, b0 + lane)) : 0u;
+        uint32_t upto = n;                     // inclusive
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, upto, off);
+            if (lane >= off) upto += v;
+        }
+        const uint32_t hit = __ballot_sync(0xffffffffu, (before + upto) * p.kv_heads > at);
+        if (hit) {
+            const int src = __ffs(hit) - 1;
+            first.b = b0 + src;
+            before += __shfl_sync(0xffffffffu, upto - n, src);
+            break;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    first.keys = paged_len(p, first.b);
+    first.n = chunks_of(first.keys);
+    first.ahead = first.b + 1u < p.batch ? paged_len(p, first.b + 1u) : 0u;
+    const uint32_t in = at - before * p.kv_heads;
+    first.g = in / first.n;
+    first.lo = in - first.g * first.n;
+    const uint32_t total = min(share, all - at);         // chunks of this CTA
+    first.hi = min(first.lo + total, first.n);
+    auto next = [&](Piece& w, uint32_t left) { // the piece after w, `left` chunks still to do
+        if (++w.g == p.kv_heads) {
+            w.g = 0u;
+            w.keys = w.ahead;
+            for (w.b++; w.keys == 0u && w.b + 1u < p.batch;) w.keys = paged_len(p, ++w.b);     // (left > 0: there is one)
+            w.n = chunks_of(w.keys);
+            w.ahead = w.b + 1u < p.batch ? paged_len(p, w.b + 1u) : 0u;
+        }
+        w.lo = 0u;
+        w.hi = min(left, w.n);
+    };
+
+    if (tid == 0) {
+        *abort_flag = 0u;
+        for (uint32_t s = 0; s < NS; s++) {
+            mbar_init(bar_full + 8u * s, 1u);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+
+    if (warp == ATT_CW) {
+        // ---- producer: one chunk = keys [t0, t0 + nk) of K and of V ------------------------------
+        Pages pages;
+        Piece w = first, then = first;         // the piece at hand, the one after it
+        uint32_t c = 0;
+        pages.next = pages.ask(p, w.b, w.lo * ATT_CK / p.block_size + lane, w.keys);
+        for (;;) {
+            const uint32_t end = c + (w.hi - w.lo);
+            pages.begin(p, w.b, w.lo * ATT_CK / p.block_size, w.keys, lane);
+            if (end < total) {
+                next(then, total - end);
+                pages.next = pages.ask(p, then.b, lane, then.keys);
+            }
+            for (uint32_t t0 = w.lo * ATT_CK; c < end; c++, t0 += ATT_CK) {
+                const uint32_t s = c % NS, nk = min((uint32_t)ATT_CK, w.keys - t0), bar = bar_full + 8u * s;
+                if (c >= NS) {
+                    named_bar_sync<ATT_BAR_FREE0>(s, ATT_THREADS);      // all consumer warps have left the stage
+                    if (*abort_flag) break;
+                }
+                float* ks = stages + s * stage_floats;
+                if (lane == 0) mbar_expect_tx(bar, 2u * nk * D * 4u);
+                __syncwarp();
+                pages.copy(p, w.g, t0, nk, w.keys, ks, ks + (size_t)ATT_CK * D, bar, lane);
+            }
+            if (c < end || c == total) break;
+            w = then;
+        }
+    } else {
+        // ---- consumers -------------------------------------------------------------------------
+        const uint32_t rg = (uint32_t)warp % p.rgp, kslot = (uint32_t)warp / p.rgp, wpg = ATT_CW / p.rgp;
+        Rows<VPL, RT, FULL> rows;
+        rows.columns(D, lane & 7);
+        const uint32_t row_bytes = D * 4u, lane_off = (uint32_t)(lane & 7) * 16u;
         const uint32_t stage0 = smem_u32(stages), stage_bytes = 2u * ATT_CK * row_bytes, v_off = ATT_CK * row_bytes;
         uint32_t c = 0;
         auto walk = [&](const Piece& w) {                                // the chunks of a piece; false: a wait gave up
-            const uint32_t t_begin = w.lo * ATT_CK, t_end = min(w.hi * ATT_CK, w.lmax);
-            uint32_t t0 = w.start(slices ? w.ahead : blockIdx.x) * ATT_CK;
+            const uint32_t t_end = min(w.hi * ATT_CK, w.keys);
+            uint32_t t0 = w.lo * ATT_CK;
             for (const uint32_t c_end = c + (w.hi - w.lo); c < c_end; c++) {
                 const uint32_t s = c % NS;
                 // one poller per CTA: warp 0 waits for the copies, the named barrier releases the other seven
@@ -491,85 +791,122 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) lux_attn_stream_
                     for (uint32_t cc = c; cc < c + NS && cc + NS < total; cc++) named_bar_arrive<ATT_BAR_FREE0>(cc % NS, ATT_THREADS);
                     return false;
                 }
-                const uint32_t nk = min((uint32_t)ATT_CK, t_end - t0);
-                const uint32_t kchunk = stage0 + s * stage_bytes + lane_off;
-                if (nk == ATT_CK && t0 + ATT_CK <= min_len) {
-                    for (uint32_t kb = kslot * 4u; kb < ATT_CK; kb += wpg * 4u) {
-                        const uint32_t ka = kchunk + (kb + (uint32_t)kg) * row_bytes;
-                        step(std::false_type{}, ka, ka + v_off, true, 0u);
-                    }
-                } else {
-                    for (uint32_t kb = kslot * 4u; kb < nk; kb += wpg * 4u) {
-                        const uint32_t key = kb + (uint32_t)kg, ka = kchunk + key * row_bytes;
-                        step(std::true_type{}, ka, ka + v_off, key < nk, t0 + key);
-                    }
-                }
+                rows.chunk(stage0 + s * stage_bytes + lane_off, v_off, row_bytes, t0, min((uint32_t)ATT_CK, t_end - t0), kslot, wpg, lane >> 3);
                 // done with the stage (not needed for the last NS chunks: nobody refills them)
                 if (c + NS < total) named_bar_arrive<ATT_BAR_FREE0>(s, ATT_THREADS);
                 t0 += ATT_CK;
-                if (t0 >= t_end) t0 = t_begin;
             }
             return true;
         };
-        if constexpr (!EVEN) {
-            begin(first);
-            if (walk(first)) finish(first);                              // (a slice past the rows' keys leaves an empty result)
-        } else {
-            // the piece lies in shared memory while its chunks are worked on: the loop has no registers left for it
-            Piece* const kept = reinterpret_cast<Piece*>(smem + 128) + warp;
-            Piece w = first;
-            for (;;) {
-                begin(w);
-                if (lane == 0) *kept = w;
-                __syncwarp();
-                if (!walk(w)) break;
-                w.load(kept);
-                finish(w);
-                if (c == total) break;
-                next(w, total - c);
-                __syncwarp();
+        // the end of a piece: the warps of each row group are merged and the rows written: the outputs of a whole item, else
+        // partial results
+        auto finish = [&](const Piece& w) {
+#pragma unroll
+            for (int i = 0; i < RT; i++) {
+                rows.fold(i);
+                rows.store(i, mrg + ((size_t)warp * RT + i) * MS, D, lane);
             }
+            named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);
+            const bool whole = w.lo == 0u && w.hi == w.n;
+            if (w.lo == 0u && tid == 0)                                  // the item may go on in the CTAs after this one
+                p.spans[w.b * p.kv_heads + w.g] = AttnSpan{(int32_t)blockIdx.x, (int32_t)(1u + (w.n - w.hi + share - 1u) / share)};
+            for (uint32_t e = tid; e < rpb * D; e += ATT_CW * 32) {
+                const uint32_t ir = e / D, d = e - ir * D;
+                if (ir >= R) continue;
+                float M, L, acc;
+                merge_warps<RT>(mrg, ir, d, D, p.rgp, wpg, M, L, acc);
+                const size_t orow = (size_t)w.b * p.heads + w.g * p.group + ir;
+                if (whole) {
+                    p.out[orow * D + d] = L > 0.0f ? acc / L : 0.0f;
+                } else {
+                    float* dst = p.part + ((size_t)(blockIdx.x * 2u + (w.lo == 0u ? 1u : 0u)) * rpb + ir) * MS;
+                    dst[d] = acc;
+                    if (d == 0) {
+                        dst[D] = M;
+                        dst[D + 1] = L;
+                    }
+                }
+            }
+            named_bar_sync_c<ATT_BAR_MERGE>(ATT_CW * 32);                // before the next piece is merged
+        };
+        // the piece lies in shared memory while its chunks are worked on: the loop has no registers left for it
+        Piece* const kept = reinterpret_cast<Piece*>(smem + ATT_HEADER) + warp;
+        Piece w = first;
+        for (;;) {
+            rows.begin(p, w.b, w.g, rg * RT, w.keys, lane & 7);
+            if (lane == 0) *kept = w;
+            __syncwarp();
+            if (!walk(w)) break;
+            w.load(kept);
+            finish(w);
+            if (c == total) break;
+            next(w, total - c);
+            __syncwarp();
         }
     }
 
     __syncthreads();               // every chunk has landed and been read
-    if (*abort_flag) {
-        // A bounded wait gave up: report it and give copies still in flight time to land in this
-        // CTA's shared memory before it is released.  The piece it was in is not written.
-        if (tid == 0 && p.status) atomicOr(p.status, ATT_STATUS_WAIT);
-        for (int i = 0; i < 64; i++) __nanosleep(1000);
-        __syncthreads();
-    }
+    if (*abort_flag) report_abort(p);          // the piece it was in is not written, nor what comes after it
 }
 
-// Merge of the partial results of one output row (paged_attention_v2_reduce, paged.wgsl:351-405, with
+// Merge of the key slices of one output row (paged_attention_v2_reduce, paged.wgsl:351-405, with
 // the statistics in the base-2 domain).  One CTA per row; resident early, it waits for the slices.
-constexpr int ATT_MAX_PARTS = 512;
-__global__ void __launch_bounds__(128) lux_attn_merge_f32(const AttnParams p) {
-    __shared__ float wgt[ATT_MAX_PARTS];
+__global__ void __launch_bounds__(128) lux_attn_merge_f32(const float* __restrict__ part, float* __restrict__ out, float* __restrict__ lse,
+                                                          const int32_t* __restrict__ context_lens, uint32_t rows_per_seq,
+                                                          uint32_t nsplit, uint32_t D) {
+    __shared__ float wgt[256];
     __shared__ float stat[2];
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t row = blockIdx.x, D = p.head_dim, MS = D + 2u, b = row / (p.heads * p.seq_q);
-    if (p.context_lens && p.context_lens[b] <= 0) return;
-    // partial result 0, partial result 1 and the step from it to each of the others
-    const float *base0, *base1;
-    size_t step;
-    uint32_t parts;
-    const uint32_t hq = row - b * (p.heads * p.seq_q), head = hq / p.seq_q, qi = hq - head * p.seq_q;
-    const AttnSpan span = p.share ? p.spans[b * p.kv_heads + head / p.group] : AttnSpan{0, 0};
+    const uint32_t row = blockIdx.x, MS = D + 2u;
+    if (context_lens && context_lens[row / rows_per_seq] <= 0) return;
+    const float* base = part + (size_t)row * nsplit * MS;
+    if (threadIdx.x < 32) {
+        float M = ATT_NEG;
+        for (uint32_t s = threadIdx.x; s < nsplit; s += 32) M = fmaxf(M, base[(size_t)s * MS + D]);
+        for (int off = 16; off; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+        float L = 0.0f;
+        for (uint32_t s = threadIdx.x; s < nsplit; s += 32) {
+            const float w = exp2f(base[(size_t)s * MS + D] - M);
+            wgt[s] = w;
+            L = fmaf(base[(size_t)s * MS + D + 1], w, L);
+        }
+        for (int off = 16; off; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
+        if (threadIdx.x == 0) {
+            stat[0] = M;
+            stat[1] = L;
+        }
+    }
+    __syncthreads();
+    const float L = stat[1], inv = L > 0.0f ? 1.0f / L : 0.0f;
+    for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
+        float acc = 0.0f;
+        for (uint32_t s = 0; s < nsplit; s++) acc = fmaf(base[(size_t)s * MS + d], wgt[s], acc);
+        out[(size_t)row * D + d] = acc * inv;
+    }
+    if (threadIdx.x == 0 && lse) lse[row] = L > 0.0f ? fmaf(stat[0], ATT_LN2, logf(L)) : -3.402823e+38f;
+}
+
+// The same for a paged cache that may have been dealt out in even shares: slices, what several CTAs did of a row, or nothing to do.
+__global__ void __launch_bounds__(128) lux_attn_merge_even_f32(const AttnParams p) {
+    __shared__ float wgt[ATT_MAX_PARTS];
+    __shared__ float denominator;
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t row = blockIdx.x, D = p.head_dim, MS = D + 2u, b = row / p.heads, head = row - b * p.heads;
+    if (p.context_lens[b] <= 0) return;
+    const AttnSpan span = p.spans[b * p.kv_heads + head / p.group];
     if (span.ctas == 1) return;                        // one CTA saw all of it and wrote the row
-    if (span.ctas == 0) {
-        base0 = p.part + (size_t)row * p.nsplit * MS;
-        base1 = base0 + MS;
-        step = MS;
-        parts = p.nsplit;
-    } else {
+    // partial result 0, partial result 1 and the step from it to each of the others
+    const float *base0 = p.part + (size_t)row * p.nsplit * MS, *base1 = base0 + MS;
+    size_t step = MS;
+    uint32_t parts = p.nsplit;
+    if (span.ctas != 0) {
         if (!span_fits(span, p.ctas)) {                // never written: a wait gave up in the CTA in which the item begins
             if (threadIdx.x == 0 && p.status) atomicOr(p.status, ATT_STATUS_WAIT);
             return;
         }
-        const uint32_t ir = qi * p.group + head % p.group;
+        const uint32_t ir = head % p.group;
         base0 = p.part + ((size_t)span_place(span, 0) * p.rpb + ir) * MS;
         base1 = p.part + ((size_t)span_place(span, 1) * p.rpb + ir) * MS;
         step = (size_t)2 * p.rpb * MS;
@@ -587,19 +924,15 @@ __global__ void __launch_bounds__(128) lux_attn_merge_f32(const AttnParams p) {
             L = fmaf(part(s)[D + 1], w, L);
         }
         for (int off = 16; off; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
-        if (threadIdx.x == 0) {
-            stat[0] = M;
-            stat[1] = L;
-        }
+        if (threadIdx.x == 0) denominator = L;
     }
     __syncthreads();
-    const float L = stat[1], inv = L > 0.0f ? 1.0f / L : 0.0f;
+    const float L = denominator, inv = L > 0.0f ? 1.0f / L : 0.0f;
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         float acc = 0.0f;
         for (uint32_t s = 0; s < parts; s++) acc = fmaf(part(s)[d], wgt[s], acc);
         p.out[(size_t)row * D + d] = acc * inv;
     }
-    if (threadIdx.x == 0 && p.lse) p.lse[row] = L > 0.0f ? fmaf(stat[0], ATT_LN2, logf(L)) : -3.402823e+38f;
 }
 
 // Any head_dim, any alignment: one CTA per output row, 256 keys per step (a thread per key for the
@@ -810,18 +1143,21 @@ uint32_t pow2ceil(uint32_t v) {
 }
 
 using AttnKernel = void (*)(const AttnParams);
-template <int VPL, int RT> AttnKernel stream_kernel(bool full, bool even) {
-    if (even) return full ? lux_attn_stream_f32<VPL, RT, true, true> : lux_attn_stream_f32<VPL, RT, false, true>;
-    return full ? lux_attn_stream_f32<VPL, RT, true, false> : lux_attn_stream_f32<VPL, RT, false, false>;
+enum Form { SLICES, SLICES_GATED, EVEN };
+template <int VPL, int RT, bool FULL> AttnKernel decode_kernel(Form f) {
+    return f == EVEN ? lux_attn_even_f32<VPL, RT, FULL> : f == SLICES_GATED ? lux_attn_stream_f32<VPL, RT, FULL, true> : lux_attn_stream_f32<VPL, RT, FULL, false>;
+}
+template <int VPL, int RT> AttnKernel decode_kernel(bool full, Form f) {
+    return full ? decode_kernel<VPL, RT, true>(f) : decode_kernel<VPL, RT, false>(f);
 }
 // full: head_dim is exactly VPL * 32, so no lane has a column to skip
-AttnKernel pick_stream(int vpl, int rt, bool full, bool even) {
+AttnKernel pick_kernel(int vpl, int rt, bool full, Form f) {
     switch (vpl * 10 + rt) {
-        case 11: return stream_kernel<1, 1>(full, even); case 12: return stream_kernel<1, 2>(full, even);
-        case 21: return stream_kernel<2, 1>(full, even); case 22: return stream_kernel<2, 2>(full, even);
-        case 31: return stream_kernel<3, 1>(full, even); case 32: return stream_kernel<3, 2>(full, even);
-        case 41: return stream_kernel<4, 1>(full, even); case 42: return stream_kernel<4, 2>(full, even);
-        case 81: return stream_kernel<8, 1>(full, even);
+        case 11: return decode_kernel<1, 1>(full, f); case 12: return decode_kernel<1, 2>(full, f);
+        case 21: return decode_kernel<2, 1>(full, f); case 22: return decode_kernel<2, 2>(full, f);
+        case 31: return decode_kernel<3, 1>(full, f); case 32: return decode_kernel<3, 2>(full, f);
+        case 41: return decode_kernel<4, 1>(full, f); case 42: return decode_kernel<4, 2>(full, f);
+        case 81: return decode_kernel<8, 1>(full, f);
     }
     return nullptr;
 }
@@ -903,7 +1239,7 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     uint32_t min_split = 1;
     if (p.block_size) {
         // a slice (a multiple of the chunk) spans at most split_keys / block_size + 2 pages
-        const uint64_t cap = ATT_PAGES / 256 * p.block_size / ATT_CK * ATT_CK;
+        const uint64_t cap = (uint64_t)(ATT_TABLE - 2) * p.block_size / ATT_CK * ATT_CK;
         min_split = (uint32_t)std::max<uint64_t>((max_keys + cap - 1) / cap, 1);
     }
     uint32_t best = min_split;
@@ -943,59 +1279,71 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     }
     geometry(g_tune.attn_splits > 0 ? std::max<uint32_t>((uint32_t)g_tune.attn_splits, min_split) : best);
     if (p.nsplit > 256) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;     // a context beyond 256 x 2046 pages
-    // A decode step over a paged cache deals its chunks out evenly over one wave of CTAs, wherever sequences begin and end
-    // (their lengths are known on the device only).  It costs a CTA some microseconds to end one item and begin another, so
-    // this is for caches that may hold 1000 keys of a sequence and more: equal items stay with the slices.
-    const uint32_t slots = (uint32_t)ctx->sm_count * (D > 128 ? 1 : ATT_CTAS_PER_SM), n = (max_keys + ATT_CK - 1) / ATT_CK;
-    const uint64_t all = (uint64_t)items * n;
+    // A paged cache whose sequences may differ in length by enough has both kernels launched (gated): even shares if more than
+    // `slack` of a full cache's chunks are missing, else slices.  A share costs a CTA some microseconds where it ends one item and
+    // begins the next, about what 7 chunks take, or 14 chunks an item where CTAs take many items each; the kernel that leaves at once 1 to 3 us.
+    // So this is for caches large enough that sequences of evenly spread lengths leave more than that missing (0.42 of a full one).
+    // Llama-3-8B heads, 16-token pages, us a step by slices / by shares / gated.  Lengths 1, .2, .5, .9, ... of the longest: 8 x 2500 37.3 / 34.3 / 37.1,
+    // 8 x 8000 83.8 / 64.6 / 66.7, 16 x 4000 90.0 / 68.4 / 71.4, 32 x 2000 85.7 / 71.2 / 73.3, 64 x 1500 107 / 97.8 / 102.8; not gated:
+    // 8 x 2000 32.3 / 31.3, 20 x 1000 39.4 / 37.0, 32 x 1000 48.5 / 48.8, 48 x 1000 64.6 / 66.2, 64 x 1000 76.2 / 79.9.  All as long as the longest: 1 x 32768
+    // 57.4 / 63.4 / 60.0, 8 x 8192 97.8 / 100.1 / 100.9, 32 x 2048 89.4 / 101.5 / 94.8.
+    const uint32_t slots = (uint32_t)ctx->sm_count * (D > 128 ? 1 : ATT_CTAS_PER_SM);
+    const uint64_t full_chunks = (uint64_t)items * chunks_of(max_keys);
     const size_t even_part = std::max((size_t)slots * 2 * rpb, out_rows * p.nsplit) * (D + 2) * 4 / 16 * 16 + 16;
-    size_t ctas = items * p.nsplit;
-    bool merge = p.nsplit > 1;
-    if (p.block_size && p.row_blocks == 1 && max_keys >= ATT_EVEN_KEYS && all < (1u << 31) && !g_tune.attn_splits && slots <= ATT_MAX_PARTS &&
-        even_part + items * sizeof(AttnSpan) <= ctx->d_attn_bytes) {
+    const uint64_t slack = g_tune.attn_even == 1 ? 0u : std::max<uint64_t>(7u * slots, 14u * items);
+    const bool gated = p.block_size && p.row_blocks == 1 && full_chunks < (1u << 31) && full_chunks * 5u >= slack * 12u && g_tune.attn_even != 2 &&
+                       !g_tune.attn_splits && slots <= ATT_MAX_PARTS && even_part + items * sizeof(AttnSpan) <= ctx->d_attn_bytes;
+    if (gated) {
+        p.full_chunks = (uint32_t)full_chunks;
+        p.slack = (uint32_t)slack;
         p.share = 4;                           // a share is no shorter than the shortest slice above
-        ctas = std::min<uint64_t>((all + p.share - 1) / p.share, slots);
-        merge = true;
+        p.ctas = (uint32_t)std::min<uint64_t>((full_chunks + p.share - 1) / p.share, slots);
         p.part = (float*)ctx->d_attn;
         p.spans = (AttnSpan*)((unsigned char*)ctx->d_attn + even_part);
-    } else if (merge) {
+    } else if (p.nsplit > 1) {
         if (out_rows * p.nsplit * (D + 2) * 4 > ctx->d_attn_bytes) {
             // fewer slices than wanted rather than an allocation inside a call
             const uint32_t fit = (uint32_t)(ctx->d_attn_bytes / (out_rows * (D + 2) * 4));
             if (std::max(fit, 1u) < min_split) return LUX_BACKEND_ERROR_OUT_OF_MEMORY;
             geometry(std::max(fit, 1u));
-            ctas = items * p.nsplit;
-            merge = p.nsplit > 1;
         }
         p.part = (float*)ctx->d_attn;
     }
-    const size_t stage_bytes = (size_t)2 * ATT_CK * D * 4;
-    const size_t fixed = ATT_HEADER + att_merge_floats(D, rt) * 4;
-    // heads wider than 128 take the whole SM's shared memory (one CTA per SM)
-    const size_t budget = D > 128 ? 2 * ATT_SMEM_BUDGET : ATT_SMEM_BUDGET;
-    p.stages = (uint32_t)std::min<size_t>(ATT_MAX_STAGES, (budget - fixed) / stage_bytes);
-    const size_t smem = fixed + p.stages * stage_bytes;
-    const bool full = D == (uint32_t)vpl * 32u;
-    AttnKernel kfn = pick_stream(vpl, rt, full, p.share != 0);
-    if (!kfn || p.stages < 2) return LUX_BACKEND_ERROR_INTERNAL;
-    static std::mutex mu;
-    static bool attr_set[16][9][3][2][2];
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        bool& done = attr_set[ctx->device & 15][vpl][rt][full ? 1 : 0][p.share ? 1 : 0];
-        if (!done) {
-            if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * ATT_SMEM_BUDGET)) != cudaSuccess)
-                return map_cuda(cudaGetLastError(), what);
-            done = true;
-        }
-    }
+    const size_t ctas = items * p.nsplit;
     if (ctas > 0x7fffffffu) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
-    p.ctas = (uint32_t)ctas;
-    cudaError_t e = launch_pdl(g_tune.pdl != 2, kfn, dim3((unsigned)ctas), dim3(ATT_THREADS), smem, ctx->stream, 1, p);
-    if (e != cudaSuccess) return map_cuda(e, what);
-    count_launch("lux_attn_stream_f32");
-    if (merge) {
-        e = launch_pdl(g_tune.pdl != 2, lux_attn_merge_f32, dim3((unsigned)out_rows), dim3(128), 0, ctx->stream, 1, p);
+    const bool full = D == (uint32_t)vpl * 32u;
+    auto launch = [&](Form form, size_t grid) {
+        const size_t stage_bytes = (size_t)2 * ATT_CK * D * 4;
+        const size_t fixed = form == EVEN ? ATT_EVEN_HEADER + att_merge_floats(D, rt) * 4 : ATT_HEADER + (p.block_size ? ATT_TABLE * 4 : 0);
+        // heads wider than 128 take the whole SM's shared memory (one CTA per SM)
+        const size_t budget = D > 128 ? 2 * ATT_SMEM_BUDGET : ATT_SMEM_BUDGET;
+        p.stages = (uint32_t)std::min<size_t>(ATT_MAX_STAGES, (budget - fixed) / stage_bytes);
+        AttnKernel kfn = pick_kernel(vpl, rt, full, form);
+        if (!kfn || p.stages < 2) return LUX_BACKEND_ERROR_INTERNAL;
+        static std::mutex mu;
+        static bool attr_set[16][9][3][2][3];
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            bool& done = attr_set[ctx->device & 15][vpl][rt][full ? 1 : 0][form];
+            if (!done) {
+                if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * ATT_SMEM_BUDGET)) != cudaSuccess)
+                    return map_cuda(cudaGetLastError(), what);
+                done = true;
+            }
+        }
+        const cudaError_t e = launch_pdl(g_tune.pdl != 2, kfn, dim3((unsigned)grid), dim3(ATT_THREADS), fixed + p.stages * stage_bytes, ctx->stream, 1, p);
+        if (e != cudaSuccess) return map_cuda(e, what);
+        count_launch(form == EVEN ? "lux_attn_even_f32" : "lux_attn_stream_f32");
+        return LUX_BACKEND_OK;
+    };
+    LuxBackendError le = gated ? launch(EVEN, p.ctas) : LUX_BACKEND_OK;
+    if (le == LUX_BACKEND_OK) le = launch(gated ? SLICES_GATED : SLICES, ctas);
+    if (le != LUX_BACKEND_OK) return le;
+    if (gated || p.nsplit > 1) {
+        const dim3 grid((unsigned)out_rows), block(128);
+        const cudaError_t e = gated ? launch_pdl(g_tune.pdl != 2, lux_attn_merge_even_f32, grid, block, 0, ctx->stream, 1, p)
+                                    : launch_pdl(g_tune.pdl != 2, lux_attn_merge_f32, grid, block, 0, ctx->stream, 1, (const float*)p.part, p.out, p.lse,
+                                                 p.context_lens, p.heads * p.seq_q, p.nsplit, D);
         if (e != cudaSuccess) return map_cuda(e, what);
         count_launch("lux_attn_merge_f32");
     }
