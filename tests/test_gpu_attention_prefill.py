@@ -415,3 +415,74 @@ def test_calls_on_two_streams_share_the_scratch_in_order(backend):
     finally:
         c.set_stream(0)
         c.destroy()
+
+
+class _Prompts:
+    """Prompts of several lengths on the GPU, each with the bits that it has alone."""
+
+    def __init__(self, backend, lengths, H=8, Hkv=2):
+        import torch
+        self.torch, self.c, self.H, self.Hkv = torch, backend.create_context(0), H, Hkv
+        self.data = []
+        for i, S in enumerate(lengths):
+            t = [torch.from_numpy(x).cuda() for x in _qkv(80 + i, 1, H, Hkv, S, S)]
+            t.append(torch.zeros_like(t[0]))
+            self.data.append((S, t, [self.c.wrap(x.data_ptr(), x.numel() * 4) for x in t]))
+        torch.cuda.synchronize()
+        self.want = []
+        for i in range(len(lengths)):
+            self.call(i, 0)
+            self.want.append(self.data[i][1][3].cpu().numpy().view(np.uint32).copy())
+            self.data[i][1][3].zero_()
+        torch.cuda.synchronize()
+
+    def call(self, i, flags=B.FLAG_NO_SYNC):
+        S, _, b = self.data[i]
+        self.c.sdpa(*b, 1, self.H, self.Hkv, S, S, 128, 1 / np.sqrt(128), flags=flags | B.FLAG_ATTN_CAUSAL)
+
+    def check(self):
+        self.torch.cuda.synchronize()
+        for (_, t, _), w in zip(self.data, self.want):
+            assert np.array_equal(t[3].cpu().numpy().view(np.uint32), w)
+
+    def clear(self):
+        for _, t, _ in self.data:
+            t[3].zero_()
+        self.torch.cuda.synchronize()
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.torch.cuda.synchronize()
+        self.c.set_stream(0)
+        self.c.destroy()
+
+
+def test_order_of_the_scratch_survives_a_capture_and_a_blocking_call(backend):
+    """A long prompt on one stream; then on another, the context having been on a capturing stream or in a blocking
+    call in between, a short one: it still begins behind the first."""
+    with _Tuned(backend, attn_prefill=1), _Prompts(backend, (4000, 700, 130), H=16, Hkv=4) as pr:
+        torch = pr.torch
+        for between in ("capture", "blocking", "same handle"):
+            a, b = torch.cuda.Stream(), torch.cuda.Stream()
+            other = torch.zeros(1 << 20, device="cuda")
+            ob = pr.c.wrap(other.data_ptr(), other.numel() * 4)
+            pr.clear()
+            pr.c.set_stream(a.cuda_stream)
+            for _ in range(4):
+                pr.call(0)
+            if between == "capture":
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=b, capture_error_mode="relaxed"):
+                    pr.c.set_stream(b.cuda_stream)
+                    pr.c.rope_precompute_cache(ob, ob, 16, 128, 1e4, B.FLAG_NO_SYNC)
+            elif between == "blocking":
+                pr.c.set_stream(b.cuda_stream)
+                pr.c.rope_precompute_cache(ob, ob, 16, 128, 1e4, 0)
+            else:
+                pr.c.set_stream(b.cuda_stream)
+                pr.c.set_stream(b.cuda_stream)
+            pr.call(1)
+            pr.call(2)
+            pr.check()

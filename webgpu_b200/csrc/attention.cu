@@ -1270,11 +1270,6 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
         f.kv_len = p.kv_len; f.kv_stride = p.kv_stride; f.causal = p.causal; f.causal_base = p.causal_base;
         f.qscale = p.qscale;
         const LuxBackendError e = launch_attn_prefill(ctx, f, g_tune.attn_prefill == 3);
-        if (e == LUX_BACKEND_OK && (flags & LUX_QMATMUL_FLAG_NO_SYNC)) {
-            cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
-            else if (st == cudaStreamCaptureStatusNone) ctx->parts_pending = cudaEventRecord(ctx->parts_event, ctx->stream) == cudaSuccess;
-        }
         return e != LUX_BACKEND_OK ? e : finish_op(ctx, (flags & LUX_QMATMUL_FLAG_NO_SYNC) != 0, what);
     }
     geometry(g_tune.attn_splits > 0 ? std::max<uint32_t>((uint32_t)g_tune.attn_splits, min_split) : best);

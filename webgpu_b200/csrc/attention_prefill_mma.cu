@@ -647,6 +647,13 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
     geo.levels = geo.by_head ? p.q_blocks : (p.q_blocks + 1) / 2;
     const char* name = "lux_attn_prefill_mma_f32";
     cudaError_t e = allow_smem((const void*)lux_attn_prefill_mma_f32, 1, SMEM, ctx->device);
+    // The scratch is the context's: this call begins behind the last one that used it, on whichever stream that was.  (What is
+    // captured is ordered by its graph.)
+    std::lock_guard<std::mutex> lk(ctx->parts_mu);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (e == cudaSuccess) e = cudaStreamIsCapturing(ctx->stream, &capture);
+    const bool direct = capture == cudaStreamCaptureStatusNone;
+    if (e == cudaSuccess && direct && ctx->parts_used && !ctx->parts_ordered) e = cudaStreamWaitEvent(ctx->stream, ctx->parts_event, 0);
     // as many (sequence, KV head) pairs at a time as have their parts in the scratch (in one call all, up to 128 k keys in total)
     for (geo.bk0 = 0; e == cudaSuccess && geo.bk0 < bks; geo.bk0 += geo.nbk) {
         geo.nbk = std::min(fit, bks - geo.bk0);
@@ -662,6 +669,10 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
         }
         e = launch_pdl(g_tune.pdl != 2, lux_attn_prefill_mma_f32, dim3(2u * geo.levels * geo.nbk * geo.units), dim3(THREADS), (size_t)SMEM, ctx->stream, 1, p, geo);
         if (e == cudaSuccess) count_launch(name);
+    }
+    if (e == cudaSuccess && direct) {
+        e = cudaEventRecord(ctx->parts_event, ctx->stream);
+        ctx->parts_used = ctx->parts_ordered = true;
     }
     return e == cudaSuccess ? LUX_BACKEND_OK : map_cuda(e, name);
 }

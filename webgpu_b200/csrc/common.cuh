@@ -53,8 +53,10 @@ struct Context {
     size_t         d_attn_bytes = 0;        // 16 MB, allocated with the context (a call takes fewer slices rather than allocate)
     void*          d_parts = nullptr;       // bf16 parts of K and V of prompt attention: 1536 bytes a key and KV head,
     size_t         d_parts_bytes = 0;       // 128 k of them, allocated with the context (a larger call goes in several passes)
-    bool           parts_pending = false;   // a call that uses them has been enqueued without a wait,
-    cudaEvent_t    parts_event = nullptr;   // and this is its end: another stream is ordered behind it (lux_cuda_context_set_stream)
+    std::mutex     parts_mu;                // held while such a call enqueues its kernels: threads do not mix theirs
+    cudaEvent_t    parts_event = nullptr;   // the end of the last such call,
+    bool           parts_used = false;      // if there was one,
+    bool           parts_ordered = false;   // and whether the context's stream runs behind it
     std::mutex     mu;                      // guards the staging buffers
     int            sm_count = 148;
     // A kernel of this library that WRITES a buffer a later matmul may bind as weights, scales or

@@ -29,7 +29,6 @@ LuxBackendError finish_op(Context* ctx, bool no_sync, const char* what) {
         return LUX_BACKEND_ERROR_DEVICE_LOST;
     }
     ctx->writer_pending = false;             // everything enqueued so far has completed
-    ctx->parts_pending = false;
     if (ctx->h_status && *(volatile uint32_t*)ctx->h_status != 0) {
         ctx->last_status = *(volatile uint32_t*)ctx->h_status;
         *(volatile uint32_t*)ctx->h_status = 0;
@@ -479,17 +478,11 @@ extern "C" {
 LuxBackendError lux_cuda_context_set_stream(LuxBackendContext* context, void* stream) {
     auto* ctx = as_ctx(context);
     if (!ctx) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
-    const cudaStream_t next = stream ? reinterpret_cast<cudaStream_t>(stream) : ctx->own_stream;
-    if (next != ctx->stream && ctx->parts_pending) {
-        // A prompt's attention may still be reading its scratch: what follows on the new stream waits for it.  (Not into a
-        // capture, whose events belong to its graph; the old stream may be gone by now and is not touched.)
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        cudaSetDevice(ctx->device);
-        if (cudaStreamIsCapturing(next, &st) != cudaSuccess ||
-            (st == cudaStreamCaptureStatusNone && cudaStreamWaitEvent(next, ctx->parts_event, 0) != cudaSuccess))
-            cudaGetLastError();
-    }
-    ctx->stream = next;
+    // A prompt's attention may still be reading its scratch: the next one on this stream waits for it (also if the handle is
+    // the same, which may by now be another stream's).
+    std::lock_guard<std::mutex> lk(ctx->parts_mu);
+    ctx->stream = stream ? reinterpret_cast<cudaStream_t>(stream) : ctx->own_stream;
+    ctx->parts_ordered = false;
     return LUX_BACKEND_OK;
 }
 
