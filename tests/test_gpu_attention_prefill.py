@@ -445,6 +445,10 @@ class _Prompts:
         for (_, t, _), w in zip(self.data, self.want):
             assert np.array_equal(t[3].cpu().numpy().view(np.uint32), w)
 
+    def check_nothing_ran(self):
+        self.torch.cuda.synchronize()
+        assert not any(t[3].any().item() for _, t, _ in self.data)
+
     def clear(self):
         for _, t, _ in self.data:
             t[3].zero_()
@@ -485,4 +489,58 @@ def test_order_of_the_scratch_survives_a_capture_and_a_blocking_call(backend):
                 pr.c.set_stream(b.cuda_stream)
             pr.call(1)
             pr.call(2)
+            pr.check()
+
+
+def test_replayed_prompts_and_direct_ones_share_nothing(backend):
+    """Graphs that hold prompts are replayed on one stream, others, and direct calls, run beside them: every output keeps
+    the bits that its call has alone.  What a graph had is given back when it is gone."""
+    with _Tuned(backend, attn_prefill=1), _Prompts(backend, (3000, 900, 130, 2000), H=16, Hkv=4) as pr:
+        torch = pr.torch
+        a, b, c = (torch.cuda.Stream() for _ in range(3))
+        def capture(stream, prompts):
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                pr.c.set_stream(stream.cuda_stream)
+                for i in prompts:
+                    pr.call(i)
+            return g
+        free = []
+        for _ in range(3):
+            pr.clear()
+            ga, gb = capture(a, (2, 0)), capture(b, (1,))           # the longer one last: a larger scratch for the same stream
+            pr.check_nothing_ran()
+            for _ in range(3):
+                with torch.cuda.stream(a):
+                    ga.replay()
+                with torch.cuda.stream(b):
+                    gb.replay()
+                pr.c.set_stream(c.cuda_stream)
+                pr.call(3)
+            pr.check()
+            del ga, gb
+            torch.cuda.synchronize()
+            pr.c.set_stream(c.cuda_stream)
+            pr.call(2, 0)
+            free.append(torch.cuda.mem_get_info()[0])
+        assert free[1] == free[2]
+
+
+def test_a_capture_that_forks_has_a_scratch_for_each_branch(backend):
+    """Two streams within one capture: the branches run side by side in a replay."""
+    with _Tuned(backend, attn_prefill=1), _Prompts(backend, (1500, 1400), H=4, Hkv=2) as pr:
+        torch = pr.torch
+        a, b = torch.cuda.Stream(), torch.cuda.Stream()
+        pr.clear()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=a):
+            b.wait_stream(a)
+            pr.c.set_stream(b.cuda_stream)
+            pr.call(1)
+            pr.c.set_stream(a.cuda_stream)
+            pr.call(0)
+            a.wait_stream(b)
+        for _ in range(3):
+            pr.clear()
+            g.replay()
             pr.check()

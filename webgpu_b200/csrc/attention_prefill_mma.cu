@@ -47,6 +47,8 @@
 #include "attention_ring.h"
 
 #include <algorithm>
+#include <cstddef>
+#include <new>
 
 namespace luxcuda {
 
@@ -621,6 +623,71 @@ cudaError_t allow_smem(const void* kfn, int which, int bytes, int device) {
     return e;
 }
 
+// Allocates and frees wherever the caller is, in a capture too (neither becomes part of it).
+struct Uncaptured {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Scratch of at least `want` bytes for a call that is being captured: the graph's own, shared by what is captured one after the other on
+// one stream, and kept until the graph and all that was instantiated from it are gone (a replay in flight included).  Null: there is none.
+const GraphParts* graph_scratch(Context* ctx, size_t want) try {
+    cudaStreamCaptureStatus st;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(ctx->stream, &st, &id, &graph) != cudaSuccess || st != cudaStreamCaptureStatusActive) return nullptr;
+    GraphParts* best = nullptr;
+    for (GraphParts& g : ctx->graph_parts) {
+        if (g.bytes < want) continue;
+        const bool live = g.live->load(std::memory_order_acquire);
+        if (live && g.capture == id && g.stream == ctx->stream) return &g;
+        if (!live && (!best || g.bytes < best->bytes)) best = &g;         // a graph that is gone left it
+    }
+    if (!best) {
+        Uncaptured scope;
+        GraphParts g{nullptr, want, 0, nullptr, std::make_shared<std::atomic<bool>>(false)};
+        ctx->graph_parts.reserve(ctx->graph_parts.size() + 1);
+        if (cudaMalloc(&g.p, want) != cudaSuccess) return nullptr;
+        ctx->graph_parts.push_back(std::move(g));
+        best = &ctx->graph_parts.back();
+    }
+    auto* held = new std::shared_ptr<std::atomic<bool>>(best->live);
+    auto release = [](void* h) {                      // may come from any thread, after the context
+        auto* flag = static_cast<std::shared_ptr<std::atomic<bool>>*>(h);
+        (*flag)->store(false, std::memory_order_release);
+        delete flag;
+    };
+    cudaUserObject_t object;
+    if (cudaUserObjectCreate(&object, held, release, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        delete held;
+        return nullptr;
+    }
+    best->live->store(true, std::memory_order_release);
+    if (cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaUserObjectRelease(object, 1);
+        return nullptr;
+    }
+    best->capture = id;
+    best->stream = ctx->stream;
+    return best;
+} catch (const std::bad_alloc&) {
+    return nullptr;
+}
+
+// Gives back what graphs that are gone have left.
+void free_idle_graph_scratch(Context* ctx) {
+    for (size_t i = 0; i < ctx->graph_parts.size();) {
+        if (ctx->graph_parts[i].live->load(std::memory_order_acquire)) {
+            i++;
+            continue;
+        }
+        Uncaptured scope;
+        cudaFree(ctx->graph_parts[i].p);
+        ctx->graph_parts.erase(ctx->graph_parts.begin() + (std::ptrdiff_t)i);
+    }
+}
+
 }  // namespace pmma
 }  // namespace
 
@@ -631,10 +698,27 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
     Geometry geo{};
     geo.all_tiles = (keys + BN - 1) / BN;
     const size_t per_bk = geo.all_tiles * (TILE_BYTES + 8);
-    const uint32_t bks = p.batch * p.kv_heads, fit = per_bk ? (uint32_t)std::min<size_t>(ctx->d_parts_bytes / per_bk, 65535) : 65535u;
+    const uint32_t bks = p.batch * p.kv_heads;
+    // The scratch is the context's, or the graph's for a call that is being captured.
+    std::lock_guard<std::mutex> lk(ctx->parts_mu);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(ctx->stream, &capture);
+    if (e != cudaSuccess) return map_cuda(e, "lux_attn_prefill_mma_f32");
+    const bool direct = capture == cudaStreamCaptureStatusNone;
+    void* scratch = ctx->d_parts;
+    size_t scratch_bytes = ctx->d_parts_bytes;
+    if (direct) {
+        free_idle_graph_scratch(ctx);
+    } else if (!f32_only && per_bk && per_bk <= scratch_bytes) {
+        const GraphParts* own = graph_scratch(ctx, std::min(bks * per_bk, scratch_bytes));
+        if (!own) cudaGetLastError();
+        scratch = own ? own->p : nullptr;
+        scratch_bytes = own ? own->bytes : 0;
+    }
+    const uint32_t fit = per_bk ? (uint32_t)std::min<size_t>(scratch_bytes / per_bk, 65535) : 65535u;
     if (f32_only || fit == 0) {                        // (128 k keys per KV head fit the scratch)
         const char* name = "lux_attn_prefill_f32";
-        cudaError_t e = allow_smem((const void*)lux_attn_prefill_f32, 0, prefill::PF_SMEM + 128, ctx->device);
+        e = allow_smem((const void*)lux_attn_prefill_f32, 0, prefill::PF_SMEM + 128, ctx->device);
         if (e == cudaSuccess)
             e = launch_pdl(g_tune.pdl != 2, lux_attn_prefill_f32, dim3(p.q_blocks * p.heads * p.batch), dim3(prefill::PF_THREADS),
                            (size_t)prefill::PF_SMEM + 128, ctx->stream, 1, p);
@@ -646,18 +730,13 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
     geo.units = geo.by_head ? p.group / 2 : p.group;
     geo.levels = geo.by_head ? p.q_blocks : (p.q_blocks + 1) / 2;
     const char* name = "lux_attn_prefill_mma_f32";
-    cudaError_t e = allow_smem((const void*)lux_attn_prefill_mma_f32, 1, SMEM, ctx->device);
-    // The scratch is the context's: this call begins behind the last one that used it, on whichever stream that was.  (What is
-    // captured is ordered by its graph.)
-    std::lock_guard<std::mutex> lk(ctx->parts_mu);
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (e == cudaSuccess) e = cudaStreamIsCapturing(ctx->stream, &capture);
-    const bool direct = capture == cudaStreamCaptureStatusNone;
+    e = allow_smem((const void*)lux_attn_prefill_mma_f32, 1, SMEM, ctx->device);
+    // behind the last call that used the context's scratch, on whichever stream that was
     if (e == cudaSuccess && direct && ctx->parts_used && !ctx->parts_ordered) e = cudaStreamWaitEvent(ctx->stream, ctx->parts_event, 0);
     // as many (sequence, KV head) pairs at a time as have their parts in the scratch (in one call all, up to 128 k keys in total)
     for (geo.bk0 = 0; e == cudaSuccess && geo.bk0 < bks; geo.bk0 += geo.nbk) {
         geo.nbk = std::min(fit, bks - geo.bk0);
-        unsigned char* parts = (unsigned char*)ctx->d_parts;
+        unsigned char* parts = (unsigned char*)scratch;
         uint32_t* flags = (uint32_t*)(parts + (size_t)geo.nbk * geo.all_tiles * TILE_BYTES);
         geo.parts = parts;
         geo.flags = flags;

@@ -9,9 +9,11 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "lux/gpu/backend_plugin.h"
 #include "lux/gpu/qmatmul_ext.h"
@@ -24,6 +26,15 @@ struct Buffer {
     size_t size;
     int    device;
     bool   owned;    // false for lux_cuda_buffer_wrap handles
+};
+
+// Scratch of the prompt attention in a captured graph.
+struct GraphParts {
+    void*  p;
+    size_t bytes;
+    unsigned long long capture;             // whose it is: calls captured on one stream come one after the other
+    cudaStream_t stream;
+    std::shared_ptr<std::atomic<bool>> live;// until the graph and all that was instantiated from it are gone
 };
 
 // Counterpart of WGPUBackendContext (src/webgpu_plugin.cpp:584-622): one device, one
@@ -57,6 +68,7 @@ struct Context {
     cudaEvent_t    parts_event = nullptr;   // the end of the last such call,
     bool           parts_used = false;      // if there was one,
     bool           parts_ordered = false;   // and whether the context's stream runs behind it
+    std::vector<GraphParts> graph_parts;    // captured calls have their own, since replays are ordered by nothing here
     std::mutex     mu;                      // guards the staging buffers
     int            sm_count = 148;
     // A kernel of this library that WRITES a buffer a later matmul may bind as weights, scales or

@@ -156,6 +156,7 @@ static void cuda_destroy_context(LuxBackendContext* context) {
     if (ctx->d_stage) cudaFree(ctx->d_stage);
     if (ctx->d_int) cudaFree(ctx->d_int);
     if (ctx->d_parts) cudaFree(ctx->d_parts);
+    for (const GraphParts& g : ctx->graph_parts) cudaFree(g.p);
     if (ctx->parts_event) cudaEventDestroy(ctx->parts_event);
     if (ctx->d_attn) cudaFree(ctx->d_attn);
     if (ctx->d_splitk) cudaFree(ctx->d_splitk);
