@@ -228,7 +228,8 @@ LUX_GPU_PLUGIN_EXPORT LuxBackendError lux_cuda_qmlp_noalloc(
  * NULL restores the context's own non-blocking stream; to name the default stream pass
  * cudaStreamLegacy or cudaStreamPerThread, not 0).  Calls share the context's scratch:
  * work enqueued without a wait on two streams (or replayed from a graph beside it) has to
- * be ordered by the caller; this call orders a prompt's attention by itself.  The reference has one implicit queue per
+ * be ordered by the caller, but for the attention of prompts, which orders itself and has a
+ * scratch of its own in a graph.  The reference has one implicit queue per
  * context (src/webgpu_plugin.cpp:584-622); this is its CUDA counterpart. */
 LUX_GPU_PLUGIN_EXPORT LuxBackendError lux_cuda_context_set_stream(LuxBackendContext* ctx, void* stream);
 LUX_GPU_PLUGIN_EXPORT void* lux_cuda_context_get_stream(LuxBackendContext* ctx);

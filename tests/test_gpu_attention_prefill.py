@@ -544,3 +544,26 @@ def test_a_capture_that_forks_has_a_scratch_for_each_branch(backend):
             pr.clear()
             g.replay()
             pr.check()
+
+
+def test_a_context_takes_the_scratch_with_its_first_prompt(backend):
+    """A host that never runs prompt attention does not pay for its scratch; one call takes it, the next no more."""
+    import torch
+    free = lambda: (torch.cuda.synchronize(), torch.cuda.mem_get_info()[0])[1]
+    q, k, v = _qkv(70, 1, 2, 1, 64, 64)
+    warm = backend.create_context(0)                 # what the first context of a process sets up
+    warm.destroy()
+    before = free()
+    c = backend.create_context(0)
+    try:
+        created = before - free()
+        assert created < 64 << 20
+        with _Tuned(backend, attn_prefill=1):
+            _sdpa(c, q, k, v, True)
+            first = before - free()
+            assert first >= 131072 * 1536
+            _sdpa(c, q, k, v, True)
+            assert before - free() == first
+    finally:
+        c.destroy()
+    assert before - free() < 32 << 20

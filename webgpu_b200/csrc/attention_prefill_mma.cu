@@ -67,6 +67,8 @@ constexpr int PART = 64 * D;              // bytes of one part of a CTA's half t
 constexpr int SLOT = 3 * PART;            // K or V of a tile, one CTA's half
 constexpr int SLOTS = 7;
 constexpr size_t TILE_BYTES = 4 * SLOT;   // scratch per tile: K of rank 0, 1, V of rank 0, 1
+constexpr size_t TILE_SCRATCH = TILE_BYTES + 8;              // and its flags
+constexpr size_t SCRATCH = 131072 / BN * TILE_SCRATCH;       // 201 MB
 // Q's l part, ring, two rows of factors, denominators and maxima, barriers and flags
 constexpr int OFF_QL = 0, OFF_RING = BM * D * 2, OFF_ALPHA = OFF_RING + SLOTS * SLOT, OFF_STAT = OFF_ALPHA + 2 * BM * 4;
 constexpr int OFF_BAR = OFF_STAT + 2 * BM * 4, OFF_FLAG = OFF_BAR + 256;
@@ -630,6 +632,19 @@ struct Uncaptured {
     ~Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
+// The context's scratch, from the first call on that needs it; less of it, or none, where memory is short.
+void context_scratch(Context* ctx) {
+    Uncaptured scope;
+    for (size_t n = SCRATCH; !ctx->d_parts && n >= 64 * TILE_SCRATCH; n /= 2) {
+        if (cudaMalloc(&ctx->d_parts, n) == cudaSuccess) {
+            ctx->d_parts_bytes = n;
+        } else {
+            ctx->d_parts = nullptr;
+            cudaGetLastError();
+        }
+    }
+}
+
 // Scratch of at least `want` bytes for a call that is being captured: the graph's own, shared by what is captured one after the other on
 // one stream, and kept until the graph and all that was instantiated from it are gone (a replay in flight included).  Null: there is none.
 const GraphParts* graph_scratch(Context* ctx, size_t want) try {
@@ -697,7 +712,7 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
     const uint32_t keys = p.causal ? (uint32_t)std::min<uint64_t>((uint64_t)p.causal_base + p.seq_q, p.kv_len) : p.kv_len;
     Geometry geo{};
     geo.all_tiles = (keys + BN - 1) / BN;
-    const size_t per_bk = geo.all_tiles * (TILE_BYTES + 8);
+    const size_t per_bk = geo.all_tiles * TILE_SCRATCH;
     const uint32_t bks = p.batch * p.kv_heads;
     // The scratch is the context's, or the graph's for a call that is being captured.
     std::lock_guard<std::mutex> lk(ctx->parts_mu);
@@ -705,12 +720,15 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
     cudaError_t e = cudaStreamIsCapturing(ctx->stream, &capture);
     if (e != cudaSuccess) return map_cuda(e, "lux_attn_prefill_mma_f32");
     const bool direct = capture == cudaStreamCaptureStatusNone;
-    void* scratch = ctx->d_parts;
-    size_t scratch_bytes = ctx->d_parts_bytes;
-    if (direct) {
-        free_idle_graph_scratch(ctx);
-    } else if (!f32_only && per_bk && per_bk <= scratch_bytes) {
-        const GraphParts* own = graph_scratch(ctx, std::min(bks * per_bk, scratch_bytes));
+    void* scratch = nullptr;
+    size_t scratch_bytes = 0;
+    if (direct) free_idle_graph_scratch(ctx);
+    if (!f32_only && per_bk && direct) {
+        context_scratch(ctx);
+        scratch = ctx->d_parts;
+        scratch_bytes = ctx->d_parts_bytes;
+    } else if (!f32_only && per_bk && per_bk <= SCRATCH) {
+        const GraphParts* own = graph_scratch(ctx, std::min(bks * per_bk, SCRATCH));
         if (!own) cudaGetLastError();
         scratch = own ? own->p : nullptr;
         scratch_bytes = own ? own->bytes : 0;

@@ -62,8 +62,8 @@ struct Context {
     size_t         d_int_bytes = 0;
     void*          d_attn = nullptr;        // partial results of attention calls that split the keys over CTAs:
     size_t         d_attn_bytes = 0;        // 16 MB, allocated with the context (a call takes fewer slices rather than allocate)
-    void*          d_parts = nullptr;       // bf16 parts of K and V of prompt attention: 1536 bytes a key and KV head,
-    size_t         d_parts_bytes = 0;       // 128 k of them, allocated with the context (a larger call goes in several passes)
+    void*          d_parts = nullptr;       // bf16 parts of K and V of prompt attention: 1536 bytes a key and KV head, allocated by
+    size_t         d_parts_bytes = 0;       // the first call that needs them, for 128 k keys (a larger call goes in several passes)
     std::mutex     parts_mu;                // held while such a call enqueues its kernels: threads do not mix theirs
     cudaEvent_t    parts_event = nullptr;   // the end of the last such call,
     bool           parts_used = false;      // if there was one,

@@ -123,15 +123,10 @@ static LuxBackendContext* cuda_create_context(int device_index) {
         ctx->d_attn_bytes = 16u << 20;
         ok = cudaMalloc(&ctx->d_attn, ctx->d_attn_bytes) == cudaSuccess;
     }
-    if (ok) {
-        ctx->d_parts_bytes = (size_t)131072 / 64 * ((64u * 1536u) + 8u);
-        ok = cudaMalloc(&ctx->d_parts, ctx->d_parts_bytes) == cudaSuccess &&
-             cudaEventCreateWithFlags(&ctx->parts_event, cudaEventDisableTiming) == cudaSuccess;
-    }
+    ok = ok && cudaEventCreateWithFlags(&ctx->parts_event, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         if (ctx->parts_event) cudaEventDestroy(ctx->parts_event);
-        if (ctx->d_parts) cudaFree(ctx->d_parts);
         if (ctx->d_attn) cudaFree(ctx->d_attn);
         if (ctx->d_splitk) cudaFree(ctx->d_splitk);
         if (ctx->d_absmax) cudaFree(ctx->d_absmax);
