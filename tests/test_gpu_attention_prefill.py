@@ -567,3 +567,37 @@ def test_a_context_takes_the_scratch_with_its_first_prompt(backend):
     finally:
         c.destroy()
     assert before - free() < 32 << 20
+
+
+@pytest.mark.parametrize("gain", [1e-6, 1.0, 1e7])
+def test_a_row_with_one_key_is_its_value_bit_for_bit(ctx, backend, gain):
+    """The first row of a causal prompt, and a row whose other keys weigh nothing, are that key's V; the log-sum-exp of such a row
+    is its score, to the rounding of the score and of a product by ln 2."""
+    q, k, v = _qkv(90, 2, 4, 2, 200, 200)
+    v *= np.float32(gain)
+    q[:, :, 150] = 0
+    q[:, :, 150, 0] = 4000.0
+    k[:, :, :, 0] = np.where(np.arange(200) == 77, 3.0, -1.0)            # scores of about 1060 and -350
+    q[:, :, 0, 0] = 0
+    with _Tuned(backend, attn_prefill=1):
+        got, lse = _sdpa(ctx, q, k, v, True)
+    assert np.array_equal(got[:, :, 0].view(np.uint32), np.repeat(v[:, :, 0], 2, axis=1).view(np.uint32))
+    assert np.array_equal(got[:, :, 150].view(np.uint32), np.repeat(v[:, :, 77], 2, axis=1).view(np.uint32))
+    want = np.einsum("bhd,bhd->bh", q[:, :, 0].astype(np.float64), np.repeat(k[:, :, 0], 2, axis=1).astype(np.float64)) / np.sqrt(128)
+    # a score is a sum of 128 products of N(0, 1) values, 1 / 11 each, with an error of 2^-24 of its largest partial sums (below 4)
+    np.testing.assert_allclose(lse[:, :, 0], want, rtol=0, atol=4 * 4 * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("peak", [1.0, 6.0])
+def test_outputs_have_no_mean_error(ctx, backend, peak):
+    """What the tensor core's chains cut off is added back: over many rows with so many keys the outputs are neither too large
+    nor too small by more than 2e-8 of themselves (3 to 8e-8 if it were not; a row of ones is off by up to 9e-8 where the
+    denominator carries the correction).  The mean of 2^18 errors of 3e-7 at most is known to 1e-9."""
+    q, k, v = _qkv(91, 4, 16, 16, 256, 256)
+    q *= np.float32(peak)
+    with _Tuned(backend, attn_prefill=1):
+        got, _ = _sdpa(ctx, q, k, v, True)
+    want = _sdpa64(q, k, v, True)
+    for lo, hi in ((1, 32), (32, 64), (64, 128), (128, 256)):
+        w, e = want[:, :, lo:hi], got[:, :, lo:hi] - want[:, :, lo:hi]
+        assert abs((e * w).sum() / (w * w).sum()) < 2e-8, (lo, hi)

@@ -33,10 +33,14 @@
 // Accumulation.  The tensor core cuts its f32 sums off at every step of 16 (measured on chains of 1 / 2 / 4 / 8 steps:
 // mean loss 1.1 / 2.4 / 4.9 / 9.4e-8 of the sum, in rms 2.5 / 3.9 / 6.5 / 11.6e-8), so chains are four steps of the large products, after
 // the small ones: a score is the f32 sum of two such chains, and the output is kept in f32 registers, to which each
-// tile of 64 keys is added by an ordinary rounded addition.  What a chain loses on average is taken off the denominator too.
+// tile of 64 keys is added by an ordinary rounded addition.  What the weighted sum of a tile loses on average (signed, N(0, 1) inputs:
+// 3.6e-8 of it with 2 keys, 4.1 with 16, 5.2 with 32, 6.5 with 48, 7.8 with 64; scores six times as large give the same) is added to the
+// quotient before its one rounding, which leaves at most 0.9e-8; a row with a single weight loses nothing and is its value bit for bit.
+// The log-sum-exp takes the denominator as it is.
 // Relative error against 64 bits, in 1e-7 (2-norm, N(0, 1) inputs, Llama-3-8B heads; streaming kernel / mma.sync form of this
-// one / this one): causal, 150 tokens 1.37 / 1.06 / 1.05, 512 1.65 / 1.20 / 1.15, 2048 2.24 / 1.39 / 1.28; unmasked,
-// 700 x 3 3.07 / 1.76 / 1.56, 1448 4.03 / 2.02 / 1.76.
+// one / this one): causal, 64 tokens 1.22 / 0.96 / 0.84, 150 1.36 / 1.08 / 0.92, 512 1.68 / 1.23 / 1.05, 2048 2.25 / 1.42 / 1.20; unmasked,
+// 700 x 3 3.12 / 1.82 / 1.50, 1448 4.05 / 2.05 / 1.70.  The log-sum-exp (rms, a unit in its last place being 4.8): 1.69 / 1.48 / 1.62 at 150,
+// 2.47 / 2.13 / 2.22 at 2048, 2.49 / 2.05 / 2.16 at 1448 (scores of both signs are cut towards zero, which takes 0.6 off it on average).
 //
 // Measured, Llama-3-8B heads, against the form with mma.sync products and the splitting in every CTA (bound by that instruction,
 // 568 TFLOP/s, and by the splitting): causal, 2048 tokens 674 -> 168 us (205 TFLOP/s of f32 products, 1.23 PFLOP/s of
@@ -69,9 +73,9 @@ constexpr int SLOTS = 7;
 constexpr size_t TILE_BYTES = 4 * SLOT;   // scratch per tile: K of rank 0, 1, V of rank 0, 1
 constexpr size_t TILE_SCRATCH = TILE_BYTES + 8;              // and its flags
 constexpr size_t SCRATCH = 131072 / BN * TILE_SCRATCH;       // 201 MB
-// Q's l part, ring, two rows of factors, denominators and maxima, barriers and flags
+// Q's l part, ring, two rows of factors, denominators, maxima and losses, barriers and flags
 constexpr int OFF_QL = 0, OFF_RING = BM * D * 2, OFF_ALPHA = OFF_RING + SLOTS * SLOT, OFF_STAT = OFF_ALPHA + 2 * BM * 4;
-constexpr int OFF_BAR = OFF_STAT + 2 * BM * 4, OFF_FLAG = OFF_BAR + 256;
+constexpr int OFF_BAR = OFF_STAT + 3 * BM * 4, OFF_FLAG = OFF_BAR + 256;
 constexpr int SMEM = OFF_FLAG + 64 + 1024;
 constexpr int OUT_PITCH = D + 4;          // floats between the rows of the output in shared memory (over the ring)
 // tensor memory columns
@@ -79,7 +83,8 @@ constexpr uint32_t T_QH = 0, T_QM = 64, T_S = 128, T_P = 256, T_O = 384;
 constexpr float NEG = -3.0e38f, LN2 = 0.6931471805599453f;
 constexpr float RAISE = 8.0f;             // the running maximum is raised when a score passes it by more: weights below 2^8
 constexpr float P_SCALE = 0x1p30f;        // of the weights before they are split
-constexpr float CHAIN_LOSS = 0x1p-24f;    // taken off the denominators: what the chains of the weighted sum lose on average (5 to 6e-8)
+constexpr float LOSS_CHAIN = 2.2e-8f, LOSS_STEP = 1.4e-8f;   // what a weighted sum of one tile loses on average: per chain, per step of 16 keys
+constexpr float LOSS = LOSS_CHAIN + LOSS_STEP * (BN / 16);
 constexpr uint32_t TOO_LARGE = (127u + 60u) << 23;           // |x| >= 2^60, infinity or NaN, as bits
 constexpr uint32_t TOO_SMALL = (127u - 100u) << 23;          // 0 < |v| < 2^-100
 constexpr uint32_t FLAG_BAD = 1u, FLAG_TINY = 2u;            // of a tile of K or V
@@ -440,7 +445,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         regs_inc<REGS_S>();
         const uint32_t len = row < rows ? row_len(q0 + row) : 0u;        // a padding row sees nothing and is not written
         const uint32_t free_bar = in_leader(s_free), ready_bar = in_leader(p_ready);
-        float m = NEG, l = 0.0f;
+        float m = NEG, l = 0.0f, kept = 0.0f;     // kept: of the loss that l stands for, what a tile's unseen keys leave out
         for (uint32_t t = 0; t < walk; t++) {
             if (!warp_wait(s_full, t & 1u, abort_flag, lane)) break;
             const bool own = t < own_tiles;
@@ -498,7 +503,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
                 }
                 float x, y;
                 unpair(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), x, y);
-                l = fmaf(x + y, 1.0f - CHAIN_LOSS, l);
+                x += y;
+                l += x;
+                if (t0 + BN > len && t0 < len) kept = x * (LOSS_STEP * (float)((t0 + BN - len) / 16u));       // (the row's last keys)
             }
             // the weighted sum before this one has read its weights
             if (t && !warp_wait(o_full, (t - 1u) & 1u, abort_flag, lane)) break;
@@ -519,6 +526,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         }
         stat[row] = l;
         stat[BM + row] = m;
+        stat[2 * BM + row] = l == 1.0f ? 0.0f : LOSS - kept / fmaxf(l, 1.0f);      // (a single weight is its value's three parts: nothing is cut off)
         __syncwarp();
         cluster_sync_all();
         regs_dec<REGS>();
@@ -594,10 +602,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
     }
     const size_t orow = ((size_t)b * p.heads + h) * p.seq_q + q0;
     for (uint32_t r = warp; r < rows; r += THREADS / 32) {
-        const float l = stat[r];
+        const float l = stat[r], inv = 1.0f / l, loss = stat[2 * BM + r];
         float4 v = *reinterpret_cast<const float4*>(out_s + r * OUT_PITCH + 4 * lane);
-        v = l > 0.0f ? make_float4(v.x / l * (1.0f / P_SCALE), v.y / l * (1.0f / P_SCALE), v.z / l * (1.0f / P_SCALE), v.w / l * (1.0f / P_SCALE))
-                     : make_float4(0.f, 0.f, 0.f, 0.f);                          // a row without keys is zero
+        // an estimate of the quotient; then what it leaves of the dividend, and the mean loss, before the one rounding that counts
+        auto quotient = [&](float a) {
+            const float c = a * inv;
+            return fmaf(fmaf(loss, a, fmaf(-c, l, a)), inv, c) * (1.0f / P_SCALE);
+        };
+        v = l > 0.0f ? make_float4(quotient(v.x), quotient(v.y), quotient(v.z), quotient(v.w)) : make_float4(0.f, 0.f, 0.f, 0.f);   // a row without keys is zero
         *reinterpret_cast<float4*>(p.out + (orow + r) * D + 4 * lane) = v;
     }
     if (p.lse && tid < (int)rows) p.lse[orow + tid] = stat[tid] > 0.0f ? fmaf(stat[BM + tid], LN2, logf(stat[tid])) : -3.402823e+38f;
