@@ -343,10 +343,10 @@ def test_an_odd_pair_with_one_block_out_of_range(ctx, backend, where):
     assert np.array_equal(got[:, :, 128:].view(np.uint32), want[:, :, 128:].view(np.uint32))
 
 
-@pytest.mark.parametrize("B_,Hkv,Skv,kernel", [(3, 50, 1000, "lux_attn_prefill_mma_f32"), (1, 1, 131073, "lux_attn_prefill_f32")])
+@pytest.mark.parametrize("B_,Hkv,Skv,kernel", [(3, 50, 1000, "lux_attn_prefill_mma_f32"), (1, 1, 131073, "lux_attn_prefill_mma_f32"), (1, 2, 90001, "lux_attn_prefill_mma_f32")])
 def test_more_keys_than_the_scratch_holds(ctx, backend, B_, Hkv, Skv, kernel):
-    """128 k keys of all KV heads have their parts in the scratch at a time: more heads go in several passes, a longer
-    head goes to the f32 kernel; either way the streaming kernel's answer to rounding."""
+    """128 k keys of all KV heads have their parts in the scratch at a time: more heads, or longer ones, go in several passes;
+    either way the streaming kernel's answer to rounding."""
     q, k, v = _qkv(23, B_, Hkv, Hkv, 66, Skv)
     outs = []
     for mode in (1, 2):
@@ -601,3 +601,59 @@ def test_outputs_have_no_mean_error(ctx, backend, peak):
     for lo, hi in ((1, 32), (32, 64), (64, 128), (128, 256)):
         w, e = want[:, :, lo:hi], got[:, :, lo:hi] - want[:, :, lo:hi]
         assert abs((e * w).sum() / (w * w).sum()) < 2e-8, (lo, hi)
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 5])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("B_,H,Hkv,Sq,Skv", [(1, 2, 2, 127, 128), (1, 1, 1, 129, 191), (2, 4, 2, 65, 65), (1, 5, 1, 300, 640), (1, 3, 3, 257, 449), (1, 8, 2, 385, 1000),
+                                             (1, 2, 2, 500, 130), (2, 2, 1, 70, 0)])
+def test_passes_over_ranges_of_the_keys(ctx, backend, B_, H, Hkv, Sq, Skv, causal, tiles):
+    """So many key tiles per pass, blocks carrying what they have from one to the next: blocks that see no key of a pass, passes that end
+    inside a block's diagonal, odd pairs; against 64 bits, and the log-sum-exp against one pass."""
+    q, k, v = _qkv(Sq + Skv + tiles, B_, H, Hkv, Sq, Skv)
+    with _Tuned(backend, attn_prefill=1):
+        one, one_lse = _sdpa(ctx, q, k, v, causal)
+    before = backend.launch_count()
+    with _Tuned(backend, attn_prefill=1, attn_pass_tiles=tiles):
+        got, lse = _sdpa(ctx, q, k, v, causal)
+        assert backend.last_kernel_name() == "lux_attn_prefill_mma_f32" and ctx.last_device_status() == 0
+    seen = -(-(min(Sq, Skv) if causal else Skv) // 64)
+    assert backend.launch_count() - before == (2 * -(-seen // tiles) if seen else 1)
+    if not Skv:
+        assert not got.any()
+        return
+    assert orc.rel_l2(got, _sdpa64(q, k, v, causal)) < TOL
+    np.testing.assert_allclose(lse, one_lse, rtol=2.0 ** -22, atol=2.0 ** -22)      # four roundings each
+
+
+@pytest.mark.parametrize("tiles", [1, 3])
+def test_passes_keep_what_one_pass_keeps(ctx, backend, tiles):
+    """The tests above on ranges, extremes and fallbacks, with their bounds, in passes."""
+    with _Tuned(backend, attn_pass_tiles=tiles):
+        for bad in (np.nan, np.inf):
+            test_values_a_row_must_not_see_do_not_reach_it(ctx, backend, bad)
+        for row in (0, 77, 149):
+            test_a_non_finite_query_is_noticed_by_every_warp(ctx, backend, row, np.nan)
+        test_no_keys_and_large_scores(ctx, backend, 1)
+        test_magnitudes_far_apart(ctx, backend)
+        for key in (63, 149):
+            for factor in (1e5, 1e30):
+                test_large_finite_values_behind_the_mask_do_not_reach_earlier_rows(ctx, backend, key, factor)
+        for lo, hi in ((-6, 12), (-30, 0)):
+            test_keys_of_very_different_magnitude(ctx, backend, lo, hi)
+        for drop in (14, 30, 80):
+            test_small_weights_under_a_dominant_key_without_a_value(ctx, backend, drop)
+        for scale in (1e-28, 1e-31, 1e-37):
+            for columns in (slice(None), slice(5, 6)):
+                test_values_close_to_the_smallest_normal_number(ctx, backend, scale, columns)
+        for qs, ks in ((1e15, 1e-15), (1e-37, 1e37)):
+            test_scores_of_ordinary_size_from_extreme_operands(ctx, backend, qs, ks)
+        for value in (np.float32(1), np.float32(3e-30)):
+            test_a_constant_v_comes_back(ctx, backend, value)
+        for where, bad in (("q", np.nan), ("k", np.inf), ("v", np.nan), ("v", 1e30)):
+            test_a_block_out_of_range_leaves_the_others_alone(ctx, backend, where, bad)
+            test_an_odd_pair_with_one_block_out_of_range(ctx, backend, where)
+        test_output_over_the_queries(ctx, backend)
+        test_replays_of_a_captured_call_do_not_remember(backend)
+        test_a_row_with_one_key_is_its_value_bit_for_bit(ctx, backend, 1.0)
+        test_outputs_have_no_mean_error(ctx, backend, 1.0)

@@ -1169,8 +1169,9 @@ bool prefill_fits(const AttnParams& p) {
 // Which of the two kernels answers a call: by what the streaming kernel takes in us on 148 SMs and what the prompt kernel
 // took when its products were mma.sync ones.  Over 178 shapes (64 .. 2049 queries, 64 .. 16384 keys, 4 .. 64 heads,
 // batch 1 .. 8) that choice was nowhere slower than the streaming kernel by more than 3 %.  The prompt kernel has become two to
-// four times faster since (attention_prefill_mma.cu), so it is the faster one wherever it is chosen; the line has stayed, and with
-// it which kernel, and so which order of sums, a call gets.
+// five times faster since (attention_prefill_mma.cu), so it is the faster one wherever it is chosen (by this line / the streaming kernel,
+// 32 heads, 8 KV heads, us: 256 queries over 4096 keys 156 / 858, over 131072 4294 / 26015) and also where it is not: 65 over 4096 151 / 236, 128
+// over 131072 4249 / 13435.  The line has stayed, and with it which kernel, and so which order of sums, a call gets.
 // The mma.sync form: a CTA per SM owned 128 queries of a head and walked all their keys, 5.5 us a tile of 32, 4.6 where half
 // of its warps had no rows.
 double prefill_us(const AttnParams& p, int sms) {

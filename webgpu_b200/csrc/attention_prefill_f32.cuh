@@ -2,7 +2,7 @@
 //
 // What lux_attn_prefill_mma_f32 does with a block in which it met values that its bf16 parts cannot carry (2^60 and
 // more, infinities, NaN; outputs below 2^-100): the block starts over here, in the same CTA, before anything of it was written, and
-// no other block notices.  lux_attn_prefill_f32 runs it for every block (more than 128 k keys per KV head; tunable attn_prefill = 3: the tests).
+// no other block notices.  lux_attn_prefill_f32 runs it for every block (no scratch to be had; tunable attn_prefill = 3: the tests).
 //
 // What bounds it.  Both contractions are f32 products of f32 operands, so the FMA pipe is the floor: 128 lanes x 148
 // SMs (72 TFLOP/s at 1.9 GHz).  A 16-byte shared-memory read costs the SM four cycles however many lanes read

@@ -16,7 +16,8 @@
 // one head) starts over by itself (attention_prefill_f32.cuh), before it has written anything: this holds with
 // out == q, and no other block, call or replay of a captured one takes part.
 //
-// Two kernels.  lux_attn_split_kv writes the parts of K and V once per call, tile by tile as the tensor core wants them in
+// Two kernels.  (Where the parts of all keys do not fit the scratch, a pair of them per pass, attention_passes.h: blocks then carry their
+// outputs, maxima and denominators from one range of keys to the next, merged by the running-maximum rule.)  lux_attn_split_kv writes the parts of K and V once per call, tile by tile as the tensor core wants them in
 // shared memory, into the context's scratch (split in every CTA instead, an element would be converted 64 times in a
 // 2048-token prompt, and the parts' way through shared memory would take as long as the products).
 // lux_attn_prefill_mma_f32 is a pair of CTAs (two heads that share a KV head and their 128 queries, or two
@@ -47,6 +48,7 @@
 // bf16 ones: 0.89 of what cuBLAS sustains under the power cap), 512 tokens 95 -> 30.5, 150 tokens 28.7 -> 16.9; unmasked
 // 700 tokens x 3 511 -> 139.  The tensor pipe is busy for 62 % of the time, at 1.63 GHz; two softmax warps per row instead of one
 // gave 1 %.
+#include "attention_passes.h"
 #include "attention_prefill_f32.cuh"
 #include "attention_ring.h"
 
@@ -71,7 +73,6 @@ constexpr int PART = 64 * D;              // bytes of one part of a CTA's half t
 constexpr int SLOT = 3 * PART;            // K or V of a tile, one CTA's half
 constexpr int SLOTS = 7;
 constexpr size_t TILE_BYTES = 4 * SLOT;   // scratch per tile: K of rank 0, 1, V of rank 0, 1
-constexpr size_t TILE_SCRATCH = TILE_BYTES + 8;              // and its flags
 constexpr size_t SCRATCH = 131072 / BN * TILE_SCRATCH;       // 201 MB
 // Q's l part, ring, two rows of factors, denominators, maxima and losses, barriers and flags
 constexpr int OFF_QL = 0, OFF_RING = BM * D * 2, OFF_ALPHA = OFF_RING + SLOTS * SLOT, OFF_STAT = OFF_ALPHA + 2 * BM * 4;
@@ -220,8 +221,17 @@ struct Geometry {
     const uint32_t* flags;
     uint32_t bk0, nbk, all_tiles;
     uint32_t by_head;            // pairs are two heads (their number per KV head is even), else two blocks of queries
-    uint32_t units, levels;      // pairs per KV head and block of queries; blocks of queries (pairs of them)
+    uint32_t units, levels;      // pairs per KV head and block of queries; blocks of queries (pairs of them),
+    uint32_t level0;             // from this one on
+    // A pass over the keys key0 .. key0 + keys.  Unless it is the first and the last, blocks carry what they have so far:
+    // CARRY_ROW floats a row, at the same block of the grid in every pass, and CARRY_BAD, FLAG_TINY.
+    uint32_t key0, keys, first, last;
+    float* carry;
+    uint32_t* carry_flags;
 };
+constexpr int CARRY_ROW = D + 4;          // the outputs, maximum, denominator, loss; whole 16 bytes
+static_assert(TILE_SCRATCH == TILE_BYTES + 8 && CARRY == BM * CARRY_ROW * 4 + 16, "tiles and carried blocks with their flags");
+constexpr uint32_t CARRY_BAD = 1u;
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn_prefill_mma_f32(const PrefillArgs p, const Geometry geo) {
     extern __shared__ unsigned char smem_raw[];
@@ -246,12 +256,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
     // blocks of late queries see the most keys under a causal mask: they come first, so that the last
     // wave is made of short ones.  Neighbouring pairs are heads of one KV head and share its tiles in L2.
     const uint32_t per_level = geo.nbk * geo.units;
-    const uint32_t level = geo.levels - 1u - (blockIdx.x >> 1) / per_level, rest = (blockIdx.x >> 1) % per_level;
+    const uint32_t level = geo.level0 + geo.levels - 1u - (blockIdx.x >> 1) / per_level, rest = (blockIdx.x >> 1) % per_level;
     const uint32_t unit = rest % geo.units, bkl = rest / geo.units, bk = geo.bk0 + bkl, b = bk / p.kv_heads;
     const uint32_t h = bk % p.kv_heads * p.group + (geo.by_head ? 2u * unit + rank : unit);
     const uint32_t qb = geo.by_head ? level : 2u * level + rank;
     const uint32_t q0 = qb * BM, rows = q0 < p.seq_q ? min((uint32_t)BM, p.seq_q - q0) : 0u;
-    auto row_len = [&](uint32_t qi) { return p.causal ? min(p.causal_base + qi + 1u, p.kv_len) : p.kv_len; };
+    auto row_len = [&](uint32_t qi) {             // of the keys of this pass
+        const uint32_t n = p.causal ? min(p.causal_base + qi + 1u, p.kv_len) : p.kv_len;
+        return min(max(n, geo.key0) - geo.key0, geo.keys);
+    };
     const uint32_t lmax = rows ? row_len(q0 + rows - 1u) : 0u, own_tiles = (lmax + BN - 1u) / BN;
     const uint32_t pair_last = min(p.seq_q, (geo.by_head ? level + 1u : 2u * level + 2u) * BM) - 1u;
     const uint32_t tiles = (row_len(pair_last) + BN - 1u) / BN;            // the pair walks them together
@@ -574,7 +587,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
                 *reinterpret_cast<float4*>(out_s + row * OUT_PITCH + 4 * j) = v;
             }
         }
-        if ((*seen & FLAG_TINY) && row < rows) {
+        if ((*seen & FLAG_TINY) && row < rows && geo.first && geo.last) {
             const float least = stat[row] * (P_SCALE * 0x1p-100f);
 #pragma unroll
             for (int j = 0; j < D / 2; j++) {
@@ -587,7 +600,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         regs_dec<REGS>();
     }
     if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
-    const bool again = __syncthreads_or(low) || bad;
+    bool again = __syncthreads_or(low) || bad;
     if (*abort_flag) {
         // a bounded wait gave up: report it, and give copies in flight time to land.  Nothing has been written.
         if (tid == 0 && p.status) atomicOr(p.status, p.status_wait);
@@ -596,6 +609,46 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) lux_attn
         return;
     }
     if (!rows) return;
+    if (!(geo.first && geo.last)) {               // this pass's part of the rows, with what the earlier ones left
+        const uint32_t before = geo.first ? 0u : __ldcg(geo.carry_flags + blockIdx.x);
+        const uint32_t so_far = before | (again ? CARRY_BAD : 0u) | (*seen & FLAG_TINY);
+        float* mine = geo.carry + (size_t)blockIdx.x * (BM * CARRY_ROW);
+        __syncthreads();                          // all have read the flags
+        if (tid == 0) __stcg(geo.carry_flags + blockIdx.x, so_far);
+        bool small = false;
+        if (!(so_far & CARRY_BAD)) {
+            for (uint32_t r = warp; r < rows; r += THREADS / 32) {
+                float l = stat[r], m = stat[BM + r], cut = stat[2 * BM + r] * l;
+                float4 v = *reinterpret_cast<const float4*>(out_s + r * OUT_PITCH + 4 * lane);
+                float* there = mine + r * CARRY_ROW;
+                if (!geo.first) {
+                    const float4 c = __ldcg(reinterpret_cast<const float4*>(there) + lane), s = __ldcg(reinterpret_cast<const float4*>(there + D));
+                    const float top = fmaxf(m, s.x), a = ex2(m - top), b = ex2(s.x - top);
+                    v = make_float4(fmaf(v.x, a, c.x * b), fmaf(v.y, a, c.y * b), fmaf(v.z, a, c.z * b), fmaf(v.w, a, c.w * b));
+                    l = fmaf(l, a, s.y * b);
+                    cut = fmaf(cut, a, s.z * b);
+                    m = top;
+                }
+                if (geo.last) {
+                    __syncwarp();                 // all lanes have read the row's numbers
+                    const float least = l * (P_SCALE * 0x1p-100f);
+                    small |= fabsf(v.x) < least || fabsf(v.y) < least || fabsf(v.z) < least || fabsf(v.w) < least;
+                    *reinterpret_cast<float4*>(out_s + r * OUT_PITCH + 4 * lane) = v;
+                    if (lane == 0) {
+                        stat[r] = l;
+                        stat[BM + r] = m;
+                        stat[2 * BM + r] = l > 0.0f ? cut / l : 0.0f;
+                    }
+                } else {
+                    __stcg(reinterpret_cast<float4*>(there) + lane, v);
+                    if (lane == 0) __stcg(reinterpret_cast<float4*>(there + D), make_float4(m, l, cut, 0.0f));
+                }
+            }
+        }
+        if (!geo.last) return;
+        again = (so_far & CARRY_BAD) || ((so_far & FLAG_TINY) && __syncthreads_or(small));
+        __syncthreads();
+    }
     if (again) {                                  // values out of range: the block starts over on the f32 pipe
         if (tid < prefill::PF_THREADS) prefill::attend_f32(p, smem, qb, h, b);
         return;
@@ -722,10 +775,12 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
     using namespace pmma;
     p.q_blocks = (p.seq_q + pmma::BM - 1) / pmma::BM;
     const uint32_t keys = p.causal ? (uint32_t)std::min<uint64_t>((uint64_t)p.causal_base + p.seq_q, p.kv_len) : p.kv_len;
+    const uint32_t tiles = (keys + BN - 1) / BN, bks = p.batch * p.kv_heads;
+    const size_t per_bk = tiles * TILE_SCRATCH;
     Geometry geo{};
-    geo.all_tiles = (keys + BN - 1) / BN;
-    const size_t per_bk = geo.all_tiles * TILE_SCRATCH;
-    const uint32_t bks = p.batch * p.kv_heads;
+    geo.by_head = p.group % 2 == 0;
+    geo.units = geo.by_head ? p.group / 2 : p.group;
+    const uint32_t levels = geo.by_head ? p.q_blocks : (p.q_blocks + 1) / 2;
     // The scratch is the context's, or the graph's for a call that is being captured.
     std::lock_guard<std::mutex> lk(ctx->parts_mu);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -739,14 +794,14 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
         context_scratch(ctx);
         scratch = ctx->d_parts;
         scratch_bytes = ctx->d_parts_bytes;
-    } else if (!f32_only && per_bk && per_bk <= SCRATCH) {
-        const GraphParts* own = graph_scratch(ctx, std::min(bks * per_bk, SCRATCH));
+    } else if (!f32_only && per_bk) {
+        const GraphParts* own = graph_scratch(ctx, per_bk > SCRATCH ? SCRATCH : std::min(bks * per_bk, SCRATCH));
         if (!own) cudaGetLastError();
         scratch = own ? own->p : nullptr;
         scratch_bytes = own ? own->bytes : 0;
     }
-    const uint32_t fit = per_bk ? (uint32_t)std::min<size_t>(scratch_bytes / per_bk, 65535) : 65535u;
-    if (f32_only || fit == 0) {                        // (128 k keys per KV head fit the scratch)
+    const Passes plan = plan_passes(bks, levels, geo.units, tiles, scratch_bytes, (uint32_t)ctx->sm_count, (uint32_t)std::max(g_tune.attn_pass_tiles, 0));
+    if (f32_only || !plan.heads) {                     // (no scratch)
         const char* name = "lux_attn_prefill_f32";
         e = allow_smem((const void*)lux_attn_prefill_f32, 0, prefill::PF_SMEM + 128, ctx->device);
         if (e == cudaSuccess)
@@ -756,28 +811,44 @@ LuxBackendError launch_attn_prefill(Context* ctx, PrefillArgs p, bool f32_only) 
         count_launch(name);
         return LUX_BACKEND_OK;
     }
-    geo.by_head = p.group % 2 == 0;
-    geo.units = geo.by_head ? p.group / 2 : p.group;
-    geo.levels = geo.by_head ? p.q_blocks : (p.q_blocks + 1) / 2;
     const char* name = "lux_attn_prefill_mma_f32";
     e = allow_smem((const void*)lux_attn_prefill_mma_f32, 1, SMEM, ctx->device);
     // behind the last call that used the context's scratch, on whichever stream that was
     if (e == cudaSuccess && direct && ctx->parts_used && !ctx->parts_ordered) e = cudaStreamWaitEvent(ctx->stream, ctx->parts_event, 0);
-    // as many (sequence, KV head) pairs at a time as have their parts in the scratch (in one call all, up to 128 k keys in total)
-    for (geo.bk0 = 0; e == cudaSuccess && geo.bk0 < bks; geo.bk0 += geo.nbk) {
-        geo.nbk = std::min(fit, bks - geo.bk0);
+    auto pass = [&](uint32_t visible) {                // `visible`: keys of all passes
         unsigned char* parts = (unsigned char*)scratch;
         uint32_t* flags = (uint32_t*)(parts + (size_t)geo.nbk * geo.all_tiles * TILE_BYTES);
         geo.parts = parts;
         geo.flags = flags;
         if (geo.all_tiles) {
-            e = launch_pdl(g_tune.pdl != 2, lux_attn_split_kv, dim3(geo.all_tiles, geo.nbk, 2), dim3(256), (size_t)0, ctx->stream, 1, p.k, p.v, parts, flags,
-                           geo.bk0, keys, p.kv_stride);
-            if (e != cudaSuccess) break;
+            const size_t at = (size_t)geo.key0 * D;
+            e = launch_pdl(g_tune.pdl != 2, lux_attn_split_kv, dim3(geo.all_tiles, geo.nbk, 2), dim3(256), (size_t)0, ctx->stream, 1, p.k + at, p.v + at, parts, flags,
+                           geo.bk0, std::min(visible - geo.key0, geo.keys), p.kv_stride);
+            if (e != cudaSuccess) return;
             count_launch("lux_attn_split_kv");
         }
         e = launch_pdl(g_tune.pdl != 2, lux_attn_prefill_mma_f32, dim3(2u * geo.levels * geo.nbk * geo.units), dim3(THREADS), (size_t)SMEM, ctx->stream, 1, p, geo);
         if (e == cudaSuccess) count_launch(name);
+    };
+    for (geo.bk0 = 0; e == cudaSuccess && geo.bk0 < bks; geo.bk0 += geo.nbk) {
+        geo.nbk = std::min(plan.heads, bks - geo.bk0);
+        for (geo.level0 = 0; e == cudaSuccess && geo.level0 < levels; geo.level0 += geo.levels) {
+            geo.levels = std::min(plan.levels, levels - geo.level0);
+            // the keys that these queries see, in passes of equal numbers of tiles
+            const uint64_t end = (uint64_t)(geo.level0 + geo.levels) * (geo.by_head ? 1u : 2u) * pmma::BM;
+            const uint32_t visible = p.causal ? (uint32_t)std::min<uint64_t>(keys, (uint64_t)p.causal_base + end) : keys;
+            const uint32_t n = (visible + BN - 1) / BN;
+            geo.carry = (float*)((unsigned char*)scratch + plan.carry_at);
+            geo.carry_flags = (uint32_t*)(geo.carry + (size_t)2u * geo.levels * geo.nbk * geo.units * (pmma::BM * CARRY_ROW));
+            for (uint32_t t = 0; e == cudaSuccess && (t < n || t == 0); t += std::max(geo.all_tiles, 1u)) {
+                geo.all_tiles = plan.pass_tiles(t, n);
+                geo.first = t == 0;
+                geo.last = t + geo.all_tiles == n;
+                geo.key0 = t * BN;
+                geo.keys = geo.all_tiles * BN;
+                pass(visible);
+            }
+        }
     }
     if (e == cudaSuccess && direct) {
         e = cudaEventRecord(ctx->parts_event, ctx->stream);

@@ -147,6 +147,7 @@ struct Tunables {
     int int_matmul_splits = 0;   // slices of K there: 0 choose, 1, 2 or 4 where K has as many stages of 128
     int attn_prefill = 0;        // attention of many queries per head: 0 choose, 1 lux_attn_prefill_mma_f32 wherever it applies, 2 never,
                                  // 3 lux_attn_prefill_f32 wherever it applies
+    int attn_pass_tiles = 0;     // prompt attention: key tiles per pass; 0 = choose
     int attn_even = 0;           // decode over a paged cache: 0 choose, 1 even shares unless all sequences are full, 2 never
     int attn_splits = 0;         // attention: slices of the keys per (sequence, KV head, row block); 0 = choose
     int gemm_wa_narrow = 0;      // weights-in-TMEM GEMM, batch <= 64: 0 narrow tile (two CTAs per SM) when the launch has more CTAs
