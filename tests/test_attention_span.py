@@ -58,6 +58,6 @@ def test_no_span_leads_outside_the_scratch(tmp_path):
 
 def test_the_merge_follows_only_spans_that_fit():
     merge = (ROOT / "webgpu_b200/csrc/attention.cu").read_text()
-    merge = merge[merge.index("lux_attn_merge_f32(const AttnParams"):]
+    merge = merge[merge.index("lux_attn_merge_even_f32(const AttnParams"):]
     merge = merge[:merge.index("\n}")]
     assert merge.index("span_fits(span, p.ctas)") < merge.index("span_place(")
