@@ -194,8 +194,12 @@ lux_qgemm_i4_tc_wa(const __grid_constant__ CUtensorMap map_x, const WaParams p) 
         load_row64<W32>(wp, nq);
         // the line some units ahead is asked for now, so that the register fetch finds it in L2; once per line of two units (a
         // request of 32 lanes in as many rows takes the load pipe 32 cycles: with every unit's, config 4 gate_up at 16 rows 25.8
-        // us against 25.0, at 64 28.6 against 27.4, down 15.3 against 15.0)
-        if (ahead && !zodd) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp + (size_t)p.prefetch * (WA_UNIT_K / 2)));
+        // us against 25.0, at 64 28.6 against 27.4, down 15.3 against 15.0).  For an odd K / 128 every second row starts in the middle
+        // of a line.  bf16 tells by the address which unit begins one (weights that L2 has not seen, 16 rows, by the unit's number / by the
+        // address: 8192 x 8064 33.7 / 31.6 us, 14208 -> 4096 54.7 / 52.3, even ones alike); f16 by the unit's number, where the
+        // address takes longer (28672 x 4224 24.2 / 24.7, x 4096 23.9 / 24.1).
+        const uint8_t* const line = wp + (size_t)p.prefetch * (WA_UNIT_K / 2);
+        if (ahead && (BF16 ? !(reinterpret_cast<uintptr_t>(line) & 64u) : !zodd)) asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
         nsh = __ldg(sp);
         if (zp) nzb = (uint32_t)__ldg(zp);
     };
