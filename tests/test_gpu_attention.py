@@ -473,20 +473,23 @@ def test_how_a_paged_cache_is_dealt_out_follows_what_is_missing(ctx, backend):
 
 @pytest.mark.parametrize("B_,H,Hkv,keys,Sq", [(1, 8, 8, 33, 1), (37, 8, 8, 32, 1), (37, 8, 8, 31, 1), (5, 32, 8, 1184, 1), (1, 32, 8, 148 * 64, 1),
                                                (2, 8, 2, 700, 4), (3, 16, 2, 2049, 2)])
-def test_contiguous_decode_dealt_out_evenly(ctx, backend, B_, H, Hkv, keys, Sq):
-    """Shares that hold whole items, parts of one, and ends of two; rows of a step that appended several tokens see
-    different numbers of keys.  One slice per item (forced) is the reference (both sum in f32)."""
+def test_contiguous_decode_in_slices(ctx, backend, B_, H, Hkv, keys, Sq):
+    """One slice of the keys and many, the last one short; rows of a step that appended several tokens see different
+    numbers of keys.  The slices that the call chooses, and one (forced), against 64 bits."""
     rng = np.random.default_rng(keys)
     q = rng.standard_normal((B_, H, Sq, 128), np.float32)
     kc, vc = (rng.standard_normal((B_, Hkv, keys, 128), np.float32) for _ in range(2))
-    outs = []
+    k, v = (np.repeat(x.astype(np.float64), H // Hkv, axis=1) for x in (kc, vc))
+    s = q.astype(np.float64) @ k.transpose(0, 1, 3, 2) * np.float64(np.float32(0.09))
+    s = np.where(np.arange(keys) <= keys - Sq + np.arange(Sq)[:, None], s, -np.inf)
+    w = np.exp(s - s.max(axis=-1, keepdims=True))
+    want = w @ v / w.sum(axis=-1, keepdims=True)
     for splits in (0, 1):
         backend.tune("attn_splits", splits)
         try:
             ob = ctx.alloc(q.nbytes)
             ctx.sdpa_kv_cache(ctx.upload(q), ctx.upload(kc), ctx.upload(vc), ob, B_, H, Hkv, Sq, keys - Sq, keys, 128, 0.09, flags=B.FLAG_ATTN_CAUSAL)
-            outs.append(ob.to_host(np.float32, q.shape))
+            assert orc.rel_l2(ob.to_host(np.float32, q.shape), want) < TOL
         finally:
             backend.tune("attn_splits", 0)
-    _close(outs[0], outs[1])
     assert ctx.last_device_status() == 0
