@@ -132,7 +132,10 @@ LUX_GPU_PLUGIN_EXPORT LuxBackendError lux_cuda_sdpa_kv_cache_f32(
  *   block_tables  i32 [num_seqs, max_blocks_per_seq], physical block of each logical block
  *   context_lens  i32 [num_seqs]; a sequence with context_len <= 0 leaves its output rows
  *                 untouched (:66-67)
- * A context_len above max_blocks_per_seq * block_size is cut there.  The shader text reduces the
+ * A context_len above max_blocks_per_seq * block_size is cut there.  The order in which a sequence is
+ * summed follows the sizes of the call, and for a large cache of sequences that differ much in length
+ * those lengths too: its last bits may change with its neighbours'.  Full caches are summed as
+ * contiguous ones.  The shader text reduces the
  * maximum and the sum through the first lane of each warp only (:112-131, :141-157); the softmax
  * over the whole context that its comments describe is what is computed here.
  */

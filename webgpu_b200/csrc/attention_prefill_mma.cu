@@ -44,9 +44,9 @@
 // 2.47 / 2.13 / 2.22 at 2048, 2.49 / 2.05 / 2.16 at 1448 (scores of both signs are cut towards zero, which takes 0.6 off it on average).
 //
 // Measured, Llama-3-8B heads, against the form with mma.sync products and the splitting in every CTA (bound by that instruction,
-// 568 TFLOP/s, and by the splitting): causal, 2048 tokens 674 -> 168 us (205 TFLOP/s of f32 products, 1.23 PFLOP/s of
-// bf16 ones: 0.89 of what cuBLAS sustains under the power cap), 512 tokens 95 -> 30.5, 150 tokens 28.7 -> 16.9; unmasked
-// 700 tokens x 3 511 -> 139.  The tensor pipe is busy for 62 % of the time, at 1.63 GHz; two softmax warps per row instead of one
+// 568 TFLOP/s, and by the splitting): causal, 2048 tokens 674 -> 167 us (206 TFLOP/s of f32 products, 1.24 PFLOP/s of
+// bf16 ones), 192 where a call follows others under the power cap, 512 tokens 95 -> 32, 150 tokens 28.7 -> 15.4; unmasked
+// 700 tokens x 3 511 -> 138.  The tensor pipe is busy for 62 % of the time, at 1.63 GHz; two softmax warps per row instead of one
 // gave 1 %.
 #include "attention_passes.h"
 #include "attention_prefill_f32.cuh"
