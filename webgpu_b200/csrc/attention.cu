@@ -1277,16 +1277,17 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
     if (p.nsplit > 256) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;     // a context beyond 256 x 2046 pages
     // A paged cache whose sequences may differ in length by enough has both kernels launched (gated): even shares if more than
     // `slack` of a full cache's chunks are missing, else slices.  A share costs a CTA some microseconds where it ends one item and
-    // begins the next, about what 7 chunks take, or 14 chunks an item where CTAs take many items each; the kernel that leaves at once 1 to 3 us.
+    // begins the next, about what 7 chunks take (9 where a few items are cut into many parts: 2 x 16000 with 9 missing a CTA 50.9 us by slices, 50.6 by
+    // shares, 4 x 8000 with 8 48.8 / 49.5), or 14 chunks an item where CTAs take many items each; the kernel that leaves at once 1 to 3 us.
     // So this is for caches large enough that sequences of evenly spread lengths leave more than that missing (0.42 of a full one).
     // Llama-3-8B heads, 16-token pages, us a step by slices / by shares / gated.  Lengths 1, .2, .5, .9, ... of the longest: 8 x 2500 37.3 / 34.3 / 37.1,
     // 8 x 8000 83.8 / 64.6 / 66.7, 16 x 4000 90.0 / 68.4 / 71.4, 32 x 2000 85.7 / 71.2 / 73.3, 64 x 1500 107 / 97.8 / 102.8; not gated:
     // 8 x 2000 32.3 / 31.3, 20 x 1000 39.4 / 37.0, 32 x 1000 48.5 / 48.8, 48 x 1000 64.6 / 66.2, 64 x 1000 76.2 / 79.9.  All as long as the longest: 1 x 32768
-    // 57.4 / 63.4 / 60.0, 8 x 8192 97.8 / 100.1 / 100.9, 32 x 2048 89.4 / 101.5 / 94.8.
+    // 57.0 / 63.4 / 58.3, 8 x 8192 97.8 / 100.1 / 100.9, 32 x 2048 89.4 / 101.5 / 94.8.
     const uint32_t slots = (uint32_t)ctx->sm_count * (D > 128 ? 1 : ATT_CTAS_PER_SM);
     const uint64_t full_chunks = (uint64_t)items * chunks_of(max_keys);
     const size_t even_part = std::max((size_t)slots * 2 * rpb, out_rows * p.nsplit) * (D + 2) * 4 / 16 * 16 + 16;
-    const uint64_t slack = g_tune.attn_even == 1 ? 0u : std::max<uint64_t>(7u * slots, 14u * items);
+    const uint64_t slack = g_tune.attn_even == 1 ? 0u : std::max<uint64_t>((items < 64 ? 9u : 7u) * slots, 14u * items);
     const bool gated = p.block_size && p.row_blocks == 1 && full_chunks < (1u << 31) && full_chunks * 5u >= slack * 12u && g_tune.attn_even != 2 &&
                        !g_tune.attn_splits && slots <= ATT_MAX_PARTS && even_part + items * sizeof(AttnSpan) <= ctx->d_attn_bytes;
     if (gated) {
@@ -1332,8 +1333,13 @@ LuxBackendError attn_launch(Context* ctx, AttnParams& p, uint32_t max_keys, uint
         count_launch(form == EVEN ? "lux_attn_even_f32" : "lux_attn_stream_f32");
         return LUX_BACKEND_OK;
     };
-    LuxBackendError le = gated ? launch(EVEN, p.ctas) : LUX_BACKEND_OK;
+    // The kernel that leaves at once costs less behind the other.  Lengths spread between 1/8 and all of the longest one, which fills the
+    // table, leave 0.44 of the other sequences' chunks missing: one sequence, or two of 16 k keys, are more likely to
+    // get slices (1 x 32768 keys 58.3 us with these first, 60.0 with shares first; 8 x 2500 ragged ones 39.7 / 37.1).
+    const bool shares_first = gated && full_chunks * 44u * (p.batch - 1u) >= slack * 100u * p.batch;
+    LuxBackendError le = shares_first ? launch(EVEN, p.ctas) : LUX_BACKEND_OK;
     if (le == LUX_BACKEND_OK) le = launch(gated ? SLICES_GATED : SLICES, ctas);
+    if (le == LUX_BACKEND_OK && gated && !shares_first) le = launch(EVEN, p.ctas);
     if (le != LUX_BACKEND_OK) return le;
     if (gated || p.nsplit > 1) {
         const dim3 grid((unsigned)out_rows), block(128);
